@@ -10,15 +10,19 @@
 // (BeatEngineCudaField.jl:102-189).
 //
 // Here: a prologue kernel forms the weighted sources p_s w_s (all frequencies
-// and excitations of a batch), then the FP32 kernel runs one CTA per (32
-// observation points, frequency) and the FP64 kernel one CTA per (observation
-// point, frequency), each sweeping the faces.  The mixed form uses the same compensated
+// and excitations of a batch), then the FP32 kernel runs one cluster per (32
+// observation points, up to four frequencies), its CTAs sharing out the faces,
+// and the FP64 kernel one CTA per (observation point, frequency).  The mixed form uses the same compensated
 // phase as the assembly (double-float k|c_g - x| per face, FP32 correction per
-// point), Kahan-compensated FP32 partial sums per thread and an FP64 block
+// point), compensated FP32 partial sums per thread and an FP64 block
 // reduction; the far field sits at kr ~ 500 rad at 16 kHz, where plain FP32
 // phase would lose ~3e-5 rad.
+#include <cooperative_groups.h>
+
 #include "bem_common.cuh"
 #include "bem_kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace bem {
 namespace {
@@ -56,149 +60,49 @@ struct FieldParamsF32 {
   float2 qscale[64];
 };
 
-__device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
-  float y = x - c;
-  float t = s + y;
-  c = (t - s) - y;
-  s = t;
+// Adds x to the running sum s; the rounding error of the addition, which two_sum gives
+// exactly, goes to c, so s + c carries the terms' sum to about 2^-44.
+__device__ __forceinline__ void comp_add(float& s, float& c, float x) {
+  const df t = two_sum(s, x);
+  s = t.hi;
+  c += t.lo;
 }
 
-// One CTA per (32 observation points, frequency): lane = observation point,
-// warp w sweeps faces w, w + 8, ...  Every lane of a warp works on the same
-// face, so face records, sources and drives are broadcast loads, and the
-// compensated phase set-up (double-float k|c_g - x|) is done once per
-// (point, face).  The Q point terms of a face are summed in FP32 and added to
-// a Kahan-compensated per-lane sum; the 8 warps' sums are added in FP64.
+// One cluster per (32 observation points, NFQ frequencies starting at NFQ * blockIdx.y):
+// lane = observation point; the cluster's CTAs and their eight warps take the faces in
+// turn (face g goes to warp g mod (8 CTAs of the cluster)).  Every lane of a warp works on
+// the same face, so face records, sources and drives are broadcast loads, and everything
+// that does not depend on the frequency is formed once per (point, face) or (point,
+// source): the double-float distance |c_g - x|, s = 2 C.d + d.d, 1/r,
+// the compensated r - |C| = s / (r + |C|) and the normal-derivative factor.  Per frequency
+// remain the reduction of k|C| mod 2 pi, the phase, e^{ikr} and
+//   fs += e^{ikr} [ (t/r)(ik - 1/r) p_s w_s - q w_s / r ] / (4 pi).
+// The Q terms of a face are summed in FP32 and added to a compensated per-lane sum
+// (comp_add: exact rounding errors, so the split of the faces over warps and CTAs moves
+// the result by about 1e-13 only); the warps' and then the CTAs' sums are added in
+// FP64 in a fixed order, the latter through distributed shared memory, so the split needs
+// no workspace.  Frequencies of the last group beyond the batch are computed on the
+// batch's last frequency and not stored.
+//
+// Bound: FP32 issue where the grid fills the GPU.  Before the faces were shared out over a
+// cluster, a call of one frequency ran one CTA per 32 points, each warp sweeping an eighth
+// of all the faces: 68 CTAs on 152 SMs for 2,146 points and 9,948 faces (2.0 ms; now
+// 0.4 ms), 5 CTAs for 146 points and 1,036 faces (0.22 ms; now 0.06 ms).
 constexpr int kFieldWarps = 8;
+constexpr int kFieldMaxSplit = 8;
 
-template <int Q, int NC>
+template <int Q, int NC, int NFQ>
 __global__ void __launch_bounds__(256) field_f32_kernel(const FaceF32* __restrict__ faces, int nf,
                                                         const float2* __restrict__ src,
                                                         const float2* __restrict__ drive,  // NC x nf
                                                         const double* __restrict__ obs, int nobs,
-                                                        const FieldParamsF32* __restrict__ prm,
+                                                        const FieldParamsF32* __restrict__ prm, int batch,
                                                         double2* __restrict__ out, FieldRule<float> fr, int ntr,
                                                         int4 trs) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int split = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int o = blockIdx.x * 32 + lane, bt = blockIdx.y;
-  const bool live = o < nobs;
-  const int oc = live ? o : nobs - 1;  // idle lanes repeat a live point; their result is dropped
-  const double xo[3] = {obs[3 * oc], obs[3 * oc + 1], obs[3 * oc + 2]};
-  float xhi[3], xlo[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    xhi[d] = (float)xo[d];
-    xlo[d] = (float)(xo[d] - (double)xhi[d]);
-  }
-  const df kdf = prm->kdf[bt];
-  const float k = prm->k[bt];
-  const float2 qs = prm->qscale[bt];
-  float ar[NC], ac[NC], br[NC], bcmp[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    ar[c] = 0.f;
-    ac[c] = 0.f;
-    br[c] = 0.f;
-    bcmp[c] = 0.f;
-  }
-  // sources: every face and, under symmetry, its images (BeatEngineCore.jl:1240-1280)
-  for (int ti = 0; ti < ntr; ++ti)
-  for (int g = wid; g < nf; g += kFieldWarps) {
-    const FaceF32& F = faces[g];
-    const int tr = ti == 0 ? trs.x : ti == 1 ? trs.y : ti == 2 ? trs.z : trs.w;
-    const float sg[3] = {(tr & 1) ? -1.f : 1.f, (tr & 2) ? -1.f : 1.f, 1.f};
-    const float nrm[3] = {sg[0] * F.normal[0], sg[1] * F.normal[1], F.normal[2]};
-    // base phase k|c_g - x| in double-float
-    df C[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      df s = two_sum(sg[d] * F.anchor_hi[d], -xhi[d]);
-      s.lo += sg[d] * F.anchor_lo[d] - xlo[d];
-      C[d] = quick_two_sum(s.hi, s.lo);
-    }
-    df r2 = df_add(df_add(df_mul(C[0], C[0]), df_mul(C[1], C[1])), df_mul(C[2], C[2]));
-    df R = df_sqrt(r2);
-    const float R0 = R.hi + R.lo;
-    const float theta0 = df_reduce_two_pi(df_mul(kdf, R));
-    const float Cf[3] = {C[0].hi + C[0].lo, C[1].hi + C[1].lo, C[2].hi + C[2].lo};
-    const float Cn = fmaf(Cf[0], nrm[0], fmaf(Cf[1], nrm[1], Cf[2] * nrm[2]));
-    float2 qg[NC], fs[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      qg[c] = cscale(cmul(qs, drive[(size_t)c * nf + g]), F.area2);
-      fs[c] = make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int n = 0; n < Q; ++n) {
-      const float d[3] = {sg[0] * F.off[3 * n], sg[1] * F.off[3 * n + 1], F.off[3 * n + 2]};
-      const float rv[3] = {Cf[0] + d[0], Cf[1] + d[1], Cf[2] + d[2]};
-      const float rr = fmaf(rv[0], rv[0], fmaf(rv[1], rv[1], rv[2] * rv[2]));
-      const float rinv = rr > 1e-30f ? rsqrt_ftz(rr) : 0.f;
-      const float r = rr * rinv;
-      const float cd = fmaf(Cf[0], d[0], fmaf(Cf[1], d[1], Cf[2] * d[2]));
-      const float dd = fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
-      const float delta = fmaf(2.f, cd, dd) * rcp_ftz(fmaxf(r + R0, 1e-30f));
-      const float th = reduce_two_pi(fmaf(k, delta, theta0));
-      float sn, cs;
-      sincos_ftz(th, &sn, &cs);
-      const float sc = rinv * BEM_INV_FOUR_PI;
-      const float2 G = make_float2(cs * sc, sn * sc);
-      // (r . n_y) / r with r . n_y = C . n + d . n (d . n = 0 for points on the face plane, kept for generality)
-      const float t = (Cn + fmaf(d[0], nrm[0], fmaf(d[1], nrm[1], d[2] * nrm[2]))) * rinv;
-      const float2 Dk = make_float2(t * (-G.x * rinv - G.y * k), t * (G.x * k - G.y * rinv));
-      const float wn = fr.w[n];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float2 ps = src[(((size_t)bt * NC + c) * nf + g) * Q + n];
-        const float2 qq = cscale(qg[c], wn);
-        fs[c] = cadd(fs[c], csub(cmul(Dk, ps), cmul(G, qq)));
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      kahan_add(ar[c], ac[c], fs[c].x);
-      kahan_add(br[c], bcmp[c], fs[c].y);
-    }
-  }
-  __shared__ double2 red[kFieldWarps][NC][32];
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-    red[wid][c][lane] = make_double2((double)ar[c] - (double)ac[c], (double)br[c] - (double)bcmp[c]);
-  __syncthreads();
-  if (wid == 0 && live) {
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      double vr = 0.0, vi = 0.0;
-      for (int w = 0; w < kFieldWarps; ++w) {
-        vr += red[w][c][lane].x;
-        vi += red[w][c][lane].y;
-      }
-      out[((size_t)bt * NC + c) * nobs + o] = make_double2(vr, vi);
-    }
-  }
-}
-
-// The same sums for NFQ frequencies of a batch per CTA (blockIdx.y = group of
-// NFQ frequencies starting at NFQ * blockIdx.y).  Everything that does not
-// depend on the frequency is formed once per (point, face) and once per
-// (point, source) and shared by the NFQ frequencies: the double-float
-// distance |c_g - x| to the face anchor, the FP32 offset geometry, 1/r, the
-// compensated r - |c_g - x| and the normal derivative factor t.  Per frequency
-// remain the reduction of k|c_g - x|, the phase of each source, e^{ikr} and the
-// accumulation, with the arithmetic and the order of every sum of
-// field_f32_kernel.  Frequencies of
-// the last group beyond the batch are computed on the batch's last frequency and
-// not stored.
-template <int Q, int NC, int NFQ>
-__global__ void __launch_bounds__(256) field_f32_freqs_kernel(const FaceF32* __restrict__ faces, int nf,
-                                                              const float2* __restrict__ src,
-                                                              const float2* __restrict__ drive,  // NC x nf
-                                                              const double* __restrict__ obs, int nobs,
-                                                              const FieldParamsF32* __restrict__ prm, int batch,
-                                                              double2* __restrict__ out, FieldRule<float> fr, int ntr,
-                                                              int4 trs) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int o = blockIdx.x * 32 + lane;
+  const int o = (blockIdx.x / split) * 32 + lane;
   const int f0 = blockIdx.y * NFQ;
   const bool live = o < nobs;
   const int oc = live ? o : nobs - 1;  // idle lanes repeat a live point; their result is dropped
@@ -230,8 +134,9 @@ __global__ void __launch_bounds__(256) field_f32_freqs_kernel(const FaceF32* __r
       br[f][c] = 0.f;
       bcmp[f][c] = 0.f;
     }
+  // sources: every face and, under symmetry, its images (BeatEngineCore.jl:1240-1280)
   for (int ti = 0; ti < ntr; ++ti)
-  for (int g = wid; g < nf; g += kFieldWarps) {
+  for (int g = rank * kFieldWarps + wid; g < nf; g += split * kFieldWarps) {
     const FaceF32& F = faces[g];
     const int tr = ti == 0 ? trs.x : ti == 1 ? trs.y : ti == 2 ? trs.z : trs.w;
     const float sg[3] = {(tr & 1) ? -1.f : 1.f, (tr & 2) ? -1.f : 1.f, 1.f};
@@ -243,13 +148,14 @@ __global__ void __launch_bounds__(256) field_f32_freqs_kernel(const FaceF32* __r
       s.lo += sg[d] * F.anchor_lo[d] - xlo[d];
       C[d] = quick_two_sum(s.hi, s.lo);
     }
-    df r2 = df_add(df_add(df_mul(C[0], C[0]), df_mul(C[1], C[1])), df_mul(C[2], C[2]));
-    df R = df_sqrt(r2);
+    const df R2 = df_add(df_add(df_mul(C[0], C[0]), df_mul(C[1], C[1])), df_mul(C[2], C[2]));
+    const df R = df_sqrt(R2);
     const float R0 = R.hi + R.lo;
     float theta0[NFQ];
 #pragma unroll
     for (int f = 0; f < NFQ; ++f) theta0[f] = df_reduce_two_pi(df_mul(kdf[f], R));
     const float Cf[3] = {C[0].hi + C[0].lo, C[1].hi + C[1].lo, C[2].hi + C[2].lo};
+    const float C2[3] = {2.f * Cf[0], 2.f * Cf[1], 2.f * Cf[2]};
     const float Cn = fmaf(Cf[0], nrm[0], fmaf(Cf[1], nrm[1], Cf[2] * nrm[2]));
     float2 qg[NFQ][NC], fs[NFQ][NC];
 #pragma unroll
@@ -257,35 +163,40 @@ __global__ void __launch_bounds__(256) field_f32_freqs_kernel(const FaceF32* __r
       const float2 dr = drive[(size_t)c * nf + g];
 #pragma unroll
       for (int f = 0; f < NFQ; ++f) {
-        qg[f][c] = cscale(cmul(qs[f], dr), F.area2);
+        // every rounding spelled out: the same bits whichever NFQ a frequency runs in
+        qg[f][c] = make_float2(__fmul_rn(fmaf(qs[f].x, dr.x, -__fmul_rn(qs[f].y, dr.y)), F.area2),
+                               __fmul_rn(fmaf(qs[f].x, dr.y, __fmul_rn(qs[f].y, dr.x)), F.area2));
         fs[f][c] = make_float2(0.f, 0.f);
       }
     }
 #pragma unroll
     for (int n = 0; n < Q; ++n) {
       const float d[3] = {sg[0] * F.off[3 * n], sg[1] * F.off[3 * n + 1], F.off[3 * n + 2]};
+      const float dd = fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
+      const float s = fmaf(C2[0], d[0], fmaf(C2[1], d[1], fmaf(C2[2], d[2], dd)));
       const float rv[3] = {Cf[0] + d[0], Cf[1] + d[1], Cf[2] + d[2]};
-      const float rr = fmaf(rv[0], rv[0], fmaf(rv[1], rv[1], rv[2] * rv[2]));
+      const float rr = fmaf(rv[0], rv[0], fmaf(rv[1], rv[1], rv[2] * rv[2]));  // not |C|^2 + s: that cancels close by
       const float rinv = rr > 1e-30f ? rsqrt_ftz(rr) : 0.f;
       const float r = rr * rinv;
-      const float cd = fmaf(Cf[0], d[0], fmaf(Cf[1], d[1], Cf[2] * d[2]));
-      const float dd = fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
-      const float delta = fmaf(2.f, cd, dd) * rcp_ftz(fmaxf(r + R0, 1e-30f));
+      const float delta = s * rcp_ftz(fmaxf(r + R0, 1e-30f));
       const float sc = rinv * BEM_INV_FOUR_PI;
-      const float t = (Cn + fmaf(d[0], nrm[0], fmaf(d[1], nrm[1], d[2] * nrm[2]))) * rinv;
-      const float wn = fr.w[n];
+      // (r . n_y) / r with r . n_y = C . n + d . n (d . n = 0 for points on the face plane, kept for generality)
+      const float t = (Cn + fmaf(d[0], nrm[0], fmaf(d[1], nrm[1], d[2] * nrm[2]))) * rinv * sc;
+      const float nta = -t * rinv;          // -(t/r)/r / (4 pi)
+      const float nscw = -sc * fr.w[n];     // -w/r / (4 pi)
 #pragma unroll
       for (int f = 0; f < NFQ; ++f) {
         const float th = reduce_two_pi(fmaf(k[f], delta, theta0[f]));
         float sn, cs;
         sincos_ftz(th, &sn, &cs);
-        const float2 G = make_float2(cs * sc, sn * sc);
-        const float2 Dk = make_float2(t * (-G.x * rinv - G.y * k[f]), t * (G.x * k[f] - G.y * rinv));
+        const float tb = t * k[f];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           const float2 ps = src[(((size_t)bt[f] * NC + c) * nf + g) * Q + n];
-          const float2 qq = cscale(qg[f][c], wn);
-          fs[f][c] = cadd(fs[f][c], csub(cmul(Dk, ps), cmul(G, qq)));
+          const float zx = fmaf(nta, ps.x, fmaf(-tb, ps.y, nscw * qg[f][c].x));
+          const float zy = fmaf(nta, ps.y, fmaf(tb, ps.x, nscw * qg[f][c].y));
+          fs[f][c].x = fmaf(cs, zx, fmaf(-sn, zy, fs[f][c].x));
+          fs[f][c].y = fmaf(cs, zy, fmaf(sn, zx, fs[f][c].y));
         }
       }
     }
@@ -293,31 +204,69 @@ __global__ void __launch_bounds__(256) field_f32_freqs_kernel(const FaceF32* __r
     for (int f = 0; f < NFQ; ++f)
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        kahan_add(ar[f][c], ac[f][c], fs[f][c].x);
-        kahan_add(br[f][c], bcmp[f][c], fs[f][c].y);
+        comp_add(ar[f][c], ac[f][c], fs[f][c].x);
+        comp_add(br[f][c], bcmp[f][c], fs[f][c].y);
       }
   }
   __shared__ double2 red[kFieldWarps][NC][32];
+  __shared__ double2 tot[NFQ][NC][32];  // this CTA's sums, read by the cluster's first CTA
 #pragma unroll
   for (int f = 0; f < NFQ; ++f) {
 #pragma unroll
     for (int c = 0; c < NC; ++c)
       red[wid][c][lane] =
-          make_double2((double)ar[f][c] - (double)ac[f][c], (double)br[f][c] - (double)bcmp[f][c]);
+          make_double2((double)ar[f][c] + (double)ac[f][c], (double)br[f][c] + (double)bcmp[f][c]);
     __syncthreads();
-    if (wid == 0 && live && f0 + f < batch) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        double vr = 0.0, vi = 0.0;
-        for (int w = 0; w < kFieldWarps; ++w) {
-          vr += red[w][c][lane].x;
-          vi += red[w][c][lane].y;
-        }
-        out[((size_t)(f0 + f) * NC + c) * nobs + o] = make_double2(vr, vi);
+    if (wid < NC) {
+      double vr = 0.0, vi = 0.0;
+      for (int w = 0; w < kFieldWarps; ++w) {
+        vr += red[w][wid][lane].x;
+        vi += red[w][wid][lane].y;
       }
+      tot[f][wid][lane] = make_double2(vr, vi);
     }
     __syncthreads();
   }
+  if (split > 1) cluster.sync();
+  if (rank == 0 && wid < NFQ * NC && live) {  // NFQ x NC <= 4 warps, one (frequency, excitation) each
+    const int f = wid / NC, c = wid - f * NC;
+    if (f0 + f < batch) {
+      double vr = 0.0, vi = 0.0;
+      for (int r = 0; r < split; ++r) {
+        const double2 v = *cluster.map_shared_rank(&tot[f][c][lane], r);
+        vr += v.x;
+        vi += v.y;
+      }
+      out[((size_t)(f0 + f) * NC + c) * nobs + o] = make_double2(vr, vi);
+    }
+  }
+  if (split > 1) cluster.sync();  // no CTA leaves while the first may still read its sums
+}
+
+// CTAs of a cluster that share the faces of 32 points: the smallest power of two that gives
+// every SM four CTAs (two keep the FP32 pipe busy; four even out the last wave), while a
+// warp keeps at least four faces.
+int field_split(long long clusters, int nf) {
+  int s = 1;
+  while (s < kFieldMaxSplit && clusters * s < 4LL * sm_count() && nf >= 2 * s * kFieldWarps * 4) s *= 2;
+  return s;
+}
+
+template <typename K, typename... A>
+cudaError_t launch_field_f32(K kern, unsigned pt_blocks, unsigned groups, int nf, cudaStream_t stream, A... args) {
+  const int split = field_split((long long)pt_blocks * groups, nf);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(pt_blocks * split, groups);
+  cfg.blockDim = dim3(kFieldWarps * 32);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 struct FieldParamsF64 {
@@ -435,24 +384,23 @@ cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const d
     }
     FieldParamsF32* dp = (FieldParamsF32*)((char*)sources + (((size_t)total * sizeof(float2) + 255) / 256) * 256);
     cudaMemcpyAsync(dp, &hp, sizeof(hp), cudaMemcpyHostToDevice, stream);
-    // NFQ frequencies per CTA share the frequency-independent geometry; the
-    // largest NFQ (4 or 2, NFQ x nc <= 4) whose grid still gives every SM a CTA
-    // (at 10k with 2,146 points and 15 frequencies: four per CTA, 272 CTAs, field
-    // 0.36 -> 0.30 ms per frequency against the twice-filled grid of two per CTA)
-    const long long pt_blocks = (nobs + 31) / 32;
+    // NFQ frequencies per cluster share the frequency-independent geometry: the largest of
+    // four, two and one with NFQ x nc <= 4 (the sums stay in registers) that the batch fills
     int nfq = 1;
     for (int cand = 4; cand >= 2; cand /= 2)
-      if (cand * nc <= 4 && cand <= batch && pt_blocks * ((batch + cand - 1) / cand) >= (long long)sm_count()) {
+      if (cand * nc <= 4 && cand <= batch) {
         nfq = cand;
         break;
       }
+    const unsigned pt_blocks = (unsigned)((nobs + 31) / 32);
     const int4 trs = make_int4(m.tr[0], m.tr[1], m.tr[2], m.tr[3]);
-    auto run = [&](auto kern, int nf_per_cta) {
-      dim3 g((unsigned)pt_blocks, (unsigned)((batch + nf_per_cta - 1) / nf_per_cta));
-      kern<<<g, 256, 0, stream>>>(m.faces32, m.nf, (const float2*)sources, (const float2*)drive, obs, nobs, dp,
-                                  batch, out, fr32, m.ntr, trs);
+    cudaError_t le = cudaSuccess;
+    auto run = [&](auto kern, int per_cluster) {
+      le = launch_field_f32(kern, pt_blocks, (unsigned)((batch + per_cluster - 1) / per_cluster), m.nf, stream,
+                            (const FaceF32*)m.faces32, m.nf, (const float2*)sources, (const float2*)drive, obs, nobs,
+                            (const FieldParamsF32*)dp, batch, out, fr32, m.ntr, trs);
     };
-#define BEM_F32(QQ, NCC, NFQQ) run(field_f32_freqs_kernel<QQ, NCC, NFQQ>, NFQQ)
+#define BEM_F32(QQ, NCC, NFQQ) run(field_f32_kernel<QQ, NCC, NFQQ>, NFQQ)
 #define BEM_F32_Q(NCC, NFQQ) \
   if (m.Q == 6)              \
     BEM_F32(6, NCC, NFQQ);   \
@@ -476,6 +424,7 @@ cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const d
     }
 #undef BEM_F32_Q
 #undef BEM_F32
+    if (le != cudaSuccess) return le;
   } else {
     field_sources_kernel<double><<<(total + 255) / 256, 256, 0, stream>>>(m.faces, m.area, m.nf, m.Q, nc,
                                                                           (const double2*)pressure, ldp,
@@ -544,19 +493,20 @@ cudaError_t launch_field_single(Precision prec, const void* faces, int nf, int Q
     fr64.phi[i] = rule_phi[i];
   }
   dim3 grid(nobs, 1);
-  dim3 grid32((nobs + 31) / 32, 1);
   if (prec == Precision::Mixed) {
     FieldParamsF32* dp = (FieldParamsF32*)params;
     write_field_params_f32<<<1, 1, 0, stream>>>(dp, k);
     const FaceF32* f = (const FaceF32*)faces;
     const float2* s = (const float2*)sources;
     const float2* d = (const float2*)drive;
-    if (Q == 6)
-      field_f32_kernel<6, 1><<<grid32, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr32, 1, make_int4(0, 0, 0, 0));
-    else if (Q == 3)
-      field_f32_kernel<3, 1><<<grid32, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr32, 1, make_int4(0, 0, 0, 0));
-    else
-      field_f32_kernel<1, 1><<<grid32, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr32, 1, make_int4(0, 0, 0, 0));
+    auto run = [&](auto kern) {
+      return launch_field_f32(kern, (unsigned)((nobs + 31) / 32), 1u, nf, stream, f, nf, s, d, obs, nobs,
+                              (const FieldParamsF32*)dp, 1, out, fr32, 1, make_int4(0, 0, 0, 0));
+    };
+    const cudaError_t le = Q == 6   ? run(field_f32_kernel<6, 1, 1>)
+                           : Q == 3 ? run(field_f32_kernel<3, 1, 1>)
+                                    : run(field_f32_kernel<1, 1, 1>);
+    if (le != cudaSuccess) return le;
   } else {
     FieldParamsF64* dp = (FieldParamsF64*)params;
     write_field_params_f64<<<1, 1, 0, stream>>>(dp, k);
