@@ -318,57 +318,59 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_cluster_kernel(typenam
 // produces go to shared memory (Lb[column][thread]).  Interchanges are virtual:
 // each thread carries the logical row index lg of its physical row, the pivot
 // search compares logical indices (LAPACK's first maximum of |re| + |im|), and
-// every row is written once, at the end, to its logical position.  A step:
-//  1. this CTA's candidate row (the smallest lg among the largest) and the
-//     candidate (value, lg) are pushed into slot j & 1 of every CTA (DSMEM
-//     stores), and the row with lg = j is copied into the local row-j slot;
-//     the writers fence (acq_rel, cluster scope);
+// every row is written once, at the end, to its logical position, which is also
+// the net row permutation that the other columns get.  A step:
+//  1. every warp takes this CTA's candidate from the warps' keys; the warp that
+//     holds the candidate row copies it from its thread's registers through a
+//     shared row and pushes it with the key into slot j & 1 of every CTA (DSMEM
+//     stores, fenced by that warp alone);
 //  2. cluster barrier (relaxed arrive, acquiring wait);
-//  3. every warp takes the pivot and reads the pivot row from its own shared
-//     memory (the pivot's U row j: columns j.. as u[0..]); rank 0 stores it;
-//     only if every candidate is NaN is row j fetched from its CTA instead;
+//  3. every warp takes the pivot from the CTAs' keys and reads the pivot row
+//     (columns j.. as u[0..]) from its own shared memory; rank 0 stores it;
 //  4. the pivot row leaves (lg = j), the row with lg = j takes the pivot's old
 //     lg; every other active row stores l = a[0] / pivot, subtracts l u and
 //     shifts; the next candidate is reduced per warp; CTA barrier.
+// A single CTA (CLUSTER = false) replaces 1 and 2 by the owner thread writing the
+// row to its own shared memory and a CTA barrier.
 // Requires a full panel (kb = 32) and chunk <= kRegPanelThreads.
+//
+// Bound: the latency of a column step (two barriers, the candidate exchange and the row
+// update, about 440 issue cycles with 640 rows on an SM).  The keys are reduced by the
+// warp-reduction instruction (two 32-bit maxima instead of five 64-bit shuffle stages),
+// one warp instead of 640 threads does the push, and no row-j copy is kept for the
+// all-NaN case (a NaN key ranks below every number, so row j itself wins it): 32 columns
+// of one matrix take 29 us with one CTA (518 rows) and 53 us with eight (4,976); 74 us before, either way.
 constexpr int kRegPanelThreads = 640;
 constexpr int kRegPanelWarps = kRegPanelThreads / 32;
 
-// Pivot candidates as one 64-bit key: the bits of |re| + |im| (non-negative,
-// so their unsigned order is the value order) above the complement of the
-// logical row, so the largest key is the first maximum (larger value, then
-// smaller row).  NaN values and rows without a candidate get key 0, which no
-// candidate key equals (the low word ~row is at least 2^31).
-__device__ __forceinline__ unsigned long long pivot_key(float v, int row) {
-  return v == v ? ((unsigned long long)__float_as_uint(v) << 32) | (unsigned)~row : 0ull;
+// Pivot candidates as two 32-bit words, compared as (hi, lo): the bits of |re| + |im|
+// plus one (non-negative floats order as their bits; 0 for NaN) and the complement of the
+// logical row, so the largest key is the first maximum (larger value, then smaller row).
+// A row that is no candidate has (0, 0), below every candidate: lo >= 2^31 for any row.
+__device__ __forceinline__ uint2 pivot_key(float v, int row) {
+  return make_uint2(v == v ? __float_as_uint(v) + 1u : 0u, (unsigned)~row);
 }
-__device__ __forceinline__ int key_row(unsigned long long key) { return (int)~(unsigned)key; }
-__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, o);
-    k = ok > k ? ok : k;
-  }
-  return k;
+__device__ __forceinline__ uint2 warp_max_key(uint2 k) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, k.x);
+  return make_uint2(hi, __reduce_max_sync(0xffffffffu, k.x == hi ? k.y : 0u));
 }
 
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float2* A, long long lda, long long strideA,
                                                                            int n, int k, int kb, int chunk, int* ipiv,
                                                                            int* info, int* rowmap) {
   constexpr int NB = 32;
   constexpr int NW = kRegPanelWarps;
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int CL = (int)cluster.num_blocks();
+  const int rank = CLUSTER ? (int)cluster.block_rank() : 0;
+  const int CL = CLUSTER ? (int)cluster.num_blocks() : 1;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* Lb = reinterpret_cast<float2*>(smem_raw);  // [NB][kRegPanelThreads] multipliers by column, thread
-  __shared__ float2 rowsC[2][16][NB];  // pushed candidate rows, by source CTA
-  __shared__ float2 pub[NB], dg[2][NB];
-  __shared__ float2 urow[NB];
-  __shared__ unsigned long long ckey[2][16], wkey[NW];
-  __shared__ int chasj[2][16];
-  __shared__ int s_pivs[NB];
+  __shared__ __align__(16) float4 rowsC[2][CLUSTER ? 16 : 1][NB / 2];  // candidate rows, by source CTA
+  __shared__ __align__(16) float4 pub[NB / 2];
+  __shared__ uint2 ckey[2][16], wkey[NW];
+  __shared__ int s_moved;  // rows that changed place (rank 0's counts for the cluster)
   float2* M = A + (size_t)blockIdx.y * strideA;
   int* piv = ipiv + (size_t)blockIdx.y * n;
   const int m = n - k;
@@ -383,69 +385,55 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
 #pragma unroll
     for (int c = 0; c < NB; ++c) a[c] = mine ? src[(size_t)c * lda] : make_float2(0.f, 0.f);
   }
-  auto candidate = [&]() {  // the warp's candidate key for the current column
-    return warp_max_key(mine && done_at < 0 ? pivot_key(abs1(a[0]), lg) : 0ull);
-  };
-  {
-    const unsigned long long key = candidate();
+  auto publish_warp_key = [&]() {  // the warp's candidate for the current column
+    const uint2 key = warp_max_key(mine && done_at < 0 ? pivot_key(abs1(a[0]), lg) : make_uint2(0u, 0u));
     if (lane == 0) wkey[wid] = key;
-  }
+  };
+  auto copy_row = [&](float4* dst) {
+#pragma unroll
+    for (int q = 0; q < NB / 2; ++q) dst[q] = make_float4(a[2 * q].x, a[2 * q].y, a[2 * q + 1].x, a[2 * q + 1].y);
+  };
+  if (tid == 0) s_moved = 0;
+  publish_warp_key();
   __syncthreads();
 #pragma unroll 1
   for (int j = 0; j < NB; ++j) {
     const int s = j & 1;
-    {  // 1. publish and push
-      const unsigned long long key = warp_max_key(lane < NW ? wkey[lane] : 0ull);
-      const bool active = mine && done_at < 0;
-      if (key != 0ull && active && lg == key_row(key)) {  // this CTA's candidate row (logical rows are distinct)
-#pragma unroll
-        for (int c = 0; c < NB; ++c) pub[c] = a[c];
+    // 1. this CTA's candidate, pushed by the warp that holds it
+    uint2 key = warp_max_key(lane < NW ? wkey[lane] : make_uint2(0u, 0u));
+    const bool own = mine && done_at < 0 && key.y != 0u && lg == (int)~key.y;  // logical rows are distinct
+    if constexpr (CLUSTER) {
+      const bool owner_warp = __ballot_sync(0xffffffffu, own) != 0u;
+      if (owner_warp) {
+        if (own) copy_row(pub);
+        __syncwarp();
+        const float4 v = pub[lane & 15];
+        for (int t = lane >> 4; t < CL; t += 2) *cluster.map_shared_rank(&rowsC[s][rank][lane & 15], t) = v;
       }
-      const bool hasj = active && lg == j;
-      if (hasj) {
-#pragma unroll
-        for (int c = 0; c < NB; ++c) dg[s][c] = a[c];
+      if (owner_warp || (key.y == 0u && wid == 0)) {  // without a candidate row, warp 0 says so
+        if (lane < CL) *cluster.map_shared_rank(&ckey[s][rank], lane) = key;
+        asm volatile("fence.acq_rel.cluster;" ::: "memory");
       }
-      const int cnt = __syncthreads_or(hasj);
-      bool wrote = hasj;
-      if (key != 0ull && tid < CL * NB) {  // the candidate row into every CTA
-        *cluster.map_shared_rank(&rowsC[s][rank][tid & (NB - 1)], tid / NB) = pub[tid & (NB - 1)];
-        wrote = true;
-      }
-      if (tid < CL) {
-        *cluster.map_shared_rank(&ckey[s][rank], tid) = key;
-        *cluster.map_shared_rank(&chasj[s][rank], tid) = cnt;
-        wrote = true;
-      }
-      if (wrote) asm volatile("fence.acq_rel.cluster;" ::: "memory");
-    }
-    // 2. the writes above were fenced by their writers; the wait acquires them
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-    // 3. pivot (logical row p, held by CTA pr), in every warp
-    const unsigned long long ck = lane < CL ? ckey[s][lane] : 0ull;
-    const unsigned long long km = warp_max_key(ck);
-    const bool fallback = km == 0ull;  // no comparable candidate (all NaN): keep row j
-    const int pr = __ffs(__ballot_sync(0xffffffffu, lane < CL && ck == km)) - 1;  // keys are distinct
-    const int p = fallback ? j : key_row(km);
-    const float2* U = &rowsC[s][fallback ? 0 : pr][0];  // the pivot row, u[c] = U(j, j + c) (zero beyond the panel)
-    if (fallback) {  // every CTA takes this branch together
-      if (wid == 0) {
-        int jr = 0;  // CTA holding logical row j
-        const unsigned hb = __ballot_sync(0xffffffffu, lane < CL && chasj[s][lane] != 0);
-        if (hb) jr = __ffs(hb) - 1;
-        urow[lane] = *cluster.map_shared_rank(&dg[s][lane], jr);
-      }
+      // 2. the writes above were fenced by their writers; the wait acquires them
+      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    } else {
+      if (own) copy_row(rowsC[s][0]);
       __syncthreads();
-      U = urow;
     }
+    // 3. pivot (logical row p, held by CTA pr), in every warp; row j itself is a candidate, so there is one
+    int pr = 0;
+    if constexpr (CLUSTER) {
+      const uint2 ck = lane < CL ? ckey[s][lane] : make_uint2(0u, 0u);
+      key = warp_max_key(ck);
+      pr = __ffs(__ballot_sync(0xffffffffu, ck.x == key.x && ck.y == key.y)) - 1;  // keys are distinct
+    }
+    const int p = (int)~key.y;
+    const float4* U = rowsC[s][pr];  // the pivot row, u[c] = U(j, j + c) (zero beyond the panel)
     if (rank == 0 && wid == 0 && lane < NB - j)  // U row j
-      M[(size_t)(k + j + lane) * lda + k + j] = U[lane];
-    if (rank == 0 && tid == 0) {
-      piv[k + j] = k + p;
-      s_pivs[j] = p;
-    }
-    const float2 d = U[0];
+      M[(size_t)(k + j + lane) * lda + k + j] = reinterpret_cast<const float2*>(U)[lane];
+    if (rank == 0 && tid == 0) piv[k + j] = k + p;
+    const float2 d = make_float2(U[0].x, U[0].y);
     float2 inv;
     if (d.x == 0.f && d.y == 0.f) {
       inv = make_float2(0.f, 0.f);
@@ -469,10 +457,14 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
         auto update = [&](auto width) {
           constexpr int W = decltype(width)::value;
 #pragma unroll
-          for (int c = 1; c < W; ++c) {
-            const float2 u = U[c];
-            a[c - 1].x = fmaf(-l.x, u.x, fmaf(l.y, u.y, a[c].x));
-            a[c - 1].y = fmaf(-l.x, u.y, fmaf(-l.y, u.x, a[c].y));
+          for (int q = 0; q < W / 2; ++q) {
+            const float4 u = U[q];
+            if (q > 0) {
+              a[2 * q - 1].x = fmaf(-l.x, u.x, fmaf(l.y, u.y, a[2 * q].x));
+              a[2 * q - 1].y = fmaf(-l.x, u.y, fmaf(-l.y, u.x, a[2 * q].y));
+            }
+            a[2 * q].x = fmaf(-l.x, u.z, fmaf(l.y, u.w, a[2 * q + 1].x));
+            a[2 * q].y = fmaf(-l.x, u.w, fmaf(-l.y, u.z, a[2 * q + 1].y));
           }
           a[W - 1] = make_float2(0.f, 0.f);
         };
@@ -486,10 +478,7 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
           update(std::integral_constant<int, 8>{});
       }
     }
-    {
-      const unsigned long long key = candidate();
-      if (lane == 0) wkey[wid] = key;  // every thread read wkey in this step's push, before the cluster barrier
-    }
+    publish_warp_key();  // every thread read wkey in this step's 1, before the barrier of 2
     __syncthreads();
   }
   // every row to its logical position: the multipliers left of its pivot column
@@ -499,8 +488,18 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
     float2* dst = M + (size_t)k * lda + k + lg;
     for (int c = 0; c < ncol; ++c) dst[(size_t)c * lda] = Lb[(size_t)c * kRegPanelThreads + tid];
   }
-  if (rank == 0 && wid == 0 && rowmap != nullptr) net_row_map<NB>(s_pivs, NB, k, rowmap + (size_t)blockIdx.y * kRowmapStride);
-  cluster.sync();  // no CTA leaves while others may still read its shared memory
+  // the net row permutation, [count, (dst row, src row) x count] in any order (at most 2 kb rows move)
+  if (rowmap != nullptr) {
+    int* rm = rowmap + (size_t)blockIdx.y * kRowmapStride;
+    if (mine && lg != r0 + tid) {
+      const int e = atomicAdd(CLUSTER ? cluster.map_shared_rank(&s_moved, 0) : &s_moved, 1);
+      rm[1 + 2 * e] = k + lg;
+      rm[2 + 2 * e] = k + r0 + tid;
+    }
+    if constexpr (!CLUSTER) __syncthreads();
+  }
+  if constexpr (CLUSTER) cluster.sync();  // no CTA leaves while others may still use its shared memory
+  if (rowmap != nullptr && rank == 0 && tid == 0) rowmap[(size_t)blockIdx.y * kRowmapStride] = s_moved;
 }
 
 // perm[i] such that (P b)[i] = b[perm[i]], from LAPACK-style interchanges.
@@ -794,9 +793,10 @@ template <typename R> bool choose_panel(int n, int want_nb, int batch, int& nb, 
     for (int c : {1, 2, 4, 8, 16}) {
       if ((n + c - 1) / c > kRegPanelThreads) continue;
       const size_t sm = (size_t)32 * kRegPanelThreads * sizeof(float2);
-      if (c > 1 && max_cluster(lu_panel_reg_kernel, kRegPanelThreads, sm) < c) continue;
-      if (c == 1 && !ensure_smem_limit((const void*)lu_panel_reg_kernel, sm)) continue;
-      const int act = active_clusters(lu_panel_reg_kernel, kRegPanelThreads, sm, c);
+      if (c > 1 && max_cluster(lu_panel_reg_kernel<true>, kRegPanelThreads, sm) < c) continue;
+      if (c == 1 && !ensure_smem_limit((const void*)lu_panel_reg_kernel<false>, sm)) continue;
+      const int act = c > 1 ? active_clusters(lu_panel_reg_kernel<true>, kRegPanelThreads, sm, c)
+                            : active_clusters(lu_panel_reg_kernel<false>, kRegPanelThreads, sm, c);
       if (act < 1) continue;
       const int waves = (std::max(batch, 1) + act - 1) / act;
       if (!found || waves < best_waves) {
@@ -866,7 +866,10 @@ int lu_resident_batch(Precision prec, int n) {
   const int chunk = (n + cl - 1) / cl;
   int act = 0;
   if (prec == Precision::Mixed && nb == 32 && chunk <= kRegPanelThreads)
-    act = active_clusters(lu_panel_reg_kernel, kRegPanelThreads, (size_t)32 * kRegPanelThreads * sizeof(float2), cl);
+    act = cl > 1 ? active_clusters(lu_panel_reg_kernel<true>, kRegPanelThreads,
+                                   (size_t)32 * kRegPanelThreads * sizeof(float2), cl)
+                 : active_clusters(lu_panel_reg_kernel<false>, kRegPanelThreads,
+                                   (size_t)32 * kRegPanelThreads * sizeof(float2), cl);
   else if (prec == Precision::Mixed)
     act = nb == 64 ? active_clusters(lu_panel_cluster_kernel<float, 64>, kPanelThreads, panel_smem<float, 64>(chunk), cl)
                    : active_clusters(lu_panel_cluster_kernel<float, 32>, kPanelThreads, panel_smem<float, 32>(chunk), cl);
@@ -884,9 +887,13 @@ cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long s
   dim3 grid(cl, batch);
   if (prec == Precision::Mixed && nb == 32 && chunk <= kRegPanelThreads && kb == 32) {
     const size_t sm = (size_t)32 * kRegPanelThreads * sizeof(float2);
-    ensure_smem_limit((const void*)lu_panel_reg_kernel, sm);
-    cudaFuncSetAttribute(lu_panel_reg_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return launch_cluster(lu_panel_reg_kernel, grid, kRegPanelThreads, sm, cl, stream, args);
+    if (cl == 1) {
+      ensure_smem_limit((const void*)lu_panel_reg_kernel<false>, sm);
+      return launch_cluster(lu_panel_reg_kernel<false>, grid, kRegPanelThreads, sm, cl, stream, args);
+    }
+    ensure_smem_limit((const void*)lu_panel_reg_kernel<true>, sm);
+    cudaFuncSetAttribute(lu_panel_reg_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return launch_cluster(lu_panel_reg_kernel<true>, grid, kRegPanelThreads, sm, cl, stream, args);
   }
   if (prec == Precision::Mixed) {
     if (nb == 64) {
