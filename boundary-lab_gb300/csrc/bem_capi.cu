@@ -952,13 +952,12 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
   int lu_launches = 0;
   ck(bem::lu_factor_batched(prec, ctx->mats.p, lda, n, B, (int*)ctx->ipiv.p, (int*)ctx->info.p, nb, ctx->cublas,
                             ctx->stream, (bem::LuGemm)o.lu_gemm, tcws, &used_tensor, &tc_err, (int*)ctx->rowmap.p,
-                            &lu_launches),
+                            &lu_launches, (int*)ctx->perm.p),
      "LU factorisation");
-  // kernels of this batch besides the assembly: the LU, the permutation, the solves
+  // kernels of this batch besides the assembly: the LU with its row permutation, the solves
   // (mixed: 6 + 6 per refinement step), the field (2, +1 mixed, per slice)
-  T.launches += lu_launches + 1;
+  T.launches += lu_launches;
   T.gemm_used = mixed ? (used_tensor ? 2 : 1) : 0;
-  ck(bem::lu_perm_batched((const int*)ctx->ipiv.p, n, B, (int*)ctx->perm.p, ctx->stream), "pivot permutation");
   prof_mark(ctx, BEM_K_LU);
   ck(cudaMemcpyAsync(info.data(), ctx->info.p, (size_t)B * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
      "copy info");

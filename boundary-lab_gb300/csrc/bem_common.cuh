@@ -172,6 +172,27 @@ BEM_D float reduce_two_pi(float t) {
   return fmaf(-n, BEM_TWO_PI_MID, t);
 }
 
+// ------------------------------------------------------- row permutation --
+// Applies a panel's net row permutation (cnt <= 128 pairs: row sdst takes row ssrc) to one
+// column of n entries, by one warp: every source row is loaded (at most 4 per lane, all in
+// flight) before any destination row is stored.
+template <typename T>
+__device__ __forceinline__ void permute_column(T* a, int n, int cnt, const int* sdst, const int* ssrc) {
+  const int lane = threadIdx.x & 31;
+  T v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int e = lane + 32 * q;
+    if (e < cnt && (unsigned)ssrc[e] < (unsigned)n) v[q] = a[ssrc[e]];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int e = lane + 32 * q;
+    if (e < cnt && (unsigned)ssrc[e] < (unsigned)n && (unsigned)sdst[e] < (unsigned)n) a[sdst[e]] = v[q];
+  }
+}
+
 // -------------------------------------------------------- status / limits --
 // Device status word written by kernels that can detect bad input; the host
 // reads it after the launch.  No kernel traps or spins without a bound.

@@ -156,7 +156,8 @@ int* tc_gemm_error_word(TcGemmPlan* p);
 // batch) bytes, may be null) enables the tensor-core update; *used_tensor tells
 // which update ran; *tc_err receives the device address of the kernel's error word.
 // rowmap (batch * kRowmapStride ints, may be null) lets the cluster panel hand
-// the net row permutation of its interchanges to the row-swap kernel.
+// the net row permutation of its interchanges to the row-swap kernel.  perm (batch * n
+// ints, may be null) receives the row permutation: (P b)[i] = b[perm[i]].
 constexpr int kRowmapStride = 512;
 // Outer block width of the two-level LU (trailing-update depth); a multiple of
 // every cluster panel width (32, 64) and at most the tcgen05 update's K (256).
@@ -165,11 +166,11 @@ constexpr int kRowmapStride = 512;
 // per frequency at n = 4,976 against 128).
 constexpr int kOuterBlock = 256;
 // Kernels the two-level LU launches for one batch (cuBLAS kernels not counted).
-int lu_launch_count(int n, int nb, int NB, bool tensor);
+int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm);
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info,
                               int nb, void* cublas_handle, cudaStream_t stream, LuGemm gemm = LuGemm::Cublas,
                               void* tc_workspace = nullptr, bool* used_tensor = nullptr, int** tc_err = nullptr,
-                              int* rowmap = nullptr, int* n_launches = nullptr);
+                              int* rowmap = nullptr, int* n_launches = nullptr, int* perm = nullptr);
 // Solve (LU) X = B in place for nrhs columns per matrix (B stride ldb*nrhs per matrix), working precision.
 cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* ipiv,
                              void* B, long long ldb, int nrhs, int nb, cudaStream_t stream);
@@ -188,10 +189,11 @@ int lu_resident_batch(Precision prec, int n);
 // the net effect of the panel's kb interchanges on any column (at most 2 kb rows).
 cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb, int nb,
                              int cl, int batch, int* ipiv, int* info, cudaStream_t stream, int* rowmap = nullptr);
-// Apply a panel's net row permutation (rowmap) to every column outside the panel.
+// Apply a panel's net row permutation (rowmap) to every column outside the panel, and to
+// perm (batch * n ints) when not null.
 cudaError_t lu_swap_rows_batched(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb,
-                                 int batch, const int* rowmap, cudaStream_t stream);
-// perm[i]: (P b)[i] = b[perm[i]]; then one cluster per right-hand side solves in place.
+                                 int batch, const int* rowmap, int* perm, cudaStream_t stream);
+// perm from the interchanges ipiv, (P b)[i] = b[perm[i]]; then one cluster per right-hand side solves in place.
 cudaError_t lu_perm_batched(const int* ipiv, int n, int batch, int* perm, cudaStream_t stream);
 cudaError_t lu_solve_cluster_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* perm,
                                      void* B, long long ldb, int nrhs, cudaStream_t stream);

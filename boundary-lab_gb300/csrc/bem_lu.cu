@@ -208,42 +208,260 @@ __global__ void lu_trsm_kernel(C2* A, long long lda, long long strideA, int n, i
   }
 }
 
-// U12 = L11^{-1} A12 for a 32-row block (mixed form): one thread per column,
-// the column's 32 complex entries in registers (the 32 x 32 substitution is
-// fully unrolled, so every index is a constant); L11 (unit lower) in shared
-// memory, read as broadcasts.  Replaces lu_trsm_kernel's shared-memory column
-// for kb = 32: 496 multiply-adds per column with no shared-memory traffic for X.
-__global__ void __launch_bounds__(128) lu_trsm32_kernel(float2* A, long long lda, long long strideA, int k,
-                                                        int c_begin, int c_end) {
-  __shared__ float2 L[32 * 32];  // column-major
+// The three steps around the 32-wide panels of the two-level LU (mixed form).  A panel of
+// one matrix takes some tens of microseconds on at most 16 SMs, so what follows it has to
+// be short as well; these kernels do the outer block's own part in plain FP32 FMAs, which
+// a K = 32 product does in less time than it takes to split its operands for the tensor
+// cores and read them back.  Measured at n = 4,976, one matrix (and 15): per 32 columns of
+// the outer block, interchanges + U rows 6 us (29) where the two kernels before took 15,
+// the rest of the block 7 us (30) where operand split + tcgen05 update took 13; per 256
+// columns, the U rows for the trailing columns 40 us (310) where eight rounds of
+// triangular solve, operand split and update took 180.  The time before was latency for
+// one matrix (LU 16.9 -> 12.3 ms) and about the same work for 15 (75.7 -> 71.9 ms for 30).
+
+// Applies a panel's net row permutation (rowmap) to every column outside the panel and
+// turns rows k .. k + 31 of the outer block's columns right of it, [k + 32, c_end), into U
+// rows: x = L11^{-1} x with the panel's unit lower triangle.  One warp per column.  The
+// first `solve_ctas` CTAs take the columns to solve: lane = row of the diagonal block, its
+// new value comes through shared memory, and the substitution broadcasts x_j from lane j.
+// The others only permute; a warp more carries the row permutation so far (perm[i] =
+// source of row i; null: none) as a column of its own.
+__global__ void __launch_bounds__(256) lu_swap_urows_kernel(float2* A, long long lda, long long strideA, int n, int k,
+                                                            int c_end, int solve_ctas,
+                                                            const int* __restrict__ rowmap, int* __restrict__ perm) {
+  __shared__ int sdst[128], ssrc[128];
+  __shared__ float2 top[8][32];
+  __shared__ float2 L[32][32];  // [column][row]
+  __shared__ int s_cnt;
+  const int* rm = rowmap + (size_t)blockIdx.y * kRowmapStride;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2* M = A + (size_t)blockIdx.y * strideA;
-  for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
-    const int r = i & 31, c = i >> 5;
-    L[i] = M[(size_t)(k + c) * lda + k + r];
+  const bool solver = (int)blockIdx.x < solve_ctas;
+  if (solver)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) L[wid + 8 * q][lane] = M[(size_t)(k + wid + 8 * q) * lda + k + lane];
+  if (threadIdx.x == 0) s_cnt = min(max(rm[0], 0), 128);
+  __syncthreads();
+  const int cnt = s_cnt;
+  for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+    sdst[e] = rm[1 + 2 * e];
+    ssrc[e] = rm[2 + 2 * e];
   }
   __syncthreads();
-  const int col = c_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= c_end) return;
-  float4* src = reinterpret_cast<float4*>(M + (size_t)col * lda + k);  // 16-byte aligned: lda and k are even
-  float2 x[32];
+  if (solver) {
+    const int c = k + 32 + blockIdx.x * 8 + wid;
+    if (c >= c_end) return;
+    float2* a = M + (size_t)c * lda;
+    float2 v[4];
+    top[wid][lane] = a[k + lane];
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const float4 v = src[q];
-    x[2 * q] = make_float2(v.x, v.y);
-    x[2 * q + 1] = make_float2(v.z, v.w);
+    for (int q = 0; q < 4; ++q) {
+      const int e = lane + 32 * q;
+      if (e < cnt && (unsigned)ssrc[e] < (unsigned)n) v[q] = a[ssrc[e]];
+    }
+    __syncwarp();  // every source is read before any destination is written
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = lane + 32 * q;
+      if (e < cnt && (unsigned)ssrc[e] < (unsigned)n && (unsigned)sdst[e] < (unsigned)n) {
+        if ((unsigned)(sdst[e] - k) < 32u)
+          top[wid][sdst[e] - k] = v[q];
+        else
+          a[sdst[e]] = v[q];
+      }
+    }
+    __syncwarp();
+    float2 x = top[wid][lane];
+#pragma unroll
+    for (int j = 0; j < 31; ++j) {
+      const float xr = __shfl_sync(0xffffffffu, x.x, j), xi = __shfl_sync(0xffffffffu, x.y, j);
+      const float2 l = L[j][lane];
+      if (lane > j) {
+        x.x = fmaf(-l.x, xr, fmaf(l.y, xi, x.x));
+        x.y = fmaf(-l.x, xi, fmaf(-l.y, xr, x.y));
+      }
+    }
+    a[k + lane] = x;
+    return;
   }
+  const int t = (blockIdx.x - solve_ctas) * 8 + wid;  // left of the panel, then right of the outer block
+  const int rest = k + (n - c_end);
+  if (cnt == 0 || t > rest) return;
+  if (t < rest)
+    permute_column(M + (size_t)(t < k ? t : c_end + (t - k)) * lda, n, cnt, sdst, ssrc);
+  else if (perm != nullptr)
+    permute_column(perm + (size_t)blockIdx.y * n, n, cnt, sdst, ssrc);
+}
+
+// A[r0 .. r0 + M, c0 .. c0 + N) -= A[r0 .., kc .. kc + 32) A[kc .. kc + 32, c0 ..): one CTA per
+// 128 x 32 tile, both operands in shared memory, each thread 4 x 4 entries in registers
+// (rows 32 apart, so every global access of a warp is one run of 256 bytes).
+__global__ void __launch_bounds__(256) lu_update32_kernel(float2* A, long long lda, long long strideA, int r0, int M,
+                                                          int c0, int N, int kc) {
+  __shared__ float2 sl[32][128];
+  __shared__ __align__(16) float2 su[32][32];
+  float2* Mx = A + (size_t)blockIdx.z * strideA;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int row0 = blockIdx.x * 128, col0 = blockIdx.y * 32;
+  {
+    const int r = tid & 127, kh = tid >> 7;
+    const bool in = row0 + r < M;
+    const float2* src = Mx + (size_t)kc * lda + r0 + row0 + r;
+    float2 v[16];
 #pragma unroll
-  for (int j = 0; j < 31; ++j) {
-    const float2 xj = x[j];
+    for (int q = 0; q < 16; ++q) v[q] = in ? src[(size_t)(2 * q + kh) * lda] : make_float2(0.f, 0.f);
+    float2 u[4];
 #pragma unroll
-    for (int i = j + 1; i < 32; ++i) {
-      const float2 l = L[j * 32 + i];
-      x[i].x = fmaf(-l.x, xj.x, fmaf(l.y, xj.y, x[i].x));
-      x[i].y = fmaf(-l.x, xj.y, fmaf(-l.y, xj.x, x[i].y));
+    for (int q = 0; q < 4; ++q) {
+      const int cc = col0 + wid + 8 * q;
+      u[q] = cc < N ? Mx[(size_t)(c0 + cc) * lda + kc + lane] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) sl[2 * q + kh][r] = v[q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) su[lane][wid + 8 * q] = u[q];
+  }
+  float2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = row0 + lane + 32 * i, c = col0 + 4 * wid + j;
+      acc[i][j] = r < M && c < N ? Mx[(size_t)(c0 + c) * lda + r0 + r] : make_float2(0.f, 0.f);
+    }
+  __syncthreads();
+#pragma unroll 8
+  for (int kk = 0; kk < 32; ++kk) {
+    const float4 ua = *reinterpret_cast<const float4*>(&su[kk][4 * wid]);
+    const float4 ub = *reinterpret_cast<const float4*>(&su[kk][4 * wid + 2]);
+    const float2 u[4] = {make_float2(ua.x, ua.y), make_float2(ua.z, ua.w), make_float2(ub.x, ub.y),
+                         make_float2(ub.z, ub.w)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 l = sl[kk][lane + 32 * i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[i][j].x = fmaf(-l.x, u[j].x, fmaf(l.y, u[j].y, acc[i][j].x));
+        acc[i][j].y = fmaf(-l.x, u[j].y, fmaf(-l.y, u[j].x, acc[i][j].y));
+      }
     }
   }
 #pragma unroll
-  for (int q = 0; q < 16; ++q) src[q] = make_float4(x[2 * q].x, x[2 * q].y, x[2 * q + 1].x, x[2 * q + 1].y);
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = row0 + lane + 32 * i, c = col0 + 4 * wid + j;
+      if (r < M && c < N) Mx[(size_t)(c0 + c) * lda + r0 + r] = acc[i][j];
+    }
+}
+
+// U rows of a whole outer block for the trailing columns: rows [k0, k0 + 256) of columns
+// [c0, c1) become L^{-1} times themselves, L the unit lower triangle of the outer block.
+// Left-looking over 32-row blocks: a warp owns CPW columns, lane = row of the current
+// block; the block first takes its products with the solved blocks (their rows in the
+// warp's shared memory, read as broadcasts), then the 32 x 32 substitution (x_j broadcast
+// from lane j).  The CTA's warps walk the triangle's 36 tiles of 32 x 32 together, each
+// tile staged once for all of them by asynchronous copies kUrowsStages - 1 tiles ahead
+// (read directly by every warp, L's latency made the kernel four times slower).  CPW = 8
+// needs the fewest shared-memory reads per FMA; 4 halves the time of a call whose columns
+// leave SMs idle.
+constexpr int kUrowsWarps = 4, kUrowsStages = 4;
+template <int CPW> constexpr size_t urows_smem() {
+  return ((size_t)kUrowsStages * 32 * 32 + (size_t)kUrowsWarps * kOuterBlock * CPW) * sizeof(float2);
+}
+template <int CPW>
+__global__ void __launch_bounds__(kUrowsWarps * 32) lu_urows_kernel(float2* A, long long lda, long long strideA, int k0,
+                                                                    int c0, int c1) {
+  constexpr int NBLK = kOuterBlock / 32, TILES = NBLK * (NBLK + 1) / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  float2* ring = reinterpret_cast<float2*>(smem_raw);                                           // [stage][column][row]
+  float2* X = ring + kUrowsStages * 32 * 32 + (size_t)wid * kOuterBlock * CPW;  // [row][CPW]
+  float2* M = A + (size_t)blockIdx.y * strideA;
+  const int cw = c0 + (blockIdx.x * kUrowsWarps + wid) * CPW;
+  const int nc = max(0, min(CPW, c1 - cw));
+  const float2* Lm = M + (size_t)k0 * lda + k0;
+  int pb = 0, pl = 0;  // next tile to stage: rows 32 pb.., columns 32 pl..
+  auto stage = [&](int slot) {
+    if (pb < NBLK) {
+      float2* dst = ring + (size_t)slot * 32 * 32;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {  // 512 pieces of 16 bytes
+        const int i = threadIdx.x + 128 * q, col = i >> 4, piece = i & 15;
+        const float2* src = Lm + (size_t)(32 * pl + col) * lda + 32 * pb + 2 * piece;
+        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + 32 * col + 2 * piece);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
+      }
+      if (++pl > pb) {
+        pl = 0;
+        ++pb;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < kUrowsStages - 1; ++i) stage(i);
+  float2 x[CPW], nx[CPW];  // the current block's rows, and the next one's
+#pragma unroll
+  for (int c = 0; c < CPW; ++c) nx[c] = c < nc ? M[(size_t)(cw + c) * lda + k0 + lane] : make_float2(0.f, 0.f);
+  int b = 0, l = 0;
+  for (int t = 0; t < TILES; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kUrowsStages - 2) : "memory");
+    __syncthreads();  // tile t is in place for every warp, and tile t - 1 is no longer read
+    stage((t + kUrowsStages - 1) % kUrowsStages);
+    const float2* T = ring + (size_t)(t % kUrowsStages) * 32 * 32 + lane;
+    if (l == 0) {
+#pragma unroll
+      for (int c = 0; c < CPW; ++c) x[c] = nx[c];
+      if (b + 1 < NBLK) {
+#pragma unroll
+        for (int c = 0; c < CPW; ++c)
+          nx[c] = c < nc ? M[(size_t)(cw + c) * lda + k0 + 32 * (b + 1) + lane] : make_float2(0.f, 0.f);
+      }
+    }
+    if (l < b) {
+      const float4* xs = reinterpret_cast<const float4*>(X + (size_t)32 * l * CPW);
+#pragma unroll 8
+      for (int kk = 0; kk < 32; ++kk) {
+        const float2 lv = T[32 * kk];
+#pragma unroll
+        for (int q = 0; q < CPW / 2; ++q) {
+          const float4 u = xs[kk * (CPW / 2) + q];
+          x[2 * q].x = fmaf(-lv.x, u.x, fmaf(lv.y, u.y, x[2 * q].x));
+          x[2 * q].y = fmaf(-lv.x, u.y, fmaf(-lv.y, u.x, x[2 * q].y));
+          x[2 * q + 1].x = fmaf(-lv.x, u.z, fmaf(lv.y, u.w, x[2 * q + 1].x));
+          x[2 * q + 1].y = fmaf(-lv.x, u.w, fmaf(-lv.y, u.z, x[2 * q + 1].y));
+        }
+      }
+      ++l;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 31; ++j) {
+        const float2 lv = T[32 * j];
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) {
+          const float xr = __shfl_sync(0xffffffffu, x[c].x, j), xi = __shfl_sync(0xffffffffu, x[c].y, j);
+          if (lane > j) {
+            x[c].x = fmaf(-lv.x, xr, fmaf(lv.y, xi, x[c].x));
+            x[c].y = fmaf(-lv.x, xi, fmaf(-lv.y, xr, x[c].y));
+          }
+        }
+      }
+      float4* xd = reinterpret_cast<float4*>(X + (size_t)(32 * b + lane) * CPW);
+#pragma unroll
+      for (int q = 0; q < CPW / 2; ++q) xd[q] = make_float4(x[2 * q].x, x[2 * q].y, x[2 * q + 1].x, x[2 * q + 1].y);
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < CPW; ++c)
+        if (c < nc) M[(size_t)(cw + c) * lda + k0 + 32 * b + lane] = x[c];
+      l = 0;
+      ++b;
+    }
+  }
+}
+
+__global__ void iota_rows_kernel(int* __restrict__ perm, int n, int total) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < total) perm[i] = i % n;
 }
 
 // One CTA per (matrix, right-hand side): P, then L (unit lower), then U.
@@ -536,6 +754,7 @@ struct LuJob {
   int* ipiv;
   int* info;
   int* rowmap;
+  int* perm;         // row permutation of the whole factorisation, built panel by panel (null: not wanted)
   TcGemmPlan* plan;  // tcgen05 updates (mixed form); null: cuBLAS
   cublasHandle_t h;
   cudaStream_t stream;
@@ -544,11 +763,6 @@ struct LuJob {
 // U rows [k, k+kb) of columns [c0, c1): U = L^{-1} A with L the unit lower triangle of A[k:k+kb, k:k+kb].
 cudaError_t trsm_cols(const LuJob& j, int k, int kb, int c0, int c1) {
   if (c1 <= c0 || kb <= 0) return cudaSuccess;
-  if (j.prec == Precision::Mixed && kb == 32 && (j.lda & 1) == 0 && (k & 1) == 0) {
-    dim3 g((unsigned)((c1 - c0 + 127) / 128), j.batch);
-    lu_trsm32_kernel<<<g, 128, 0, j.stream>>>((float2*)j.A, j.lda, j.strideA, k, c0, c1);
-    return cudaGetLastError();
-  }
   const int tpb = 128;
   dim3 g((unsigned)((c1 - c0 + tpb - 1) / tpb), j.batch);
   if (j.prec == Precision::Mixed) {
@@ -592,33 +806,75 @@ cudaError_t block_update(const LuJob& j, int r0, int M, int c0, int N, int kc, i
     if (e_ != cudaSuccess) return e_;       \
   } while (0)
 
+// U rows of outer block k0 (kOuterBlock wide) for columns [c0, c1).
+cudaError_t outer_urows(const LuJob& j, int k0, int c0, int c1) {
+  auto run = [&](auto cpw_c) {
+    constexpr int CPW = decltype(cpw_c)::value;
+    constexpr size_t sm = urows_smem<CPW>();
+    ensure_smem_limit((const void*)lu_urows_kernel<CPW>, sm);
+    dim3 g((unsigned)((c1 - c0 + kUrowsWarps * CPW - 1) / (kUrowsWarps * CPW)), j.batch);
+    lu_urows_kernel<CPW><<<g, kUrowsWarps * 32, sm, j.stream>>>((float2*)j.A, j.lda, j.strideA, k0, c0, c1);
+    return cudaGetLastError();
+  };
+  // 8 columns per warp where that still gives every SM a CTA, else 4
+  const long long cols = (long long)(c1 - c0) * j.batch;
+  if (cols >= 8LL * kUrowsWarps * sm_count()) return run(std::integral_constant<int, 8>{});
+  return run(std::integral_constant<int, 4>{});
+}
+
 // Two-level right-looking LU.  The matrix is factored in outer block columns of
 // width NB (kOuterBlock, 256): each is factored as sub-panels of width nb (the cluster panel
 // width, 32 or 64) with their row interchanges applied to every other column
 // and the rest of the outer block updated after each sub-panel; then the outer
-// block's U rows are solved block by block and the trailing matrix takes one
+// block's U rows are solved and the trailing matrix takes one
 // update of depth NB.  The trailing matrix is read and written once per NB
 // columns instead of once per nb, which at block depth 64 bounds the LU by HBM.
+// Sub-panels of 32 columns (the mixed form's) take the three FP32 kernels above; 64-wide
+// ones (options.lu_block) the general triangular solve and updates.
 cudaError_t lu_two_level(const LuJob& j, int NB) {
   const int n = j.n, nb = j.nb;
+  const bool narrow = j.prec == Precision::Mixed && nb == 32;
+  float2* A32 = (float2*)j.A;
+  if (j.perm) {
+    const int total = n * j.batch;
+    iota_rows_kernel<<<(total + 255) / 256, 256, 0, j.stream>>>(j.perm, n, total);
+  }
   for (int k0 = 0; k0 < n; k0 += NB) {
     const int KB = std::min(NB, n - k0);
     for (int j0 = 0; j0 < KB; j0 += nb) {
       const int kb = std::min(nb, KB - j0), kk = k0 + j0;
       BEM_TRY(lu_panel_cluster(j.prec, j.A, j.lda, j.strideA, n, kk, kb, nb, j.cl, j.batch, j.ipiv, j.info, j.stream,
                                j.rowmap));
-      BEM_TRY(lu_swap_rows_batched(j.prec, j.A, j.lda, j.strideA, n, kk, kb, j.batch, j.rowmap, j.stream));
+      if (narrow && kb == 32) {
+        const int rest = k0 + KB - kk - 32;  // the rest of the outer block
+        const int solve_ctas = (rest + 7) / 8;
+        dim3 gs((unsigned)(solve_ctas + (kk + n - k0 - KB + (j.perm ? 1 : 0) + 7) / 8), j.batch);
+        if (gs.x > 0)
+          lu_swap_urows_kernel<<<gs, 256, 0, j.stream>>>(A32, j.lda, j.strideA, n, kk, k0 + KB, solve_ctas, j.rowmap,
+                                                         j.perm);
+        if (rest > 0) {
+          dim3 gu((unsigned)((n - kk - 32 + 127) / 128), (unsigned)((rest + 31) / 32), j.batch);
+          lu_update32_kernel<<<gu, 256, 0, j.stream>>>(A32, j.lda, j.strideA, kk + 32, n - kk - 32, kk + 32, rest, kk);
+        }
+        BEM_TRY(cudaGetLastError());
+        continue;
+      }
+      BEM_TRY(lu_swap_rows_batched(j.prec, j.A, j.lda, j.strideA, n, kk, kb, j.batch, j.rowmap, j.perm, j.stream));
       if (j0 + kb < KB) {  // the rest of the outer block
         BEM_TRY(trsm_cols(j, kk, kb, kk + kb, k0 + KB));
         BEM_TRY(block_update(j, kk + kb, n - kk - kb, kk + kb, k0 + KB - kk - kb, kk, kb));
       }
     }
     if (k0 + KB < n) {
-      // U rows of the outer block for the trailing columns: blocked forward substitution
-      for (int i0 = 0; i0 < KB; i0 += nb) {
-        const int kb = std::min(nb, KB - i0), kk = k0 + i0;
-        BEM_TRY(trsm_cols(j, kk, kb, k0 + KB, n));
-        if (i0 + kb < KB) BEM_TRY(block_update(j, kk + kb, k0 + KB - kk - kb, k0 + KB, n - k0 - KB, kk, kb));
+      if (narrow) {
+        BEM_TRY(outer_urows(j, k0, k0 + KB, n));
+      } else {
+        // U rows of the outer block for the trailing columns: blocked forward substitution
+        for (int i0 = 0; i0 < KB; i0 += nb) {
+          const int kb = std::min(nb, KB - i0), kk = k0 + i0;
+          BEM_TRY(trsm_cols(j, kk, kb, k0 + KB, n));
+          if (i0 + kb < KB) BEM_TRY(block_update(j, kk + kb, k0 + KB - kk - kb, k0 + KB, n - k0 - KB, kk, kb));
+        }
       }
       BEM_TRY(block_update(j, k0 + KB, n - k0 - KB, k0 + KB, n - k0 - KB, k0, KB));
     }
@@ -628,18 +884,22 @@ cudaError_t lu_two_level(const LuJob& j, int NB) {
 
 }  // namespace
 
-int lu_launch_count(int n, int nb, int NB, bool tensor) {
+int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm) {
   const int per_update = tensor ? 2 : 0;  // operand split + tcgen05 kernel (cuBLAS kernels are not counted)
-  int count = 0;
+  const bool narrow = tensor && nb == 32;
+  int count = perm ? 1 : 0;
   for (int k0 = 0; k0 < n; k0 += NB) {
     const int KB = std::min(NB, n - k0);
     for (int j0 = 0; j0 < KB; j0 += nb) {
       const int kb = std::min(nb, KB - j0);
-      count += 2;                                        // panel, row swaps
-      if (j0 + kb < KB) count += 1 + (n - k0 - j0 - kb > 0 ? per_update : 0);
+      count += 2;                                        // panel, row swaps (narrow: with the U rows)
+      if (j0 + kb < KB) count += narrow ? 1 : 1 + (n - k0 - j0 - kb > 0 ? per_update : 0);
     }
     if (k0 + KB < n) {
-      for (int i0 = 0; i0 < KB; i0 += nb) count += 1 + (i0 + std::min(nb, KB - i0) < KB ? per_update : 0);
+      if (narrow)
+        count += 1;
+      else
+        for (int i0 = 0; i0 < KB; i0 += nb) count += 1 + (i0 + std::min(nb, KB - i0) < KB ? per_update : 0);
       count += per_update;
     }
   }
@@ -648,7 +908,7 @@ int lu_launch_count(int n, int nb, int NB, bool tensor) {
 
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info, int nb,
                               void* cublas_handle, cudaStream_t stream, LuGemm gemm, void* tc_workspace,
-                              bool* used_tensor, int** tc_err, int* rowmap, int* n_launches) {
+                              bool* used_tensor, int** tc_err, int* rowmap, int* n_launches, int* perm) {
   cublasHandle_t h = (cublasHandle_t)cublas_handle;
   cublasSetStream(h, stream);
   const long long strideA = lda * (long long)n;
@@ -677,8 +937,8 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
   // form, or lu_gemm = 1) keeps one level: its kernels for the skinny panel
   // shapes of the two-level schedule are slow.
   if (cluster_panel && rowmap && plan) {
-    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, plan, h, stream};
-    if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, plan != nullptr);
+    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, h, stream};
+    if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, plan != nullptr, perm != nullptr);
     return lu_two_level(job, kOuterBlock);
   }
   if (n_launches) *n_launches = 0;
@@ -693,7 +953,7 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
     else
       lu_panel_kernel<double><<<batch, 1024, 0, stream>>>((double2*)A, lda, strideA, n, k, kb, ipiv, info);
     if (n - kb > 0 && cluster_panel && rowmap) {
-      cudaError_t e = lu_swap_rows_batched(prec, A, lda, strideA, n, k, kb, batch, rowmap, stream);
+      cudaError_t e = lu_swap_rows_batched(prec, A, lda, strideA, n, k, kb, batch, rowmap, nullptr, stream);
       if (e != cudaSuccess) return e;
     } else if (n - kb > 0) {
       dim3 g((n - kb + 127) / 128, batch);
@@ -735,6 +995,10 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
         if (st != CUBLAS_STATUS_SUCCESS) return cudaErrorUnknown;
       }
     }
+  }
+  if (perm) {
+    if (n_launches) *n_launches += 1;
+    return lu_perm_batched(ipiv, n, batch, perm, stream);
   }
   return cudaGetLastError();
 }

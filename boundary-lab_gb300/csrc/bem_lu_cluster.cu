@@ -124,12 +124,11 @@ template <int NB> __device__ void net_row_map(const int* pivs, int kb, int k, in
   }
 }
 
-// Apply a net row permutation to the columns outside the panel: one warp per
-// column loads every source row (at most 4 per lane, all in flight), then
-// stores every destination row.
+// Apply a net row permutation to the columns outside the panel, one warp per column.  One
+// warp more does the same to the row permutation so far (perm, null: none).
 template <typename C2>
 __global__ void __launch_bounds__(256) lu_swap_rows_kernel(C2* A, long long lda, long long strideA, int n, int k,
-                                                          int kb, const int* rowmap) {
+                                                          int kb, const int* rowmap, int* perm) {
   __shared__ int sdst[128], ssrc[128];
   __shared__ int s_cnt;
   const int* rm = rowmap + (size_t)blockIdx.y * kRowmapStride;
@@ -141,23 +140,12 @@ __global__ void __launch_bounds__(256) lu_swap_rows_kernel(C2* A, long long lda,
     ssrc[e] = rm[2 + 2 * e];
   }
   __syncthreads();
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * (blockDim.x >> 5) + wid;
-  if (cnt == 0 || t >= n - kb) return;
-  const int c = t < k ? t : t + kb;
-  C2* a = A + (size_t)blockIdx.y * strideA + (size_t)c * lda;
-  C2 v[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = lane + 32 * q;
-    if (e < cnt && (unsigned)ssrc[e] < (unsigned)n) v[q] = a[ssrc[e]];
-  }
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = lane + 32 * q;
-    if (e < cnt && (unsigned)ssrc[e] < (unsigned)n && (unsigned)sdst[e] < (unsigned)n) a[sdst[e]] = v[q];
-  }
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (cnt == 0 || t > n - kb) return;
+  if (t < n - kb)
+    permute_column(A + (size_t)blockIdx.y * strideA + (size_t)(t < k ? t : t + kb) * lda, n, cnt, sdst, ssrc);
+  else if (perm != nullptr)
+    permute_column(perm + (size_t)blockIdx.y * n, n, cnt, sdst, ssrc);
 }
 
 // One column step has a single cluster barrier.  Before it, every CTA
@@ -920,13 +908,14 @@ cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long s
 }
 
 cudaError_t lu_swap_rows_batched(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb,
-                                 int batch, const int* rowmap, cudaStream_t stream) {
-  if (n - kb <= 0) return cudaSuccess;
-  dim3 g((unsigned)((n - kb + 7) / 8), batch);
+                                 int batch, const int* rowmap, int* perm, cudaStream_t stream) {
+  const int warps = n - kb + (perm ? 1 : 0);
+  if (warps <= 0) return cudaSuccess;
+  dim3 g((unsigned)((warps + 7) / 8), batch);
   if (prec == Precision::Mixed)
-    lu_swap_rows_kernel<float2><<<g, 256, 0, stream>>>((float2*)A, lda, strideA, n, k, kb, rowmap);
+    lu_swap_rows_kernel<float2><<<g, 256, 0, stream>>>((float2*)A, lda, strideA, n, k, kb, rowmap, perm);
   else
-    lu_swap_rows_kernel<double2><<<g, 256, 0, stream>>>((double2*)A, lda, strideA, n, k, kb, rowmap);
+    lu_swap_rows_kernel<double2><<<g, 256, 0, stream>>>((double2*)A, lda, strideA, n, k, kb, rowmap, perm);
   return cudaGetLastError();
 }
 
