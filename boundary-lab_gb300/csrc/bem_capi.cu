@@ -86,11 +86,12 @@ struct bem_context {
   cublasHandle_t cublas = nullptr;
   std::string err;
   cudaMemPool_t pool = nullptr;
-  DevBuf rext, mats, mats2, ipiv, perm, info, sblocks, rb, b32, b64, x64, r64, d32, fsrc, fout, norms, pout, tcws, rowmap;
+  DevBuf rext, mats, mats2, ipiv, perm, info, sblocks, rb, b32, x64, r64, d32, fsrc, fout, norms, pout, tcws, rowmap;
+  DevBuf inv;                          // inverted diagonal blocks of a batch's factors
   DevBuf ftrace_p, ftrace_q, fpoints;  // bem_evaluate_field: boundary traces and points
   DevBuf xsplit;                       // the refinement's x as float hi / lo pairs
   std::vector<DevBuf*> scratch() {
-    return {&rext, &mats, &mats2, &ipiv, &perm, &info, &sblocks, &rb, &b32, &b64, &x64, &r64, &d32, &fsrc, &fout, &norms,
+    return {&rext, &mats, &mats2, &ipiv, &perm, &info, &sblocks, &rb, &b32, &inv, &x64, &r64, &d32, &fsrc, &fout, &norms,
             &pout, &tcws, &rowmap, &ftrace_p, &ftrace_q, &fpoints, &xsplit};
   }
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -880,9 +881,9 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
   const size_t vecn = (size_t)B * nc * ldb;
   ck(ctx->b32.ensure(vecn * esz), "alloc rhs");
   if (mixed) {
-    ck(ctx->b64.ensure(vecn * sizeof(double2)), "alloc rhs64");
     ck(ctx->x64.ensure(vecn * sizeof(double2)), "alloc x");
-    ck(ctx->r64.ensure(vecn * sizeof(double2)), "alloc r");
+    ck(ctx->r64.ensure(vecn * sizeof(double2) * bem::residual_splits(n, B * nc)), "alloc residual parts");
+    if (bem::lu_solve_blocks_fits(n)) ck(ctx->inv.ensure(bem::lu_inverse_bytes(n, B)), "alloc block inverses");
     ck(ctx->d32.ensure(vecn * sizeof(float2)), "alloc d");
     ck(ctx->xsplit.ensure(vecn * sizeof(float4)), "alloc x split");
     ck(ctx->norms.ensure((size_t)B * nc * 2 * sizeof(double)), "alloc norms");
@@ -955,7 +956,7 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
                             &lu_launches, (int*)ctx->perm.p),
      "LU factorisation");
   // kernels of this batch besides the assembly: the LU with its row permutation, the solves
-  // (mixed: 6 + 6 per refinement step), the field (2, +1 mixed, per slice)
+  // (mixed: 5 + 4 per refinement step), the field (2, +1 mixed, per slice)
   T.launches += lu_launches;
   T.gemm_used = mixed ? (used_tensor ? 2 : 1) : 0;
   prof_mark(ctx, BEM_K_LU);
@@ -969,21 +970,23 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
     T.launches += 1;
   } else {
     double2* x = (double2*)ctx->x64.p;
-    double2* r = (double2*)ctx->r64.p;
-    double2* b64 = (double2*)ctx->b64.p;
     float2* d = (float2*)ctx->d32.p;
-    ck(bem::convert_f32_to_f64((const float2*)ctx->b32.p, b64, nvec, ctx->stream), "convert rhs");
+    const bool blocks = bem::lu_solve_blocks_fits(n);
+    if (blocks) ck(bem::lu_block_inverses(ctx->mats.p, lda, n, B, ctx->inv.p, ctx->stream), "block inverses");
     ck(cudaMemcpyAsync(d, ctx->b32.p, nvec * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream), "copy rhs");
-    ck(bem::lu_solve_cluster_batched(prec, ctx->mats.p, lda, n, B, (const int*)ctx->perm.p, d, ldb, nc, ctx->stream),
-       "LU solve");
-    ck(cudaMemsetAsync(x, 0, nvec * sizeof(double2), ctx->stream), "memset x");
-    ck(bem::axpy_f32_into_f64(d, x, nvec, ctx->stream), "axpy");
     int steps = 0;
     double worst = 0;
     for (;;) {
-      ck(bem::residual_batched(prec, ctx->mats2.p, lda, n, B, x, b64, ldb, nc, r, ctx->xsplit.p, ctx->stream),
+      // x += (LU)^{-1} d, then d = b - A x
+      ck(blocks ? bem::lu_solve_blocks_batched(ctx->mats.p, lda, n, B, ctx->inv.p, (const int*)ctx->perm.p, d, ldb, nc,
+                                               ctx->stream)
+                : bem::lu_solve_cluster_batched(prec, ctx->mats.p, lda, n, B, (const int*)ctx->perm.p, d, ldb, nc,
+                                                ctx->stream),
+         "LU solve");
+      ck(bem::refine_update_x(steps == 0, d, x, ctx->xsplit.p, nvec, ctx->stream), "update x");
+      ck(bem::refine_residual(ctx->mats2.p, lda, n, B, ctx->xsplit.p, (const float2*)ctx->b32.p, ldb, nc,
+                              (double2*)ctx->r64.p, d, (double*)ctx->norms.p, ctx->stream),
          "residual");
-      ck(bem::norms_batched(r, b64, ldb, n, B * nc, (double*)ctx->norms.p, ctx->stream), "norms");
       ck(cudaMemcpyAsync(norms.data(), ctx->norms.p, (size_t)B * nc * 2 * sizeof(double), cudaMemcpyDeviceToHost,
                          ctx->stream),
          "copy norms");
@@ -995,16 +998,11 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
         else worst = std::max(worst, rel);
       }
       if (worst <= o.refine_tol || steps >= o.max_refine || !std::isfinite(worst)) break;
-      ck(bem::convert_f64_to_f32(r, d, nvec, ctx->stream), "convert residual");
-      ck(bem::lu_solve_cluster_batched(prec, ctx->mats.p, lda, n, B, (const int*)ctx->perm.p, d, ldb, nc,
-                                       ctx->stream),
-         "LU solve");
-      ck(bem::axpy_f32_into_f64(d, x, nvec, ctx->stream), "axpy");
       ++steps;
     }
     T.max_steps = std::max(T.max_steps, steps);
     T.max_res = std::max(T.max_res, worst);
-    T.launches += 6 + 6LL * steps;  // 3 + (x split, residual, norms) per check + (convert, solve, axpy) per step
+    T.launches += (blocks ? 1 : 0) + 4LL * (steps + 1);  // inverses; solve, x, residual parts and sum per round
   }
   prof_mark(ctx, BEM_K_SOLVE);
   cudaEventRecord(ctx->ev[2], ctx->stream);
@@ -1128,7 +1126,8 @@ long long bem_estimate_device_bytes(int nv, int nf, int npairs, int nrhs, int np
   bytes += (long long)batch * lda * nv * esz * (precision == BEM_PRECISION_MIXED ? 2 : 1);  // matrices (+copy)
   bytes += (long long)npairs * (12 * esz * group + 24 * 8 + 48 + (bem::kPairRec + bem::kPairGeoDf) * 4 + 96 +
                                 bem::kChebN * 24 * 4);  // singular blocks, moments, pairs, records, scatter plan, Chebyshev moments
-  bytes += (long long)batch * nrhs * lda * (esz + 3 * 16 + 16);             // rhs, x, r, b64, d
+  bytes += (long long)batch * nrhs * lda * (esz + (2 + bem::kResidualSplits) * 16 + 16);  // rhs, x, residual parts, d
+  if (precision == BEM_PRECISION_MIXED) bytes += (long long)bem::lu_inverse_bytes(nv, batch);  // block inverses
   bytes += (long long)batch * nrhs * ((long long)nf * 6 * esz + (long long)npts * 16);  // field sources + out
   bytes += (long long)nf * (2 * 160 + 288 + 64);                            // face records (+ lane-group copy), maps
   if (precision == BEM_PRECISION_MIXED)                                      // tensor-core update operands

@@ -174,12 +174,25 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
 // Solve (LU) X = B in place for nrhs columns per matrix (B stride ldb*nrhs per matrix), working precision.
 cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* ipiv,
                              void* B, long long ldb, int nrhs, int nb, cudaStream_t stream);
-// r = b - A x in FP64 arithmetic: A (complex64 or complex128), x, b, r complex128.
-cudaError_t residual_batched(Precision prec, const void* A, long long lda, int n, int batch, const double2* x,
-                             const double2* b, long long ldb, int nrhs, double2* r, void* xsplit, cudaStream_t stream);
-// Per (matrix, rhs): out[2*i] = ||r_i||^2 and out[2*i+1] = ||b_i||^2.
-cudaError_t norms_batched(const double2* r, const double2* b, long long ldb, int n, int count, double* out,
-                          cudaStream_t stream);
+// Solves and refinement of the mixed form (bem_lu_solve.cu).  lu_block_inverses inverts the
+// 256 x 256 diagonal blocks of the factors into inv (lu_inverse_bytes); the solves then take
+// B (column stride ldb, nrhs per matrix) to x in place.  lu_solve_blocks_fits: whether order
+// n is in their range (else lu_solve_cluster_batched).
+size_t lu_inverse_bytes(int n, int batch);
+bool lu_solve_blocks_fits(int n);
+cudaError_t lu_block_inverses(const void* LU, long long lda, int n, int batch, void* inv, cudaStream_t stream);
+cudaError_t lu_solve_blocks_batched(const void* LU, long long lda, int n, int batch, const void* inv, const int* perm,
+                                    void* B, long long ldb, int nrhs, cudaStream_t stream);
+// x = d (first) or x += d, and x split into float pairs (4 floats per value) for the residual.
+cudaError_t refine_update_x(bool first, const float2* d, double2* x, void* xsplit, long long count,
+                            cudaStream_t stream);
+// d = b - A x rounded to FP32 (A and b FP32, x as split above, FP64-accurate sums), and per
+// system norms[2 i] = ||b - A x||^2, norms[2 i + 1] = ||b||^2.  parts: kResidualSplits x
+// systems x ldb values at most.
+constexpr int kResidualSplits = 8;
+int residual_splits(int n, int systems);
+cudaError_t refine_residual(const void* A, long long lda, int n, int batch, const void* xsplit, const float2* b,
+                            long long ldb, int nrhs, double2* parts, float2* d, double* norms, cudaStream_t stream);
 // Cluster-resident panel (bem_lu_cluster.cu).  lu_cluster_plan picks the panel
 // width (64 or 32) and cluster size for an n x n matrix; false when no cluster
 // configuration fits (then the single-CTA panel is used).
@@ -197,10 +210,7 @@ cudaError_t lu_swap_rows_batched(Precision prec, void* A, long long lda, long lo
 cudaError_t lu_perm_batched(const int* ipiv, int n, int batch, int* perm, cudaStream_t stream);
 cudaError_t lu_solve_cluster_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* perm,
                                      void* B, long long ldb, int nrhs, cudaStream_t stream);
-// x += d (d complex64) ; copy / convert helpers
-cudaError_t axpy_f32_into_f64(const float2* d, double2* x, long long n, cudaStream_t stream);
 cudaError_t convert_f64_to_f32(const double2* src, float2* dst, long long n, cudaStream_t stream);
-cudaError_t convert_f32_to_f64(const float2* src, double2* dst, long long n, cudaStream_t stream);
 
 // far field (bem_field.cu)
 cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const double* k, const double2* qscale,

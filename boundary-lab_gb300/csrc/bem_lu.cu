@@ -1,5 +1,4 @@
-// Dense complex LU with partial pivoting, triangular solves and the FP64
-// residual for iterative refinement (sm_103a).
+// Dense complex LU with partial pivoting: driver, trailing updates and U rows (sm_103a).
 //
 // The reference solves each Burton-Miller system with CUDA.jl's `\`
 // (cuSOLVER getrf + getrs, src/blab/solvers/julia_local/src/
@@ -566,172 +565,9 @@ __global__ void __launch_bounds__(1024) lu_solve_kernel(const typename CT<R>::C2
   }
 }
 
-template <typename C2>
-__global__ void residual_kernel(const C2* __restrict__ A, long long lda, long long strideA, int n,
-                                const double2* __restrict__ x, const double2* __restrict__ b, long long ldb, int nrhs,
-                                double2* __restrict__ r) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  const int mat = blockIdx.y / nrhs, rhs = blockIdx.y % nrhs;
-  if (row >= n) return;
-  const C2* M = A + (size_t)mat * strideA;
-  const size_t off = ((size_t)mat * nrhs + rhs) * ldb;
-  const double2* xv = x + off;
-  double sr = 0.0, si = 0.0;
-  for (int j = 0; j < n; ++j) {
-    const C2 a = M[(size_t)j * lda + row];
-    const double2 xj = xv[j];
-    const double ar = (double)a.x, ai = (double)a.y;
-    sr = fma(ar, xj.x, sr);
-    sr = fma(-ai, xj.y, sr);
-    si = fma(ar, xj.y, si);
-    si = fma(ai, xj.x, si);
-  }
-  const double2 bb = b[off + row];
-  r[off + row] = make_double2(bb.x - sr, bb.y - si);
-}
-
-// r = b - A x for an FP32 matrix A and FP64 x (the mixed form's refinement
-// residual) with no FP64 arithmetic in the inner loop: this part's FP64 rate is
-// a small fraction of its FP32 rate.  Per tile of 256 columns, x is split into
-// float pairs x = xh + xl in shared memory; every product a * xh is formed
-// exactly as p + fma(a, xh, -p), the p are summed in double-float (two_sum),
-// and the small terms (product errors and a * xl) in FP32.  The tile sums are
-// added in FP64, so the result carries about 2^-40 relative error per tile:
-// far below the 1e-10 refinement target.
-__device__ __forceinline__ void acc_exact_prod(float& sh, float& sl, float& e, float a, float xh, float xl) {
-  const float p = a * xh;
-  const float pe = fmaf(a, xh, -p);
-  const float t = sh + p;
-  const float bb = t - sh;
-  sl += (sh - (t - bb)) + (p - bb);
-  sh = t;
-  e = fmaf(a, xl, e + pe);
-}
-
-// x (FP64) as float hi / lo pairs (re hi, im hi, re lo, im lo), once per residual,
-// so the residual kernel below runs no FP64 instruction in its inner loop.
-__global__ void split_x_kernel(const double2* __restrict__ x, float4* __restrict__ xs, long long count) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const double2 v = x[i];
-  const float hr = (float)v.x, hi = (float)v.y;
-  xs[i] = make_float4(hr, hi, (float)(v.x - (double)hr), (float)(v.y - (double)hi));
-}
-
-// r = b - A x with A in FP32 and x in FP64: every product a * (x_hi + x_lo) is
-// formed exactly (two FMAs) and summed in double-float, so r carries the
-// accuracy of an FP64 product with the FP32 matrix.  A CTA covers 64 rows; its
-// four groups of 64 threads take interleaved 64-column slices of each
-// 256-column block of x staged in shared memory, each thread keeping two
-// independent double-float sums (even / odd columns).  The four partial sums of
-// a row are added in a fixed order at the end (deterministic).
-__global__ void __launch_bounds__(256) residual_f32a_kernel(const float2* __restrict__ A, long long lda,
-                                                            long long strideA, int n, const float4* __restrict__ xs,
-                                                            const double2* __restrict__ b, long long ldb, int nrhs,
-                                                            double2* __restrict__ r) {
-  __shared__ float4 xsh[256];
-  __shared__ double part[2][4][64];
-  const int rl = threadIdx.x & 63, cg = threadIdx.x >> 6;
-  const int row = blockIdx.x * 64 + rl;
-  const int mat = blockIdx.y / nrhs, rhs = blockIdx.y % nrhs;
-  const float2* M = A + (size_t)mat * strideA;
-  const size_t off = ((size_t)mat * nrhs + rhs) * ldb;
-  const float4* xv = xs + off;
-  float srh = 0.f, srl = 0.f, er = 0.f, sih = 0.f, sil = 0.f, ei = 0.f;      // even columns
-  float trh = 0.f, trl = 0.f, fr = 0.f, tih = 0.f, til = 0.f, fi = 0.f;      // odd columns
-  for (int j0 = 0; j0 < n; j0 += 256) {
-    __syncthreads();
-    {
-      const int j = j0 + threadIdx.x;
-      xsh[threadIdx.x] = j < n ? xv[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
-    const int cb = j0 + cg * 64;
-    const int jn = min(64, n - cb);
-    if (row < n && jn > 0) {
-      const float2* col = M + (size_t)cb * lda + row;
-      const float4* xg = xsh + cg * 64;
-      int t = 0;
-#pragma unroll 4
-      for (; t + 1 < jn; t += 2) {
-        const float2 a0 = col[(size_t)t * lda], a1 = col[(size_t)(t + 1) * lda];
-        const float4 x0 = xg[t], x1 = xg[t + 1];
-        // re += a.x xr - a.y xi ; im += a.x xi + a.y xr
-        acc_exact_prod(srh, srl, er, a0.x, x0.x, x0.z);
-        acc_exact_prod(srh, srl, er, -a0.y, x0.y, x0.w);
-        acc_exact_prod(sih, sil, ei, a0.x, x0.y, x0.w);
-        acc_exact_prod(sih, sil, ei, a0.y, x0.x, x0.z);
-        acc_exact_prod(trh, trl, fr, a1.x, x1.x, x1.z);
-        acc_exact_prod(trh, trl, fr, -a1.y, x1.y, x1.w);
-        acc_exact_prod(tih, til, fi, a1.x, x1.y, x1.w);
-        acc_exact_prod(tih, til, fi, a1.y, x1.x, x1.z);
-      }
-      if (t < jn) {
-        const float2 a0 = col[(size_t)t * lda];
-        const float4 x0 = xg[t];
-        acc_exact_prod(srh, srl, er, a0.x, x0.x, x0.z);
-        acc_exact_prod(srh, srl, er, -a0.y, x0.y, x0.w);
-        acc_exact_prod(sih, sil, ei, a0.x, x0.y, x0.w);
-        acc_exact_prod(sih, sil, ei, a0.y, x0.x, x0.z);
-      }
-    }
-  }
-  part[0][cg][rl] = ((double)srh + ((double)srl + (double)er)) + ((double)trh + ((double)trl + (double)fr));
-  part[1][cg][rl] = ((double)sih + ((double)sil + (double)ei)) + ((double)tih + ((double)til + (double)fi));
-  __syncthreads();
-  if (cg == 0 && row < n) {
-    const double accr = ((part[0][0][rl] + part[0][1][rl]) + part[0][2][rl]) + part[0][3][rl];
-    const double acci = ((part[1][0][rl] + part[1][1][rl]) + part[1][2][rl]) + part[1][3][rl];
-    const double2 bb = b[off + row];
-    r[off + row] = make_double2(bb.x - accr, bb.y - acci);
-  }
-}
-
-__global__ void norms_kernel(const double2* __restrict__ r, const double2* __restrict__ b, long long ldb, int n,
-                             double* out) {
-  const double2* rv = r + (size_t)blockIdx.x * ldb;
-  const double2* bv = b + (size_t)blockIdx.x * ldb;
-  double sr = 0.0, sb = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    sr += rv[i].x * rv[i].x + rv[i].y * rv[i].y;
-    sb += bv[i].x * bv[i].x + bv[i].y * bv[i].y;
-  }
-  __shared__ double s1[32], s2[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-    sb += __shfl_xor_sync(0xffffffffu, sb, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    s1[threadIdx.x >> 5] = sr;
-    s2[threadIdx.x >> 5] = sb;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0, c = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      a += s1[w];
-      c += s2[w];
-    }
-    out[2 * blockIdx.x] = a;
-    out[2 * blockIdx.x + 1] = c;
-  }
-}
-
-__global__ void axpy_kernel(const float2* d, double2* x, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    x[i].x += (double)d[i].x;
-    x[i].y += (double)d[i].y;
-  }
-}
 __global__ void f64_to_f32_kernel(const double2* s, float2* d, long long n) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) d[i] = make_float2((float)s[i].x, (float)s[i].y);
-}
-__global__ void f32_to_f64_kernel(const float2* s, double2* d, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] = make_double2((double)s[i].x, (double)s[i].y);
 }
 
 }  // namespace
@@ -1015,38 +851,8 @@ cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int 
   return cudaGetLastError();
 }
 
-cudaError_t residual_batched(Precision prec, const void* A, long long lda, int n, int batch, const double2* x,
-                             const double2* b, long long ldb, int nrhs, double2* r, void* xsplit, cudaStream_t stream) {
-  const long long strideA = lda * (long long)n;
-  if (prec == Precision::Mixed) {
-    const long long count = (long long)batch * nrhs * ldb;
-    split_x_kernel<<<(unsigned)((count + 255) / 256), 256, 0, stream>>>(x, (float4*)xsplit, count);
-    dim3 g((n + 63) / 64, batch * nrhs);
-    residual_f32a_kernel<<<g, 256, 0, stream>>>((const float2*)A, lda, strideA, n, (const float4*)xsplit, b, ldb,
-                                                 nrhs, r);
-  } else {
-    dim3 g((n + 255) / 256, batch * nrhs);
-    residual_kernel<double2><<<g, 256, 0, stream>>>((const double2*)A, lda, strideA, n, x, b, ldb, nrhs, r);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t norms_batched(const double2* r, const double2* b, long long ldb, int n, int count, double* out,
-                          cudaStream_t stream) {
-  norms_kernel<<<count, 256, 0, stream>>>(r, b, ldb, n, out);
-  return cudaGetLastError();
-}
-
-cudaError_t axpy_f32_into_f64(const float2* d, double2* x, long long n, cudaStream_t stream) {
-  axpy_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(d, x, n);
-  return cudaGetLastError();
-}
 cudaError_t convert_f64_to_f32(const double2* src, float2* dst, long long n, cudaStream_t stream) {
   f64_to_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(src, dst, n);
-  return cudaGetLastError();
-}
-cudaError_t convert_f32_to_f64(const float2* src, double2* dst, long long n, cudaStream_t stream) {
-  f32_to_f64_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(src, dst, n);
   return cudaGetLastError();
 }
 
