@@ -40,7 +40,7 @@ bool ensure_smem_limit(const void* func, size_t bytes) {
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   std::lock_guard<std::mutex> lock(mu);
   size_t& cur = limit[{dev, func}];
-  if (bytes <= std::max<size_t>(cur, 48 * 1024)) return true;
+  if (bytes <= std::max<size_t>(cur, 32 * 1024)) return true;  // below the default 48 KB even beside static arrays
   if (cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
   cur = bytes;
   return true;
@@ -460,7 +460,194 @@ __global__ void __launch_bounds__(WARPS * 32, RegularOccupancy<NFQ>::kCtasPerSm)
 }
 
 // ------------------------------------------------------------------------
-// Regular pairs, FP64 (the plain FP64 form).
+// Regular pairs, FP64, Burton-Miller operator (cD arbitrary, cH / cD = -i/k): NFQ
+// frequencies at once, in the weights of regular_f32_kernel.  With that ratio the
+// hypersingular part joins the double layer's,
+//   H = e^{ikr} E'',  E'' = -t/r^2 + i k (t + n_f . n_g) / r,  t = (r . n_g) / r,
+// and per test point the trial-basis sums Hs[b] = sum_n cw[b][n] H and Gs = sum_n w_n
+// e^{ikr} / r are folded into W[a][b] and S0, each pair adding
+//   jac (cD W[a][b] + (curl_a . curl_b) cH S0).
+//
+// Bound: the FP64 pipe (two lanes per SM and clock).  Per quadrature pair 19 FP64
+// instructions of geometry shared by the NFQ frequencies and about 32 per frequency (phase,
+// table sine and cosine, E'' and its product, sums), against 113 of the one-frequency
+// kernel with library sincos, square root, divide and nine-entry sums of each operator:
+// 1,280 triangles, 16 frequencies: 10.6 -> 5.5 ms per frequency; 3,984 triangles: 91 -> 48.  Two frequencies per
+// launch: four would need 224 KB of accumulators per CTA and spill.
+// ------------------------------------------------------------------------
+template <int NFQ> struct RegParamsF64BM {
+  double k[NFQ];
+  double2 cD[NFQ], cH[NFQ];  // with the 1 / (4 pi) of the Green's function
+  double cw[3 * kMaxQ], w[kMaxQ];
+};
+
+template <int Q, int WARPS, int NFQ>
+__global__ void __launch_bounds__(WARPS * 32, 2)
+    regular_f64_bm_kernel(const FaceF64* __restrict__ faces, int nf, const int* __restrict__ tile_group_ptr,
+                          const LaneSlot* __restrict__ slots, const int* __restrict__ tile_row_base, int max_rows,
+                          double2* __restrict__ Rext, long long ldR, long long strideR, RegParamsF64BM<NFQ> p,
+                          int ntr, int4 trs, const unsigned char* __restrict__ fix_mask,
+                          const double2* __restrict__ trig) {
+  extern __shared__ double2 smem_acc64[];
+  __shared__ double2 tab[kSincosTable];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.y;
+  const int g = blockIdx.x * WARPS + warp;
+  const int base = tile_row_base[tile];
+  const int rows = tile_row_base[tile + 1] - base;
+  double2* acc = smem_acc64 + (size_t)warp * NFQ * 3 * max_rows;  // [NFQ][3][max_rows]
+  for (int i = lane; i < NFQ * 3 * max_rows; i += 32) acc[i] = make_double2(0.0, 0.0);
+  load_sincos_table(tab, trig);
+  __syncthreads();
+  if (g >= nf) return;
+  const FaceF64& T = faces[g];
+  double ag[3], ng[3], og[Q][3], ogn[Q], cg[9];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    ag[d] = T.anchor[d];
+    ng[d] = T.normal[d];
+  }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) cg[i] = T.curls[i];
+#pragma unroll
+  for (int n = 0; n < Q; ++n) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) og[n][d] = T.off[3 * n + d];
+    ogn[n] = og[n][0] * ng[0] + og[n][1] * ng[1] + og[n][2] * ng[2];
+  }
+  const double a2g = T.area2;
+  const int gv0 = T.verts[0], gv1 = T.verts[1], gv2 = T.verts[2];
+  const int g0 = tile_group_ptr[tile], g1 = tile_group_ptr[tile + 1];
+  int prev_tr = 0;
+  for (int ti = 0; ti < ntr; ++ti) {  // symmetry images, as in regular_f32_kernel
+    const int tr = ti == 0 ? trs.x : ti == 1 ? trs.y : ti == 2 ? trs.z : trs.w;
+    {
+      const int dlt = tr ^ prev_tr;
+      const double fx = (dlt & 1) ? -1.0 : 1.0, fy = (dlt & 2) ? -1.0 : 1.0, dr = fx * fy;
+      ag[0] *= fx;
+      ag[1] *= fy;
+      ng[0] *= fx;
+      ng[1] *= fy;
+#pragma unroll
+      for (int n = 0; n < Q; ++n) {  // og . n_g is unchanged by a reflection
+        og[n][0] *= fx;
+        og[n][1] *= fy;
+      }
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        cg[3 * b] *= fx * dr;
+        cg[3 * b + 1] *= fy * dr;
+        cg[3 * b + 2] *= dr;
+      }
+      prev_tr = tr;
+    }
+    const int sv0 = (tr == 0 || (fix_mask[gv0] & tr) == tr) ? gv0 : -2;
+    const int sv1 = (tr == 0 || (fix_mask[gv1] & tr) == tr) ? gv1 : -2;
+    const int sv2 = (tr == 0 || (fix_mask[gv2] & tr) == tr) ? gv2 : -2;
+    for (int grp = g0; grp < g1; ++grp) {
+      const LaneSlot s = slots[(size_t)grp * 32 + lane];
+      if (s.face >= 0) {
+        const FaceF64& F = faces[s.face];
+        const int fv[3] = {F.verts[0], F.verts[1], F.verts[2]};
+        if (!share_vertex(fv, sv0, sv1, sv2)) {
+          const double C[3] = {ag[0] - F.anchor[0], ag[1] - F.anchor[1], ag[2] - F.anchor[2]};
+          const double nn = F.normal[0] * ng[0] + F.normal[1] * ng[1] + F.normal[2] * ng[2];
+          double2 W[NFQ][3][3], S0[NFQ];
+#pragma unroll
+          for (int f = 0; f < NFQ; ++f) {
+            S0[f] = make_double2(0., 0.);
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+              for (int b = 0; b < 3; ++b) W[f][a][b] = make_double2(0., 0.);
+          }
+#pragma unroll 1
+          for (int m = 0; m < Q; ++m) {
+            const double cm[3] = {C[0] - F.off[3 * m], C[1] - F.off[3 * m + 1], C[2] - F.off[3 * m + 2]};
+            const double cmn = cm[0] * ng[0] + cm[1] * ng[1] + cm[2] * ng[2];
+            double2 Hs[NFQ][3], Gs[NFQ];
+#pragma unroll
+            for (int f = 0; f < NFQ; ++f) {
+              Gs[f] = make_double2(0., 0.);
+#pragma unroll
+              for (int b = 0; b < 3; ++b) Hs[f][b] = make_double2(0., 0.);
+            }
+#pragma unroll
+            for (int n = 0; n < Q; ++n) {
+              const double rv[3] = {cm[0] + og[n][0], cm[1] + og[n][1], cm[2] + og[n][2]};
+              const double r2 = fma(rv[0], rv[0], fma(rv[1], rv[1], rv[2] * rv[2]));
+              if (r2 == 0.0) continue;
+              const double rinv = rsqrt_step(r2), r = r2 * rinv;
+              const double tq = (cmn + ogn[n]) * rinv * rinv;  // t / r
+              const double ex = -tq * rinv, tn = fma(nn, rinv, tq), wr = p.w[n] * rinv;
+#pragma unroll
+              for (int f = 0; f < NFQ; ++f) {
+                double sn, cs;
+                sincos_table(p.k[f] * r, tab, &sn, &cs);
+                const double ey = p.k[f] * tn;
+                const double2 H = make_double2(fma(cs, ex, -sn * ey), fma(cs, ey, sn * ex));
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                  Hs[f][b].x = fma(p.cw[b * Q + n], H.x, Hs[f][b].x);
+                  Hs[f][b].y = fma(p.cw[b * Q + n], H.y, Hs[f][b].y);
+                }
+                Gs[f].x = fma(wr, cs, Gs[f].x);
+                Gs[f].y = fma(wr, sn, Gs[f].y);
+              }
+            }
+#pragma unroll
+            for (int f = 0; f < NFQ; ++f) {
+#pragma unroll
+              for (int a = 0; a < 3; ++a) {
+                const double c = p.cw[a * Q + m];
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                  W[f][a][b].x = fma(c, Hs[f][b].x, W[f][a][b].x);
+                  W[f][a][b].y = fma(c, Hs[f][b].y, W[f][a][b].y);
+                }
+              }
+              S0[f].x = fma(p.w[m], Gs[f].x, S0[f].x);
+              S0[f].y = fma(p.w[m], Gs[f].y, S0[f].y);
+            }
+          }
+          const double jac = F.area2 * a2g;
+          double2 cDj[NFQ], Bc[NFQ];
+#pragma unroll
+          for (int f = 0; f < NFQ; ++f) {
+            cDj[f] = cscale(p.cD[f], jac);
+            Bc[f] = cmul(cscale(p.cH[f], jac), S0[f]);
+          }
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            const double c0 = F.curls[3 * a], c1 = F.curls[3 * a + 1], c2 = F.curls[3 * a + 2];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+              const double cc = c0 * cg[3 * b] + c1 * cg[3 * b + 1] + c2 * cg[3 * b + 2];
+#pragma unroll
+              for (int f = 0; f < NFQ; ++f) {
+                double2* dst = &acc[(f * 3 + b) * max_rows + s.loc[a]];
+                double2 o = *dst;
+                const double2 w = W[f][a][b];
+                o.x = fma(cc, Bc[f].x, fma(cDj[f].x, w.x, fma(-cDj[f].y, w.y, o.x)));
+                o.y = fma(cc, Bc[f].y, fma(cDj[f].x, w.y, fma(cDj[f].y, w.x, o.y)));
+                *dst = o;
+              }
+            }
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }  // symmetry transforms
+  for (int i = lane; i < NFQ * 3 * rows; i += 32) {
+    const int fb = i / rows, loc = i - fb * rows;
+    const int f = fb / 3, b = fb - 3 * f;
+    Rext[(size_t)f * strideR + (size_t)(3 * g + b) * ldR + base + loc] = acc[fb * max_rows + loc];
+  }
+}
+
+// ------------------------------------------------------------------------
+// Regular pairs, FP64, any combination of operators (the inspection entry points).
 // ------------------------------------------------------------------------
 struct RegParamsF64 {
   double k, k2;
@@ -898,97 +1085,99 @@ template <> struct SingParams<double> {
 constexpr int kSingOut = 12;
 
 // The plain FP64 form's singular kernel (the mixed form uses singular_dyn_f32_kernel below).
-template <typename R>
+// A warp per pair, lanes over the Duffy points.  Bound by the FP64 pipe: about 110 FP64
+// instructions per point (table sine and cosine, the factors hr fy, hi fy, hr fx, hi fx
+// formed once, 21 complex sums: the single-layer sums SR[a] are the sums of IR[a][b] over b,
+// as the P1 trial basis sums to one), against 190 with library sincos and a product chain
+// per sum: 1,280 triangles: 5.2 -> 4.1 ms per frequency.
 __global__ void __launch_bounds__(256, 1)
     singular_dyn_kernel(SingularGeom geo, const SingularPair* __restrict__ pairs, int npairs,
-                                    const int* __restrict__ rule_ptr, const R* __restrict__ duffy,
-                                    const double* __restrict__ moments, const double* __restrict__ curls,
-                                    const double* __restrict__ area, const double* __restrict__ m11m10,
-                                    SingParams<R> p, typename cplx<R>::type* __restrict__ out) {
-  typedef typename cplx<R>::type C2;
+                        const int* __restrict__ rule_ptr, const double* __restrict__ duffy,
+                        const double* __restrict__ moments, const double* __restrict__ curls,
+                        const double* __restrict__ area, const double* __restrict__ m11m10, SingParams<double> p,
+                        const double2* __restrict__ trig, double2* __restrict__ out) {
+  __shared__ double2 tab[kSincosTable];
+  load_sincos_table(tab, trig);
+  __syncthreads();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= npairs) return;
   const SingularPair P = pairs[warp];
   const int* ft = geo.faces + 3 * P.test;
   const int* fr = geo.faces + 3 * P.trial;
-  R e1t[3], e2t[3], d0[3], e1r[3], e2r[3], nt[3], nr[3];
+  double e1t[3], e2t[3], d0[3], e1r[3], e2r[3], nt[3], nr[3];
   for (int d = 0; d < 3; ++d) {
     const double sd = d == 0 ? tr_sign_x(P.tr) : d == 1 ? tr_sign_y(P.tr) : 1.0;  // image pairs: S p
     const double t0 = geo.verts[3 * ft[0] + d];
     const double r0 = sd * geo.verts[3 * fr[0] + d];
-    e1t[d] = (R)(geo.verts[3 * ft[1] + d] - t0);
-    e2t[d] = (R)(geo.verts[3 * ft[2] + d] - t0);
-    d0[d] = (R)(r0 - t0);
-    e1r[d] = (R)(sd * geo.verts[3 * fr[1] + d] - r0);
-    e2r[d] = (R)(sd * geo.verts[3 * fr[2] + d] - r0);
-    nt[d] = (R)geo.normal[3 * P.test + d];
-    nr[d] = (R)(sd * geo.normal[3 * P.trial + d]);
+    e1t[d] = geo.verts[3 * ft[1] + d] - t0;
+    e2t[d] = geo.verts[3 * ft[2] + d] - t0;
+    d0[d] = r0 - t0;
+    e1r[d] = sd * geo.verts[3 * fr[1] + d] - r0;
+    e2r[d] = sd * geo.verts[3 * fr[2] + d] - r0;
+    nt[d] = geo.normal[3 * P.test + d];
+    nr[d] = sd * geo.normal[3 * P.trial + d];
   }
-  // accumulators: SR[3], IR[9], IDh[9], IKh[3] (complex) = 48 reals
-  R acc[48];
+  // accumulators: IR[9], IDh[9], IKh[3] (complex) = 42 reals
+  double acc[42];
 #pragma unroll
-  for (int i = 0; i < 48; ++i) acc[i] = R(0);
-  const R inv4pi = R(0.25 / CUDART_PI);
+  for (int i = 0; i < 42; ++i) acc[i] = 0.0;
+  const double inv4pi = 0.25 / CUDART_PI, half_k = 0.5 * p.k;
   const int q0 = rule_ptr[P.rule], q1 = rule_ptr[P.rule + 1];
   for (int q = q0 + lane; q < q1; q += 32) {
-    const R* pt = duffy + 5 * (size_t)q;
-    const R tu = pt[0], tv = pt[1], ru = pt[2], rvv = pt[3], w = pt[4];
-    const R px[3] = {R(1) - tu - tv, tu, tv};
-    const R py[3] = {R(1) - ru - rvv, ru, rvv};
-    R rv[3];
+    const double* pt = duffy + 5 * (size_t)q;
+    const double tu = pt[0], tv = pt[1], ru = pt[2], rvv = pt[3], w = pt[4];
+    const double wp[3] = {w * (1.0 - tu - tv), w * tu, w * tv};
+    const double py[3] = {1.0 - ru - rvv, ru, rvv};
+    double rv[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) rv[d] = (d0[d] + ru * e1r[d] + rvv * e2r[d]) - (tu * e1t[d] + tv * e2t[d]);
-    const R r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-    if (r2 == R(0)) continue;
-    R sh, ch;
-    const R rinv = rsqrt(r2);
-    const R r = r2 * rinv;
-    sincos(R(0.5) * p.k * r, &sh, &ch);
-    const R z = p.k * r;
-    const R s = rinv * inv4pi;
-    const R sinz = R(2) * sh * ch;
-    const R omc = R(2) * sh * sh;  // 1 - cos z
-    const R cosz = R(1) - omc;
+    const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
+    if (r2 == 0.0) continue;
+    const double rinv = rsqrt_step(r2), r = r2 * rinv;
+    double sh, ch;
+    sincos_table(half_k * r, tab, &sh, &ch);
+    const double z = p.k * r, s = rinv * inv4pi;
+    const double sh2 = sh + sh, sinz = sh2 * ch, omc = sh2 * sh;  // omc = 1 - cos z
     // R = s (cos z - 1 + i sin z)
-    const R Rr = -s * omc, Ri = s * sinz;
+    const double Rr = -s * omc, Ri = s * sinz;
     // h(z) = (1 - cos z - z sin z) + i (z cos z - sin z)
-    const R hr = omc - z * sinz, hi = z * cosz - sinz;
-    const R fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * s * rinv * rinv;
-    const R fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * s * rinv * rinv;
+    const double hr = fma(-z, sinz, omc), hi = fma(z, 1.0 - omc, -sinz);
+    const double sr2 = s * rinv * rinv;
+    const double fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * sr2;
+    const double fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * sr2;
+    const double hyr = hr * fy, hyi = hi * fy, hxr = hr * fx, hxi = hi * fx;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const R wa = w * px[a];
-      acc[2 * a] += wa * Rr;
-      acc[2 * a + 1] += wa * Ri;
-      acc[42 + 2 * a] += wa * hr * fx;
-      acc[42 + 2 * a + 1] += wa * hi * fx;
+      acc[36 + 2 * a] = fma(wp[a], hxr, acc[36 + 2 * a]);
+      acc[36 + 2 * a + 1] = fma(wp[a], hxi, acc[36 + 2 * a + 1]);
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
-        const R wab = wa * py[b];
-        acc[6 + 2 * (3 * a + b)] += wab * Rr;
-        acc[6 + 2 * (3 * a + b) + 1] += wab * Ri;
-        acc[24 + 2 * (3 * a + b)] += wab * hr * fy;
-        acc[24 + 2 * (3 * a + b) + 1] += wab * hi * fy;
+        const double wab = wp[a] * py[b];
+        const int i = 2 * (3 * a + b);
+        acc[i] = fma(wab, Rr, acc[i]);
+        acc[i + 1] = fma(wab, Ri, acc[i + 1]);
+        acc[18 + i] = fma(wab, hyr, acc[18 + i]);
+        acc[18 + i + 1] = fma(wab, hyi, acc[18 + i + 1]);
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 48; ++i) acc[i] = warp_sum(acc[i]);
+  for (int i = 0; i < 42; ++i) acc[i] = warp_sum(acc[i]);
   if (lane != 0) return;
   const double* M = moments + (size_t)kStatic * warp;
-  const R jac = (R)P.jac;
-  C2 SR[3], IR[9], IDh[9], IKh[3];
-  for (int a = 0; a < 3; ++a) {
-    SR[a] = cplx<R>::make(acc[2 * a] * jac, acc[2 * a + 1] * jac);
-    IKh[a] = cplx<R>::make(acc[42 + 2 * a] * jac, acc[42 + 2 * a + 1] * jac);
-  }
+  const double jac = P.jac;
+  double2 SR[3], IR[9], IDh[9], IKh[3];
   for (int i = 0; i < 9; ++i) {
-    IR[i] = cplx<R>::make(acc[6 + 2 * i] * jac, acc[6 + 2 * i + 1] * jac);
-    IDh[i] = cplx<R>::make(acc[24 + 2 * i] * jac, acc[24 + 2 * i + 1] * jac);
+    IR[i] = make_double2(acc[2 * i] * jac, acc[2 * i + 1] * jac);
+    IDh[i] = make_double2(acc[18 + 2 * i] * jac, acc[18 + 2 * i + 1] * jac);
+  }
+  for (int a = 0; a < 3; ++a) {
+    SR[a] = cadd(cadd(IR[3 * a], IR[3 * a + 1]), IR[3 * a + 2]);
+    IKh[a] = make_double2(acc[36 + 2 * a] * jac, acc[36 + 2 * a + 1] * jac);
   }
   // S0 = sum w G (static + dynamic)
-  C2 S0 = cplx<R>::make((R)(M[0] + M[1] + M[2]), R(0));
+  double2 S0 = make_double2(M[0] + M[1] + M[2], 0.0);
   for (int a = 0; a < 3; ++a) S0 = cadd(S0, SR[a]);
   const double* ct = curls + 9 * (size_t)P.test;
   const double* cr0 = curls + 9 * (size_t)P.trial;
@@ -1001,25 +1190,25 @@ __global__ void __launch_bounds__(256, 1)
       cr[3 * b + 2] = det * cr0[3 * b + 2];
     }
   }
-  const R kk_nn = p.k2 * (R)P.nprod;
+  const double kk_nn = p.k2 * P.nprod;
   const bool coincident = P.kind == 1 && P.tr == 0;  // mass terms: the face with itself, never with an image
-  const R a2 = (R)(2.0 * area[P.test]);
-  C2* o = out + (size_t)kSingOut * warp;
+  const double a2 = 2.0 * area[P.test];
+  double2* o = out + (size_t)kSingOut * warp;
   for (int a = 0; a < 3; ++a) {
     for (int b = 0; b < 3; ++b) {
-      const R cc = (R)(ct[3 * a] * cr[3 * b] + ct[3 * a + 1] * cr[3 * b + 1] + ct[3 * a + 2] * cr[3 * b + 2]);
+      const double cc = ct[3 * a] * cr[3 * b] + ct[3 * a + 1] * cr[3 * b + 1] + ct[3 * a + 2] * cr[3 * b + 2];
       const int i = 3 * a + b;
-      C2 D = cplx<R>::make((R)M[12 + i] + IDh[i].x, IDh[i].y);
-      C2 IGt = cplx<R>::make((R)M[3 + i] + IR[i].x, IR[i].y);
-      C2 H = cplx<R>::make(cc * S0.x - kk_nn * IGt.x, cc * S0.y - kk_nn * IGt.y);
-      C2 L = cadd(cmul(p.cD, D), cmul(p.cH, H));
-      if (coincident) L = cadd(L, cscale(p.cM, a2 * (R)m11m10[i]));
+      const double2 D = make_double2(M[12 + i] + IDh[i].x, IDh[i].y);
+      const double2 IGt = make_double2(M[3 + i] + IR[i].x, IR[i].y);
+      const double2 H = make_double2(cc * S0.x - kk_nn * IGt.x, cc * S0.y - kk_nn * IGt.y);
+      double2 L = cadd(cmul(p.cD, D), cmul(p.cH, H));
+      if (coincident) L = cadd(L, cscale(p.cM, a2 * m11m10[i]));
       o[i] = L;
     }
-    C2 S = cplx<R>::make((R)M[a] + SR[a].x, SR[a].y);
-    C2 K = cplx<R>::make((R)M[21 + a] + IKh[a].x, IKh[a].y);
-    C2 rhs = cadd(cmul(p.cS, S), cmul(p.cK, K));
-    if (coincident) rhs = cadd(rhs, cscale(p.cM10, a2 * (R)m11m10[9 + a]));
+    const double2 S = make_double2(M[a] + SR[a].x, SR[a].y);
+    const double2 K = make_double2(M[21 + a] + IKh[a].x, IKh[a].y);
+    double2 rhs = cadd(cmul(p.cS, S), cmul(p.cK, K));
+    if (coincident) rhs = cadd(rhs, cscale(p.cM10, a2 * m11m10[9 + a]));
     o[9 + a] = rhs;
   }
 }
@@ -1052,8 +1241,8 @@ __device__ __forceinline__ void warp_reduce_halving(float* v, int lane) {
   }
 }
 
-// The mixed form's singular kernel: the same Duffy remainder as
-// singular_dyn_kernel<float>, with every per-pair FP64 quantity (geometry,
+// The mixed form's singular kernel: the Duffy remainder of
+// singular_dyn_kernel in FP32, with every per-pair FP64 quantity (geometry,
 // curl products, static moments) read from the pair record instead of being
 // formed from FP64 data per frequency.  One warp per pair, lanes over the
 // Duffy points; after the warp reduction (every lane holds every sum) lanes
@@ -1565,7 +1754,7 @@ __device__ __forceinline__ void rhs_pair_f32(const FaceF32& F, const FaceF32& Gf
 
 template <int Q>
 __device__ __forceinline__ void rhs_pair_f64(const FaceF64& F, const FaceF64& Gf, const RhsParams<double>& p,
-                                             double2 S[3], double2 K[3], double sx = 1.0, double sy = 1.0) {
+                                             double2 S[3], double2 K[3], double sx, double sy, const double2* tab) {
   const double sg[3] = {sx, sy, 1.0};
   const double C[3] = {sx * Gf.anchor[0] - F.anchor[0], sy * Gf.anchor[1] - F.anchor[1], Gf.anchor[2] - F.anchor[2]};
 #pragma unroll
@@ -1582,18 +1771,17 @@ __device__ __forceinline__ void rhs_pair_f64(const FaceF64& F, const FaceF64& Gf
       for (int d = 0; d < 3; ++d) rv[d] = C[d] + (sg[d] * Gf.off[3 * n + d] - F.off[3 * m + d]);
       const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
       if (r2 == 0.0) continue;
-      const double r = sqrt(r2), rinv = 1.0 / r;
+      const double rinv = rsqrt_step(r2), r = r2 * rinv;
       double s, c;
-      sincos(p.k * r, &s, &c);
-      const double sc = rinv * (0.25 / CUDART_PI);
-      const double2 G = make_double2(c * sc, s * sc);
+      sincos_table(p.k * r, tab, &s, &c);
+      // w G (1, t (ik - 1/r)), G = e^{ikr} / (4 pi r), t = -(r . n_x) / r
+      const double wn = (p.cw[n] + p.cw[Q + n] + p.cw[2 * Q + n]) * (0.25 / CUDART_PI);
       const double t = -(rv[0] * F.normal[0] + rv[1] * F.normal[1] + rv[2] * F.normal[2]) * rinv;
-      const double2 Kk = make_double2(t * (-G.x * rinv - G.y * p.k), t * (G.x * p.k - G.y * rinv));
-      const double wn = p.cw[n] + p.cw[Q + n] + p.cw[2 * Q + n];
-      us.x += wn * G.x;
-      us.y += wn * G.y;
-      uk.x += wn * Kk.x;
-      uk.y += wn * Kk.y;
+      const double g = wn * rinv, gt = g * t, gr = -gt * rinv, gk = gt * p.k;
+      us.x = fma(g, c, us.x);
+      us.y = fma(g, s, us.y);
+      uk.x = fma(gr, c, fma(-gk, s, uk.x));
+      uk.y = fma(gr, s, fma(gk, c, uk.y));
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -1619,8 +1807,13 @@ __global__ void rhs_faces_kernel(const typename FaceRec<R>::type* __restrict__ f
                                  const SingularPair* __restrict__ pairs, const int* __restrict__ by_test_ptr,
                                  const int* __restrict__ by_test, const typename cplx<R>::type* __restrict__ sblocks,
                                  RhsParams<R> p, typename cplx<R>::type* __restrict__ rb, int ntr, int4 trs,
-                                 const unsigned char* __restrict__ fix_mask) {
+                                 const unsigned char* __restrict__ fix_mask, const double2* __restrict__ trig) {
   typedef typename cplx<R>::type C2;
+  __shared__ double2 tab[sizeof(R) == 8 ? kSincosTable : 1];
+  if constexpr (sizeof(R) == 8) {
+    load_sincos_table(tab, trig);
+    __syncthreads();
+  }
   const int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (f >= nf) return;
@@ -1644,7 +1837,7 @@ __global__ void rhs_faces_kernel(const typename FaceRec<R>::type* __restrict__ f
     if constexpr (sizeof(R) == 4)
       rhs_pair_f32<Q>(F, Gf, p, S, K, (float)tr_sign_x(tr), (float)tr_sign_y(tr));
     else
-      rhs_pair_f64<Q>(F, Gf, p, S, K, tr_sign_x(tr), tr_sign_y(tr));
+      rhs_pair_f64<Q>(F, Gf, p, S, K, tr_sign_x(tr), tr_sign_y(tr), tab);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const C2 q = cmul(p.qscale, drive[(size_t)c * nf + g]);
@@ -1935,7 +2128,46 @@ cudaError_t launch_regular_f32(const DeviceMesh& m, const double* k, const doubl
     launch(regular_f32_kernel<1, W, NFQ, DT>);
   return cudaGetLastError();
 }
+
+template <int NFQ>
+cudaError_t launch_regular_f64_bm(const DeviceMesh& m, const double* k, const double2* cD, const double2* cH,
+                                  double2* Rext, long long ldR, long long strideR, cudaStream_t stream) {
+  constexpr int W = 4;
+  RegParamsF64BM<NFQ> p;
+  const double inv4pi = 0.25 / 3.14159265358979323846;
+  for (int f = 0; f < NFQ; ++f) {
+    p.k[f] = k[f];
+    p.cD[f] = make_double2(cD[f].x * inv4pi, cD[f].y * inv4pi);
+    p.cH[f] = make_double2(cH[f].x * inv4pi, cH[f].y * inv4pi);
+  }
+  for (int i = 0; i < 3 * kMaxQ; ++i) p.cw[i] = m.rule_cw[i];
+  for (int q = 0; q < kMaxQ; ++q) p.w[q] = m.rule_w[q];
+  const dim3 grid((m.nf + W - 1) / W, m.n_tiles);
+  const size_t sm = (size_t)W * NFQ * 3 * m.max_tile_rows * sizeof(double2);
+  auto launch = [&](auto kern) {
+    ensure_smem_limit((const void*)kern, sm);
+    kern<<<grid, W * 32, sm, stream>>>(m.faces64, m.nf, m.tile_group_ptr, m.lane_slots, m.tile_row_base,
+                                       m.max_tile_rows, Rext, ldR, strideR, p, m.ntr,
+                                       make_int4(m.tr[0], m.tr[1], m.tr[2], m.tr[3]), m.fix_mask, m.trig);
+  };
+  if (m.Q == 6)
+    launch(regular_f64_bm_kernel<6, W, NFQ>);
+  else if (m.Q == 3)
+    launch(regular_f64_bm_kernel<3, W, NFQ>);
+  else
+    launch(regular_f64_bm_kernel<1, W, NFQ>);
+  return cudaGetLastError();
+}
 }  // namespace
+
+// Frequencies per launch of the FP64 Burton-Miller kernel: two where their accumulators
+// (and the 8 KB table) fit in a CTA's shared memory (570 tile rows), else one; 0 beyond
+// 1,160 rows, where the general kernel without the table runs.
+int regular_width_f64(const DeviceMesh& m) {
+  for (int w = 2; w >= 1; --w)
+    if ((size_t)4 * w * 3 * m.max_tile_rows * sizeof(double2) <= (size_t)218 * 1024) return w;
+  return 0;
+}
 
 // Frequencies per regular-kernel launch for a group of n that all carry the
 // double-layer term: the widest NFQ (4, else 3, else 2) whose per-warp
@@ -1951,8 +2183,8 @@ int regular_width(const DeviceMesh& m) {
 int regular_split(int n, int width, int* sizes) {
   int cnt = 0;
   if (width <= 2) {
-    for (; n >= 2; n -= 2) sizes[cnt++] = 2;
-    if (n) sizes[cnt++] = 1;
+    for (; n >= width; n -= width) sizes[cnt++] = width;
+    if (n) sizes[cnt++] = n;
     return cnt;
   }
   int q = n / width, r = n % width;
@@ -2000,19 +2232,28 @@ cudaError_t launch_regular(const DeviceMesh& m, Precision prec, int nfreq, const
     }
     return cudaSuccess;
   }
-  for (int f = 0; f < nfreq; ++f) {
-    cudaError_t e = launch_regular_f64(m, k[f], cD[f], cH[f], (double2*)Rext + (size_t)f * strideR, ldR, stream);
+  // the Burton-Miller ratio cH / cD = -i/k (to rounding): two frequencies per launch; any
+  // other combination one at a time through the general kernel
+  auto bm = [&](int i) {
+    const double d = cD[i].x * cD[i].x + cD[i].y * cD[i].y;
+    if (!(d > 0.0)) return false;
+    const double qx = (cH[i].x * cD[i].x + cH[i].y * cD[i].y) / d, qy = (cH[i].y * cD[i].x - cH[i].x * cD[i].y) / d;
+    return fabs(k[i] * qx) <= 4e-16 && fabs(k[i] * qy + 1.0) <= 4e-16;
+  };
+  for (int f = 0; f < nfreq;) {
+    double2* R = (double2*)Rext + (size_t)f * strideR;
+    const int w = !bm(f) ? 0 : std::min(regular_width_f64(m), f + 1 < nfreq && bm(f + 1) ? 2 : 1);
+    const cudaError_t e = w == 2   ? launch_regular_f64_bm<2>(m, k + f, cD + f, cH + f, R, ldR, strideR, stream)
+                          : w == 1 ? launch_regular_f64_bm<1>(m, k + f, cD + f, cH + f, R, ldR, strideR, stream)
+                                   : launch_regular_f64(m, k[f], cD[f], cH[f], R, ldR, stream);
     if (e != cudaSuccess) return e;
+    f += std::max(w, 1);
   }
   return cudaSuccess;
 }
 
 int regular_groups(const DeviceMesh& m, Precision prec, int nfreq, int* sizes) {
-  if (prec != Precision::Mixed) {
-    for (int i = 0; i < nfreq; ++i) sizes[i] = 1;
-    return nfreq;
-  }
-  return regular_split(nfreq, regular_width(m), sizes);
+  return regular_split(nfreq, prec == Precision::Mixed ? regular_width(m) : std::max(1, regular_width_f64(m)), sizes);
 }
 
 double regular_flop_per_qpair(int w) {
@@ -2260,8 +2501,8 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
     p.cS = c[f].cS;
     p.cK = c[f].cK;
     p.cM10 = c[f].cM10;
-    singular_dyn_kernel<double><<<nblk, threads, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
-                                                              m.moments, m.curls, m.area, m.m11m10, p,
+    singular_dyn_kernel<<<nblk, threads, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
+                                                              m.moments, m.curls, m.area, m.m11m10, p, m.trig,
                                                               (double2*)blocks + (size_t)f * blocks_stride);
   }
   if (launched) *launched += nfreq;
@@ -2328,7 +2569,7 @@ cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const Oper
                                                                  m.pairs_by_test_ptr, m.pairs_by_test,       \
                                                                  (const float2*)sblocks, p, (float2*)rb,     \
                                                                  m.ntr, make_int4(m.tr[0], m.tr[1], m.tr[2], \
-                                                                 m.tr[3]), m.fix_mask)
+                                                                 m.tr[3]), m.fix_mask, nullptr)
 #define BEM_RHS32_Q(NCC)        \
   if (m.Q == 6)                 \
     BEM_RHS32(6, NCC);          \
@@ -2359,7 +2600,7 @@ cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const Oper
                                                                   m.pairs_by_test_ptr, m.pairs_by_test,      \
                                                                   (const double2*)sblocks, p, (double2*)rb,  \
                                                                   m.ntr, make_int4(m.tr[0], m.tr[1], m.tr[2], \
-                                                                  m.tr[3]), m.fix_mask)
+                                                                  m.tr[3]), m.fix_mask, m.trig)
 #define BEM_RHS64_Q(NCC)        \
   if (m.Q == 6)                 \
     BEM_RHS64(6, NCC);          \

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/gb300_bem.h"
+#include "bem_common.cuh"
 #include "bem_internal.h"
 #include "bem_kernels.h"
 
@@ -572,6 +573,16 @@ int bem_upload_mesh_symmetric(bem_context* ctx, const double* vertices, int n_ve
       std::vector<double> mm(12);
       for (int i = 0; i < 9; ++i) mm[i] = P.m11[i];
       for (int i = 0; i < 3; ++i) mm[9 + i] = P.m10[i];
+      // (cos, sin) of the FP64 kernels' table angles, from the first octant (where the
+      // rounded angle costs nothing) by symmetry
+      std::vector<double2> trig(kSincosTable);
+      for (int i = 0; i < kSincosTable; ++i) {
+        constexpr int kQuarter = kSincosTable / 4;
+        const int q = i / kQuarter, j = i % kQuarter, o = std::min(j, kQuarter - j);
+        const double a = 2.0 * M_PI * o / kSincosTable;
+        const double c = j == o ? std::cos(a) : std::sin(a), s = j == o ? std::sin(a) : std::cos(a);
+        trig[i] = q == 0 ? make_double2(c, s) : q == 1 ? make_double2(-s, c) : q == 2 ? make_double2(-c, -s) : make_double2(s, -c);
+      }
       UploadPack pack;
       if (P.symmetry != 0) {
         pack.add(d.fix_mask, P.fix_mask);
@@ -610,6 +621,7 @@ int bem_upload_mesh_symmetric(bem_context* ctx, const double* vertices, int n_ve
       pack.add(d.curls, P.curls);
       pack.add(d.area, P.area);
       pack.add(d.m11m10, mm);
+      pack.add(d.trig, trig);
       pack.commit(m);
       for (int q = 0; q < P.Q; ++q) {
         const double u = P.rule_pts[2 * q], v = P.rule_pts[2 * q + 1];
@@ -1121,7 +1133,7 @@ long long bem_estimate_device_bytes(int nv, int nf, int npairs, int nrhs, int np
   const long long lda = round_up(nv, 32);
   const long long n_ext = (long long)(nv * 1.3) + 64;
   long long bytes = 0;
-  const long long group = precision == BEM_PRECISION_MIXED ? 4 : 1;        // frequencies assembled together
+  const long long group = precision == BEM_PRECISION_MIXED ? 4 : 2;        // frequencies assembled together
   bytes += round_up(n_ext, 32) * 3LL * nf * esz * group;                    // extended rows
   bytes += (long long)batch * lda * nv * esz * (precision == BEM_PRECISION_MIXED ? 2 : 1);  // matrices (+copy)
   bytes += (long long)npairs * (12 * esz * group + 24 * 8 + 48 + (bem::kPairRec + bem::kPairGeoDf) * 4 + 96 +

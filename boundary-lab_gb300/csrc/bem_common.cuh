@@ -172,6 +172,54 @@ BEM_D float reduce_two_pi(float t) {
   return fmaf(-n, BEM_TWO_PI_MID, t);
 }
 
+// -------------------------------------------------------- FP64 on this part --
+// FP64 issues at 1/64 of the FP32 rate here, so an FP64 kernel's time is its count of FP64
+// instructions; everything else (table reads, FP32, integer work) is nearly free beside it.
+//
+// sin and cos by table: theta = n 2pi/512 + x, |x| <= pi/512, with the table entry of n mod
+// 512 and Taylor polynomials of x (sin to x^5, cos to x^6: truncation below 7e-20 and
+// 1e-22), combined by the addition theorem.  16 FP64 instructions for the pair.  Errors: the
+// reduction's (2pi/512 in two doubles, the product exact in the fma) and the table's, about
+// 1.5e-16 absolute; for |theta| <= pi/512 the entry is (1, 0) and the sine has full relative
+// accuracy.  |theta| < 2^22.
+constexpr int kSincosTable = 512;
+// The table (cos, sin) into shared memory, by the whole CTA (synchronise before use): from
+// its copy beside the mesh, or computed where there is none (src null; about 5% of a small
+// CTA's FP64 work).
+BEM_D void load_sincos_table(double2* tab, const double2* src) {
+  for (int i = threadIdx.x; i < kSincosTable; i += blockDim.x) {
+    if (src != nullptr) {
+      tab[i] = src[i];
+    } else {
+      double s, c;
+      sincospi(i * (2.0 / kSincosTable), &s, &c);
+      tab[i] = make_double2(c, s);
+    }
+  }
+}
+BEM_D void sincos_table(double theta, const double2* tab, double* s, double* c) {
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
+  const double t = fma(theta, 81.48733086305042, kMagic);
+  const double n = t - kMagic;
+  double x = fma(n, -0.01227184630308513, theta);
+  x = fma(n, -4.783776559169348e-19, x);
+  const double2 e = tab[__double2loint(t) & (kSincosTable - 1)];
+  const double x2 = x * x;
+  const double sx = fma(x * x2, fma(x2, 1.0 / 120.0, -1.0 / 6.0), x);
+  const double cm1 = x2 * fma(x2, fma(x2, -1.0 / 720.0, 1.0 / 24.0), -0.5);  // cos x - 1
+  *c = fma(e.x, cm1, fma(-e.y, sx, e.x));
+  *s = fma(e.y, cm1, fma(e.x, sx, e.y));
+}
+// 1 / sqrt(a), a > 0 normal: the hardware approximation (about 2^-20) and one third-order
+// step, y + y e (1/2 + 3/8 e) with e = 1 - a y^2; five FP64 instructions, relative error
+// about 2^-52.
+BEM_D double rsqrt_step(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-(a * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
 // ------------------------------------------------------- row permutation --
 // Applies a panel's net row permutation (cnt <= 128 pairs: row sdst takes row ssrc) to one
 // column of n entries, by one warp: every source row is loaded (at most 4 per lane, all in

@@ -281,7 +281,10 @@ __global__ void __launch_bounds__(256) field_f64_kernel(const FaceF64* __restric
                                                         const double* __restrict__ obs, int nobs,
                                                         const FieldParamsF64* __restrict__ prm,
                                                         double2* __restrict__ out, FieldRule<double> fr, int ntr,
-                                                        int4 trs) {
+                                                        int4 trs, const double2* __restrict__ trig) {
+  __shared__ double2 tab[kSincosTable];
+  load_sincos_table(tab, trig);
+  __syncthreads();
   const int o = blockIdx.x, bt = blockIdx.y;
   const double xo[3] = {obs[3 * o], obs[3 * o + 1], obs[3 * o + 2]};
   const double k = prm->k[bt];
@@ -304,19 +307,20 @@ __global__ void __launch_bounds__(256) field_f64_kernel(const FaceF64* __restric
       for (int d = 0; d < 3; ++d) rv[d] = (sg[d] * F.anchor[d] - xo[d]) + sg[d] * F.off[3 * n + d];
       const double rr = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
       if (rr == 0.0) continue;
-      const double r = sqrt(rr), rinv = 1.0 / r;
+      const double rinv = rsqrt_step(rr), r = rr * rinv;
       double sn, cs;
-      sincos(k * r, &sn, &cs);
+      sincos_table(k * r, tab, &sn, &cs);
       const double sc = rinv * (0.25 / CUDART_PI);
-      const double2 G = make_double2(cs * sc, sn * sc);
-      const double t = (rv[0] * sg[0] * F.normal[0] + rv[1] * sg[1] * F.normal[1] + rv[2] * F.normal[2]) * rinv;
-      const double2 Dk = make_double2(t * (-G.x * rinv - G.y * k), t * (G.x * k - G.y * rinv));
-      const double wn = fr.w[n];
+      // e^{ikr} [ (t/r)(ik - 1/r) p_s w_s - q w_s / r ] / (4 pi), t = (r . n_y) / r
+      const double t = (rv[0] * sg[0] * F.normal[0] + rv[1] * sg[1] * F.normal[1] + rv[2] * F.normal[2]) * rinv * sc;
+      const double nta = -t * rinv, tb = t * k, nscw = -sc * fr.w[n];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const double2 ps = src[(((size_t)bt * NC + c) * nf + g) * Q + n];
-        const double2 qq = cscale(qg[c], wn);
-        acc[c] = cadd(acc[c], csub(cmul(Dk, ps), cmul(G, qq)));
+        const double zx = fma(nta, ps.x, fma(-tb, ps.y, nscw * qg[c].x));
+        const double zy = fma(nta, ps.y, fma(tb, ps.x, nscw * qg[c].y));
+        acc[c].x = fma(cs, zx, fma(-sn, zy, acc[c].x));
+        acc[c].y = fma(cs, zy, fma(sn, zx, acc[c].y));
       }
     }
   }
@@ -439,7 +443,7 @@ cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const d
 #define BEM_F64(QQ, NCC)                                                                                   \
   field_f64_kernel<QQ, NCC><<<grid, 256, 0, stream>>>(m.faces64, m.nf, (const double2*)sources,            \
                                                       (const double2*)drive, obs, nobs, dp, out, fr64, m.ntr, \
-                                                      make_int4(m.tr[0], m.tr[1], m.tr[2], m.tr[3]))
+                                                      make_int4(m.tr[0], m.tr[1], m.tr[2], m.tr[3]), m.trig)
 #define BEM_F64_Q(NCC)    \
   if (m.Q == 6)           \
     BEM_F64(6, NCC);      \
@@ -514,11 +518,14 @@ cudaError_t launch_field_single(Precision prec, const void* faces, int nf, int Q
     const double2* s = (const double2*)sources;
     const double2* d = (const double2*)drive;
     if (Q == 6)
-      field_f64_kernel<6, 1><<<grid, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr64, 1, make_int4(0, 0, 0, 0));
+      field_f64_kernel<6, 1><<<grid, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr64, 1, make_int4(0, 0, 0, 0),
+                                                     nullptr);
     else if (Q == 3)
-      field_f64_kernel<3, 1><<<grid, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr64, 1, make_int4(0, 0, 0, 0));
+      field_f64_kernel<3, 1><<<grid, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr64, 1, make_int4(0, 0, 0, 0),
+                                                     nullptr);
     else
-      field_f64_kernel<1, 1><<<grid, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr64, 1, make_int4(0, 0, 0, 0));
+      field_f64_kernel<1, 1><<<grid, 256, 0, stream>>>(f, nf, s, d, obs, nobs, dp, out, fr64, 1, make_int4(0, 0, 0, 0),
+                                                     nullptr);
   }
   return cudaGetLastError();
 }

@@ -75,6 +75,7 @@ struct DeviceMesh {
   double* curls = nullptr;
   double* area = nullptr;
   double* m11m10 = nullptr;  // 9 + 3 doubles
+  double2* trig = nullptr;   // (cos, sin) table of the FP64 kernels (kSincosTable entries)
   float m11m10f[12] = {0};   // the same, rounded to float (host copy, passed as a kernel parameter)
   int* driven = nullptr;
   // symmetry: transforms applied to trial faces (0 identity, 1 x, 2 y, 3 xy),
@@ -97,7 +98,7 @@ cudaError_t launch_regular(const DeviceMesh& m, Precision prec, int nfreq, const
                            const double2* cH, void* Rext, long long ldR, long long strideR, cudaStream_t stream);
 // Frequencies assembled per regular-kernel launch for a batch of nfreq (mixed:
 // fours, or twos when four frequencies' accumulators do not fit two CTAs per SM;
-// FP64: ones); writes the group sizes (nfreq <= 64) and returns their count.
+// FP64: twos); writes the group sizes (nfreq <= 64) and returns their count.
 int regular_groups(const DeviceMesh& m, Precision prec, int nfreq, int* sizes);
 int regular_launches(const DeviceMesh& m, Precision prec, int nfreq);
 // FP32 flop per quadrature pair and frequency of the mixed-form regular kernel
