@@ -103,10 +103,17 @@ def read_gmsh22(path: str | Path, scale: float = 1.0) -> BoundaryMesh:
         elem_end = lines.index("$EndElements")
     except ValueError as exc:
         raise ValueError("Only Gmsh 2.2 ASCII meshes with Nodes and Elements sections are supported.") from exc
+    node_lines, elem_lines = lines[node_start + 2 : node_end], lines[elem_start + 2 : elem_end]
+    mesh = _gmsh22_arrays(node_lines, elem_lines, scale)
+    return mesh if mesh is not None else _gmsh22_lines(node_lines, elem_lines, scale)
 
+
+def _gmsh22_lines(node_lines: list[str], elem_lines: list[str], scale: float) -> BoundaryMesh:
+    """The sections line by line: what _gmsh22_arrays has to agree with, and the path of
+    files that are not plain numbers."""
     node_index: dict[int, int] = {}
     coords: list[tuple[float, float, float]] = []
-    for line in lines[node_start + 2 : node_end]:
+    for line in node_lines:
         parts = line.split()
         if len(parts) < 4:
             continue
@@ -115,7 +122,7 @@ def read_gmsh22(path: str | Path, scale: float = 1.0) -> BoundaryMesh:
 
     faces: list[tuple[int, int, int]] = []
     tags: list[int] = []
-    for line in lines[elem_start + 2 : elem_end]:
+    for line in elem_lines:
         parts = line.split()
         if len(parts) < 8 or int(parts[1]) != 2:
             continue
@@ -132,6 +139,65 @@ def read_gmsh22(path: str | Path, scale: float = 1.0) -> BoundaryMesh:
         np.asarray(faces, dtype=np.int32).reshape(-1, 3),
         np.asarray(tags, dtype=np.int32),
     )
+
+
+def _tokens_per_line(lines: list[str], n_tokens: int) -> np.ndarray | None:
+    """Tokens of each line of a section separated by single spaces (n_tokens in all); None
+    where the spacing is another."""
+    counts = np.array([line.count(" ") for line in lines], np.int64) + 1
+    return counts if counts.sum() == n_tokens else None  # a line holds at most spaces + 1 tokens
+
+
+def _integers(data: bytes) -> np.ndarray | None:
+    """The non-negative integers of at most nine digits in a text of digits, spaces and newlines."""
+    if data.translate(None, b"0123456789 \n"):
+        return None
+    raw = np.frombuffer(b" " + data + b" ", np.uint8)
+    digit = raw > 32
+    edge = np.nonzero(digit[1:] != digit[:-1])[0]
+    first, last = edge[::2] + 1, edge[1::2]
+    length = last - first + 1
+    if len(first) == 0 or length.max() > 9:
+        return None
+    value = np.zeros(len(first), np.int64)
+    for j in range(int(length.max())):  # the digit of weight 10^j
+        value += np.where(j < length, raw[np.maximum(last - j, 0)].astype(np.int64) - 48, 0) * 10**j
+    return value
+
+
+def _gmsh22_arrays(node_lines: list[str], elem_lines: list[str], scale: float) -> BoundaryMesh | None:
+    """The sections parsed as whole arrays (a quarter of the time of the loop over lines); None
+    where the loop has to decide: node lines that are not an id and three numbers, other text
+    than non-negative integers in the elements, ids that repeat or are far from dense."""
+    try:
+        elem_data = "\n".join(elem_lines).encode("ascii")
+        tokens = "\n".join(node_lines).split()
+        counts = _tokens_per_line(node_lines, len(tokens))
+        if counts is None or (counts != 4).any():
+            return None
+        ids = _integers(" ".join(tokens[::4]).encode("ascii"))
+        coords = np.array([list(map(float, tokens[i::4])) for i in (1, 2, 3)]).T * scale
+    except (UnicodeEncodeError, ValueError):
+        return None
+    values = _integers(elem_data)
+    if ids is None or values is None or ids.max() > 20 * len(ids) + 1000:
+        return None
+    counts = _tokens_per_line(elem_lines, len(values))
+    if counts is None:
+        return None
+    index = np.full(int(ids.max()) + 1, -1, np.int64)
+    index[ids] = np.arange(len(ids))
+    if (index[ids] != np.arange(len(ids))).any():  # repeated ids
+        return None
+    end = np.cumsum(counts)
+    first, end = (end - counts)[counts >= 8], end[counts >= 8]
+    keep = values[first + 1] == 2
+    first, end = first[keep], end[keep]
+    refs = np.stack([values[end - 3], values[end - 2], values[end - 1]], axis=1)
+    faces = np.where(refs < len(index), index[np.minimum(refs, len(index) - 1)], -1)
+    ok = (faces >= 0).all(axis=1)
+    return BoundaryMesh(np.ascontiguousarray(coords), faces[ok].astype(np.int32),
+                        values[first + 3][ok].astype(np.int32))
 
 
 def combine_meshes(meshes: Sequence[BoundaryMesh], translations: Sequence[Sequence[float]] | None = None) -> BoundaryMesh:

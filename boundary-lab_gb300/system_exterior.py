@@ -232,19 +232,23 @@ def component_impedance(mesh: meshmod.BoundaryMesh, pressure: np.ndarray, excita
     return complex(force.real / 2.0, -force.imag / 2.0)
 
 
-def complex_array_wire(values, complex_dtype) -> dict:
-    """{"dtype", "shape", "real", "imag"}, values row-major (coupled_solver.jl:125-142)."""
+def complex_array_wire(values, complex_dtype, arrays: bool = False):
+    """{"dtype", "shape", "real", "imag"}, values row-major (coupled_solver.jl:125-142); with
+    ``arrays`` the array itself, for a result that stays in this process."""
     arr = np.asarray(values).astype(complex_dtype)
+    if arrays:
+        return arr
     return {"dtype": np.dtype(complex_dtype).name, "shape": list(arr.shape),
             "real": arr.real.ravel().tolist(), "imag": arr.imag.ravel().tolist()}
 
 
-def quantity_wire(output: dict, values, unit: str, axes: list[str], complex_dtype, metadata=None) -> dict:
+def quantity_wire(output: dict, values, unit: str, axes: list[str], complex_dtype, metadata=None,
+                  arrays: bool = False) -> dict:
     """coupled_solver.jl:144-154."""
     targets = output.get("target_ids") or []
     return {"id": str(output["id"]), "quantity": str(output["quantity"]), "unit": unit,
             "target_id": None if not targets else str(targets[0]), "axes": axes,
-            "values": complex_array_wire(values, complex_dtype), "metadata": metadata or {}}
+            "values": complex_array_wire(values, complex_dtype, arrays), "metadata": metadata or {}}
 
 
 class ExteriorSystemJob:
@@ -358,8 +362,9 @@ class ExteriorSystemJob:
         return bool(self.cancel_path) and os.path.isfile(str(self.cancel_path))
 
     # ------------------------------------------------------------- results --
-    def results(self, stop: Callable[[], bool] | None = None) -> Iterator[dict]:
-        """The result dict of each frequency in request order (coupled_solver.jl:361-549).
+    def results(self, stop: Callable[[], bool] | None = None, arrays: bool = False) -> Iterator[dict]:
+        """The result dict of each frequency in request order (coupled_solver.jl:361-549); with
+        ``arrays`` the quantities' values are arrays instead of wire dicts of lists.
         Raises SystemJobCancelled when a cancel request is seen between frequencies."""
         if self._cancel_requested(stop):
             raise SystemJobCancelled(0)
@@ -384,7 +389,7 @@ class ExteriorSystemJob:
                 if i > 0 and self._cancel_requested(stop):
                     raise SystemJobCancelled(solved)
                 t_post = time.perf_counter()
-                quantities = self._quantities(float(freq), res.pressure[i], res.field[i])
+                quantities = self._quantities(float(freq), res.pressure[i], res.field[i], arrays)
                 timings = {
                     "assembly_s": float(st.get("assembly_s", 0.0) * scale),
                     "solve_s": float(st.get("solve_s", 0.0) * scale),
@@ -418,7 +423,7 @@ class ExteriorSystemJob:
                 }
                 solved += 1
 
-    def _quantities(self, freq: float, pressure: np.ndarray, field: np.ndarray) -> list[dict]:
+    def _quantities(self, freq: float, pressure: np.ndarray, field: np.ndarray, arrays: bool = False) -> list[dict]:
         """pressure [n_ports, n_vertices], field [n_ports, n_points] for one frequency."""
         omega = 2.0 * np.pi * freq
         out = []
@@ -427,12 +432,14 @@ class ExteriorSystemJob:
             if q == "exterior_pressure":
                 values = field[:, self.point_slices[str(output["id"])]]
                 out.append(quantity_wire(output, values, "Pa", ["excitation", "observation"], self.complex_dtype,
-                                         metadata={"points_m": output["options"]["points_m"]}))
+                                         metadata={"points_m": output["options"]["points_m"]}, arrays=arrays))
             elif q == "bem_boundary_pressure":
-                out.append(quantity_wire(output, pressure, "Pa", ["excitation", "bem_node"], self.complex_dtype))
+                out.append(quantity_wire(output, pressure, "Pa", ["excitation", "bem_node"], self.complex_dtype,
+                                         arrays=arrays))
             elif q == "bem_boundary_neumann":
                 neumann = self.drives * (1j * self.density * omega)
-                out.append(quantity_wire(output, neumann, "Pa/m", ["excitation", "bem_face"], self.complex_dtype))
+                out.append(quantity_wire(output, neumann, "Pa/m", ["excitation", "bem_face"], self.complex_dtype,
+                                         arrays=arrays))
             else:  # radiation_impedance, one value per component of the system
                 by_component = {e.component_id: (e, pressure[i]) for i, e in enumerate(self.excitations)}
                 values = []
@@ -443,7 +450,7 @@ class ExteriorSystemJob:
                     e, p = by_component[cid]
                     values.append(component_impedance(self.mesh, p, e, self.symmetry))
                 out.append(quantity_wire(output, np.asarray(values, dtype=np.complex128), "Pa*s/m^3", ["radiator"],
-                                         self.complex_dtype))
+                                         self.complex_dtype, arrays=arrays))
         return out
 
 
@@ -493,8 +500,10 @@ def _reference_contract():
         return None
 
 
-def array_from_wire(raw: dict) -> np.ndarray:
+def array_from_wire(raw) -> np.ndarray:
     """The inverse of complex_array_wire (system_contract.py:372-386)."""
+    if isinstance(raw, np.ndarray):
+        return raw
     dtype = np.dtype(str(raw["dtype"]))
     shape = tuple(int(v) for v in raw.get("shape", ()))
     if dtype.kind == "c":
@@ -506,8 +515,15 @@ def array_from_wire(raw: dict) -> np.ndarray:
     return values.reshape(shape)
 
 
-def system_frequency_result_from_wire(raw: dict):
-    ref = _reference_contract()
+_LOOK_UP = object()
+
+
+def system_frequency_result_from_wire(raw: dict, ref=_LOOK_UP):
+    """raw as a SystemFrequencyResult: the reference's own class when its contract imports (then
+    raw is the wire dict), else this module's.  ``ref`` is that contract or None, where the
+    caller has looked it up."""
+    if ref is _LOOK_UP:
+        ref = _reference_contract()
     if ref is not None:
         return ref.system_frequency_result_from_dict(raw)
     return SystemFrequencyResult(
@@ -557,11 +573,13 @@ class Gb300SystemSession:
         def stop() -> bool:
             return self._stop.is_set() or (stop_requested is not None and stop_requested())
 
+        ref = _reference_contract()
         try:
-            for result in self._job.results(stop=stop):
+            # without the reference's classes to build, the values need no trip through lists
+            for result in self._job.results(stop=stop, arrays=ref is None):
                 if stop():
                     return
-                yield system_frequency_result_from_wire(result)
+                yield system_frequency_result_from_wire(result, ref)
         except SystemJobCancelled:
             return
         except Exception as exc:
