@@ -19,6 +19,10 @@
 // phase would lose ~3e-5 rad.
 #include <cooperative_groups.h>
 
+#include <map>
+#include <mutex>
+#include <tuple>
+
 #include "bem_common.cuh"
 #include "bem_kernels.h"
 
@@ -243,18 +247,56 @@ __global__ void __launch_bounds__(256) field_f32_kernel(const FaceF32* __restric
   if (split > 1) cluster.sync();  // no CTA leaves while the first may still read its sums
 }
 
-// CTAs of a cluster that share the faces of 32 points: the smallest power of two that gives
-// every SM four CTAs (two keep the FP32 pipe busy; four even out the last wave), while a
-// warp keeps at least four faces.
-int field_split(long long clusters, int nf) {
-  int s = 1;
-  while (s < kFieldMaxSplit && clusters * s < 4LL * sm_count() && nf >= 2 * s * kFieldWarps * 4) s *= 2;
-  return s;
+// Clusters of `split` CTAs of a field kernel that are resident at once (asked of the driver
+// once per device, kernel and size).
+int resident_clusters(const void* kern, int split) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = known.find({dev, kern, split});
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(split);
+  cfg.blockDim = dim3(kFieldWarps * 32);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = std::max(1, 2 * sm_count() / split);
+  }
+  known[{dev, kern, split}] = n;
+  return n;
+}
+
+// CTAs of a cluster that share the faces of 32 points.  The time goes as (waves of clusters)
+// / split: 157 clusters of four, one wave and a bit, took 0.88 ms where the sevens' two full
+// waves take 0.67 (5,000 points, 9,948 faces, three-point rule).  A warp keeps at least
+// four faces.
+int field_split(const void* kern, long long clusters, int nf) {
+  int best = 1;
+  double best_time = 1e300;
+  for (int s = 1; s <= kFieldMaxSplit && (s == 1 || nf >= s * kFieldWarps * 4); ++s) {
+    const long long cap = resident_clusters(kern, s);
+    const double time = (double)((clusters + cap - 1) / cap) / s;
+    if (time < 0.999 * best_time) {
+      best = s;
+      best_time = time;
+    }
+  }
+  return best;
 }
 
 template <typename K, typename... A>
 cudaError_t launch_field_f32(K kern, unsigned pt_blocks, unsigned groups, int nf, cudaStream_t stream, A... args) {
-  const int split = field_split((long long)pt_blocks * groups, nf);
+  const int split = field_split((const void*)kern, (long long)pt_blocks * groups, nf);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pt_blocks * split, groups);
   cfg.blockDim = dim3(kFieldWarps * 32);
