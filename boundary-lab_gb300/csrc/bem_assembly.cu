@@ -1629,30 +1629,34 @@ __global__ void __launch_bounds__(128)
 template <typename C2>
 __global__ void singular_scatter_kernel(const int* __restrict__ scat_col, const int* __restrict__ scat_row,
                                         const int* __restrict__ scat_ptr, const int* __restrict__ scat_src,
-                                        int n_entries, const C2* __restrict__ blocks, C2* __restrict__ Rext,
-                                        long long ldR) {
+                                        int n_entries, const C2* __restrict__ blocks, long long blocks_stride,
+                                        C2* __restrict__ Rext, long long ldR, long long strideR) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_entries) return;
+  blocks += (size_t)blockIdx.y * blocks_stride;  // frequency
+  Rext += (size_t)blockIdx.y * strideR;
   C2* dst = &Rext[(size_t)scat_col[i] * ldR + scat_row[i]];
   C2 v = *dst;
   for (int s = scat_ptr[i]; s < scat_ptr[i + 1]; ++s) v = cadd(v, blocks[scat_src[s]]);
   *dst = v;
 }
 
-// One CTA per column: A[:, j] in permuted row order.
+// One CTA per column and frequency (blockIdx.y): A[:, j] in permuted row order.
 template <typename C2>
-__global__ void gather_columns_kernel(const C2* __restrict__ Rext, long long ldR, const int* __restrict__ col_ptr,
+__global__ void gather_columns_kernel(const C2* __restrict__ Rext, long long ldR, long long strideR,
+                                      const int* __restrict__ col_ptr,
                                       const int* __restrict__ col_fb, const int* __restrict__ ext_row,
                                       const int* __restrict__ halo_slot_of_ext, const int* __restrict__ halo_row_ptr,
                                       const int* __restrict__ halo_row, int n_ext, int n_halo_rows,
-                                      C2* __restrict__ A, long long lda, C2* __restrict__ A2, int col0,
+                                      C2* __restrict__ A, long long lda, long long strideA, C2* __restrict__ A2,
                                       const double* __restrict__ row_weight) {
   extern __shared__ unsigned char smem_raw[];
   C2* hb = reinterpret_cast<C2*>(smem_raw);
-  const int j = col0 + blockIdx.x;
+  const int j = blockIdx.x;
   const int k0 = col_ptr[j], k1 = col_ptr[j + 1];
-  C2* Aj = A + (size_t)j * lda;
-  C2* A2j = A2 ? A2 + (size_t)j * lda : nullptr;
+  Rext += (size_t)blockIdx.y * strideR;
+  C2* Aj = A + (size_t)blockIdx.y * strideA + (size_t)j * lda;
+  C2* A2j = A2 ? A2 + (size_t)blockIdx.y * strideA + (size_t)j * lda : nullptr;
   for (int e = threadIdx.x; e < n_ext; e += blockDim.x) {
     C2 v;
     v.x = 0;
@@ -1881,12 +1885,18 @@ template <int NFQ> struct RhsParamsF32N {
   df kdf[NFQ];
   float k[NFQ];
   float2 cS[NFQ], cK[NFQ], qscale[NFQ];
+};
+// The groups of NFQ frequencies of one launch (blockIdx.y) and the rule they share.
+constexpr int kRhsGroups = 16;
+template <int NFQ> struct RhsBatchF32N {
+  RhsParamsF32N<NFQ> g[kRhsGroups];
   float cw[3 * kMaxQ];
 };
 
 template <int Q, int NFQ>
 __device__ __forceinline__ void rhs_pair_f32_freqs(const FaceF32& F, const FaceF32& Gf, const RhsParamsF32N<NFQ>& p,
-                                                   float2 S[NFQ][3], float2 K[NFQ][3], float sx, float sy) {
+                                                   const float* cw, float2 S[NFQ][3], float2 K[NFQ][3], float sx,
+                                                   float sy) {
   const float ghi[3] = {sx * Gf.anchor_hi[0], sy * Gf.anchor_hi[1], Gf.anchor_hi[2]};
   const float glo[3] = {sx * Gf.anchor_lo[0], sy * Gf.anchor_lo[1], Gf.anchor_lo[2]};
   const PairGeomF32 P = pair_geom_f32(ghi, glo, F.anchor_hi, F.anchor_lo);
@@ -1927,7 +1937,7 @@ __device__ __forceinline__ void rhs_pair_f32_freqs(const FaceF32& F, const FaceF
       const float sc = rinv * BEM_INV_FOUR_PI;
       // adjoint double layer: G (-1/r + ik) * (-(r . n_x)/r)
       const float t = -fmaf(rv[0], F.normal[0], fmaf(rv[1], F.normal[1], rv[2] * F.normal[2])) * rinv;
-      const float wn = p.cw[n] + p.cw[Q + n] + p.cw[2 * Q + n];  // DP0 trial basis
+      const float wn = cw[n] + cw[Q + n] + cw[2 * Q + n];  // DP0 trial basis
 #pragma unroll
       for (int fq = 0; fq < NFQ; ++fq) {
         const float theta = reduce_two_pi(fmaf(p.k[fq], delta, th0[fq]));
@@ -1943,7 +1953,7 @@ __device__ __forceinline__ void rhs_pair_f32_freqs(const FaceF32& F, const FaceF
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const float c = p.cw[a * Q + m];
+      const float c = cw[a * Q + m];
 #pragma unroll
       for (int fq = 0; fq < NFQ; ++fq) {
         S[fq][a].x = fmaf(c, us[fq].x, S[fq][a].x);
@@ -1968,7 +1978,11 @@ __global__ void __launch_bounds__(128) rhs_faces_f32_freqs_kernel(
     const FaceF32* __restrict__ faces, int nf, const int* __restrict__ driven, int ndriven,
     const float2* __restrict__ drive, const SingularPair* __restrict__ pairs, const int* __restrict__ by_test_ptr,
     const int* __restrict__ by_test, const float2* __restrict__ sblocks, long long sblocks_stride,
-    RhsParamsF32N<NFQ> p, float2* __restrict__ rb, int ntr, int4 trs, const unsigned char* __restrict__ fix_mask) {
+    const __grid_constant__ RhsBatchF32N<NFQ> batch, float2* __restrict__ rb, int ntr, int4 trs,
+    const unsigned char* __restrict__ fix_mask) {
+  const RhsParamsF32N<NFQ>& p = batch.g[blockIdx.y];
+  sblocks += (size_t)blockIdx.y * NFQ * sblocks_stride;
+  rb += (size_t)blockIdx.y * NFQ * NC * nf * 3;
   const int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (f >= nf) return;
@@ -1991,7 +2005,7 @@ __global__ void __launch_bounds__(128) rhs_faces_f32_freqs_kernel(
       for (int b = 0; b < 3; ++b) sv[b] = (tr == 0 || (fix_mask[Gf.verts[b]] & tr) == tr) ? Gf.verts[b] : -2;
       if (share_vertex(F.verts, sv[0], sv[1], sv[2])) continue;
       float2 S[NFQ][3], K[NFQ][3];
-      rhs_pair_f32_freqs<Q, NFQ>(F, Gf, p, S, K, (float)tr_sign_x(tr), (float)tr_sign_y(tr));
+      rhs_pair_f32_freqs<Q, NFQ>(F, Gf, p, batch.cw, S, K, (float)tr_sign_x(tr), (float)tr_sign_y(tr));
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const float2 dg = drive[(size_t)c * nf + g];
@@ -2037,13 +2051,15 @@ __global__ void __launch_bounds__(128) rhs_faces_f32_freqs_kernel(
       for (int c = 0; c < NC; ++c) rb[(((size_t)fq * NC + c) * nf + f) * 3 + a] = acc[fq][a][c];
 }
 
-// b[row(j)][c] = sum over (f, a) in star(j) of rb[c][f][a]
+// b[row(j)][c] = sum over (f, a) in star(j) of rb[c][f][a], for one frequency per blockIdx.y
 template <typename C2>
 __global__ void rhs_gather_kernel(const C2* __restrict__ rb, int nf, int nc, const int* __restrict__ col_ptr,
                                   const int* __restrict__ col_fb, const int* __restrict__ vertex_row, int nv,
                                   C2* __restrict__ b, long long ldb, const double* __restrict__ row_weight) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nv) return;
+  rb += (size_t)blockIdx.y * nc * nf * 3;
+  b += (size_t)blockIdx.y * nc * ldb;
   for (int c = 0; c < nc; ++c) {
     C2 s;
     s.x = 0;
@@ -2057,10 +2073,12 @@ __global__ void rhs_gather_kernel(const C2* __restrict__ rb, int nf, int nc, con
 // Rows/columns of vertices that no face references: identity (pressure 0).
 template <typename C2>
 __global__ void isolated_identity_kernel(const int* __restrict__ iso, int n, const int* __restrict__ vertex_row,
-                                         C2* A, long long lda, C2* A2) {
+                                         C2* A, long long lda, long long strideA, C2* A2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int v = iso[i];
+  A += (size_t)blockIdx.y * strideA;
+  if (A2) A2 += (size_t)blockIdx.y * strideA;
   C2 one;
   one.x = 1;
   one.y = 0;
@@ -2509,50 +2527,49 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_singular_scatter(const DeviceMesh& m, Precision prec, const void* blocks, void* Rext,
-                                    long long ldR, cudaStream_t stream) {
+cudaError_t launch_singular_scatter(const DeviceMesh& m, Precision prec, int nfreq, const void* blocks,
+                                    long long blocks_stride, void* Rext, long long ldR, long long strideR,
+                                    cudaStream_t stream) {
   if (m.n_scat == 0) return cudaSuccess;
   const int threads = 256;
-  const int nblk = (m.n_scat + threads - 1) / threads;
+  const dim3 grid((m.n_scat + threads - 1) / threads, nfreq);
   if (prec == Precision::Mixed)
-    singular_scatter_kernel<float2><<<nblk, threads, 0, stream>>>(m.scat_col, m.scat_row, m.scat_ptr, m.scat_src,
-                                                                  m.n_scat, (const float2*)blocks, (float2*)Rext, ldR);
+    singular_scatter_kernel<float2><<<grid, threads, 0, stream>>>(m.scat_col, m.scat_row, m.scat_ptr, m.scat_src,
+                                                                  m.n_scat, (const float2*)blocks, blocks_stride,
+                                                                  (float2*)Rext, ldR, strideR);
   else
-    singular_scatter_kernel<double2><<<nblk, threads, 0, stream>>>(m.scat_col, m.scat_row, m.scat_ptr, m.scat_src,
-                                                                   m.n_scat, (const double2*)blocks, (double2*)Rext,
-                                                                   ldR);
+    singular_scatter_kernel<double2><<<grid, threads, 0, stream>>>(m.scat_col, m.scat_row, m.scat_ptr, m.scat_src,
+                                                                   m.n_scat, (const double2*)blocks, blocks_stride,
+                                                                   (double2*)Rext, ldR, strideR);
   return cudaGetLastError();
 }
 
-cudaError_t launch_gather(const DeviceMesh& m, Precision prec, const void* Rext, long long ldR, void* A, long long lda,
-                          void* A2, cudaStream_t stream) {
+cudaError_t launch_gather(const DeviceMesh& m, Precision prec, int nfreq, const void* Rext, long long ldR,
+                          long long strideR, void* A, long long lda, long long strideA, void* A2,
+                          cudaStream_t stream) {
   const int threads = 256;
-  const int n_halo = m.n_halo;
-  if (prec == Precision::Mixed) {
-    size_t sm = (size_t)std::max(1, n_halo) * sizeof(float2);
-    if (sm > 48 * 1024) ensure_smem_limit((const void*)gather_columns_kernel<float2>, sm);
-    gather_columns_kernel<float2><<<m.nv, threads, sm, stream>>>(
-        (const float2*)Rext, ldR, m.col_ptr, m.col_fb, m.ext_row, m.halo_slot_of_ext, m.halo_row_ptr, m.halo_row,
-        m.n_ext, m.n_halo_rows, (float2*)A, lda, (float2*)A2, 0, m.row_weight);
+  const dim3 grid(m.nv, nfreq), iso((m.n_isolated + 127) / 128, nfreq);
+  auto run = [&](auto zero) {
+    using C2 = decltype(zero);
+    const size_t sm = (size_t)std::max(1, m.n_halo) * sizeof(C2);
+    if (sm > 48 * 1024) ensure_smem_limit((const void*)gather_columns_kernel<C2>, sm);
+    gather_columns_kernel<C2><<<grid, threads, sm, stream>>>(
+        (const C2*)Rext, ldR, strideR, m.col_ptr, m.col_fb, m.ext_row, m.halo_slot_of_ext, m.halo_row_ptr, m.halo_row,
+        m.n_ext, m.n_halo_rows, (C2*)A, lda, strideA, (C2*)A2, m.row_weight);
     if (m.n_isolated)
-      isolated_identity_kernel<float2><<<(m.n_isolated + 127) / 128, 128, 0, stream>>>(
-          m.isolated, m.n_isolated, m.vertex_row, (float2*)A, lda, (float2*)A2);
-  } else {
-    size_t sm = (size_t)std::max(1, n_halo) * sizeof(double2);
-    if (sm > 48 * 1024) ensure_smem_limit((const void*)gather_columns_kernel<double2>, sm);
-    gather_columns_kernel<double2><<<m.nv, threads, sm, stream>>>(
-        (const double2*)Rext, ldR, m.col_ptr, m.col_fb, m.ext_row, m.halo_slot_of_ext, m.halo_row_ptr,
-        m.halo_row, m.n_ext, m.n_halo_rows, (double2*)A, lda, (double2*)A2, 0, m.row_weight);
-    if (m.n_isolated)
-      isolated_identity_kernel<double2><<<(m.n_isolated + 127) / 128, 128, 0, stream>>>(
-          m.isolated, m.n_isolated, m.vertex_row, (double2*)A, lda, (double2*)A2);
-  }
+      isolated_identity_kernel<C2><<<iso, 128, 0, stream>>>(m.isolated, m.n_isolated, m.vertex_row, (C2*)A, lda,
+                                                            strideA, (C2*)A2);
+  };
+  if (prec == Precision::Mixed)
+    run(float2{});
+  else
+    run(double2{});
   return cudaGetLastError();
 }
 
-cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const OperatorCoeffs& c, double2 qscale,
-                       const void* drive, int nc, const void* sblocks, void* rb, void* b, long long ldb,
-                       cudaStream_t stream) {
+// The face kernel of one frequency's right-hand side (rb as launch_rhs_freqs lays it out).
+static cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const OperatorCoeffs& c, double2 qscale,
+                       const void* drive, int nc, const void* sblocks, void* rb, cudaStream_t stream) {
   const int threads = 128;
   const int nblk = (int)(((long long)m.nf * 32 + threads - 1) / threads);
   if (prec == Precision::Mixed) {
@@ -2584,9 +2601,6 @@ cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const Oper
       case 4: BEM_RHS32_Q(4) break;
       default: return cudaErrorInvalidValue;
     }
-    rhs_gather_kernel<float2><<<(m.nv + 127) / 128, 128, 0, stream>>>((const float2*)rb, m.nf, nc, m.col_ptr,
-                                                                       m.col_fb, m.vertex_row, m.nv, (float2*)b,
-                                                                       ldb, m.row_weight);
   } else {
     RhsParams<double> p;
     p.k = k;
@@ -2615,9 +2629,6 @@ cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const Oper
       case 4: BEM_RHS64_Q(4) break;
       default: return cudaErrorInvalidValue;
     }
-    rhs_gather_kernel<double2><<<(m.nv + 127) / 128, 128, 0, stream>>>((const double2*)rb, m.nf, nc, m.col_ptr,
-                                                                        m.col_fb, m.vertex_row, m.nv,
-                                                                        (double2*)b, ldb, m.row_weight);
   }
   return cudaGetLastError();
 }
@@ -2628,37 +2639,41 @@ int rhs_width(Precision prec, int nc) { return prec == Precision::Mixed ? (nc ==
 
 cudaError_t launch_rhs_freqs(const DeviceMesh& m, Precision prec, int nfreq, const double* k, const OperatorCoeffs* c,
                              const double2* qscale, const void* drive, int nc, const void* sblocks,
-                             long long sblocks_stride, void* rb, void* const* b, long long ldb, cudaStream_t stream) {
+                             long long sblocks_stride, void* rb, void* b, long long ldb, cudaStream_t stream) {
   const int width = rhs_width(prec, nc);
   const size_t esz = prec == Precision::Mixed ? sizeof(float2) : sizeof(double2);
   for (int f0 = 0; f0 < nfreq;) {
     const int w = std::min(width, nfreq - f0);
+    const char* sb = (const char*)sblocks + (size_t)f0 * sblocks_stride * esz;
+    char* rbf = (char*)rb + (size_t)f0 * nc * m.nf * 3 * esz;
     if (w == 1) {
-      const cudaError_t e = launch_rhs(m, prec, k[f0], c[f0], qscale[f0], drive, nc,
-                                       (const char*)sblocks + (size_t)f0 * sblocks_stride * esz, rb, b[f0], ldb, stream);
+      const cudaError_t e = launch_rhs(m, prec, k[f0], c[f0], qscale[f0], drive, nc, sb, rbf, stream);
       if (e != cudaSuccess) return e;
       ++f0;
       continue;
     }
+    // all full groups of w frequencies in one launch (then the remainder's)
+    const int groups = std::min((nfreq - f0) / w, kRhsGroups);
     const int threads = 128;
-    const int nblk = (int)(((long long)m.nf * 32 + threads - 1) / threads);
-    const float2* sb = (const float2*)sblocks + (size_t)f0 * sblocks_stride;
+    const dim3 grid((unsigned)(((long long)m.nf * 32 + threads - 1) / threads), groups);
     const int4 trs = make_int4(m.tr[0], m.tr[1], m.tr[2], m.tr[3]);
     auto run = [&](auto nfq_c, auto nc_c) {
       constexpr int NFQ = decltype(nfq_c)::value, NC = decltype(nc_c)::value;
-      RhsParamsF32N<NFQ> p;
-      for (int i = 0; i < NFQ; ++i) {
-        p.kdf[i] = make_df(k[f0 + i]);
-        p.k[i] = (float)k[f0 + i];
-        p.cS[i] = f2(c[f0 + i].cS);
-        p.cK[i] = f2(c[f0 + i].cK);
-        p.qscale[i] = f2(qscale[f0 + i]);
+      RhsBatchF32N<NFQ> p;
+      for (int j = 0; j < groups * NFQ; ++j) {
+        RhsParamsF32N<NFQ>& g = p.g[j / NFQ];
+        const int i = j % NFQ, f = f0 + j;
+        g.kdf[i] = make_df(k[f]);
+        g.k[i] = (float)k[f];
+        g.cS[i] = f2(c[f].cS);
+        g.cK[i] = f2(c[f].cK);
+        g.qscale[i] = f2(qscale[f]);
       }
       for (int i = 0; i < 3 * kMaxQ; ++i) p.cw[i] = (float)m.rule_cw[i];
       auto go = [&](auto kern) {
-        kern<<<nblk, threads, 0, stream>>>(m.faces32, m.nf, m.driven, m.ndriven, (const float2*)drive, m.pairs,
-                                           m.pairs_by_test_ptr, m.pairs_by_test, sb, sblocks_stride, p, (float2*)rb,
-                                           m.ntr, trs, m.fix_mask);
+        kern<<<grid, threads, 0, stream>>>(m.faces32, m.nf, m.driven, m.ndriven, (const float2*)drive, m.pairs,
+                                           m.pairs_by_test_ptr, m.pairs_by_test, (const float2*)sb, sblocks_stride, p,
+                                           (float2*)rbf, m.ntr, trs, m.fix_mask);
       };
       if (m.Q == 6)
         go(rhs_faces_f32_freqs_kernel<6, NC, NFQ>);
@@ -2675,19 +2690,23 @@ cudaError_t launch_rhs_freqs(const DeviceMesh& m, Precision prec, int nfreq, con
       run(std::integral_constant<int, 3>{}, std::integral_constant<int, 1>{});
     else
       run(std::integral_constant<int, 2>{}, std::integral_constant<int, 1>{});
-    for (int i = 0; i < w; ++i)
-      rhs_gather_kernel<float2><<<(m.nv + 127) / 128, 128, 0, stream>>>(
-          (const float2*)rb + (size_t)i * nc * m.nf * 3, m.nf, nc, m.col_ptr, m.col_fb, m.vertex_row, m.nv,
-          (float2*)b[f0 + i], ldb, m.row_weight);
-    f0 += w;
+    f0 += groups * w;
   }
+  const dim3 gg((m.nv + 127) / 128, nfreq);
+  if (prec == Precision::Mixed)
+    rhs_gather_kernel<float2><<<gg, 128, 0, stream>>>((const float2*)rb, m.nf, nc, m.col_ptr, m.col_fb, m.vertex_row,
+                                                      m.nv, (float2*)b, ldb, m.row_weight);
+  else
+    rhs_gather_kernel<double2><<<gg, 128, 0, stream>>>((const double2*)rb, m.nf, nc, m.col_ptr, m.col_fb, m.vertex_row,
+                                                       m.nv, (double2*)b, ldb, m.row_weight);
   return cudaGetLastError();
 }
 
 // Kernel launches of launch_rhs_freqs for nfreq frequencies.
 int rhs_launches(Precision prec, int nc, int nfreq) {
   const int width = rhs_width(prec, nc);
-  return nfreq + (nfreq + width - 1) / width;  // one gather per frequency, one face kernel per group
+  if (width == 1) return nfreq + 1;
+  return (nfreq >= width ? 1 : 0) + (nfreq % width ? 1 : 0) + 1;  // full groups, the remainder, the gather
 }
 
 }  // namespace bem

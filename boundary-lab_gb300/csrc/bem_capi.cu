@@ -318,75 +318,92 @@ void ensure_cheb(bem_context* ctx, bem_mesh* m, const double* k, int n) {
   d.cheb_n = nterms;
 }
 
-// Assemble the LHS (c[i].cD, cH, cM) of cnt frequencies into A[i] (and A2[i] if
-// given; column-major, leading dimension lda) and, if nc > 0, the RHS into b[i]
-// (nc columns, leading dimension ldb, permuted rows).  lda / ldb <= 0: the mesh's
-// own layout.  Returns the number of kernels launched.
+// Extended rows held at once: as many frequencies as fit 1 GiB, and at least those that share
+// a regular launch.  A small mesh's batch then takes one launch of each of the scatter, gather
+// and right-hand-side kernels instead of one per frequency (1,036 triangles, 16 frequencies:
+// 0.49 -> 0.17 ms for the three); from about 5,000 triangles on the regular launch's
+// frequencies fill the GPU by themselves.
+constexpr size_t kRextBytes = (size_t)1 << 30;
+
+// Assemble the LHS (c[i].cD, cH, cM) of cnt frequencies into A + i matrices (and A2, if
+// given; column-major, leading dimension lda, lda * order apart) and, if nc > 0, the RHS into
+// b + i (nc ldb) (permuted rows).  lda / ldb <= 0: the mesh's own layout.  Returns the number
+// of kernels launched.
 long long assemble_frequencies(bem_context* ctx, bem_mesh* m, bem::Precision prec, int cnt, const double* k,
-                               const bem::OperatorCoeffs* c, void* const* A, void* const* A2, const double2* qscale,
-                               int nc, const void* drive, void* const* b, long long lda = 0, long long ldb = 0,
+                               const bem::OperatorCoeffs* c, void* A, void* A2, const double2* qscale, int nc,
+                               const void* drive, void* b, int order, long long lda = 0, long long ldb = 0,
                                double* regular_flop = nullptr, long long* cheb_freqs = nullptr,
                                bool use_cheb = false) {
   const bem::DeviceMesh& dm = m->dm;
   Layout L = layout_for(dm, prec);
   if (lda > 0) L.lda = lda;
   if (ldb > 0) L.ldb = ldb;
+  const long long strideA = L.lda * order;
   int sizes[64];
   const int ngroups = bem::regular_groups(dm, prec, cnt, sizes);
-  int G = 1;
-  for (int i = 0; i < ngroups; ++i) G = std::max(G, sizes[i]);
   const size_t rext_n = (size_t)L.ldR * 3 * dm.nf;         // elements per extended-row buffer
   const size_t sblk_n = (size_t)std::max(dm.npairs, 1) * 12;  // elements per singular-block buffer
+  // groups of regular launches that are scattered and gathered together
+  const int fit = (int)std::min<size_t>(64, kRextBytes / (rext_n * L.esz));
+  auto take = [&](int gi, int* g) {
+    *g = sizes[gi++];
+    while (gi < ngroups && *g + sizes[gi] <= fit) *g += sizes[gi++];
+    return gi;
+  };
+  int G = 1;
+  for (int gi = 0, g = 0; gi < ngroups; G = std::max(G, g)) gi = take(gi, &g);
   ck(ctx->rext.ensure(rext_n * L.esz * G), "alloc extended rows");
   ck(ctx->sblocks.ensure(sblk_n * L.esz * G), "alloc singular blocks");
-  if (nc > 0) ck(ctx->rb.ensure((size_t)std::max(4, nc) * dm.nf * 3 * L.esz), "alloc rhs faces");
-  auto rext = [&](int i) { return (void*)((char*)ctx->rext.p + rext_n * L.esz * i); };
-  auto sblk = [&](int i) { return (void*)((char*)ctx->sblocks.p + sblk_n * L.esz * i); };
+  if (nc > 0) ck(ctx->rb.ensure((size_t)G * nc * dm.nf * 3 * L.esz), "alloc rhs faces");
+  void *rext = ctx->rext.p, *sblk = ctx->sblocks.p;
   long long launches = 0;
   int f0 = 0;
-  for (int gi = 0; gi < ngroups; f0 += sizes[gi], ++gi) {
-    const int g = sizes[gi];
-    double2 cD[4], cH[4];
+  for (int gi = 0, g = 0; gi < ngroups; f0 += g) {
+    const int g_lo = gi;
+    gi = take(gi, &g);
+    std::vector<double2> cD(g), cH(g);
     for (int i = 0; i < g; ++i) {
       cD[i] = c[f0 + i].cD;
       cH[i] = c[f0 + i].cH;
     }
     // regular pairs first: on a freshly uploaded mesh they run while the side stream
     // still integrates the FP64 singular moments that the singular kernel reads
-    ck(bem::launch_regular(dm, prec, g, k + f0, cD, cH, rext(0), L.ldR, (long long)rext_n, ctx->stream),
+    ck(bem::launch_regular(dm, prec, g, k + f0, cD.data(), cH.data(), rext, L.ldR, (long long)rext_n, ctx->stream),
        "regular kernel");
     prof_mark(ctx, BEM_K_REGULAR);
     if (m->moments_ready) ck(cudaStreamWaitEvent(ctx->stream, m->moments_ready, 0), "wait for singular moments");
     if (m->cheb_ready) ck(cudaStreamWaitEvent(ctx->stream, m->cheb_ready, 0), "wait for Chebyshev moments");
     long long sing_launches = 0;
-    ck(bem::launch_singular_dyn(dm, prec, g, k + f0, c + f0, sblk(0), (long long)sblk_n, ctx->stream,
-                                &sing_launches, cheb_freqs, use_cheb),
+    ck(bem::launch_singular_dyn(dm, prec, g, k + f0, c + f0, sblk, (long long)sblk_n, ctx->stream, &sing_launches,
+                                cheb_freqs, use_cheb),
        "singular kernel");
     prof_mark(ctx, BEM_K_SINGULAR);
-    for (int i = 0; i < g; ++i) {
-      void* Ai = A[f0 + i];
-      void* A2i = A2 ? A2[f0 + i] : nullptr;
-      ck(bem::launch_singular_scatter(dm, prec, sblk(i), rext(i), L.ldR, ctx->stream), "singular scatter");
-      if (dm.n_isolated) {
-        ck(cudaMemsetAsync(Ai, 0, (size_t)L.lda * dm.nv * L.esz, ctx->stream), "memset");
-        if (A2i) ck(cudaMemsetAsync(A2i, 0, (size_t)L.lda * dm.nv * L.esz, ctx->stream), "memset");
+    char* Ag = (char*)A + (size_t)f0 * strideA * L.esz;
+    char* A2g = A2 ? (char*)A2 + (size_t)f0 * strideA * L.esz : nullptr;
+    ck(bem::launch_singular_scatter(dm, prec, g, sblk, (long long)sblk_n, rext, L.ldR, (long long)rext_n, ctx->stream),
+       "singular scatter");
+    if (dm.n_isolated)
+      for (int i = 0; i < g; ++i) {
+        const size_t off = (size_t)i * strideA * L.esz, bytes = (size_t)L.lda * dm.nv * L.esz;
+        ck(cudaMemsetAsync(Ag + off, 0, bytes, ctx->stream), "memset");
+        if (A2g) ck(cudaMemsetAsync(A2g + off, 0, bytes, ctx->stream), "memset");
       }
-      ck(bem::launch_gather(dm, prec, rext(i), L.ldR, Ai, L.lda, A2i, ctx->stream), "gather kernel");
-    }
+    ck(bem::launch_gather(dm, prec, g, rext, L.ldR, (long long)rext_n, Ag, L.lda, strideA, A2g, ctx->stream),
+       "gather kernel");
     prof_mark(ctx, BEM_K_GATHER);
     if (nc > 0) {
-      ck(bem::launch_rhs_freqs(dm, prec, g, k + f0, c + f0, qscale + f0, drive, nc, sblk(0), (long long)sblk_n,
-                               ctx->rb.p, b + f0, L.ldb, ctx->stream),
+      ck(bem::launch_rhs_freqs(dm, prec, g, k + f0, c + f0, qscale + f0, drive, nc, sblk, (long long)sblk_n,
+                               ctx->rb.p, (char*)b + (size_t)f0 * nc * L.ldb * L.esz, L.ldb, ctx->stream),
          "rhs kernel");
       prof_mark(ctx, BEM_K_RHS);
     }
-    // per frequency: scatter, gather (+ isolated rows); per group the regular, singular and
-    // right-hand-side launches
-    launches += (long long)g * (2 + (dm.n_isolated ? 1 : 0)) + (nc > 0 ? bem::rhs_launches(prec, nc, g) : 0) +
+    // the scatter (where there are singular pairs), the gather (and the isolated rows'
+    // identity), the regular, singular and right-hand-side launches
+    launches += (dm.n_scat ? 1 : 0) + 1 + (dm.n_isolated ? 1 : 0) + (nc > 0 ? bem::rhs_launches(prec, nc, g) : 0) +
                 bem::regular_launches(dm, prec, g) + sing_launches;
     if (regular_flop && prec == bem::Precision::Mixed) {
       const double qpairs = ((double)dm.ntr * dm.nf * dm.nf - dm.npairs) * dm.Q * dm.Q;
-      *regular_flop += g * qpairs * bem::regular_flop_per_qpair(g);
+      for (int i = g_lo; i < gi; ++i) *regular_flop += sizes[i] * qpairs * bem::regular_flop_per_qpair(sizes[i]);
     }
   }
   return launches;
@@ -398,8 +415,8 @@ void assemble_one(bem_mesh* m, bem::Precision prec, double k, const bem::Operato
                   double2 qscale, int nc, const void* drive, void* b) {
   const bool cheb = prec == bem::Precision::Mixed;
   if (cheb) ensure_cheb(m->ctx, m, &k, 1);
-  assemble_frequencies(m->ctx, m, prec, 1, &k, &c, &A, A2 ? &A2 : nullptr, &qscale, nc, drive, &b, 0, 0, nullptr,
-                       nullptr, cheb);
+  assemble_frequencies(m->ctx, m, prec, 1, &k, &c, A, A2, &qscale, nc, drive, b, m->dm.nv, 0, 0, nullptr, nullptr,
+                       cheb);
 }
 
 void free_mesh_device(bem_mesh* m) {
@@ -937,9 +954,9 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
     if (nvm < n)
       ck(cudaMemsetAsync(bs[i0], 0, (size_t)x.cnt * nc * ldb * esz, ctx->stream), "memset padded rhs");
     const void* drive = mixed ? x.m->drive32.p : x.m->drive64.p;
-    T.launches += assemble_frequencies(ctx, x.m, prec, x.cnt, ks.data() + i0, cs.data() + i0, As.data() + i0,
-                                       mixed ? A2s.data() + i0 : nullptr, qs.data() + i0, nc, drive, bs.data() + i0,
-                                       lda, ldb, &T.regular_flop, &T.cheb_freqs, x.cheb);
+    T.launches += assemble_frequencies(ctx, x.m, prec, x.cnt, ks.data() + i0, cs.data() + i0, As[i0],
+                                       mixed ? A2s[i0] : nullptr, qs.data() + i0, nc, drive, bs[i0], n, lda, ldb,
+                                       &T.regular_flop, &T.cheb_freqs, x.cheb);
     if (nvm < n) {
       dim3 g((unsigned)n, (unsigned)x.cnt);
       if (mixed)
@@ -1133,8 +1150,12 @@ long long bem_estimate_device_bytes(int nv, int nf, int npairs, int nrhs, int np
   const long long lda = round_up(nv, 32);
   const long long n_ext = (long long)(nv * 1.3) + 64;
   long long bytes = 0;
-  const long long group = precision == BEM_PRECISION_MIXED ? 4 : 2;        // frequencies assembled together
-  bytes += round_up(n_ext, 32) * 3LL * nf * esz * group;                    // extended rows
+  // frequencies assembled together: those of a regular launch, or a batch's within kRextBytes
+  const long long rext = round_up(n_ext, 32) * 3LL * nf * esz;
+  const long long group = std::max<long long>(precision == BEM_PRECISION_MIXED ? 4 : 2,
+                                              std::min<long long>(batch, (long long)kRextBytes / std::max(rext, 1LL)));
+  bytes += rext * group;                                                    // extended rows
+  bytes += (long long)nf * 3 * nrhs * esz * group;                          // right-hand-side face values
   bytes += (long long)batch * lda * nv * esz * (precision == BEM_PRECISION_MIXED ? 2 : 1);  // matrices (+copy)
   bytes += (long long)npairs * (12 * esz * group + 24 * 8 + 48 + (bem::kPairRec + bem::kPairGeoDf) * 4 + 96 +
                                 bem::kChebN * 24 * 4);  // singular blocks, moments, pairs, records, scatter plan, Chebyshev moments

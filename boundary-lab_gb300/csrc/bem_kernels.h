@@ -126,20 +126,20 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
 int cheb_terms(double k, double R);
 // The mesh's Chebyshev moments for the first nterms terms into m.cheb (after the pair setup).
 cudaError_t launch_cheb_moments(const DeviceMesh& m, int nterms, cudaStream_t stream);
-cudaError_t launch_singular_scatter(const DeviceMesh& m, Precision prec, const void* blocks, void* Rext,
-                                    long long ldR, cudaStream_t stream);
-cudaError_t launch_gather(const DeviceMesh& m, Precision prec, const void* Rext, long long ldR, void* A, long long lda,
-                          void* A2, cudaStream_t stream);
-cudaError_t launch_rhs(const DeviceMesh& m, Precision prec, double k, const OperatorCoeffs& c, double2 qscale,
-                       const void* drive, int nc, const void* sblocks, void* rb, void* b, long long ldb,
-                       cudaStream_t stream);
-// Right-hand sides of nfreq frequencies, up to rhs_width(prec, nc) per face-kernel launch;
-// frequency f's singular blocks start at element f * sblocks_stride of sblocks, and rb needs
-// room for max(4, nc) * nf * 3 complex values.
+// The three below take nfreq frequencies per launch: frequency f's blocks, extended rows,
+// matrices and right-hand sides start f strides (in elements) after the first's.
+cudaError_t launch_singular_scatter(const DeviceMesh& m, Precision prec, int nfreq, const void* blocks,
+                                    long long blocks_stride, void* Rext, long long ldR, long long strideR,
+                                    cudaStream_t stream);
+cudaError_t launch_gather(const DeviceMesh& m, Precision prec, int nfreq, const void* Rext, long long ldR,
+                          long long strideR, void* A, long long lda, long long strideA, void* A2,
+                          cudaStream_t stream);
+// Right-hand sides of nfreq frequencies (b stride nc * ldb), rhs_width(prec, nc) sharing each
+// q-pair's geometry; rb needs room for nfreq * nc * nf * 3 complex values.
 int rhs_width(Precision prec, int nc);
 cudaError_t launch_rhs_freqs(const DeviceMesh& m, Precision prec, int nfreq, const double* k, const OperatorCoeffs* c,
                              const double2* qscale, const void* drive, int nc, const void* sblocks,
-                             long long sblocks_stride, void* rb, void* const* b, long long ldb, cudaStream_t stream);
+                             long long sblocks_stride, void* rb, void* b, long long ldb, cudaStream_t stream);
 int rhs_launches(Precision prec, int nc, int nfreq);
 
 // dense LU and solves (bem_lu.cu).  Matrices are column-major, batched with a
