@@ -310,24 +310,29 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_cluster_kernel(typenam
 // the net row permutation that the other columns get.  A step:
 //  1. every warp takes this CTA's candidate from the warps' keys; the warp that
 //     holds the candidate row copies it from its thread's registers through a
-//     shared row and pushes it with the key into slot j & 1 of every CTA (DSMEM
-//     stores, fenced by that warp alone);
-//  2. cluster barrier (relaxed arrive, acquiring wait);
-//  3. every warp takes the pivot from the CTAs' keys and reads the pivot row
-//     (columns j.. as u[0..]) from its own shared memory; rank 0 stores it;
+//     shared row and pushes it with the key into slot j & 1 of every CTA (DSMEM);
+//  2. every 64-bit word pushed carries the step's number beside its 32 bits of
+//     payload, so the receivers poll their own shared memory for it: no fence, no
+//     cluster barrier, one DSMEM store's latency per step.  A slot is rewritten at
+//     step j + 2, by a CTA that has seen every CTA's step j + 1, which those push
+//     after the barrier that ends their reading of step j;
+//  3. every warp takes the pivot from the CTAs' keys, waits for the pivot row
+//     (columns j.. as u[0..]) and lays it out for broadcast reads; rank 0 stores it;
 //  4. the pivot row leaves (lg = j), the row with lg = j takes the pivot's old
 //     lg; every other active row stores l = a[0] / pivot, subtracts l u and
 //     shifts; the next candidate is reduced per warp; CTA barrier.
+// The polls are bounded: a CTA that waits in vain ends its panel with info = -1.
 // A single CTA (CLUSTER = false) replaces 1 and 2 by the owner thread writing the
 // row to its own shared memory and a CTA barrier.
 // Requires a full panel (kb = 32) and chunk <= kRegPanelThreads.
 //
-// Bound: the latency of a column step (two barriers, the candidate exchange and the row
+// Bound: the latency of a column step (the candidate exchange, one CTA barrier and the row
 // update, about 440 issue cycles with 640 rows on an SM).  The keys are reduced by the
 // warp-reduction instruction (two 32-bit maxima instead of five 64-bit shuffle stages),
 // one warp instead of 640 threads does the push, and no row-j copy is kept for the
 // all-NaN case (a NaN key ranks below every number, so row j itself wins it): 32 columns
-// of one matrix take 29 us with one CTA (518 rows) and 53 us with eight (4,976); 74 us before, either way.
+// of one matrix took 74 us, then 29 us with one CTA (518 rows) and 53 us with eight (4,976)
+// exchanging through a fence and a cluster barrier, 49 us through tagged words.
 constexpr int kRegPanelThreads = 640;
 constexpr int kRegPanelWarps = kRegPanelThreads / 32;
 
@@ -343,6 +348,33 @@ __device__ __forceinline__ uint2 warp_max_key(uint2 k) {
   return make_uint2(hi, __reduce_max_sync(0xffffffffu, k.x == hi ? k.y : 0u));
 }
 
+// Words of the exchange: 32 bits of payload with the step's tag above them, written and read
+// whole (64-bit accesses are single-copy atomic).  Keys pack (hi, lo): lo's 16 low bits are
+// those of ~row (rows < 10,240; 0 only where there is no candidate), its high ones the tag.
+constexpr int kPollLimit = 1 << 16;
+__device__ __forceinline__ void push_words(void* dst, unsigned long long a, unsigned long long b) {
+  asm volatile("st.relaxed.cluster.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void push_word(void* dst, unsigned long long a) {
+  asm volatile("st.relaxed.cluster.b64 [%0], %1;" ::"l"(dst), "l"(a) : "memory");
+}
+__device__ __forceinline__ unsigned long long poll_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.cluster.shared::cta.b64 %0, [%1];"
+               : "=l"(v)
+               : "r"((unsigned)__cvta_generic_to_shared(p))
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ ulonglong2 poll_words(const unsigned long long* p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];"
+               : "=l"(v.x), "=l"(v.y)
+               : "r"((unsigned)__cvta_generic_to_shared(p))
+               : "memory");
+  return v;
+}
+
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float2* A, long long lda, long long strideA,
                                                                            int n, int k, int kb, int chunk, int* ipiv,
@@ -355,9 +387,12 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* Lb = reinterpret_cast<float2*>(smem_raw);  // [NB][kRegPanelThreads] multipliers by column, thread
-  __shared__ __align__(16) float4 rowsC[2][CLUSTER ? 16 : 1][NB / 2];  // candidate rows, by source CTA
+  __shared__ __align__(16) unsigned long long rowsT[2][CLUSTER ? 16 : 1][2 * NB];  // pushed rows (tagged re, im), by source CTA
+  __shared__ unsigned long long keyT[2][16];                                      // pushed keys, by source CTA
+  __shared__ __align__(16) float4 urow[2][NB / 2];  // the pivot row for broadcast reads (CLUSTER: [0]; else by step parity)
   __shared__ __align__(16) float4 pub[NB / 2];
-  __shared__ uint2 ckey[2][16], wkey[NW];
+  __shared__ uint2 wkey[2][NW];  // by step parity
+  __shared__ int s_failed;
   __shared__ int s_moved;  // rows that changed place (rank 0's counts for the cluster)
   float2* M = A + (size_t)blockIdx.y * strideA;
   int* piv = ipiv + (size_t)blockIdx.y * n;
@@ -373,51 +408,77 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
 #pragma unroll
     for (int c = 0; c < NB; ++c) a[c] = mine ? src[(size_t)c * lda] : make_float2(0.f, 0.f);
   }
-  auto publish_warp_key = [&]() {  // the warp's candidate for the current column
+  auto publish_warp_key = [&](int parity) {  // the warp's candidate for the current column
     const uint2 key = warp_max_key(mine && done_at < 0 ? pivot_key(abs1(a[0]), lg) : make_uint2(0u, 0u));
-    if (lane == 0) wkey[wid] = key;
+    if (lane == 0) wkey[parity][wid] = key;
   };
   auto copy_row = [&](float4* dst) {
 #pragma unroll
     for (int q = 0; q < NB / 2; ++q) dst[q] = make_float4(a[2 * q].x, a[2 * q].y, a[2 * q + 1].x, a[2 * q + 1].y);
   };
-  if (tid == 0) s_moved = 0;
-  publish_warp_key();
-  __syncthreads();
+  if (tid == 0) {
+    s_moved = 0;
+    s_failed = 0;
+  }
+  publish_warp_key(0);
+  if constexpr (CLUSTER) {  // no tag of an earlier use in the slots when the first push arrives
+    for (int i = tid; i < 2 * 16 * 2 * NB; i += kRegPanelThreads) (&rowsT[0][0][0])[i] = 0ull;
+    if (tid < 32) (&keyT[0][0])[tid] = 0ull;
+    cluster.sync();
+  } else {
+    __syncthreads();
+  }
 #pragma unroll 1
   for (int j = 0; j < NB; ++j) {
     const int s = j & 1;
+    const unsigned tag = (unsigned)(j + 1);
     // 1. this CTA's candidate, pushed by the warp that holds it
-    uint2 key = warp_max_key(lane < NW ? wkey[lane] : make_uint2(0u, 0u));
+    uint2 key = warp_max_key(lane < NW ? wkey[s][lane] : make_uint2(0u, 0u));
     const bool own = mine && done_at < 0 && key.y != 0u && lg == (int)~key.y;  // logical rows are distinct
     if constexpr (CLUSTER) {
       const bool owner_warp = __ballot_sync(0xffffffffu, own) != 0u;
+      // the key first: every CTA can decide while the rows are still on their way
+      if ((owner_warp || (key.y == 0u && wid == 0)) && lane < CL)  // without a candidate row, warp 0 says so
+        push_word(cluster.map_shared_rank(&keyT[s][rank], lane),
+                  ((unsigned long long)key.x << 32) | (tag << 16) | (key.y & 0xffffu));
       if (owner_warp) {
         if (own) copy_row(pub);
         __syncwarp();
-        const float4 v = pub[lane & 15];
-        for (int t = lane >> 4; t < CL; t += 2) *cluster.map_shared_rank(&rowsC[s][rank][lane & 15], t) = v;
+        const float2 v = reinterpret_cast<const float2*>(pub)[lane];
+        const unsigned long long wr = ((unsigned long long)tag << 32) | __float_as_uint(v.x);
+        const unsigned long long wi = ((unsigned long long)tag << 32) | __float_as_uint(v.y);
+#pragma unroll 4
+        for (int t = 0; t < CL; ++t) push_words(cluster.map_shared_rank(&rowsT[s][rank][2 * lane], t), wr, wi);
       }
-      if (owner_warp || (key.y == 0u && wid == 0)) {  // without a candidate row, warp 0 says so
-        if (lane < CL) *cluster.map_shared_rank(&ckey[s][rank], lane) = key;
-        asm volatile("fence.acq_rel.cluster;" ::: "memory");
-      }
-      // 2. the writes above were fenced by their writers; the wait acquires them
-      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     } else {
-      if (own) copy_row(rowsC[s][0]);
+      if (own) copy_row(urow[s]);
       __syncthreads();
     }
     // 3. pivot (logical row p, held by CTA pr), in every warp; row j itself is a candidate, so there is one
-    int pr = 0;
+    const float4* U = urow[CLUSTER ? 0 : s];  // the pivot row, u[c] = U(j, j + c) (zero beyond the panel)
+    int p = (int)~key.y;
     if constexpr (CLUSTER) {
-      const uint2 ck = lane < CL ? ckey[s][lane] : make_uint2(0u, 0u);
+      unsigned long long kw = 0ull;
+      bool ok = false;
+      for (int it = 0; it < kPollLimit && !ok; ++it) {
+        if (lane < CL) kw = poll_word(&keyT[s][lane]);
+        ok = __all_sync(0xffffffffu, lane >= CL || ((unsigned)kw >> 16) == tag);
+      }
+      const uint2 ck = lane < CL ? make_uint2((unsigned)(kw >> 32), (unsigned)kw & 0xffffu) : make_uint2(0u, 0u);
       key = warp_max_key(ck);
-      pr = __ffs(__ballot_sync(0xffffffffu, ck.x == key.x && ck.y == key.y)) - 1;  // keys are distinct
+      const int pr = __ffs(__ballot_sync(0xffffffffu, ck.x == key.x && ck.y == key.y)) - 1;  // keys are distinct
+      p = (int)(~key.y & 0xffffu);
+      ulonglong2 u = make_ulonglong2(0ull, 0ull);
+      bool got = false;
+      for (int it = 0; it < kPollLimit && ok && !got; ++it) {
+        u = poll_words(&rowsT[s][pr][2 * lane]);
+        got = __all_sync(0xffffffffu, (unsigned)(u.x >> 32) == tag && (unsigned)(u.y >> 32) == tag);
+      }
+      if (!got) s_failed = 1;
+      // every warp writes the same values; the barrier that ends the step keeps step j + 1's away
+      reinterpret_cast<float2*>(urow[0])[lane] = make_float2(__uint_as_float((unsigned)u.x), __uint_as_float((unsigned)u.y));
+      __syncwarp();
     }
-    const int p = (int)~key.y;
-    const float4* U = rowsC[s][pr];  // the pivot row, u[c] = U(j, j + c) (zero beyond the panel)
     if (rank == 0 && wid == 0 && lane < NB - j)  // U row j
       M[(size_t)(k + j + lane) * lda + k + j] = reinterpret_cast<const float2*>(U)[lane];
     if (rank == 0 && tid == 0) piv[k + j] = k + p;
@@ -426,8 +487,9 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
     if (d.x == 0.f && d.y == 0.f) {
       inv = make_float2(0.f, 0.f);
       if (rank == 0 && tid == 0 && info[blockIdx.y] == 0) info[blockIdx.y] = k + j + 1;
-    } else {
-      inv = inverse(d);
+    } else {  // one reciprocal instead of two divisions on the step's critical path
+      const float rm = __frcp_rn(fmaf(d.x, d.x, d.y * d.y));
+      inv = make_float2(d.x * rm, -d.y * rm);
     }
     // 4. this thread's row
     if (mine && done_at < 0) {
@@ -466,8 +528,12 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
           update(std::integral_constant<int, 8>{});
       }
     }
-    publish_warp_key();  // every thread read wkey in this step's 1, before the barrier of 2
+    publish_warp_key(s ^ 1);
     __syncthreads();
+    if (CLUSTER && s_failed) {  // uniform in the CTA; the other CTAs wait in vain in turn
+      if (tid == 0) info[blockIdx.y] = -1;
+      break;
+    }
   }
   // every row to its logical position: the multipliers left of its pivot column
   // (all 32 for rows that never became the pivot)
