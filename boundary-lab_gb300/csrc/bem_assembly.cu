@@ -475,9 +475,14 @@ __global__ void __launch_bounds__(WARPS * 32, RegularOccupancy<NFQ>::kCtasPerSm)
 // 1,280 triangles, 16 frequencies: 10.6 -> 5.5 ms per frequency; 3,984 triangles: 91 -> 48.  Two frequencies per
 // launch: four would need 224 KB of accumulators per CTA and spill.
 // ------------------------------------------------------------------------
+// A launch takes up to kRegGroups64 groups of NFQ (blockIdx.z): a small mesh's launches
+// would each end in a partly filled wave (1,280 triangles: 3.2 waves).
+constexpr int kRegGroups64 = 32;
 template <int NFQ> struct RegParamsF64BM {
-  double k[NFQ];
-  double2 cD[NFQ], cH[NFQ];  // with the 1 / (4 pi) of the Green's function
+  struct Group {
+    double k[NFQ];
+    double2 cD[NFQ], cH[NFQ];  // with the 1 / (4 pi) of the Green's function
+  } g[kRegGroups64];
   double cw[3 * kMaxQ], w[kMaxQ];
 };
 
@@ -485,8 +490,8 @@ template <int Q, int WARPS, int NFQ>
 __global__ void __launch_bounds__(WARPS * 32, 2)
     regular_f64_bm_kernel(const FaceF64* __restrict__ faces, int nf, const int* __restrict__ tile_group_ptr,
                           const LaneSlot* __restrict__ slots, const int* __restrict__ tile_row_base, int max_rows,
-                          double2* __restrict__ Rext, long long ldR, long long strideR, RegParamsF64BM<NFQ> p,
-                          int ntr, int4 trs, const unsigned char* __restrict__ fix_mask,
+                          double2* __restrict__ Rext, long long ldR, long long strideR,
+                          const __grid_constant__ RegParamsF64BM<NFQ> p, int ntr, int4 trs, const unsigned char* __restrict__ fix_mask,
                           const double2* __restrict__ trig) {
   extern __shared__ double2 smem_acc64[];
   __shared__ double2 tab[kSincosTable];
@@ -496,6 +501,11 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
   const int base = tile_row_base[tile];
   const int rows = tile_row_base[tile + 1] - base;
   double2* acc = smem_acc64 + (size_t)warp * NFQ * 3 * max_rows;  // [NFQ][3][max_rows]
+  const auto& G = p.g[blockIdx.z];
+  Rext += (size_t)blockIdx.z * NFQ * strideR;
+  double k[NFQ];
+#pragma unroll
+  for (int f = 0; f < NFQ; ++f) k[f] = G.k[f];
   for (int i = lane; i < NFQ * 3 * max_rows; i += 32) acc[i] = make_double2(0.0, 0.0);
   load_sincos_table(tab, trig);
   __syncthreads();
@@ -583,8 +593,8 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
 #pragma unroll
               for (int f = 0; f < NFQ; ++f) {
                 double sn, cs;
-                sincos_table(p.k[f] * r, tab, &sn, &cs);
-                const double ey = p.k[f] * tn;
+                sincos_table(k[f] * r, tab, &sn, &cs);
+                const double ey = k[f] * tn;
                 const double2 H = make_double2(fma(cs, ex, -sn * ey), fma(cs, ey, sn * ex));
 #pragma unroll
                 for (int b = 0; b < 3; ++b) {
@@ -614,8 +624,8 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
           double2 cDj[NFQ], Bc[NFQ];
 #pragma unroll
           for (int f = 0; f < NFQ; ++f) {
-            cDj[f] = cscale(p.cD[f], jac);
-            Bc[f] = cmul(cscale(p.cH[f], jac), S0[f]);
+            cDj[f] = cscale(G.cD[f], jac);
+            Bc[f] = cmul(cscale(G.cH[f], jac), S0[f]);
           }
 #pragma unroll
           for (int a = 0; a < 3; ++a) {
@@ -1622,6 +1632,173 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// The same expansion for the FP64 form: moments and contraction in FP64, with the terms at
+// which the coefficients reach rounding (cheb_terms with tolerance kChebTol64), so the sums
+// are those of the Duffy points to rounding.  Per point and chunk of four terms about 160
+// FP64 instructions, 640 for 16 terms: four frequencies point by point, once per mesh; a
+// frequency through the moments then costs a fortieth of one (1,280 triangles: 4.1 ->
+// 0.10 ms, the moments 17.5 ms once).  Per pair 21 sums per term: IR[9], IDh[9],
+// IKh[3] (SR[a] is the sum of IR[a][b] over b), stored [pair][term][kCheb64Sums].
+constexpr int kCheb64Sums = 21;
+
+__global__ void __launch_bounds__(128)
+    singular_cheb64_moments_kernel(SingularGeom geo, const SingularPair* __restrict__ pairs, int npairs,
+                                   const int* __restrict__ rule_ptr, const double* __restrict__ duffy,
+                                   double two_over_R, int nterms, double* __restrict__ cheb) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (warp >= npairs) return;
+  const SingularPair P = pairs[warp];
+  const int* ft = geo.faces + 3 * P.test;
+  const int* fr = geo.faces + 3 * P.trial;
+  double e1t[3], e2t[3], d0[3], e1r[3], e2r[3], nt[3], nr[3];
+  for (int d = 0; d < 3; ++d) {
+    const double sd = d == 0 ? tr_sign_x(P.tr) : d == 1 ? tr_sign_y(P.tr) : 1.0;  // image pairs: S p
+    const double t0 = geo.verts[3 * ft[0] + d];
+    const double r0 = sd * geo.verts[3 * fr[0] + d];
+    e1t[d] = geo.verts[3 * ft[1] + d] - t0;
+    e2t[d] = geo.verts[3 * ft[2] + d] - t0;
+    d0[d] = r0 - t0;
+    e1r[d] = sd * geo.verts[3 * fr[1] + d] - r0;
+    e2r[d] = sd * geo.verts[3 * fr[2] + d] - r0;
+    nt[d] = geo.normal[3 * P.test + d];
+    nr[d] = sd * geo.normal[3 * P.trial + d];
+  }
+  const double inv4pi = 0.25 / CUDART_PI;
+  const int q0 = rule_ptr[P.rule], q1 = rule_ptr[P.rule + 1];
+  constexpr int NCH = 4;
+  for (int n0 = 0; n0 < nterms; n0 += NCH) {
+    double v[NCH][kCheb64Sums];
+#pragma unroll
+    for (int j = 0; j < NCH; ++j)
+#pragma unroll
+      for (int i = 0; i < kCheb64Sums; ++i) v[j][i] = 0.0;
+    for (int q = q0 + lane; q < q1; q += 32) {
+      const double* pt = duffy + 5 * (size_t)q;
+      const double tu = pt[0], tv = pt[1], ru = pt[2], rvv = pt[3], w = pt[4];
+      double rv[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) rv[d] = (d0[d] + ru * e1r[d] + rvv * e2r[d]) - (tu * e1t[d] + tv * e2t[d]);
+      const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
+      if (r2 == 0.0) continue;
+      const double rinv = rsqrt_step(r2), r = r2 * rinv, s = rinv * inv4pi;
+      const double fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * s;   // (r . n_r) / (4 pi r)
+      const double fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * s;  // -(r . n_t) / (4 pi r)
+      const double x = fmin(1.0, fma(r, two_over_R, -1.0)), x2 = x + x;
+      // T_n(x) from n0 on by the three-term recurrence
+      double ta = 1.0, tb = x;  // T_n, T_(n+1)
+      for (int n = 0; n < n0; ++n) {
+        const double tc = fma(x2, tb, -ta);
+        ta = tb;
+        tb = tc;
+      }
+      const double wp[3] = {w * (1.0 - tu - tv), w * tu, w * tv}, py[3] = {1.0 - ru - rvv, ru, rvv};
+      double wab[9], wfy[9], wfx[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        wfx[a] = wp[a] * fx;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          wab[3 * a + b] = wp[a] * py[b];
+          wfy[3 * a + b] = wab[3 * a + b] * fy;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NCH; ++j) {
+        const double tg = ta * inv4pi;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+          v[j][i] = fma(wab[i], tg, v[j][i]);
+          v[j][9 + i] = fma(wfy[i], ta, v[j][9 + i]);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[j][18 + a] = fma(wfx[a], ta, v[j][18 + a]);
+        const double tc = fma(x2, tb, -ta);
+        ta = tb;
+        tb = tc;
+      }
+    }
+    // sums over the lanes; lane i keeps sum i of every term of the chunk
+    double* o = cheb + ((size_t)warp * kChebN + n0) * kCheb64Sums;
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) {
+      double mine = 0.0;
+#pragma unroll
+      for (int i = 0; i < kCheb64Sums; ++i) {
+        const double t = warp_sum(v[j][i]);
+        if (lane == i) mine = t;
+      }
+      if (lane < kCheb64Sums) o[j * kCheb64Sums + lane] = mine;
+    }
+  }
+}
+
+struct ChebParamsF64 {
+  double2 c1[kChebN], c2[kChebN];
+  SingParams<double> p;
+};
+
+// Lane i < 21 forms sum i from the pair's moments; the outputs as in singular_dyn_kernel.
+__global__ void __launch_bounds__(128)
+    singular_cheb64_kernel(const SingularPair* __restrict__ pairs, int npairs, const double* __restrict__ cheb,
+                           int nterms, const double* __restrict__ moments, const double* __restrict__ curls,
+                           const double* __restrict__ area, const double* __restrict__ m11m10,
+                           const __grid_constant__ ChebParamsF64 cp, double2* __restrict__ out) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (warp >= npairs) return;
+  const SingularPair P = pairs[warp];
+  double2 acc = make_double2(0.0, 0.0);
+  if (lane < kCheb64Sums) {
+    const double* M = cheb + (size_t)warp * kChebN * kCheb64Sums + lane;
+    const double2* c = lane < 9 ? cp.c1 : cp.c2;
+    for (int n = 0; n < nterms; ++n) {
+      const double m = M[(size_t)n * kCheb64Sums];
+      acc.x = fma(c[n].x, m, acc.x);
+      acc.y = fma(c[n].y, m, acc.y);
+    }
+    acc = cscale(acc, P.jac);
+  }
+  auto sum = [&](int i) {
+    return make_double2(__shfl_sync(0xffffffffu, acc.x, i), __shfl_sync(0xffffffffu, acc.y, i));
+  };
+  double2 SR[3], S0;
+  const double* M = moments + (size_t)kStatic * warp;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) SR[a] = cadd(cadd(sum(3 * a), sum(3 * a + 1)), sum(3 * a + 2));
+  const double2 IDh = make_double2(__shfl_sync(0xffffffffu, acc.x, (lane + 9) & 31),
+                                   __shfl_sync(0xffffffffu, acc.y, (lane + 9) & 31));  // lanes 0-8; IKh in lanes 9-11
+  if (lane >= 12) return;
+  S0 = make_double2(M[0] + M[1] + M[2], 0.0);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) S0 = cadd(S0, SR[a]);
+  const SingParams<double>& p = cp.p;
+  const bool coincident = P.kind == 1 && P.tr == 0;  // mass terms: the face with itself, never with an image
+  const double a2 = 2.0 * area[P.test];
+  double2* o = out + (size_t)kSingOut * warp;
+  if (lane < 9) {
+    const int a = lane / 3, b = lane - 3 * a;
+    const double* ct = curls + 9 * (size_t)P.test + 3 * a;
+    const double* cr = curls + 9 * (size_t)P.trial + 3 * b;
+    // image pairs: reflected curls det(S) S c
+    const double sx = tr_sign_x(P.tr), sy = tr_sign_y(P.tr), det = sx * sy;
+    const double cc = ct[0] * (det * sx * cr[0]) + ct[1] * (det * sy * cr[1]) + ct[2] * (det * cr[2]);
+    const double kk_nn = p.k2 * P.nprod;
+    const double2 D = make_double2(M[12 + lane] + IDh.x, IDh.y), IGt = make_double2(M[3 + lane] + acc.x, acc.y);
+    const double2 H = make_double2(cc * S0.x - kk_nn * IGt.x, cc * S0.y - kk_nn * IGt.y);
+    double2 L = cadd(cmul(p.cD, D), cmul(p.cH, H));
+    if (coincident) L = cadd(L, cscale(p.cM, a2 * m11m10[lane]));
+    o[lane] = L;
+  } else {
+    const int a = lane - 9;
+    const double2 sr = a == 0 ? SR[0] : a == 1 ? SR[1] : SR[2];
+    const double2 S = make_double2(M[a] + sr.x, sr.y), K = make_double2(M[21 + a] + IDh.x, IDh.y);
+    double2 rhs = cadd(cmul(p.cS, S), cmul(p.cK, K));
+    if (coincident) rhs = cadd(rhs, cscale(p.cM10, a2 * m11m10[9 + a]));
+    o[9 + a] = rhs;
+  }
+}
+
 // The singular blocks into the extended rows: one thread per distinct target
 // entry (planned once per mesh), adding that entry's contributions in pair order,
 // so the sums are those of one thread walking each trial face's pairs, without
@@ -2148,19 +2325,21 @@ cudaError_t launch_regular_f32(const DeviceMesh& m, const double* k, const doubl
 }
 
 template <int NFQ>
-cudaError_t launch_regular_f64_bm(const DeviceMesh& m, const double* k, const double2* cD, const double2* cH,
-                                  double2* Rext, long long ldR, long long strideR, cudaStream_t stream) {
+cudaError_t launch_regular_f64_bm(const DeviceMesh& m, int groups, const double* k, const double2* cD,
+                                  const double2* cH, double2* Rext, long long ldR, long long strideR,
+                                  cudaStream_t stream) {
   constexpr int W = 4;
   RegParamsF64BM<NFQ> p;
   const double inv4pi = 0.25 / 3.14159265358979323846;
-  for (int f = 0; f < NFQ; ++f) {
-    p.k[f] = k[f];
-    p.cD[f] = make_double2(cD[f].x * inv4pi, cD[f].y * inv4pi);
-    p.cH[f] = make_double2(cH[f].x * inv4pi, cH[f].y * inv4pi);
+  for (int f = 0; f < groups * NFQ; ++f) {
+    auto& g = p.g[f / NFQ];
+    g.k[f % NFQ] = k[f];
+    g.cD[f % NFQ] = make_double2(cD[f].x * inv4pi, cD[f].y * inv4pi);
+    g.cH[f % NFQ] = make_double2(cH[f].x * inv4pi, cH[f].y * inv4pi);
   }
   for (int i = 0; i < 3 * kMaxQ; ++i) p.cw[i] = m.rule_cw[i];
   for (int q = 0; q < kMaxQ; ++q) p.w[q] = m.rule_w[q];
-  const dim3 grid((m.nf + W - 1) / W, m.n_tiles);
+  const dim3 grid((m.nf + W - 1) / W, m.n_tiles, groups);
   const size_t sm = (size_t)W * NFQ * 3 * m.max_tile_rows * sizeof(double2);
   auto launch = [&](auto kern) {
     ensure_smem_limit((const void*)kern, sm);
@@ -2258,14 +2437,22 @@ cudaError_t launch_regular(const DeviceMesh& m, Precision prec, int nfreq, const
     const double qx = (cH[i].x * cD[i].x + cH[i].y * cD[i].y) / d, qy = (cH[i].y * cD[i].x - cH[i].x * cD[i].y) / d;
     return fabs(k[i] * qx) <= 4e-16 && fabs(k[i] * qy + 1.0) <= 4e-16;
   };
+  const int width = regular_width_f64(m);
   for (int f = 0; f < nfreq;) {
     double2* R = (double2*)Rext + (size_t)f * strideR;
-    const int w = !bm(f) ? 0 : std::min(regular_width_f64(m), f + 1 < nfreq && bm(f + 1) ? 2 : 1);
-    const cudaError_t e = w == 2   ? launch_regular_f64_bm<2>(m, k + f, cD + f, cH + f, R, ldR, strideR, stream)
-                          : w == 1 ? launch_regular_f64_bm<1>(m, k + f, cD + f, cH + f, R, ldR, strideR, stream)
-                                   : launch_regular_f64(m, k[f], cD[f], cH[f], R, ldR, stream);
+    int run = 0;  // consecutive frequencies of the operator
+    while (f + run < nfreq && bm(f + run)) ++run;
+    if (run == 0 || width == 0) {
+      const cudaError_t e = launch_regular_f64(m, k[f], cD[f], cH[f], R, ldR, stream);
+      if (e != cudaSuccess) return e;
+      ++f;
+      continue;
+    }
+    const int w = std::min(width, run), groups = std::min(run / w, kRegGroups64);
+    const cudaError_t e = w == 2 ? launch_regular_f64_bm<2>(m, groups, k + f, cD + f, cH + f, R, ldR, strideR, stream)
+                                 : launch_regular_f64_bm<1>(m, groups, k + f, cD + f, cH + f, R, ldR, strideR, stream);
     if (e != cudaSuccess) return e;
-    f += std::max(w, 1);
+    f += groups * w;
   }
   return cudaSuccess;
 }
@@ -2285,6 +2472,10 @@ double regular_flop_per_qpair(int w) {
 
 int regular_launches(const DeviceMesh& m, Precision prec, int nfreq) {
   int sizes[64];
+  if (prec == Precision::FP64) {  // the full groups in one launch, the remainder in another
+    const int w = regular_width_f64(m);
+    return w == 0 ? nfreq : (nfreq >= w ? (nfreq / w + kRegGroups64 - 1) / kRegGroups64 : 0) + (nfreq % w ? 1 : 0);
+  }
   return regular_groups(m, prec, nfreq, sizes);
 }
 
@@ -2336,13 +2527,25 @@ namespace {
 // z^(n-2) / n!), which has no cancellation.  Returns false when the last two coefficients
 // of either are above 1e-9 of its largest: the expansion has not converged (kR too large
 // for N terms) and the caller integrates point by point instead.
-bool cheb_coefficients(double k, double R, int N, double2* c1, double2* c2) {
+// The FP64 form asks for the rounding level and takes the Taylor series to z = 2: the
+// direct forms lose 1 / z^2 of their accuracy there.
+constexpr double kChebTol = 1e-9, kChebTol64 = 5e-16;
+bool cheb_coefficients(double k, double R, int N, double2* c1, double2* c2, double tol) {
+  const double taylor = tol < 1e-12 ? 2.0 : 0.5;
   typedef std::complex<double> cd;
   cd f1[kChebN], g2[kChebN];
   const double pi = 3.14159265358979323846;
+  // cos(pi m / 2N) for m = 0 .. 2N from arguments below pi / 4, the others by symmetry: the
+  // rounding of an argument of up to 24 pi would put 3e-15 into the last coefficients and
+  // hide that they have converged
+  double cosines[2 * kChebN + 1];
+  for (int m = 0; m <= N; ++m) {
+    cosines[m] = 2 * m <= N ? std::cos(pi * m / (2 * N)) : std::sin(pi * (N - m) / (2 * N));
+    cosines[2 * N - m] = -cosines[m];
+  }
   for (int j = 0; j < N; ++j) {
-    const double x = std::cos(pi * (j + 0.5) / N), r = 0.5 * R * (1.0 + x), z = k * r;
-    if (z < 0.5) {
+    const double x = cosines[2 * j + 1], r = 0.5 * R * (1.0 + x), z = k * r;
+    if (z < taylor) {
       cd s1(0.0, 0.0), s2(0.0, 0.0), ipow(0.0, 1.0);  // ipow = i^n, from n = 1
       double zp1 = 1.0, zp2 = 0.0, fact = 1.0;        // z^(n-1), z^(n-2), n!
       for (int n = 1; n <= 30; ++n) {
@@ -2367,7 +2570,8 @@ bool cheb_coefficients(double k, double R, int N, double2* c1, double2* c2) {
   for (int n = 0; n < N; ++n) {
     cd s1(0.0, 0.0), s2(0.0, 0.0);
     for (int j = 0; j < N; ++j) {
-      const double t = std::cos(pi * n * (j + 0.5) / N);
+      const int m = (2 * j + 1) * n % (4 * N);
+      const double t = cosines[m > 2 * N ? 4 * N - m : m];
       s1 += f1[j] * t;
       s2 += g2[j] * t;
     }
@@ -2380,16 +2584,31 @@ bool cheb_coefficients(double k, double R, int N, double2* c1, double2* c2) {
     c2[n] = make_double2(a2[n].real(), a2[n].imag());
   }
   const double t1 = std::abs(a1[N - 1]) + std::abs(a1[N - 2]), t2 = std::abs(a2[N - 1]) + std::abs(a2[N - 2]);
-  return t1 <= 1e-9 * m1 && t2 <= 1e-9 * m2;
+  return t1 <= tol * m1 && t2 <= tol * m2;
 }
 }  // namespace
 
-int cheb_terms(double k, double R) {
+int cheb_terms(Precision prec, double k, double R) {
   if (!(R > 0.0)) return 0;
   double2 c1[kChebN], c2[kChebN];
   for (int n = 8; n <= kChebN; n += 4)
-    if (cheb_coefficients(k, R, n, c1, c2)) return n;
+    if (cheb_coefficients(k, R, n, c1, c2, prec == Precision::Mixed ? kChebTol : kChebTol64)) return n;
   return 0;
+}
+
+size_t cheb_moment_bytes(Precision prec, int npairs) {
+  return (size_t)npairs * kChebN * (prec == Precision::Mixed ? 24 * sizeof(float) : kCheb64Sums * sizeof(double));
+}
+
+cudaError_t launch_cheb64_moments(const DeviceMesh& m, int nterms, cudaStream_t stream) {
+  if (m.npairs == 0 || !m.cheb64 || nterms < 4 || nterms > kChebN || nterms % 4 || !(m.cheb_R > 0.0))
+    return cudaErrorInvalidValue;
+  SingularGeom geo{m.verts, m.faces, m.normal};
+  const int threads = 128;
+  const int blocks = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
+  singular_cheb64_moments_kernel<<<blocks, threads, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
+                                                                 2.0 / m.cheb_R, nterms, m.cheb64);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_cheb_moments(const DeviceMesh& m, int nterms, cudaStream_t stream) {
@@ -2458,9 +2677,9 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
     std::vector<int> good, bad, terms(nfreq, 0);
     for (int f = 0; f < nfreq; ++f) {
       if (use_cheb && m.cheb != nullptr && m.cheb_n > 0 && m.cheb_R > 0.0) {
-        const int nt = cheb_terms(k[f], m.cheb_R);
+        const int nt = cheb_terms(prec, k[f], m.cheb_R);
         if (nt > 0 && nt <= m.cheb_n &&
-            cheb_coefficients(k[f], m.cheb_R, nt, &c1[(size_t)f * kChebN], &c2[(size_t)f * kChebN]))
+            cheb_coefficients(k[f], m.cheb_R, nt, &c1[(size_t)f * kChebN], &c2[(size_t)f * kChebN], kChebTol))
           terms[f] = nt;
       }
       (terms[f] > 0 ? good : bad).push_back(f);
@@ -2519,6 +2738,18 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
     p.cS = c[f].cS;
     p.cK = c[f].cK;
     p.cM10 = c[f].cM10;
+    // through the mesh's Chebyshev moments where they hold the terms the frequency needs
+    const int nt = use_cheb && m.cheb64 != nullptr && m.cheb64_n > 0 ? cheb_terms(prec, k[f], m.cheb_R) : 0;
+    if (nt > 0 && nt <= m.cheb64_n) {
+      ChebParamsF64 cp{};
+      cheb_coefficients(k[f], m.cheb_R, nt, cp.c1, cp.c2, kChebTol64);
+      cp.p = p;
+      singular_cheb64_kernel<<<(m.npairs + 3) / 4, 128, 0, stream>>>(m.pairs, m.npairs, m.cheb64, nt, m.moments,
+                                                                     m.curls, m.area, m.m11m10, cp,
+                                                                     (double2*)blocks + (size_t)f * blocks_stride);
+      if (cheb_freqs) ++*cheb_freqs;
+      continue;
+    }
     singular_dyn_kernel<<<nblk, threads, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
                                                               m.moments, m.curls, m.area, m.m11m10, p, m.trig,
                                                               (double2*)blocks + (size_t)f * blocks_stride);

@@ -279,7 +279,7 @@ Layout layout_for(const bem::DeviceMesh& dm, bem::Precision prec) {
   return L;
 }
 
-// Frequencies a mixed-form call needs before its singular remainders go through the mesh's
+// Frequencies a call needs before its singular remainders go through the mesh's
 // Chebyshev moments: forming them costs about as much as six frequencies of the point-by-
 // point singular kernel at 16 terms (more at more terms, at most 24), and each frequency
 // through them costs a fifteenth of one.  A shorter call runs point by point even when the
@@ -290,15 +290,18 @@ constexpr int kChebMinFreqs = 12;
 // wavenumbers k[0..n): with the fewest terms (a multiple of four) that cover every
 // frequency whose expansion converges within kChebN terms, or twice the terms the moments
 // had, up to kChebN.  Nothing when no frequency converges (those run point by point).
-void ensure_cheb(bem_context* ctx, bem_mesh* m, const double* k, int n) {
+void ensure_cheb(bem_context* ctx, bem_mesh* m, bem::Precision prec, const double* k, int n) {
   bem::DeviceMesh& d = m->dm;
   if (d.npairs == 0 || !(d.cheb_R > 0.0)) return;
+  const bool mixed = prec == bem::Precision::Mixed;
+  int& have = mixed ? d.cheb_n : d.cheb64_n;
   int need = 0;
-  for (int i = 0; i < n; ++i) need = std::max(need, bem::cheb_terms(k[i], d.cheb_R));
-  if (need == 0 || d.cheb_n >= need) return;
-  const int nterms = std::min(bem::kChebN, std::max(need, 2 * d.cheb_n));
-  if (!d.cheb)
-    d.cheb = (float*)mesh_alloc(m, (size_t)d.npairs * bem::kChebN * 24 * sizeof(float), "allocate Chebyshev moments");
+  for (int i = 0; i < n; ++i) need = std::max(need, bem::cheb_terms(prec, k[i], d.cheb_R));
+  if (need == 0 || have >= need) return;
+  const int nterms = std::min(bem::kChebN, std::max(need, 2 * have));
+  const size_t bytes = bem::cheb_moment_bytes(prec, d.npairs);
+  if (mixed && !d.cheb) d.cheb = (float*)mesh_alloc(m, bytes, "allocate Chebyshev moments");
+  if (!mixed && !d.cheb64) d.cheb64 = (double*)mesh_alloc(m, bytes, "allocate Chebyshev moments");
   // the side stream must see the allocation (made on the context's stream), the pair
   // records (written on the side stream) are in order there, and no singular kernel of an
   // earlier sweep may still read the moments being rewritten
@@ -312,10 +315,11 @@ void ensure_cheb(bem_context* ctx, bem_mesh* m, const double* k, int n) {
     ck(cudaStreamWaitEvent(ctx->side, ev, 0), "wait for an earlier stream");
     cudaEventDestroy(ev);
   }
-  ck(bem::launch_cheb_moments(d, nterms, ctx->side), "Chebyshev moments kernel");
+  ck(mixed ? bem::launch_cheb_moments(d, nterms, ctx->side) : bem::launch_cheb64_moments(d, nterms, ctx->side),
+     "Chebyshev moments kernel");
   if (!m->cheb_ready) ck(cudaEventCreateWithFlags(&m->cheb_ready, cudaEventDisableTiming), "create event");
   ck(cudaEventRecord(m->cheb_ready, ctx->side), "record event");
-  d.cheb_n = nterms;
+  have = nterms;
 }
 
 // Extended rows held at once: as many frequencies as fit 1 GiB, and at least those that share
@@ -414,7 +418,7 @@ long long assemble_frequencies(bem_context* ctx, bem_mesh* m, bem::Precision pre
 void assemble_one(bem_mesh* m, bem::Precision prec, double k, const bem::OperatorCoeffs& c, void* A, void* A2,
                   double2 qscale, int nc, const void* drive, void* b) {
   const bool cheb = prec == bem::Precision::Mixed;
-  if (cheb) ensure_cheb(m->ctx, m, &k, 1);
+  if (cheb) ensure_cheb(m->ctx, m, prec, &k, 1);
   assemble_frequencies(m->ctx, m, prec, 1, &k, &c, A, A2, &qscale, nc, drive, b, m->dm.nv, 0, 0, nullptr, nullptr,
                        cheb);
 }
@@ -1160,7 +1164,7 @@ long long bem_estimate_device_bytes(int nv, int nf, int npairs, int nrhs, int np
   bytes += (long long)nf * 3 * nrhs * esz * group;                          // right-hand-side face values
   bytes += (long long)batch * lda * nv * esz * (precision == BEM_PRECISION_MIXED ? 2 : 1);  // matrices (+copy)
   bytes += (long long)npairs * (12 * esz * group + 24 * 8 + 48 + (bem::kPairRec + bem::kPairGeoDf) * 4 + 96 +
-                                bem::kChebN * 24 * 4);  // singular blocks, moments, pairs, records, scatter plan, Chebyshev moments
+                                (long long)bem::cheb_moment_bytes(precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64, 1));  // singular blocks, moments, pairs, records, scatter plan, Chebyshev moments
   bytes += (long long)batch * nrhs * lda * (esz + (2 + bem::kResidualSplits) * 16 + 16);  // rhs, x, residual parts, d
   if (precision == BEM_PRECISION_MIXED) bytes += (long long)bem::lu_inverse_bytes(nv, batch);  // block inverses
   bytes += (long long)batch * nrhs * ((long long)nf * 6 * esz + (long long)npts * 16);  // field sources + out
@@ -1184,11 +1188,11 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
     if (field_out && m->nobs < 1) return fail(ctx, BEM_ERR_INVALID_ARGUMENT, "no observation points set");
     if (!valid_options(ctx, o)) return BEM_ERR_INVALID_ARGUMENT;
     const bem::Precision prec = o.precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64;
-    const bool cheb = prec == bem::Precision::Mixed && n_freq >= kChebMinFreqs;
+    const bool cheb = n_freq >= kChebMinFreqs;
     if (cheb) {
       std::vector<double> kw(n_freq);
       for (int i = 0; i < n_freq; ++i) kw[i] = 2.0 * M_PI * freqs_hz[i] / o.sound_speed;
-      ensure_cheb(ctx, m, kw.data(), n_freq);
+      ensure_cheb(ctx, m, prec, kw.data(), n_freq);
     }
     const bem::DeviceMesh& dm = m->dm;
     const int nv = dm.nv, nc = m->nc;

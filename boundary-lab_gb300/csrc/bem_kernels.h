@@ -69,6 +69,8 @@ struct DeviceMesh {
   float* cheb = nullptr;
   double cheb_R = 0.0;
   int cheb_n = 0;  // terms the moments hold (0: none yet)
+  double* cheb64 = nullptr;  // the same of the FP64 form (kChebN x 21 doubles per pair)
+  int cheb64_n = 0;
   double* verts = nullptr;
   int* faces = nullptr;
   double* normal = nullptr;
@@ -114,7 +116,7 @@ constexpr int kPairGeoDf = 48;
 cudaError_t launch_singular_static(const DeviceMesh& m, double* moments, float* pairrec, cudaStream_t stream);
 // Singular blocks of nfreq frequencies; frequency f's blocks start at element
 // f * blocks_stride of blocks (the mixed form takes two frequencies per launch).
-// use_cheb (mixed form): take the mesh's Chebyshev moments for the frequencies whose
+// use_cheb: take the mesh's Chebyshev moments for the frequencies whose
 // expansion they cover.  Adds the kernels it launched to *launched and the frequencies it
 // formed from the moments to *cheb_freqs (when not null).
 cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, const double* k,
@@ -122,10 +124,13 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
                                 long long* launched = nullptr, long long* cheb_freqs = nullptr,
                                 bool use_cheb = false);
 // Chebyshev terms (a multiple of four, 8..kChebN) that expand the singular remainder of
-// wavenumber k on [0, R] to 1e-9; 0 when kChebN terms are not enough.
-int cheb_terms(double k, double R);
-// The mesh's Chebyshev moments for the first nterms terms into m.cheb (after the pair setup).
+// wavenumber k on [0, R] to 1e-9 (mixed) or to rounding (FP64); 0 when kChebN are not enough.
+int cheb_terms(Precision prec, double k, double R);
+size_t cheb_moment_bytes(Precision prec, int npairs);
+// The mesh's Chebyshev moments for the first nterms terms into m.cheb (after the pair setup),
+// or of the FP64 form into m.cheb64.
 cudaError_t launch_cheb_moments(const DeviceMesh& m, int nterms, cudaStream_t stream);
+cudaError_t launch_cheb64_moments(const DeviceMesh& m, int nterms, cudaStream_t stream);
 // The three below take nfreq frequencies per launch: frequency f's blocks, extended rows,
 // matrices and right-hand sides start f strides (in elements) after the first's.
 cudaError_t launch_singular_scatter(const DeviceMesh& m, Precision prec, int nfreq, const void* blocks,

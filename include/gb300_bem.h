@@ -156,8 +156,8 @@ typedef struct bem_solve_stats {
   double regular_flop;    /* mixed form: FP32 flop (FMA = 2) the regular-pair kernel executed in the call,
                              counted from its source per quadrature pair and frequency: 35.67 + 26.83 / w,
                              w = frequencies sharing one launch's frequency-independent geometry */
-  long long singular_cheb_freqs; /* mixed form: frequencies whose singular remainder was formed from the
-                                    mesh's Chebyshev moments (calls of at least 12 frequencies, where the
+  long long singular_cheb_freqs; /* frequencies whose singular remainder was formed from the mesh's
+                                    Chebyshev moments (calls of at least 12 frequencies, where the
                                     expansion converges); the rest point by point on the Duffy rules */
 } bem_solve_stats;
 
