@@ -207,6 +207,69 @@ __global__ void lu_trsm_kernel(C2* A, long long lda, long long strideA, int n, i
   }
 }
 
+// The FP64 form's U rows of a full panel: X = L11^{-1} X for 32 columns per CTA.  Each
+// quarter of an SM has half an FP64 lane per clock, so one instruction of one warp takes 64
+// cycles and four warps of a CTA work at once: warp w keeps rows w, w + 4, .. of its 32
+// columns in registers (lane = column), the rows' new values go through shared memory, one
+// barrier per row.  A thread per column left three quarters of each SM idle and waited for
+// its shared-memory stores (the compiler cannot tell L from X).
+// Two matrices of order 1,994, 32 rows: 157 -> 23 us (64 rows took 500).  With the panels
+// of 32 the factorisation of both takes 56.4 ms where it took 81.5 (35 are the products at
+// the FP64 pipe's rate); 16 of order 642: 24.6 -> 16.4 ms.  One level of 32-deep products is
+// faster than two levels of 64, 128 or 256 (65.1 against 68.7, 70.5 and 71.2 ms before the
+// triangular solve's change): cuBLAS loses more on the skinny shapes inside an outer block.
+template <int KB>
+__global__ void __launch_bounds__(128) lu_trsm64_kernel(double2* A, long long lda, long long strideA, int k,
+                                                        int c_begin, int c_end) {
+  extern __shared__ unsigned char smem_raw[];
+  double2* L = reinterpret_cast<double2*>(smem_raw);  // KB x KB, column-major
+  double2* X = L + KB * KB;                           // KB x 33
+  constexpr int ldx = 33, RW = KB / 4;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double2* M = A + (size_t)blockIdx.y * strideA;
+  const int c0 = c_begin + blockIdx.x * 32;
+  const int ncol = min(32, c_end - c0);
+#pragma unroll 8
+  for (int c = wid; c < KB; c += 4)
+#pragma unroll
+    for (int r = lane; r < KB; r += 32) L[c * KB + r] = M[(size_t)(k + c) * lda + k + r];
+#pragma unroll 8
+  for (int c = wid; c < 32; c += 4)
+#pragma unroll
+    for (int r = lane; r < KB; r += 32)
+      X[r * ldx + c] = c < ncol ? M[(size_t)(c0 + c) * lda + k + r] : make_double2(0., 0.);
+  __syncthreads();
+  double2 v[RW];
+#pragma unroll
+  for (int q = 0; q < RW; ++q) v[q] = X[(4 * q + wid) * ldx + lane];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < KB; ++j) {
+    if (wid == (j & 3)) X[j * ldx + lane] = v[j >> 2];
+    __syncthreads();
+    const double2 xj = X[j * ldx + lane];
+#pragma unroll
+    for (int q = j >> 2; q < RW; ++q) {
+      if (q == (j >> 2) && wid <= (j & 3)) continue;
+      const double2 l = L[j * KB + 4 * q + wid];
+      v[q].x = fma(-l.x, xj.x, fma(l.y, xj.y, v[q].x));
+      v[q].y = fma(-l.x, xj.y, fma(-l.y, xj.x, v[q].y));
+    }
+  }
+  for (int c = wid; c < ncol; c += 4)
+#pragma unroll
+    for (int r = lane; r < KB; r += 32) M[(size_t)(c0 + c) * lda + k + r] = X[r * ldx + c];
+}
+
+template <int KB>
+cudaError_t trsm64(double2* A, long long lda, long long strideA, int k, int c0, int c1, int batch, cudaStream_t stream) {
+  constexpr size_t sm = (size_t)KB * (KB + 33) * sizeof(double2);
+  if (sm > 32 * 1024) ensure_smem_limit((const void*)lu_trsm64_kernel<KB>, sm);
+  dim3 g((unsigned)((c1 - c0 + 31) / 32), batch);
+  lu_trsm64_kernel<KB><<<g, 128, sm, stream>>>(A, lda, strideA, k, c0, c1);
+  return cudaGetLastError();
+}
+
 // The three steps around the 32-wide panels of the two-level LU (mixed form).  A panel of
 // one matrix takes some tens of microseconds on at most 16 SMs, so what follows it has to
 // be short as well; these kernels do the outer block's own part in plain FP32 FMAs, which
@@ -819,8 +882,14 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
             (cuComplex*)(base + (k + kb) + (size_t)(k + kb) * lda), (int)lda, strideA, batch);
         if (st != CUBLAS_STATUS_SUCCESS) return cudaErrorUnknown;
       } else {
-        if (sm > 48 * 1024) ensure_smem_limit((const void*)lu_trsm_kernel<double2>, sm);
-        lu_trsm_kernel<double2><<<g, tpb, sm, stream>>>((double2*)A, lda, strideA, n, k, kb, k + kb, n);
+        if (kb == 32 || kb == 64) {
+          const cudaError_t e = kb == 32 ? trsm64<32>((double2*)A, lda, strideA, k, k + kb, n, batch, stream)
+                                         : trsm64<64>((double2*)A, lda, strideA, k, k + kb, n, batch, stream);
+          if (e != cudaSuccess) return e;
+        } else {
+          if (sm > 48 * 1024) ensure_smem_limit((const void*)lu_trsm_kernel<double2>, sm);
+          lu_trsm_kernel<double2><<<g, tpb, sm, stream>>>((double2*)A, lda, strideA, n, k, kb, k + kb, n);
+        }
         const cuDoubleComplex alpha = make_cuDoubleComplex(-1.0, 0.0), beta = make_cuDoubleComplex(1.0, 0.0);
         double2* base = (double2*)A;
         cublasStatus_t st = cublasZgemmStridedBatched(

@@ -556,6 +556,206 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
   if (rowmap != nullptr && rank == 0 && tid == 0) rowmap[(size_t)blockIdx.y * kRowmapStride] = s_moved;
 }
 
+// The register-resident panel of the FP64 form: the algorithm of lu_panel_reg_kernel with
+// the row's 32 complex doubles in 128 registers (256 threads), always on a cluster.  What
+// differs:
+//  - pivot keys are three words, (hi, lo) of |re| + |im| plus one in hi, and the complement
+//    of the logical row: the same first maximum, exactly;
+//  - the pivot's reciprocal is formed by the owner's thread and pushed behind the row: with
+//    two FP64 lanes per SM an instruction of one warp takes 16 cycles of the pipe, so the
+//    two divisions in every warp would cost more than the rest of the step's overhead;
+//  - the cluster is as wide as the batch leaves room for (choose_panel): the row update is
+//    bound by the FP64 pipe, 2 lanes per SM and clock, not by latency alone.
+// Two matrices of order 1,994: 64 columns in two panels of 156 us on 2 x 16 SMs, where the
+// shared-memory panel of 64 took 775 us.  Of a step's 4.9 us the row update is 2.4 us (one
+// warp per quarter of an SM), exchange and reciprocal the rest.
+constexpr int kReg64Threads = 256;
+constexpr int kReg64Warps = kReg64Threads / 32;
+
+__device__ __forceinline__ uint3 pivot_key64(double v, int row) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  return v == v ? make_uint3(hi + 1u, lo, (unsigned)~row) : make_uint3(0u, 0u, (unsigned)~row);
+}
+__device__ __forceinline__ uint3 warp_max_key(uint3 k) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, k.x);
+  const unsigned lo = __reduce_max_sync(0xffffffffu, k.x == hi ? k.y : 0u);
+  return make_uint3(hi, lo, __reduce_max_sync(0xffffffffu, k.x == hi && k.y == lo ? k.z : 0u));
+}
+__device__ __forceinline__ unsigned long long tagged(unsigned tag, int word) {
+  return ((unsigned long long)tag << 32) | (unsigned)word;
+}
+__device__ __forceinline__ double untagged(ulonglong2 w) { return __hiloint2double((int)(unsigned)w.x, (int)(unsigned)w.y); }
+
+__global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double2* A, long long lda, long long strideA,
+                                                                          int n, int k, int kb, int chunk, int* ipiv,
+                                                                          int* info, int* rowmap) {
+  constexpr int NB = 32;
+  constexpr int NW = kReg64Warps;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), CL = (int)cluster.num_blocks();
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* Lb = reinterpret_cast<double2*>(smem_raw);  // [NB][kReg64Threads] multipliers by column, thread
+  // pushed rows by source CTA, (hi, lo) of re and im per column, then the reciprocal
+  __shared__ __align__(16) unsigned long long rowsT[2][16][4 * (NB + 1)];
+  __shared__ __align__(16) unsigned long long keyT[2][16][2];  // pushed keys, by source CTA
+  __shared__ __align__(16) double2 pub[NB + 1];                // the candidate row and its reciprocal
+  __shared__ __align__(16) double2 urow[NB + 1];               // the pivot row and its reciprocal
+  __shared__ uint3 wkey[2][NW];                                // by step parity
+  __shared__ int s_failed;
+  __shared__ int s_moved;  // rows that changed place (rank 0's counts for the cluster)
+  double2* M = A + (size_t)blockIdx.y * strideA;
+  int* piv = ipiv + (size_t)blockIdx.y * n;
+  const int m = n - k;
+  const int r0 = rank * chunk;
+  const int rows = max(0, min(chunk, m - r0));
+  const bool mine = tid < rows;
+  int lg = r0 + tid;  // logical row of this thread's physical row
+  int done_at = -1;   // step at which this row became the pivot row
+  double2 a[NB];
+  {
+    const double2* src = M + (size_t)k * lda + k + r0 + tid;
+#pragma unroll
+    for (int c = 0; c < NB; ++c) a[c] = mine ? src[(size_t)c * lda] : make_double2(0., 0.);
+  }
+  auto publish_warp_key = [&](int parity) {  // the warp's candidate for the current column
+    const uint3 key = warp_max_key(mine && done_at < 0 ? pivot_key64(abs1(a[0]), lg) : make_uint3(0u, 0u, 0u));
+    if (lane == 0) wkey[parity][wid] = key;
+  };
+  if (tid == 0) {
+    s_moved = 0;
+    s_failed = 0;
+  }
+  publish_warp_key(0);
+  // no tag of an earlier use in the slots when the first push arrives
+  for (int i = tid; i < 2 * 16 * 4 * (NB + 1); i += kReg64Threads) (&rowsT[0][0][0])[i] = 0ull;
+  if (tid < 64) (&keyT[0][0][0])[tid] = 0ull;
+  cluster.sync();
+#pragma unroll 1
+  for (int j = 0; j < NB; ++j) {
+    const int s = j & 1;
+    const unsigned tag = (unsigned)(j + 1);
+    // 1. this CTA's candidate, pushed by the warp that holds it, the key first
+    uint3 key = warp_max_key(lane < NW ? wkey[s][lane] : make_uint3(0u, 0u, 0u));
+    const bool own = mine && done_at < 0 && key.z != 0u && lg == (int)~key.z;  // logical rows are distinct
+    const bool owner_warp = __ballot_sync(0xffffffffu, own) != 0u;
+    if ((owner_warp || (key.z == 0u && wid == 0)) && lane < CL)  // without a candidate row, warp 0 says so
+      push_words(cluster.map_shared_rank(&keyT[s][rank][0], lane),
+                 ((unsigned long long)key.x << 32) | (tag << 16) | (key.z & 0xffffu),
+                 ((unsigned long long)key.y << 32) | tag);
+    if (owner_warp) {
+      if (own) {
+#pragma unroll
+        for (int q = 0; q < NB; ++q) pub[q] = a[q];
+        if (a[0].x == 0. && a[0].y == 0.) {
+          pub[NB] = make_double2(0., 0.);
+        } else {  // one reciprocal instead of two divisions on the step's critical path
+          const double rm = __drcp_rn(fma(a[0].x, a[0].x, a[0].y * a[0].y));
+          pub[NB] = make_double2(a[0].x * rm, -a[0].y * rm);
+        }
+      }
+      __syncwarp();
+      for (int c = lane; c < NB + 1; c += 32) {
+        const double2 v = pub[c];
+        const unsigned long long w0 = tagged(tag, __double2hiint(v.x)), w1 = tagged(tag, __double2loint(v.x));
+        const unsigned long long w2 = tagged(tag, __double2hiint(v.y)), w3 = tagged(tag, __double2loint(v.y));
+#pragma unroll 4
+        for (int t = 0; t < CL; ++t) {
+          unsigned long long* dst = cluster.map_shared_rank(&rowsT[s][rank][4 * c], t);
+          push_words(dst, w0, w1);
+          push_words(dst + 2, w2, w3);
+        }
+      }
+    }
+    // 2. pivot (logical row p, held by CTA pr), in every warp; row j itself is a candidate, so there is one
+    ulonglong2 kw = make_ulonglong2(0ull, 0ull);
+    bool ok = false;
+    for (int it = 0; it < kPollLimit && !ok; ++it) {
+      if (lane < CL) kw = poll_words(&keyT[s][lane][0]);
+      ok = __all_sync(0xffffffffu, lane >= CL || (((unsigned)kw.x >> 16) == tag && (unsigned)kw.y == tag));
+    }
+    const uint3 ck = lane < CL ? make_uint3((unsigned)(kw.x >> 32), (unsigned)(kw.y >> 32), (unsigned)kw.x & 0xffffu)
+                               : make_uint3(0u, 0u, 0u);
+    key = warp_max_key(ck);
+    const int pr = __ffs(__ballot_sync(0xffffffffu, ck.x == key.x && ck.y == key.y && ck.z == key.z)) - 1;  // distinct
+    const int p = (int)(~key.z & 0xffffu);
+    bool got = false;
+    for (int it = 0; it < kPollLimit && ok && !got; ++it) {
+      const unsigned long long* src = rowsT[s][pr];
+      const ulonglong2 re = poll_words(src + 4 * lane), im = poll_words(src + 4 * lane + 2);
+      const ulonglong2 ire = poll_words(src + 4 * NB), iim = poll_words(src + 4 * NB + 2);
+      auto here = [&](ulonglong2 w) { return (unsigned)(w.x >> 32) == tag && (unsigned)(w.y >> 32) == tag; };
+      got = __all_sync(0xffffffffu, here(re) && here(im) && here(ire) && here(iim));
+      // every warp writes the same values; the barrier that ends the step keeps step j + 1's away
+      if (got) {
+        urow[lane] = make_double2(untagged(re), untagged(im));
+        if (lane == 0) urow[NB] = make_double2(untagged(ire), untagged(iim));
+      }
+    }
+    if (!got) s_failed = 1;
+    __syncwarp();
+    if (rank == 0 && wid == 0 && lane < NB - j) M[(size_t)(k + j + lane) * lda + k + j] = urow[lane];  // U row j
+    if (rank == 0 && tid == 0) {
+      piv[k + j] = k + p;
+      if (urow[0].x == 0. && urow[0].y == 0. && info[blockIdx.y] == 0) info[blockIdx.y] = k + j + 1;
+    }
+    // 3. this thread's row
+    if (mine && done_at < 0) {
+      if (lg == p) {  // the pivot row: it is logical row j now, finished
+        lg = j;
+        done_at = j;
+      } else {
+        if (lg == j) lg = p;  // the old row j moves to the pivot's place
+        const double2 l = cmul(a[0], urow[NB]);
+        Lb[(size_t)j * kReg64Threads + tid] = l;
+        // a[c - 1] = a[c] - l u[c] for columns j + 1.., over the smallest multiple of 4 that
+        // covers the 32 - j live columns (the columns beyond are zero)
+        auto update = [&](auto width) {
+          constexpr int W = decltype(width)::value;
+#pragma unroll
+          for (int c = 1; c < W; ++c) {
+            const double2 u = urow[c];
+            a[c - 1].x = fma(-l.x, u.x, fma(l.y, u.y, a[c].x));
+            a[c - 1].y = fma(-l.x, u.y, fma(-l.y, u.x, a[c].y));
+          }
+          a[W - 1] = make_double2(0., 0.);
+        };
+        switch (j >> 2) {
+          case 0: update(std::integral_constant<int, 32>{}); break;
+          case 1: update(std::integral_constant<int, 28>{}); break;
+          case 2: update(std::integral_constant<int, 24>{}); break;
+          case 3: update(std::integral_constant<int, 20>{}); break;
+          case 4: update(std::integral_constant<int, 16>{}); break;
+          case 5: update(std::integral_constant<int, 12>{}); break;
+          case 6: update(std::integral_constant<int, 8>{}); break;
+          default: update(std::integral_constant<int, 4>{}); break;
+        }
+      }
+    }
+    publish_warp_key(s ^ 1);
+    __syncthreads();
+    if (s_failed) {  // uniform in the CTA; the other CTAs wait in vain in turn
+      if (tid == 0) info[blockIdx.y] = -1;
+      break;
+    }
+  }
+  // every row to its logical position: the multipliers left of its pivot column
+  // (all 32 for rows that never became the pivot)
+  if (mine) {
+    const int ncol = done_at < 0 ? NB : done_at;
+    double2* dst = M + (size_t)k * lda + k + lg;
+    for (int c = 0; c < ncol; ++c) dst[(size_t)c * lda] = Lb[(size_t)c * kReg64Threads + tid];
+  }
+  if (rowmap != nullptr && mine && lg != r0 + tid) {  // the net row permutation, as above
+    int* rm = rowmap + (size_t)blockIdx.y * kRowmapStride;
+    const int e = atomicAdd(cluster.map_shared_rank(&s_moved, 0), 1);
+    rm[1 + 2 * e] = k + lg;
+    rm[2 + 2 * e] = k + r0 + tid;
+  }
+  cluster.sync();  // no CTA leaves while others may still use its shared memory
+  if (rowmap != nullptr && rank == 0 && tid == 0) rowmap[(size_t)blockIdx.y * kRowmapStride] = s_moved;
+}
+
 // perm[i] such that (P b)[i] = b[perm[i]], from LAPACK-style interchanges.
 __global__ void lu_perm_kernel(const int* __restrict__ ipiv, int n, int* __restrict__ perm) {
   extern __shared__ int sp[];
@@ -805,6 +1005,7 @@ template <typename K> int max_cluster(K kern, int threads, size_t smem) {
 }
 
 constexpr size_t kPanelSmemBudget = 200 * 1024;
+constexpr size_t kReg64Smem = (size_t)32 * kReg64Threads * sizeof(double2);
 
 template <typename R, int NB> size_t panel_smem(int chunk) {
   typedef typename CT2<R>::C2 C2;
@@ -856,6 +1057,26 @@ template <typename R> bool choose_panel(int n, int want_nb, int batch, int& nb, 
       if (!found || waves < best_waves) {
         found = true;
         best_waves = waves;
+        nb = 32;
+        cl = c;
+      }
+    }
+    if (found) return true;
+  }
+  if (sizeof(R) == 8 && (want_nb == 0 || want_nb == 32)) {
+    // the FP64 form's: a column step takes about 1.4 us of exchange and, at 2 FP64 lanes per
+    // SM and clock, 20 ns per row of a CTA while all 32 columns are live (10 ns on average
+    // over a factorisation's shrinking panels), so a wider cluster pays until it costs a wave
+    double best = 0.0;
+    for (int c : {2, 4, 8, 16}) {
+      if ((n + c - 1) / c > kReg64Threads) continue;
+      if (max_cluster(lu_panel_reg64_kernel, kReg64Threads, kReg64Smem) < c) continue;
+      const int act = active_clusters(lu_panel_reg64_kernel, kReg64Threads, kReg64Smem, c);
+      if (act < 1) continue;
+      const double cost = (std::max(batch, 1) + act - 1) / act * (1.4 + 0.01 * n / c);
+      if (!found || cost < best) {
+        found = true;
+        best = cost;
         nb = 32;
         cl = c;
       }
@@ -927,6 +1148,8 @@ int lu_resident_batch(Precision prec, int n) {
   else if (prec == Precision::Mixed)
     act = nb == 64 ? active_clusters(lu_panel_cluster_kernel<float, 64>, kPanelThreads, panel_smem<float, 64>(chunk), cl)
                    : active_clusters(lu_panel_cluster_kernel<float, 32>, kPanelThreads, panel_smem<float, 32>(chunk), cl);
+  else if (nb == 32 && chunk <= kReg64Threads)
+    act = active_clusters(lu_panel_reg64_kernel, kReg64Threads, kReg64Smem, cl);
   else
     act = nb == 64 ? active_clusters(lu_panel_cluster_kernel<double, 64>, kPanelThreads, panel_smem<double, 64>(chunk), cl)
                    : active_clusters(lu_panel_cluster_kernel<double, 32>, kPanelThreads, panel_smem<double, 32>(chunk), cl);
@@ -960,6 +1183,11 @@ cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long s
     ensure_smem_limit((const void*)lu_panel_cluster_kernel<float, 32>, sm);
     cudaFuncSetAttribute(lu_panel_cluster_kernel<float, 32>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return launch_cluster(lu_panel_cluster_kernel<float, 32>, grid, kPanelThreads, sm, cl, stream, args);
+  }
+  if (nb == 32 && kb == 32 && chunk <= kReg64Threads) {
+    ensure_smem_limit((const void*)lu_panel_reg64_kernel, kReg64Smem);
+    cudaFuncSetAttribute(lu_panel_reg64_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return launch_cluster(lu_panel_reg64_kernel, grid, kReg64Threads, kReg64Smem, cl, stream, args);
   }
   if (nb == 64) {
     const size_t sm = panel_smem<double, 64>(chunk);
