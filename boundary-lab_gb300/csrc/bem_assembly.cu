@@ -992,8 +992,9 @@ __device__ __forceinline__ void warp_reduce_halving_df(df* v, int lane) {
 // above (renormalised every eight points).  The lanes' partial
 // sums are combined by a reduce-scatter in full df_add; lane 4 j then holds
 // sums 3 j .. 3 j + 2 and writes moments = jac * sum in FP64 and their float
-// copies into the pair record; lane 0 also writes the record's S0 term.
-__global__ void __launch_bounds__(256)
+// copies into the pair record; lane 0 also writes the record's S0 term.  CTAs of one warp, as
+// pairs differ in length (14,076 pairs: 580 -> 520 us).
+__global__ void __launch_bounds__(32)
     singular_moments_df_kernel(const SingularPair* __restrict__ pairs, int npairs, const int* __restrict__ rule_ptr,
                                const float* __restrict__ duffy_df, const float* __restrict__ geo_df,
                                double* __restrict__ moments, float* __restrict__ rec) {
@@ -1094,13 +1095,89 @@ template <> struct SingParams<double> {
 // Per pair output: 9 LHS block entries then 3 RHS-operator entries (complex).
 constexpr int kSingOut = 12;
 
+// Warp reduce-scatter by recursive halving of N = 3 x 2^j values per lane (N <= 96).  At
+// exchange offset O a lane keeps one half of its values (the upper half when bit O of its
+// lane index is set) and adds its partner's copy of that half, so each level moves half as
+// many values as the one before; once three values remain, the remaining offsets are plain
+// butterflies.  Afterwards v[0..3) of lane l hold the warp sums of entries 3 (l >> s) ..
+// 3 (l >> s) + 2, s = 5 - log2(N / 3).  For 96 values the five levels move 48 + 24 + 12 +
+// 6 + 3 values per lane, against 5 x 96 for a butterfly of every value.
+template <int N, int O, typename T>
+__device__ __forceinline__ void warp_reduce_halving(T* v, int lane) {
+  if constexpr (O > 0) {
+    if constexpr (N > 3) {
+      constexpr int H = N / 2;
+      const bool upper = (lane & O) != 0;
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const T send = upper ? v[i] : v[H + i];
+        const T keep = upper ? v[H + i] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      warp_reduce_halving<H, O / 2>(v, lane);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], O);
+      warp_reduce_halving<N, O / 2>(v, lane);
+    }
+  }
+}
+
+// A pair's outputs from its 21 sums, sum i in lane i: IR[9], IDh[9], IKh[3], already times
+// jac (SR[a] is the sum of IR[a][b] over b).  Lanes 0-8 form the nine LHS entries, lanes
+// 9-11 the three RHS-operator entries.
+__device__ __forceinline__ void singular_outputs_f64(int lane, const SingularPair& P, double2 acc,
+                                                     const double* __restrict__ M, const double* __restrict__ curls,
+                                                     const double* __restrict__ area,
+                                                     const double* __restrict__ m11m10, const SingParams<double>& p,
+                                                     double2* __restrict__ o) {
+  auto sum = [&](int i) {
+    return make_double2(__shfl_sync(0xffffffffu, acc.x, i), __shfl_sync(0xffffffffu, acc.y, i));
+  };
+  double2 SR[3], S0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) SR[a] = cadd(cadd(sum(3 * a), sum(3 * a + 1)), sum(3 * a + 2));
+  const double2 IDh = make_double2(__shfl_sync(0xffffffffu, acc.x, (lane + 9) & 31),
+                                   __shfl_sync(0xffffffffu, acc.y, (lane + 9) & 31));  // lanes 0-8; IKh in lanes 9-11
+  if (lane >= 12) return;
+  S0 = make_double2(M[0] + M[1] + M[2], 0.0);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) S0 = cadd(S0, SR[a]);
+  const bool coincident = P.kind == 1 && P.tr == 0;  // mass terms: the face with itself, never with an image
+  const double a2 = 2.0 * area[P.test];
+  if (lane < 9) {
+    const int a = lane / 3, b = lane - 3 * a;
+    const double* ct = curls + 9 * (size_t)P.test + 3 * a;
+    const double* cr = curls + 9 * (size_t)P.trial + 3 * b;
+    // image pairs: reflected curls det(S) S c
+    const double sx = tr_sign_x(P.tr), sy = tr_sign_y(P.tr), det = sx * sy;
+    const double cc = ct[0] * (det * sx * cr[0]) + ct[1] * (det * sy * cr[1]) + ct[2] * (det * cr[2]);
+    const double kk_nn = p.k2 * P.nprod;
+    const double2 D = make_double2(M[12 + lane] + IDh.x, IDh.y), IGt = make_double2(M[3 + lane] + acc.x, acc.y);
+    const double2 H = make_double2(cc * S0.x - kk_nn * IGt.x, cc * S0.y - kk_nn * IGt.y);
+    double2 L = cadd(cmul(p.cD, D), cmul(p.cH, H));
+    if (coincident) L = cadd(L, cscale(p.cM, a2 * m11m10[lane]));
+    o[lane] = L;
+  } else {
+    const int a = lane - 9;
+    const double2 sr = a == 0 ? SR[0] : a == 1 ? SR[1] : SR[2];
+    const double2 S = make_double2(M[a] + sr.x, sr.y), K = make_double2(M[21 + a] + IDh.x, IDh.y);
+    double2 rhs = cadd(cmul(p.cS, S), cmul(p.cK, K));
+    if (coincident) rhs = cadd(rhs, cscale(p.cM10, a2 * m11m10[9 + a]));
+    o[9 + a] = rhs;
+  }
+}
+
 // The plain FP64 form's singular kernel (the mixed form uses singular_dyn_f32_kernel below).
 // A warp per pair, lanes over the Duffy points.  Bound by the FP64 pipe: about 110 FP64
 // instructions per point (table sine and cosine, the factors hr fy, hi fy, hr fx, hi fx
 // formed once, 21 complex sums: the single-layer sums SR[a] are the sums of IR[a][b] over b,
 // as the P1 trial basis sums to one), against 190 with library sincos and a product chain
-// per sum: 1,280 triangles: 5.2 -> 4.1 ms per frequency.
-__global__ void __launch_bounds__(256, 1)
+// per sum: 1,280 triangles: 5.2 -> 4.1 ms per frequency.  A pair of 512 points costs 16
+// steps, so what follows the points counts: sums by reduce-scatter (48 additions instead of
+// 210), outputs on twelve lanes instead of one, and CTAs of four warps, whose slots free up
+// sooner than those of eight when pairs differ in length: 3,984 triangles 13.9 -> 10.5 ms.
+__global__ void __launch_bounds__(128, 2)
     singular_dyn_kernel(SingularGeom geo, const SingularPair* __restrict__ pairs, int npairs,
                         const int* __restrict__ rule_ptr, const double* __restrict__ duffy,
                         const double* __restrict__ moments, const double* __restrict__ curls,
@@ -1128,10 +1205,10 @@ __global__ void __launch_bounds__(256, 1)
     nt[d] = geo.normal[3 * P.test + d];
     nr[d] = sd * geo.normal[3 * P.trial + d];
   }
-  // accumulators: IR[9], IDh[9], IKh[3] (complex) = 42 reals
-  double acc[42];
+  // accumulators: IR[9], IDh[9], IKh[3] (complex) = 42 reals, padded for the reduction
+  double acc[48];
 #pragma unroll
-  for (int i = 0; i < 42; ++i) acc[i] = 0.0;
+  for (int i = 0; i < 48; ++i) acc[i] = 0.0;
   const double inv4pi = 0.25 / CUDART_PI, half_k = 0.5 * p.k;
   const int q0 = rule_ptr[P.rule], q1 = rule_ptr[P.rule + 1];
   for (int q = q0 + lane; q < q1; q += 32) {
@@ -1172,83 +1249,19 @@ __global__ void __launch_bounds__(256, 1)
       }
     }
   }
+  // reduce-scatter: lanes 2m and 2m + 1 end with sums 3m .. 3m + 2, which go to the lanes of
+  // their outputs through shared memory
+  warp_reduce_halving<48, 16>(acc, lane);
+  __shared__ double red[4][48];
+  double* r = red[threadIdx.x >> 5];
+  if ((lane & 1) == 0) {
 #pragma unroll
-  for (int i = 0; i < 42; ++i) acc[i] = warp_sum(acc[i]);
-  if (lane != 0) return;
-  const double* M = moments + (size_t)kStatic * warp;
-  const double jac = P.jac;
-  double2 SR[3], IR[9], IDh[9], IKh[3];
-  for (int i = 0; i < 9; ++i) {
-    IR[i] = make_double2(acc[2 * i] * jac, acc[2 * i + 1] * jac);
-    IDh[i] = make_double2(acc[18 + 2 * i] * jac, acc[18 + 2 * i + 1] * jac);
+    for (int j = 0; j < 3; ++j) r[3 * (lane >> 1) + j] = acc[j];
   }
-  for (int a = 0; a < 3; ++a) {
-    SR[a] = cadd(cadd(IR[3 * a], IR[3 * a + 1]), IR[3 * a + 2]);
-    IKh[a] = make_double2(acc[36 + 2 * a] * jac, acc[36 + 2 * a + 1] * jac);
-  }
-  // S0 = sum w G (static + dynamic)
-  double2 S0 = make_double2(M[0] + M[1] + M[2], 0.0);
-  for (int a = 0; a < 3; ++a) S0 = cadd(S0, SR[a]);
-  const double* ct = curls + 9 * (size_t)P.test;
-  const double* cr0 = curls + 9 * (size_t)P.trial;
-  double cr[9];  // image pairs: reflected curls det(S) S c
-  {
-    const double sx = tr_sign_x(P.tr), sy = tr_sign_y(P.tr), det = sx * sy;
-    for (int b = 0; b < 3; ++b) {
-      cr[3 * b] = det * sx * cr0[3 * b];
-      cr[3 * b + 1] = det * sy * cr0[3 * b + 1];
-      cr[3 * b + 2] = det * cr0[3 * b + 2];
-    }
-  }
-  const double kk_nn = p.k2 * P.nprod;
-  const bool coincident = P.kind == 1 && P.tr == 0;  // mass terms: the face with itself, never with an image
-  const double a2 = 2.0 * area[P.test];
-  double2* o = out + (size_t)kSingOut * warp;
-  for (int a = 0; a < 3; ++a) {
-    for (int b = 0; b < 3; ++b) {
-      const double cc = ct[3 * a] * cr[3 * b] + ct[3 * a + 1] * cr[3 * b + 1] + ct[3 * a + 2] * cr[3 * b + 2];
-      const int i = 3 * a + b;
-      const double2 D = make_double2(M[12 + i] + IDh[i].x, IDh[i].y);
-      const double2 IGt = make_double2(M[3 + i] + IR[i].x, IR[i].y);
-      const double2 H = make_double2(cc * S0.x - kk_nn * IGt.x, cc * S0.y - kk_nn * IGt.y);
-      double2 L = cadd(cmul(p.cD, D), cmul(p.cH, H));
-      if (coincident) L = cadd(L, cscale(p.cM, a2 * m11m10[i]));
-      o[i] = L;
-    }
-    const double2 S = make_double2(M[a] + SR[a].x, SR[a].y);
-    const double2 K = make_double2(M[21 + a] + IKh[a].x, IKh[a].y);
-    double2 rhs = cadd(cmul(p.cS, S), cmul(p.cK, K));
-    if (coincident) rhs = cadd(rhs, cscale(p.cM10, a2 * m11m10[9 + a]));
-    o[9 + a] = rhs;
-  }
-}
-
-// Warp reduce-scatter by recursive halving of N = 3 x 2^j values per lane (N <= 96).  At
-// exchange offset O a lane keeps one half of its values (the upper half when bit O of its
-// lane index is set) and adds its partner's copy of that half, so each level moves half as
-// many values as the one before; once three values remain, the remaining offsets are plain
-// butterflies.  Afterwards v[0..3) of lane l hold the warp sums of entries 3 (l >> s) ..
-// 3 (l >> s) + 2, s = 5 - log2(N / 3).  For 96 values the five levels move 48 + 24 + 12 +
-// 6 + 3 values per lane, against 5 x 96 for a butterfly of every value.
-template <int N, int O>
-__device__ __forceinline__ void warp_reduce_halving(float* v, int lane) {
-  if constexpr (O > 0) {
-    if constexpr (N > 3) {
-      constexpr int H = N / 2;
-      const bool upper = (lane & O) != 0;
-#pragma unroll
-      for (int i = 0; i < H; ++i) {
-        const float send = upper ? v[i] : v[H + i];
-        const float keep = upper ? v[H + i] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-      }
-      warp_reduce_halving<H, O / 2>(v, lane);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], O);
-      warp_reduce_halving<N, O / 2>(v, lane);
-    }
-  }
+  __syncwarp();
+  const double2 sum = lane < 21 ? make_double2(r[2 * lane] * P.jac, r[2 * lane + 1] * P.jac) : make_double2(0.0, 0.0);
+  singular_outputs_f64(lane, P, sum, moments + (size_t)kStatic * warp, curls, area, m11m10, p,
+                       out + (size_t)kSingOut * warp);
 }
 
 // The mixed form's singular kernel: the Duffy remainder of
@@ -1256,7 +1269,9 @@ __device__ __forceinline__ void warp_reduce_halving(float* v, int lane) {
 // curl products, static moments) read from the pair record instead of being
 // formed from FP64 data per frequency.  One warp per pair, lanes over the
 // Duffy points; after the warp reduction (every lane holds every sum) lanes
-// 0-8 form the nine LHS entries and lanes 9-11 the three RHS-operator entries.
+// 0-8 form the nine LHS entries and lanes 9-11 the three RHS-operator entries.  Pairs have
+// 512 to 1,536 points, so a CTA is one warp: registers are free again when its pair is
+// done, not when the longest of eight is (9,960 triangles, one frequency: 0.79 -> 0.68 ms).
 struct SingParamsF32 {
   float k, k2;
   float2 cD, cH, cM, cS, cK, cM10;
@@ -1271,7 +1286,7 @@ template <int NFQ> struct SingParamsF32N {
 };
 
 template <int NFQ>
-__global__ void __launch_bounds__(NFQ == 1 ? 256 : 128, NFQ == 1 ? 2 : 3)
+__global__ void __launch_bounds__(32, NFQ == 1 ? 16 : 12)
     singular_dyn_f32_kernel(const SingularPair* __restrict__ pairs, int npairs, const int* __restrict__ rule_ptr,
                             const float* __restrict__ duffy, const float* __restrict__ rec, SingParamsF32N<NFQ> pn,
                             float2* __restrict__ out, long long out_stride) {
@@ -1362,8 +1377,7 @@ __global__ void __launch_bounds__(NFQ == 1 ? 256 : 128, NFQ == 1 ? 2 : 3)
   // at 48 f + 2 i, .y next to it); with one, lanes 2m and 2m + 1 both hold sums 3m .. 3m + 2.
   // The sums go through shared memory to the lanes that form the outputs.
   constexpr int T = NFQ * 48;
-  constexpr int WPB = (NFQ == 1 ? 256 : 128) / 32;
-  __shared__ float red[WPB][T];
+  __shared__ float red[T];
   {
     float v[T];
 #pragma unroll
@@ -1374,7 +1388,7 @@ __global__ void __launch_bounds__(NFQ == 1 ? 256 : 128, NFQ == 1 ? 2 : 3)
         v[48 * f + 2 * i + 1] = acc2[f][i].y;
       }
     warp_reduce_halving<T, 16>(v, lane);
-    float* r = red[threadIdx.x >> 5];
+    float* r = red;
     constexpr int sh = NFQ == 2 ? 0 : 1;
     if ((lane & ((1 << sh) - 1)) == 0) {
 #pragma unroll
@@ -1382,7 +1396,7 @@ __global__ void __launch_bounds__(NFQ == 1 ? 256 : 128, NFQ == 1 ? 2 : 3)
     }
     __syncwarp();
   }
-  const float* red_w = red[threadIdx.x >> 5];
+  const float* red_w = red;
   auto sum2 = [&](int f, int i) { return make_float2(red_w[48 * f + 2 * i], red_w[48 * f + 2 * i + 1]); };
 #pragma unroll
   for (int f = 0; f < NFQ; ++f) {
@@ -1445,7 +1459,7 @@ __global__ void __launch_bounds__(NFQ == 1 ? 256 : 128, NFQ == 1 ? 2 : 3)
 // contiguous in cheb[((pair kChebN) + n) 24 + i].  The single-layer sums SR[a] (entries
 // 0-2) are not formed: the P1 trial basis sums to one, so SR[a] = IR[a][0] + IR[a][1] +
 // IR[a][2], and the per-frequency kernel adds them up there.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32)
     singular_cheb_moments_kernel(const SingularPair* __restrict__ pairs, int npairs, const int* __restrict__ rule_ptr,
                                  const float* __restrict__ duffy, const float* __restrict__ rec, float two_over_R,
                                  int nterms, float* __restrict__ cheb) {
@@ -1637,11 +1651,11 @@ __global__ void __launch_bounds__(128)
 // are those of the Duffy points to rounding.  Per point and chunk of four terms about 160
 // FP64 instructions, 640 for 16 terms: four frequencies point by point, once per mesh; a
 // frequency through the moments then costs a fortieth of one (1,280 triangles: 4.1 ->
-// 0.10 ms, the moments 17.5 ms once).  Per pair 21 sums per term: IR[9], IDh[9],
+// 0.10 ms, the moments 15.4 ms once for 16 terms; 17.5 with butterfly sums).  Per pair 21 sums per term: IR[9], IDh[9],
 // IKh[3] (SR[a] is the sum of IR[a][b] over b), stored [pair][term][kCheb64Sums].
 constexpr int kCheb64Sums = 21;
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32)
     singular_cheb64_moments_kernel(SingularGeom geo, const SingularPair* __restrict__ pairs, int npairs,
                                    const int* __restrict__ rule_ptr, const double* __restrict__ duffy,
                                    double two_over_R, int nterms, double* __restrict__ cheb) {
@@ -1668,11 +1682,9 @@ __global__ void __launch_bounds__(128)
   const int q0 = rule_ptr[P.rule], q1 = rule_ptr[P.rule + 1];
   constexpr int NCH = 4;
   for (int n0 = 0; n0 < nterms; n0 += NCH) {
-    double v[NCH][kCheb64Sums];
+    double v[NCH * 24];  // kCheb64Sums of each term, padded to 24
 #pragma unroll
-    for (int j = 0; j < NCH; ++j)
-#pragma unroll
-      for (int i = 0; i < kCheb64Sums; ++i) v[j][i] = 0.0;
+    for (int i = 0; i < NCH * 24; ++i) v[i] = 0.0;
     for (int q = q0 + lane; q < q1; q += 32) {
       const double* pt = duffy + 5 * (size_t)q;
       const double tu = pt[0], tv = pt[1], ru = pt[2], rvv = pt[3], w = pt[4];
@@ -1708,27 +1720,22 @@ __global__ void __launch_bounds__(128)
         const double tg = ta * inv4pi;
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
-          v[j][i] = fma(wab[i], tg, v[j][i]);
-          v[j][9 + i] = fma(wfy[i], ta, v[j][9 + i]);
+          v[24 * j + i] = fma(wab[i], tg, v[24 * j + i]);
+          v[24 * j + 9 + i] = fma(wfy[i], ta, v[24 * j + 9 + i]);
         }
 #pragma unroll
-        for (int a = 0; a < 3; ++a) v[j][18 + a] = fma(wfx[a], ta, v[j][18 + a]);
+        for (int a = 0; a < 3; ++a) v[24 * j + 18 + a] = fma(wfx[a], ta, v[24 * j + 18 + a]);
         const double tc = fma(x2, tb, -ta);
         ta = tb;
         tb = tc;
       }
     }
-    // sums over the lanes; lane i keeps sum i of every term of the chunk
-    double* o = cheb + ((size_t)warp * kChebN + n0) * kCheb64Sums;
+    // reduce-scatter over the chunk's 4 x 24 values: lane L ends with 3L .. 3L + 2
+    warp_reduce_halving<NCH * 24, 16>(v, lane);
+    double* o = cheb + ((size_t)warp * kChebN + n0 + (lane >> 3)) * kCheb64Sums + 3 * (lane & 7);
+    if ((lane & 7) < 7) {
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-      double mine = 0.0;
-#pragma unroll
-      for (int i = 0; i < kCheb64Sums; ++i) {
-        const double t = warp_sum(v[j][i]);
-        if (lane == i) mine = t;
-      }
-      if (lane < kCheb64Sums) o[j * kCheb64Sums + lane] = mine;
+      for (int j = 0; j < 3; ++j) o[j] = v[j];
     }
   }
 }
@@ -1759,44 +1766,8 @@ __global__ void __launch_bounds__(128)
     }
     acc = cscale(acc, P.jac);
   }
-  auto sum = [&](int i) {
-    return make_double2(__shfl_sync(0xffffffffu, acc.x, i), __shfl_sync(0xffffffffu, acc.y, i));
-  };
-  double2 SR[3], S0;
-  const double* M = moments + (size_t)kStatic * warp;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) SR[a] = cadd(cadd(sum(3 * a), sum(3 * a + 1)), sum(3 * a + 2));
-  const double2 IDh = make_double2(__shfl_sync(0xffffffffu, acc.x, (lane + 9) & 31),
-                                   __shfl_sync(0xffffffffu, acc.y, (lane + 9) & 31));  // lanes 0-8; IKh in lanes 9-11
-  if (lane >= 12) return;
-  S0 = make_double2(M[0] + M[1] + M[2], 0.0);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) S0 = cadd(S0, SR[a]);
-  const SingParams<double>& p = cp.p;
-  const bool coincident = P.kind == 1 && P.tr == 0;  // mass terms: the face with itself, never with an image
-  const double a2 = 2.0 * area[P.test];
-  double2* o = out + (size_t)kSingOut * warp;
-  if (lane < 9) {
-    const int a = lane / 3, b = lane - 3 * a;
-    const double* ct = curls + 9 * (size_t)P.test + 3 * a;
-    const double* cr = curls + 9 * (size_t)P.trial + 3 * b;
-    // image pairs: reflected curls det(S) S c
-    const double sx = tr_sign_x(P.tr), sy = tr_sign_y(P.tr), det = sx * sy;
-    const double cc = ct[0] * (det * sx * cr[0]) + ct[1] * (det * sy * cr[1]) + ct[2] * (det * cr[2]);
-    const double kk_nn = p.k2 * P.nprod;
-    const double2 D = make_double2(M[12 + lane] + IDh.x, IDh.y), IGt = make_double2(M[3 + lane] + acc.x, acc.y);
-    const double2 H = make_double2(cc * S0.x - kk_nn * IGt.x, cc * S0.y - kk_nn * IGt.y);
-    double2 L = cadd(cmul(p.cD, D), cmul(p.cH, H));
-    if (coincident) L = cadd(L, cscale(p.cM, a2 * m11m10[lane]));
-    o[lane] = L;
-  } else {
-    const int a = lane - 9;
-    const double2 sr = a == 0 ? SR[0] : a == 1 ? SR[1] : SR[2];
-    const double2 S = make_double2(M[a] + sr.x, sr.y), K = make_double2(M[21 + a] + IDh.x, IDh.y);
-    double2 rhs = cadd(cmul(p.cS, S), cmul(p.cK, K));
-    if (coincident) rhs = cadd(rhs, cscale(p.cM10, a2 * m11m10[9 + a]));
-    o[9 + a] = rhs;
-  }
+  singular_outputs_f64(lane, P, acc, moments + (size_t)kStatic * warp, curls, area, m11m10, cp.p,
+                       out + (size_t)kSingOut * warp);
 }
 
 // The singular blocks into the extended rows: one thread per distinct target
@@ -2512,9 +2483,7 @@ cudaError_t launch_singular_static(const DeviceMesh& m, double* moments, float* 
   SingularGeom geo{m.verts, m.faces, m.normal};
   pair_setup_kernel<<<(m.npairs + 127) / 128, 128, 0, stream>>>(geo, m.pairs, m.npairs, m.curls, m.area, m.pairgeo_df,
                                                                 pairrec);
-  const int threads = 256;
-  const int blocks = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
-  singular_moments_df_kernel<<<blocks, threads, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy_df, m.pairgeo_df,
+  singular_moments_df_kernel<<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy_df, m.pairgeo_df,
                                                              moments, pairrec);
   return cudaGetLastError();
 }
@@ -2604,9 +2573,7 @@ cudaError_t launch_cheb64_moments(const DeviceMesh& m, int nterms, cudaStream_t 
   if (m.npairs == 0 || !m.cheb64 || nterms < 4 || nterms > kChebN || nterms % 4 || !(m.cheb_R > 0.0))
     return cudaErrorInvalidValue;
   SingularGeom geo{m.verts, m.faces, m.normal};
-  const int threads = 128;
-  const int blocks = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
-  singular_cheb64_moments_kernel<<<blocks, threads, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
+  singular_cheb64_moments_kernel<<<m.npairs, 32, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
                                                                  2.0 / m.cheb_R, nterms, m.cheb64);
   return cudaGetLastError();
 }
@@ -2614,9 +2581,7 @@ cudaError_t launch_cheb64_moments(const DeviceMesh& m, int nterms, cudaStream_t 
 cudaError_t launch_cheb_moments(const DeviceMesh& m, int nterms, cudaStream_t stream) {
   if (m.npairs == 0 || !m.cheb || nterms < 4 || nterms > kChebN || nterms % 4 || !(m.cheb_R > 0.0))
     return cudaErrorInvalidValue;
-  const int threads = 256;
-  const int blocks = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
-  singular_cheb_moments_kernel<<<blocks, threads, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32, m.pairrec,
+  singular_cheb_moments_kernel<<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32, m.pairrec,
                                                                (float)(2.0 / m.cheb_R), nterms, m.cheb);
   return cudaGetLastError();
 }
@@ -2649,17 +2614,13 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
           SingParamsF32N<2> pn;
           pn.f[0] = params(f);
           pn.f[1] = params(f + 1);
-          const int threads = 128;
-          const int nblk = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
-          singular_dyn_f32_kernel<2><<<nblk, threads, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32,
+          singular_dyn_f32_kernel<2><<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32,
                                                                    m.pairrec, pn, o, blocks_stride);
           f += 2;
         } else {
           SingParamsF32N<1> pn;
           pn.f[0] = params(f);
-          const int threads = 256;
-          const int nblk = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
-          singular_dyn_f32_kernel<1><<<nblk, threads, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32,
+          singular_dyn_f32_kernel<1><<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32,
                                                                    m.pairrec, pn, o, blocks_stride);
           f += 1;
         }
@@ -2726,7 +2687,7 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
     if (launched) *launched += nl;
     return cudaGetLastError();
   }
-  const int threads = 256;
+  const int threads = 128;
   const int nblk = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
   for (int f = 0; f < nfreq; ++f) {
     SingParams<double> p;
