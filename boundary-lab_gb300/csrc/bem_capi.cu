@@ -286,6 +286,18 @@ Layout layout_for(const bem::DeviceMesh& dm, bem::Precision prec) {
 // moments exist, so a call's results depend on its own inputs only.
 constexpr int kChebMinFreqs = 12;
 
+// Batch of a call that one automatic batch would hold and that may use two lanes: split in
+// two, so that one half's latency-bound LU panels, solves and last waves overlap the other's
+// assembly.  The first half is a multiple of four, the frequencies that share a regular
+// launch's geometry (5 + 5 or 6 + 6 lost 1 % at 10,000 triangles where 8 + 4 gains 1 %); a
+// second half below four gains nothing (2 + 2: 2 to 12 % slower).  Measured, one lane and
+// two: 1,000 triangles, 16 frequencies 2.87 -> 2.58 ms; 2,500, 12: 8.7 -> 8.2; 5,000, 30:
+// 59.5 -> 58.1; FP64 form, 1,280, 16: 114.2 -> 112.4.
+int lane_split(int n_freq) {
+  const int half = ((n_freq + 1) / 2 + 3) / 4 * 4;
+  return n_freq - half >= 4 ? half : n_freq;
+}
+
 // Forms (or extends) the mesh's Chebyshev moments on the side stream for the call's
 // wavenumbers k[0..n): with the fewest terms (a multiple of four) that cover every
 // frequency whose expansion converges within kChebN terms, or twice the terms the moments
@@ -1157,9 +1169,10 @@ long long bem_estimate_device_bytes(int nv, int nf, int npairs, int nrhs, int np
   const long long n_ext = (long long)(nv * 1.3) + 64;
   long long bytes = 0;
   // frequencies assembled together: those of a regular launch, or a batch's within kRextBytes
+  // (on each of two lanes)
   const long long rext = round_up(n_ext, 32) * 3LL * nf * esz;
   const long long group = std::max<long long>(precision == BEM_PRECISION_MIXED ? 4 : 2,
-                                              std::min<long long>(batch, (long long)kRextBytes / std::max(rext, 1LL)));
+                                              std::min<long long>(batch, 2LL * kRextBytes / std::max(rext, 1LL)));
   bytes += rext * group;                                                    // extended rows
   bytes += (long long)nf * 3 * nrhs * esz * group;                          // right-hand-side face values
   bytes += (long long)batch * lda * nv * esz * (precision == BEM_PRECISION_MIXED ? 2 : 1);  // matrices (+copy)
@@ -1198,6 +1211,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
     const int nv = dm.nv, nc = m->nc;
     int B = o.batch > 0 ? std::min(o.batch, 64) : auto_batch(m, prec, n_freq);
     B = std::min(B, n_freq);
+    if (o.batch <= 0 && o.lanes >= 2 && B == n_freq) B = lane_split(n_freq);
     ctx->prof = o.profile != 0;
     const int nbatch = (n_freq + B - 1) / B;
     auto slice_of = [&](int bi) {
