@@ -15,6 +15,31 @@
 #define BEM_HD __host__ __device__ __forceinline__
 #define BEM_D __device__ __forceinline__
 
+// Programmatic dependent launch, for chains of short kernels: a kernel launched with
+// launch_chained may start while its predecessor in the stream drains.  It calls grid_wait
+// before its first access to memory that an earlier kernel writes or reads (the wait ends
+// when all earlier grids are complete and their writes visible), and reads such memory with
+// plain loads, never through the read-only path.  A predecessor that never calls
+// grid_trigger lets it start when it ends, as an ordinary launch does.
+BEM_D void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+BEM_D void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                                  A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // -------------------------------------------------------------- complex ----
 BEM_HD float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 BEM_HD double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }

@@ -402,6 +402,16 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
   const bool mine = tid < rows;
   int lg = r0 + tid;         // logical row of this thread's physical row
   int done_at = -1;          // step at which this row became the pivot row
+  if (tid == 0) {
+    s_moved = 0;
+    s_failed = 0;
+  }
+  if constexpr (CLUSTER) {  // no tag of an earlier use in the slots when the first push arrives
+    for (int i = tid; i < 2 * 16 * 2 * NB; i += kRegPanelThreads) (&rowsT[0][0][0])[i] = 0ull;
+    if (tid < 32) (&keyT[0][0])[tid] = 0ull;
+    cluster.sync();
+  }
+  grid_wait();
   float2 a[NB];
   {
     const float2* src = M + (size_t)k * lda + k + r0 + tid;
@@ -416,18 +426,8 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
 #pragma unroll
     for (int q = 0; q < NB / 2; ++q) dst[q] = make_float4(a[2 * q].x, a[2 * q].y, a[2 * q + 1].x, a[2 * q + 1].y);
   };
-  if (tid == 0) {
-    s_moved = 0;
-    s_failed = 0;
-  }
   publish_warp_key(0);
-  if constexpr (CLUSTER) {  // no tag of an earlier use in the slots when the first push arrives
-    for (int i = tid; i < 2 * 16 * 2 * NB; i += kRegPanelThreads) (&rowsT[0][0][0])[i] = 0ull;
-    if (tid < 32) (&keyT[0][0])[tid] = 0ull;
-    cluster.sync();
-  } else {
-    __syncthreads();
-  }
+  __syncthreads();
 #pragma unroll 1
   for (int j = 0; j < NB; ++j) {
     const int s = j & 1;
@@ -535,6 +535,7 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
       break;
     }
   }
+  grid_trigger();
   // every row to its logical position: the multipliers left of its pivot column
   // (all 32 for rows that never became the pivot)
   if (mine) {
@@ -972,19 +973,21 @@ __global__ void __launch_bounds__(kSolveThreads) lu_solve_cluster_kernel(const t
 
 template <typename K>
 cudaError_t launch_cluster(K kern, dim3 grid, int threads, size_t smem, int cl, cudaStream_t stream,
-                           void** args) {
+                           void** args, bool chained = false) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cl;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 2 : 1;  // chained: the kernel calls grid_wait
   return cudaLaunchKernelExC(&cfg, (const void*)kern, args);
 }
 
@@ -1166,11 +1169,11 @@ cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long s
     const size_t sm = (size_t)32 * kRegPanelThreads * sizeof(float2);
     if (cl == 1) {
       ensure_smem_limit((const void*)lu_panel_reg_kernel<false>, sm);
-      return launch_cluster(lu_panel_reg_kernel<false>, grid, kRegPanelThreads, sm, cl, stream, args);
+      return launch_cluster(lu_panel_reg_kernel<false>, grid, kRegPanelThreads, sm, cl, stream, args, true);
     }
     ensure_smem_limit((const void*)lu_panel_reg_kernel<true>, sm);
     cudaFuncSetAttribute(lu_panel_reg_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return launch_cluster(lu_panel_reg_kernel<true>, grid, kRegPanelThreads, sm, cl, stream, args);
+    return launch_cluster(lu_panel_reg_kernel<true>, grid, kRegPanelThreads, sm, cl, stream, args, true);
   }
   if (prec == Precision::Mixed) {
     if (nb == 64) {
