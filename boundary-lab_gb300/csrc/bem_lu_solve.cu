@@ -9,7 +9,8 @@
 // rows and no serial chain inside a block: x_K = inv(L_KK) b_K is a matrix-vector product
 // shared by the cluster's CTAs, and so is the update of the rows below.  One solve: 1.88 ->
 // 0.43 ms for one matrix of order 4,976, 0.68 ms for 15 (0.44 ms is their HBM time); 153 ->
-// 33 us at order 518; the inverses take 0.11 ms (one), 0.97 ms (15).
+// 33 us at order 518; the inverses take 0.09 ms (one), 0.34 ms (16 of
+// order 2,524).
 //
 // The substitution arithmetic stays FP32; the refinement loop around it takes the residual
 // of the FP32 matrix with exact products and compensated sums as before.
@@ -27,7 +28,7 @@ namespace cg = cooperative_groups;
 namespace bem {
 namespace {
 
-constexpr int kInvWarps = 4, kInvStages = 4;
+constexpr int kInvWarps = 8, kInvStages = 4;
 constexpr int kInvBlk = kOuterBlock / 32;
 
 template <int CPW> constexpr size_t inverse_smem() {
@@ -45,8 +46,10 @@ __device__ __forceinline__ float2 cinv_or_zero(float2 d) {
 // lower one, so both sides run the same left-looking substitution: a warp owns CPW columns
 // of the identity, lane = row of the current 32-row block, the 32 x 32 tiles of the triangle
 // pass through shared memory once per CTA (the scheme of lu_urows_kernel).  A slab (the
-// CTA's 4 CPW columns) starts at the block row of its columns: the rows above are zero.
-// Grid (256 / (4 CPW) slabs x 2 sides, blocks, batch).
+// CTA's 8 CPW columns) starts at the block row of its columns: the rows above are zero.
+// Grid (256 / (8 CPW) slabs x 2 sides, blocks, batch).  Bound by latency (the substitutions'
+// shuffles) at two warps per scheduler, so eight warps of four columns share a tile where
+// four of eight did: 32 matrices of order 600 348 -> 225 us, one of order 520 48 -> 35.
 template <int SIDE, int CPW>
 __device__ void block_inverse(const float2* __restrict__ D, long long lda, int KB, float2* __restrict__ out, int col0,
                               float2* ring, float2* X) {
@@ -59,8 +62,8 @@ __device__ void block_inverse(const float2* __restrict__ D, long long lda, int K
       float2* dst = ring + (size_t)slot * 32 * 32;
       const int rb = REV ? kInvBlk - 1 - pb : pb, cb = REV ? kInvBlk - 1 - pl : pl;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = threadIdx.x + 128 * q, col = i >> 4, piece = i & 15;
+      for (int q = 0; q < 16 / kInvWarps; ++q) {
+        const int i = threadIdx.x + 32 * kInvWarps * q, col = i >> 4, piece = i & 15;
         const int c = 32 * cb + col, r = 32 * rb + 2 * piece;
         // entries beyond the matrix are zero-filled (a piece may straddle its last row)
         const int bytes = c < KB ? min(max(KB - r, 0), 2) * (int)sizeof(float2) : 0;
@@ -494,10 +497,10 @@ cudaError_t lu_block_inverses(const void* LU, long long lda, int n, int batch, v
                                                                     (float2*)inv);
     return cudaGetLastError();
   };
-  // 8 columns per warp need the fewest shared-memory reads per FMA; 4 shorten the chain of a
-  // call that leaves SMs idle (n = 518, one matrix: 95 us with 8, 48 us with 4)
-  if (2LL * 8 * blocks * batch >= 2LL * sm_count()) return run(std::integral_constant<int, 8>{});
-  return run(std::integral_constant<int, 4>{});
+  // 4 columns per warp need fewer shared-memory reads per FMA; 2 shorten the chain of a
+  // call that leaves SMs idle
+  if (2LL * 8 * blocks * batch >= 2LL * sm_count()) return run(std::integral_constant<int, 4>{});
+  return run(std::integral_constant<int, 2>{});
 }
 
 cudaError_t lu_solve_blocks_batched(const void* LU, long long lda, int n, int batch, const void* inv, const int* perm,
