@@ -172,7 +172,7 @@ constexpr int kRowmapStride = 512;
 // per frequency at n = 4,976 against 128).
 constexpr int kOuterBlock = 256;
 // Kernels the two-level LU launches for one batch (cuBLAS kernels not counted).
-int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm);
+int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm, int batch);
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info,
                               int nb, void* cublas_handle, cudaStream_t stream, LuGemm gemm = LuGemm::Cublas,
                               void* tc_workspace = nullptr, bool* used_tensor = nullptr, int** tc_err = nullptr,
