@@ -1,19 +1,20 @@
 // Cluster-resident LU panel factorisation and cluster triangular solves (sm_103a).
 //
-// Panel: the m x nb panel of one matrix is spread over the shared memory of a
+// Panels: lu_panel_reg_kernel (mixed form) and lu_panel_reg64_kernel (FP64 form) keep a row
+// of 32 columns per thread in registers and exchange pivot candidates as tagged words
+// (described at the kernels); they serve every order whose rows fit a cluster of 16.
+// lu_panel_cluster_kernel takes the rest (64-wide panels, partial last panels, larger
+// orders): the m x nb panel of one matrix is spread over the shared memory of a
 // thread-block cluster (CL CTAs, each holding a contiguous block of panel rows,
 // column-major).  Each column step does a local pivot search, publishes the
 // CTA's candidate row, one cluster barrier, a pivot decision from the CL
 // candidates read through distributed shared memory (DSMEM), then the swap,
 // scaling and rank-1 update entirely in shared memory.
-// Nothing touches global memory between the initial load and the final store,
-// where the previous single-CTA kernel streamed the whole panel through L2 at
-// every column.  Pivot choice is LAPACK's (first maximum of |re| + |im|).
+// Pivot choice is LAPACK's (first maximum of |re| + |im|) in all three.
 //
-// Solves: pivots are turned into a row permutation once per factorisation
-// (lu_perm_kernel, in shared memory); each right-hand side is then solved by
-// one cluster whose CTAs own blocks of rows: the owner of a 32-row diagonal
-// block solves it with one warp, publishes the 32 values in a double-buffered
+// Solves (FP64 form, and orders whose rows bem_lu_solve.cu cannot hold): each right-hand
+// side is solved by one cluster whose CTAs own blocks of rows: the owner of a 32-row
+// diagonal block solves it with one warp, publishes the 32 values in a double-buffered
 // shared slot, and after one cluster barrier every CTA applies the block's
 // columns to its own rows.
 //
