@@ -504,8 +504,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
   const auto& G = p.g[blockIdx.z];
   Rext += (size_t)blockIdx.z * NFQ * strideR;
   double k[NFQ];
+  AngleUnits ku[NFQ];
 #pragma unroll
-  for (int f = 0; f < NFQ; ++f) k[f] = G.k[f];
+  for (int f = 0; f < NFQ; ++f) {
+    k[f] = G.k[f];
+    ku[f] = angle_units(k[f]);
+  }
   for (int i = lane; i < NFQ * 3 * max_rows; i += 32) acc[i] = make_double2(0.0, 0.0);
   load_sincos_table(tab, trig);
   __syncthreads();
@@ -586,14 +590,14 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
             for (int n = 0; n < Q; ++n) {
               const double rv[3] = {cm[0] + og[n][0], cm[1] + og[n][1], cm[2] + og[n][2]};
               const double r2 = fma(rv[0], rv[0], fma(rv[1], rv[1], rv[2] * rv[2]));
-              if (r2 == 0.0) continue;
+              if (is_zero(r2)) continue;
               const double rinv = rsqrt_step(r2), r = r2 * rinv;
               const double tq = (cmn + ogn[n]) * rinv * rinv;  // t / r
               const double ex = -tq * rinv, tn = fma(nn, rinv, tq), wr = p.w[n] * rinv;
 #pragma unroll
               for (int f = 0; f < NFQ; ++f) {
                 double sn, cs;
-                sincos_table(k[f] * r, tab, &sn, &cs);
+                sincos_table(r, ku[f], tab, &sn, &cs);
                 const double ey = k[f] * tn;
                 const double2 H = make_double2(fma(cs, ex, -sn * ey), fma(cs, ey, sn * ex));
 #pragma unroll
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(WARPS * 32) regular_f64_kernel(const FaceF64* 
           for (int n = 0; n < Q; ++n) {
             const double rv[3] = {C[0] + (og[n][0] - of[0]), C[1] + (og[n][1] - of[1]), C[2] + (og[n][2] - of[2])};
             const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-            if (r2 == 0.0) continue;
+            if (is_zero(r2)) continue;
             const double r = sqrt(r2);
             const double rinv = 1.0 / r;
             double s, c;
@@ -1209,7 +1213,8 @@ __global__ void __launch_bounds__(128, 2)
   double acc[48];
 #pragma unroll
   for (int i = 0; i < 48; ++i) acc[i] = 0.0;
-  const double inv4pi = 0.25 / CUDART_PI, half_k = 0.5 * p.k;
+  const double inv4pi = 0.25 / CUDART_PI;
+  const AngleUnits half_k = angle_units(0.5 * p.k);
   const int q0 = rule_ptr[P.rule], q1 = rule_ptr[P.rule + 1];
   for (int q = q0 + lane; q < q1; q += 32) {
     const double* pt = duffy + 5 * (size_t)q;
@@ -1220,10 +1225,10 @@ __global__ void __launch_bounds__(128, 2)
 #pragma unroll
     for (int d = 0; d < 3; ++d) rv[d] = (d0[d] + ru * e1r[d] + rvv * e2r[d]) - (tu * e1t[d] + tv * e2t[d]);
     const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-    if (r2 == 0.0) continue;
+    if (is_zero(r2)) continue;
     const double rinv = rsqrt_step(r2), r = r2 * rinv;
     double sh, ch;
-    sincos_table(half_k * r, tab, &sh, &ch);
+    sincos_table(r, half_k, tab, &sh, &ch);
     const double z = p.k * r, s = rinv * inv4pi;
     const double sh2 = sh + sh, sinz = sh2 * ch, omc = sh2 * sh;  // omc = 1 - cos z
     // R = s (cos z - 1 + i sin z)
@@ -1692,7 +1697,7 @@ __global__ void __launch_bounds__(32)
 #pragma unroll
       for (int d = 0; d < 3; ++d) rv[d] = (d0[d] + ru * e1r[d] + rvv * e2r[d]) - (tu * e1t[d] + tv * e2t[d]);
       const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-      if (r2 == 0.0) continue;
+      if (is_zero(r2)) continue;
       const double rinv = rsqrt_step(r2), r = r2 * rinv, s = rinv * inv4pi;
       const double fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * s;   // (r . n_r) / (4 pi r)
       const double fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * s;  // -(r . n_t) / (4 pi r)
@@ -1907,6 +1912,7 @@ __device__ __forceinline__ void rhs_pair_f32(const FaceF32& F, const FaceF32& Gf
 template <int Q>
 __device__ __forceinline__ void rhs_pair_f64(const FaceF64& F, const FaceF64& Gf, const RhsParams<double>& p,
                                              double2 S[3], double2 K[3], double sx, double sy, const double2* tab) {
+  const AngleUnits ku = angle_units(p.k);
   const double sg[3] = {sx, sy, 1.0};
   const double C[3] = {sx * Gf.anchor[0] - F.anchor[0], sy * Gf.anchor[1] - F.anchor[1], Gf.anchor[2] - F.anchor[2]};
 #pragma unroll
@@ -1922,10 +1928,10 @@ __device__ __forceinline__ void rhs_pair_f64(const FaceF64& F, const FaceF64& Gf
       double rv[3];
       for (int d = 0; d < 3; ++d) rv[d] = C[d] + (sg[d] * Gf.off[3 * n + d] - F.off[3 * m + d]);
       const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-      if (r2 == 0.0) continue;
+      if (is_zero(r2)) continue;
       const double rinv = rsqrt_step(r2), r = r2 * rinv;
       double s, c;
-      sincos_table(p.k * r, tab, &s, &c);
+      sincos_table(r, ku, tab, &s, &c);
       // w G (1, t (ik - 1/r)), G = e^{ikr} / (4 pi r), t = -(r . n_x) / r
       const double wn = (p.cw[n] + p.cw[Q + n] + p.cw[2 * Q + n]) * (0.25 / CUDART_PI);
       const double t = -(rv[0] * F.normal[0] + rv[1] * F.normal[1] + rv[2] * F.normal[2]) * rinv;

@@ -201,40 +201,60 @@ BEM_D float reduce_two_pi(float t) {
 // FP64 issues at 1/64 of the FP32 rate here, so an FP64 kernel's time is its count of FP64
 // instructions; everything else (table reads, FP32, integer work) is nearly free beside it.
 //
-// sin and cos by table: theta = n 2pi/512 + x, |x| <= pi/512, with the table entry of n mod
-// 512 and Taylor polynomials of x (sin to x^5, cos to x^6: truncation below 7e-20 and
-// 1e-22), combined by the addition theorem.  16 FP64 instructions for the pair.  Errors: the
-// reduction's (2pi/512 in two doubles, the product exact in the fma) and the table's, about
-// 1.5e-16 absolute; for |theta| <= pi/512 the entry is (1, 0) and the sine has full relative
-// accuracy.  |theta| < 2^22.
-constexpr int kSincosTable = 512;
-// The table (cos, sin) into shared memory, by the whole CTA (synchronise before use): from
-// its copy beside the mesh, or computed where there is none (src null; about 5% of a small
-// CTA's FP64 work).
+// sin and cos of k r by table, in units of h = 2 pi / 2048: u = r (k / h), n its nearest
+// integer, x = u - n.  The table holds (cos, sin) of the first quadrant's 512 units; the other
+// quadrants follow by exchanging and negating words, which is integer work.  With the units in
+// the polynomials' coefficients there is no product k r and no reduction of it, and |x| <= 1/2
+// (pi / 2048) needs two terms each: sin to x^3 with the cubic coefficient moved by 0.87 of
+// half a unit's x^5 / 120 (error 1e-17), cos to x^4 (2e-20), combined by the addition theorem:
+// 13 FP64 instructions for the pair, against 17 with 512 units to the circle, an angle in
+// radians and its two-term reduction.  Errors: the roundings of
+// x and the table's entry, with the result's about 2e-16 absolute (k / h is held in two doubles); for |k r| <= h / 2 the entry is (1, 0) and the sine has
+// full relative accuracy.  |u| < 2^31.
+constexpr int kSincosTable = 512, kSincosUnits = 4 * kSincosTable;
+struct AngleUnits {
+  double hi, lo;  // k / h
+};
+BEM_D AngleUnits angle_units(double k) {
+  AngleUnits a;
+  a.hi = k * 325.94932345220167;
+  a.lo = fma(k, 325.94932345220167, -a.hi) + k * -2.0150964915386866e-14;
+  return a;
+}
+// The table into shared memory, by the whole CTA (synchronise before use): from its copy
+// beside the mesh, or computed where there is none (src null; about 5% of a small CTA's FP64
+// work).
 BEM_D void load_sincos_table(double2* tab, const double2* src) {
   for (int i = threadIdx.x; i < kSincosTable; i += blockDim.x) {
     if (src != nullptr) {
       tab[i] = src[i];
     } else {
       double s, c;
-      sincospi(i * (2.0 / kSincosTable), &s, &c);
+      sincospi(i * (2.0 / kSincosUnits), &s, &c);
       tab[i] = make_double2(c, s);
     }
   }
 }
-BEM_D void sincos_table(double theta, const double2* tab, double* s, double* c) {
+BEM_D void sincos_table(double r, AngleUnits k, const double2* tab, double* s, double* c) {
   constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
-  const double t = fma(theta, 81.48733086305042, kMagic);
-  const double n = t - kMagic;
-  double x = fma(n, -0.01227184630308513, theta);
-  x = fma(n, -4.783776559169348e-19, x);
-  const double2 e = tab[__double2loint(t) & (kSincosTable - 1)];
+  const double t = fma(r, k.hi, kMagic);
+  const double x = fma(r, k.lo, fma(r, k.hi, -(t - kMagic)));
+  const int n = __double2loint(t);
+  const double2 q = tab[n & (kSincosTable - 1)];
+  // quadrant 0 (c, s), 1 (-s, c), 2 (-c, -s), 3 (s, -c)
+  const bool odd = (n & kSincosTable) != 0;
+  const int ssign = (n << 21) & 0x80000000, csign = ((n << 22) ^ (n << 21)) & 0x80000000;
+  const double a = odd ? q.y : q.x, b = odd ? q.x : q.y;
+  const double ec = __hiloint2double(__double2hiint(a) ^ csign, __double2loint(a));
+  const double es = __hiloint2double(__double2hiint(b) ^ ssign, __double2loint(b));
   const double x2 = x * x;
-  const double sx = fma(x * x2, fma(x2, 1.0 / 120.0, -1.0 / 6.0), x);
-  const double cm1 = x2 * fma(x2, fma(x2, -1.0 / 720.0, 1.0 / 24.0), -0.5);  // cos x - 1
-  *c = fma(e.x, cm1, fma(-e.y, sx, e.x));
-  *s = fma(e.y, cm1, fma(e.x, sx, e.y));
+  const double sx = x * fma(x2, -4.812807078551805e-09, 0.0030679615757712823);
+  const double cm1 = x2 * fma(x2, 3.691377174997586e-12, -4.706194115204505e-06);  // cos - 1
+  *c = fma(ec, cm1, fma(-es, sx, ec));
+  *s = fma(es, cm1, fma(ec, sx, es));
 }
+// a == 0 for a sum of squares, in integer instructions.
+BEM_D bool is_zero(double a) { return (__double2hiint(a) | __double2loint(a)) == 0; }
 // 1 / sqrt(a), a > 0 normal: the hardware approximation (about 2^-20) and one third-order
 // step, y + y e (1/2 + 3/8 e) with e = 1 - a y^2; five FP64 instructions, relative error
 // about 2^-52.

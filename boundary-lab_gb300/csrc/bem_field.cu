@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(256) field_f64_kernel(const FaceF64* __restric
   const int o = blockIdx.x, bt = blockIdx.y;
   const double xo[3] = {obs[3 * o], obs[3 * o + 1], obs[3 * o + 2]};
   const double k = prm->k[bt];
+  const AngleUnits ku = angle_units(k);
   const double2 qs = prm->qscale[bt];
   double2 acc[NC];
 #pragma unroll
@@ -348,10 +349,10 @@ __global__ void __launch_bounds__(256) field_f64_kernel(const FaceF64* __restric
 #pragma unroll
       for (int d = 0; d < 3; ++d) rv[d] = (sg[d] * F.anchor[d] - xo[d]) + sg[d] * F.off[3 * n + d];
       const double rr = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-      if (rr == 0.0) continue;
+      if (is_zero(rr)) continue;
       const double rinv = rsqrt_step(rr), r = rr * rinv;
       double sn, cs;
-      sincos_table(k * r, tab, &sn, &cs);
+      sincos_table(r, ku, tab, &sn, &cs);
       const double sc = rinv * (0.25 / CUDART_PI);
       // e^{ikr} [ (t/r)(ik - 1/r) p_s w_s - q w_s / r ] / (4 pi), t = (r . n_y) / r
       const double t = (rv[0] * sg[0] * F.normal[0] + rv[1] * sg[1] * F.normal[1] + rv[2] * F.normal[2]) * rinv * sc;
