@@ -1181,11 +1181,20 @@ __device__ __forceinline__ void singular_outputs_f64(int lane, const SingularPai
 // steps, so what follows the points counts: sums by reduce-scatter (48 additions instead of
 // 210), outputs on twelve lanes instead of one, and CTAs of four warps, whose slots free up
 // sooner than those of eight when pairs differ in length: 3,984 triangles 13.9 -> 10.5 ms.
+// Two frequencies of a call share a point's geometry, 45 of the 110 instructions (a few
+// registers of pair geometry spill): 10.2 -> 8.2 ms per frequency.
+template <int NFQ> struct SingParamsF64N {
+  SingParams<double> f[NFQ];
+  long long off[NFQ];  // frequency f's blocks at out + off[f]
+};
+
+template <int NFQ>
 __global__ void __launch_bounds__(128, 2)
     singular_dyn_kernel(SingularGeom geo, const SingularPair* __restrict__ pairs, int npairs,
                         const int* __restrict__ rule_ptr, const double* __restrict__ duffy,
                         const double* __restrict__ moments, const double* __restrict__ curls,
-                        const double* __restrict__ area, const double* __restrict__ m11m10, SingParams<double> p,
+                        const double* __restrict__ area, const double* __restrict__ m11m10,
+                        const __grid_constant__ SingParamsF64N<NFQ> pn,
                         const double2* __restrict__ trig, double2* __restrict__ out) {
   __shared__ double2 tab[kSincosTable];
   load_sincos_table(tab, trig);
@@ -1210,11 +1219,13 @@ __global__ void __launch_bounds__(128, 2)
     nr[d] = sd * geo.normal[3 * P.trial + d];
   }
   // accumulators: IR[9], IDh[9], IKh[3] (complex) = 42 reals, padded for the reduction
-  double acc[48];
+  double acc[NFQ * 48];
 #pragma unroll
-  for (int i = 0; i < 48; ++i) acc[i] = 0.0;
+  for (int i = 0; i < NFQ * 48; ++i) acc[i] = 0.0;
   const double inv4pi = 0.25 / CUDART_PI;
-  const AngleUnits half_k = angle_units(0.5 * p.k);
+  AngleUnits half_k[NFQ];
+#pragma unroll
+  for (int f = 0; f < NFQ; ++f) half_k[f] = angle_units(0.5 * pn.f[f].k);
   const int q0 = rule_ptr[P.rule], q1 = rule_ptr[P.rule + 1];
   for (int q = q0 + lane; q < q1; q += 32) {
     const double* pt = duffy + 5 * (size_t)q;
@@ -1227,46 +1238,55 @@ __global__ void __launch_bounds__(128, 2)
     const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
     if (is_zero(r2)) continue;
     const double rinv = rsqrt_step(r2), r = r2 * rinv;
-    double sh, ch;
-    sincos_table(r, half_k, tab, &sh, &ch);
-    const double z = p.k * r, s = rinv * inv4pi;
-    const double sh2 = sh + sh, sinz = sh2 * ch, omc = sh2 * sh;  // omc = 1 - cos z
-    // R = s (cos z - 1 + i sin z)
-    const double Rr = -s * omc, Ri = s * sinz;
-    // h(z) = (1 - cos z - z sin z) + i (z cos z - sin z)
-    const double hr = fma(-z, sinz, omc), hi = fma(z, 1.0 - omc, -sinz);
-    const double sr2 = s * rinv * rinv;
+    const double s = rinv * inv4pi, sr2 = s * rinv * rinv;
     const double fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * sr2;
     const double fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * sr2;
-    const double hyr = hr * fy, hyi = hi * fy, hxr = hr * fx, hxi = hi * fx;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      acc[36 + 2 * a] = fma(wp[a], hxr, acc[36 + 2 * a]);
-      acc[36 + 2 * a + 1] = fma(wp[a], hxi, acc[36 + 2 * a + 1]);
+    for (int f = 0; f < NFQ; ++f) {
+      double* af = acc + 48 * f;
+      double sh, ch;
+      sincos_table(r, half_k[f], tab, &sh, &ch);
+      const double z = pn.f[f].k * r;
+      const double sh2 = sh + sh, sinz = sh2 * ch, omc = sh2 * sh;  // omc = 1 - cos z
+      // R = s (cos z - 1 + i sin z)
+      const double Rr = -s * omc, Ri = s * sinz;
+      // h(z) = (1 - cos z - z sin z) + i (z cos z - sin z)
+      const double hr = fma(-z, sinz, omc), hi = fma(z, 1.0 - omc, -sinz);
+      const double hyr = hr * fy, hyi = hi * fy, hxr = hr * fx, hxi = hi * fx;
 #pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const double wab = wp[a] * py[b];
-        const int i = 2 * (3 * a + b);
-        acc[i] = fma(wab, Rr, acc[i]);
-        acc[i + 1] = fma(wab, Ri, acc[i + 1]);
-        acc[18 + i] = fma(wab, hyr, acc[18 + i]);
-        acc[18 + i + 1] = fma(wab, hyi, acc[18 + i + 1]);
+      for (int a = 0; a < 3; ++a) {
+        af[36 + 2 * a] = fma(wp[a], hxr, af[36 + 2 * a]);
+        af[36 + 2 * a + 1] = fma(wp[a], hxi, af[36 + 2 * a + 1]);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          const double wab = wp[a] * py[b];
+          const int i = 2 * (3 * a + b);
+          af[i] = fma(wab, Rr, af[i]);
+          af[i + 1] = fma(wab, Ri, af[i + 1]);
+          af[18 + i] = fma(wab, hyr, af[18 + i]);
+          af[18 + i + 1] = fma(wab, hyi, af[18 + i + 1]);
+        }
       }
     }
   }
-  // reduce-scatter: lanes 2m and 2m + 1 end with sums 3m .. 3m + 2, which go to the lanes of
-  // their outputs through shared memory
-  warp_reduce_halving<48, 16>(acc, lane);
-  __shared__ double red[4][48];
+  // reduce-scatter: with one frequency lanes 2m and 2m + 1 end with sums 3m .. 3m + 2, with two
+  // lane m does; they go to the lanes of their outputs through shared memory
+  warp_reduce_halving<NFQ * 48, 16>(acc, lane);
+  __shared__ double red[4][NFQ * 48];
   double* r = red[threadIdx.x >> 5];
-  if ((lane & 1) == 0) {
+  constexpr int kShift = NFQ == 2 ? 0 : 1;
+  if ((lane & kShift) == 0) {
 #pragma unroll
-    for (int j = 0; j < 3; ++j) r[3 * (lane >> 1) + j] = acc[j];
+    for (int j = 0; j < 3; ++j) r[3 * (lane >> kShift) + j] = acc[j];
   }
   __syncwarp();
-  const double2 sum = lane < 21 ? make_double2(r[2 * lane] * P.jac, r[2 * lane + 1] * P.jac) : make_double2(0.0, 0.0);
-  singular_outputs_f64(lane, P, sum, moments + (size_t)kStatic * warp, curls, area, m11m10, p,
-                       out + (size_t)kSingOut * warp);
+#pragma unroll
+  for (int f = 0; f < NFQ; ++f) {
+    const double* rf = r + 48 * f;
+    const double2 sum = lane < 21 ? make_double2(rf[2 * lane] * P.jac, rf[2 * lane + 1] * P.jac) : make_double2(0.0, 0.0);
+    singular_outputs_f64(lane, P, sum, moments + (size_t)kStatic * warp, curls, area, m11m10, pn.f[f],
+                         out + pn.off[f] + (size_t)kSingOut * warp);
+  }
 }
 
 // The mixed form's singular kernel: the Duffy remainder of
@@ -2699,9 +2719,7 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
     if (launched) *launched += nl;
     return cudaGetLastError();
   }
-  const int threads = 128;
-  const int nblk = (int)(((long long)m.npairs * 32 + threads - 1) / threads);
-  for (int f = 0; f < nfreq; ++f) {
+  auto params = [&](int f) {
     SingParams<double> p;
     p.k = k[f];
     p.k2 = k[f] * k[f];
@@ -2711,23 +2729,47 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
     p.cS = c[f].cS;
     p.cK = c[f].cK;
     p.cM10 = c[f].cM10;
+    return p;
+  };
+  const int nblk = (m.npairs + 3) / 4;
+  std::vector<int> direct;
+  for (int f = 0; f < nfreq; ++f) {
     // through the mesh's Chebyshev moments where they hold the terms the frequency needs
     const int nt = use_cheb && m.cheb64 != nullptr && m.cheb64_n > 0 ? cheb_terms(prec, k[f], m.cheb_R) : 0;
-    if (nt > 0 && nt <= m.cheb64_n) {
-      ChebParamsF64 cp{};
-      cheb_coefficients(k[f], m.cheb_R, nt, cp.c1, cp.c2, kChebTol64);
-      cp.p = p;
-      singular_cheb64_kernel<<<(m.npairs + 3) / 4, 128, 0, stream>>>(m.pairs, m.npairs, m.cheb64, nt, m.moments,
-                                                                     m.curls, m.area, m.m11m10, cp,
-                                                                     (double2*)blocks + (size_t)f * blocks_stride);
-      if (cheb_freqs) ++*cheb_freqs;
+    if (nt == 0 || nt > m.cheb64_n) {
+      direct.push_back(f);
       continue;
     }
-    singular_dyn_kernel<<<nblk, threads, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy,
-                                                              m.moments, m.curls, m.area, m.m11m10, p, m.trig,
-                                                              (double2*)blocks + (size_t)f * blocks_stride);
+    ChebParamsF64 cp{};
+    cheb_coefficients(k[f], m.cheb_R, nt, cp.c1, cp.c2, kChebTol64);
+    cp.p = params(f);
+    singular_cheb64_kernel<<<nblk, 128, 0, stream>>>(m.pairs, m.npairs, m.cheb64, nt, m.moments, m.curls, m.area,
+                                                     m.m11m10, cp, (double2*)blocks + (size_t)f * blocks_stride);
+    if (cheb_freqs) ++*cheb_freqs;
+    ++nl;
   }
-  if (launched) *launched += nfreq;
+  // the others point by point, two frequencies sharing each point's geometry
+  auto run = [&](auto nfq_c, size_t i) {
+    constexpr int NFQ = decltype(nfq_c)::value;
+    SingParamsF64N<NFQ> pn;
+    for (int j = 0; j < NFQ; ++j) {
+      pn.f[j] = params(direct[i + j]);
+      pn.off[j] = (long long)direct[i + j] * blocks_stride;
+    }
+    singular_dyn_kernel<NFQ><<<nblk, 128, 0, stream>>>(geo, m.pairs, m.npairs, m.rule_ptr, m.duffy, m.moments, m.curls,
+                                                       m.area, m.m11m10, pn, m.trig, (double2*)blocks);
+    ++nl;
+  };
+  for (size_t i = 0; i < direct.size();) {
+    if (i + 1 < direct.size()) {
+      run(std::integral_constant<int, 2>{}, i);
+      i += 2;
+    } else {
+      run(std::integral_constant<int, 1>{}, i);
+      i += 1;
+    }
+  }
+  if (launched) *launched += nl;
   return cudaGetLastError();
 }
 
