@@ -504,7 +504,7 @@ def main() -> None:
 
     if fp64_workload:
         result["roofline"] = None
-        result["roofline_note"] = "FP64 workload: the regular assembly runs regular_f64_kernel on the FP64 pipe"
+        result["roofline_note"] = "FP64 workload: the regular assembly runs regular_f64_bm_kernel on the FP64 pipe"
 
     if not args.no_extras and rank == 0 and fp64_workload:
         # the FP64 GPU form against the FP64 CPU oracle on one frequency

@@ -468,12 +468,12 @@ __global__ void __launch_bounds__(WARPS * 32, RegularOccupancy<NFQ>::kCtasPerSm)
 // e^{ikr} / r are folded into W[a][b] and S0, each pair adding
 //   jac (cD W[a][b] + (curl_a . curl_b) cH S0).
 //
-// Bound: the FP64 pipe (two lanes per SM and clock).  Per quadrature pair 19 FP64
-// instructions of geometry shared by the NFQ frequencies and about 32 per frequency (phase,
-// table sine and cosine, E'' and its product, sums), against 113 of the one-frequency
-// kernel with library sincos, square root, divide and nine-entry sums of each operator:
-// 1,280 triangles, 16 frequencies: 10.6 -> 5.5 ms per frequency; 3,984 triangles: 91 -> 48.  Two frequencies per
-// launch: four would need 224 KB of accumulators per CTA and spill.
+// Bound: the FP64 pipe (two lanes per SM and clock).  Per quadrature pair 18 FP64
+// instructions of geometry shared by the NFQ frequencies and about 29 per frequency (table
+// sine and cosine, E'' and its product, sums), against 113 of the one-frequency kernel with
+// library sincos, square root, divide and nine-entry sums of each operator: 1,280 triangles,
+// 16 frequencies: 10.6 -> 4.7 ms per frequency; 3,984 triangles: 91 -> 45.  Two frequencies
+// share the geometry: four would need 224 KB of accumulators per CTA and spill.
 // ------------------------------------------------------------------------
 // A launch takes up to kRegGroups64 groups of NFQ (blockIdx.z): a small mesh's launches
 // would each end in a partly filled wave (1,280 triangles: 3.2 waves).
