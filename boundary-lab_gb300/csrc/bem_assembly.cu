@@ -1319,6 +1319,7 @@ __global__ void __launch_bounds__(32, NFQ == 1 ? 16 : 12)
                             float2* __restrict__ out, long long out_stride) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  grid_trigger();
   if (warp >= npairs) return;
   const SingularPair P = pairs[warp];
   const float* G = rec + (size_t)kPairRec * warp;
@@ -1460,6 +1461,7 @@ __global__ void __launch_bounds__(32, NFQ == 1 ? 16 : 12)
       o[9 + a] = rhs;
     }
   }
+  grid_wait();  // chained launches end in order
 }
 
 // ------------------------------------------------------------------------
@@ -2651,6 +2653,16 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
       return p;
     };
     // point by point: two frequencies per launch share each point's geometry; a lone last one runs alone
+    // (launches after the call's first are chained: they share nothing that is written)
+    bool first = true;
+    auto launch = [&](auto kern, const auto& pn, float2* o) {
+      if (first)
+        kern<<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32, m.pairrec, pn, o, blocks_stride);
+      else
+        launch_chained(kern, dim3(m.npairs), 32, 0, stream, m.pairs, m.npairs, m.rule_ptr, m.duffy32, m.pairrec, pn, o,
+                       blocks_stride);
+      first = false;
+    };
     auto direct = [&](int f0, int count) {
       for (int f = f0; f < f0 + count;) {
         float2* o = (float2*)blocks + (size_t)f * blocks_stride;
@@ -2658,14 +2670,12 @@ cudaError_t launch_singular_dyn(const DeviceMesh& m, Precision prec, int nfreq, 
           SingParamsF32N<2> pn;
           pn.f[0] = params(f);
           pn.f[1] = params(f + 1);
-          singular_dyn_f32_kernel<2><<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32,
-                                                                   m.pairrec, pn, o, blocks_stride);
+          launch(singular_dyn_f32_kernel<2>, pn, o);
           f += 2;
         } else {
           SingParamsF32N<1> pn;
           pn.f[0] = params(f);
-          singular_dyn_f32_kernel<1><<<m.npairs, 32, 0, stream>>>(m.pairs, m.npairs, m.rule_ptr, m.duffy32,
-                                                                   m.pairrec, pn, o, blocks_stride);
+          launch(singular_dyn_f32_kernel<1>, pn, o);
           f += 1;
         }
         ++nl;
