@@ -102,6 +102,7 @@ struct bem_context {
   // the extra lanes of a multi-lane sweep (options.lanes > 1): contexts of their own on the
   // same device whose streams and scratch take their share of the batches; created on first use
   std::vector<bem_context*> lanes;
+  int panel_polls = bem::kPanelPolls;  // bem_set_exchange_limit
   // optional per-kernel-family timing (options.profile)
   bool prof = false;
   std::vector<cudaEvent_t> pev;
@@ -553,6 +554,12 @@ long long bem_context_scratch_bytes(const bem_context* ctx) {
   return total;
 }
 
+int bem_set_exchange_limit(bem_context* ctx, int reads) {
+  if (!ctx) return BEM_ERR_INVALID_ARGUMENT;
+  ctx->panel_polls = reads < 0 ? bem::kPanelPolls : reads;
+  return BEM_OK;
+}
+
 int bem_upload_mesh(bem_context* ctx, const double* vertices, int n_vertices, const int* faces, int n_faces,
                     int regular_order, int singular_order, bem_mesh** out) {
   return bem_upload_mesh_symmetric(ctx, vertices, n_vertices, faces, n_faces, regular_order, singular_order,
@@ -996,7 +1003,7 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
   int lu_launches = 0;
   ck(bem::lu_factor_batched(prec, ctx->mats.p, lda, n, B, (int*)ctx->ipiv.p, (int*)ctx->info.p, nb, ctx->cublas,
                             ctx->stream, (bem::LuGemm)o.lu_gemm, tcws, &used_tensor, &tc_err, (int*)ctx->rowmap.p,
-                            &lu_launches, (int*)ctx->perm.p),
+                            &lu_launches, (int*)ctx->perm.p, ctx->panel_polls),
      "LU factorisation");
   // kernels of this batch besides the assembly: the LU with its row permutation, the solves
   // (mixed: 5 + 4 per refinement step), the field (2, +1 mixed, per slice)
@@ -1235,6 +1242,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
       for (int l = 1; l < nl; ++l) {
         bem_context* cl = ctx->lanes[l - 1];
         cl->prof = ctx->prof;
+        cl->panel_polls = ctx->panel_polls;
         threads.emplace_back([&, l, cl] {
           cudaSetDevice(ctx->device);
           try {
@@ -1384,7 +1392,8 @@ int bem_lu_factor_dense(bem_context* ctx, int n, double* a, int* ipiv, int preci
     bool used_tensor = false;
     int* tc_err = nullptr;
     ck(bem::lu_factor_batched(prec, ctx->mats.p, lda, n, 1, (int*)ctx->ipiv.p, (int*)ctx->info.p, 0, ctx->cublas,
-                              ctx->stream, (bem::LuGemm)lu_gemm, tcws, &used_tensor, &tc_err, (int*)ctx->rowmap.p),
+                              ctx->stream, (bem::LuGemm)lu_gemm, tcws, &used_tensor, &tc_err, (int*)ctx->rowmap.p, nullptr,
+                              nullptr, ctx->panel_polls),
        "LU factorisation");
     int info = 0;
     ck(cudaMemcpyAsync(host.data(), ctx->mats.p, host.size(), cudaMemcpyDeviceToHost, ctx->stream), "copy factors");

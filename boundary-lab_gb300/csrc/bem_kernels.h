@@ -165,6 +165,9 @@ int* tc_gemm_error_word(TcGemmPlan* p);
 // the net row permutation of its interchanges to the row-swap kernel.  perm (batch * n
 // ints, may be null) receives the row permutation: (P b)[i] = b[perm[i]].
 constexpr int kRowmapStride = 512;
+// Reads of a word that a register panel's CTA waits for before it gives up (info = -1): two
+// milliseconds or so, where the word takes a microsecond.
+constexpr int kPanelPolls = 1 << 16;
 // Outer block width of the two-level LU (trailing-update depth); a multiple of
 // every cluster panel width (32, 64) and at most the tcgen05 update's K (256).
 // At 256 the trailing matrix is read and written once per 256 columns: with the
@@ -176,7 +179,8 @@ int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm, int batch);
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info,
                               int nb, void* cublas_handle, cudaStream_t stream, LuGemm gemm = LuGemm::Cublas,
                               void* tc_workspace = nullptr, bool* used_tensor = nullptr, int** tc_err = nullptr,
-                              int* rowmap = nullptr, int* n_launches = nullptr, int* perm = nullptr);
+                              int* rowmap = nullptr, int* n_launches = nullptr, int* perm = nullptr,
+                              int polls = kPanelPolls);
 // Solve (LU) X = B in place for nrhs columns per matrix (B stride ldb*nrhs per matrix), working precision.
 cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* ipiv,
                              void* B, long long ldb, int nrhs, int nb, cudaStream_t stream);
@@ -207,7 +211,8 @@ int lu_resident_batch(Precision prec, int n);
 // rowmap: if not null, receives per matrix [count, (dst row, src row) x count]:
 // the net effect of the panel's kb interchanges on any column (at most 2 kb rows).
 cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb, int nb,
-                             int cl, int batch, int* ipiv, int* info, cudaStream_t stream, int* rowmap = nullptr);
+                             int cl, int batch, int* ipiv, int* info, cudaStream_t stream, int* rowmap = nullptr,
+                             int polls = kPanelPolls);
 // Apply a panel's net row permutation (rowmap) to every column outside the panel, and to
 // perm (batch * n ints) when not null.
 cudaError_t lu_swap_rows_batched(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb,

@@ -662,6 +662,7 @@ struct LuJob {
   TcGemmPlan* plan;  // tcgen05 updates (mixed form); null: cuBLAS
   cublasHandle_t h;
   cudaStream_t stream;
+  int polls;         // of the panels' exchange
 };
 
 // U rows [k, k+kb) of columns [c0, c1): U = L^{-1} A with L the unit lower triangle of A[k:k+kb, k:k+kb].
@@ -765,7 +766,7 @@ cudaError_t lu_two_level(const LuJob& j, int NB) {
     for (int j0 = 0; j0 < KB; j0 += nb) {
       const int kb = std::min(nb, KB - j0), kk = k0 + j0;
       BEM_TRY(lu_panel_cluster(j.prec, j.A, j.lda, j.strideA, n, kk, kb, nb, j.cl, j.batch, j.ipiv, j.info, j.stream,
-                               j.rowmap));
+                               j.rowmap, j.polls));
       if (narrow && kb == 32) {
         const int rest = k0 + KB - kk - 32;  // the rest of the outer block
         const int solve_ctas = (rest + 7) / 8;
@@ -830,7 +831,7 @@ int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm, int batch) {
 
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info, int nb,
                               void* cublas_handle, cudaStream_t stream, LuGemm gemm, void* tc_workspace,
-                              bool* used_tensor, int** tc_err, int* rowmap, int* n_launches, int* perm) {
+                              bool* used_tensor, int** tc_err, int* rowmap, int* n_launches, int* perm, int polls) {
   cublasHandle_t h = (cublasHandle_t)cublas_handle;
   cublasSetStream(h, stream);
   const long long strideA = lda * (long long)n;
@@ -859,7 +860,7 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
   // form, or lu_gemm = 1) keeps one level: its kernels for the skinny panel
   // shapes of the two-level schedule are slow.
   if (cluster_panel && rowmap && plan) {
-    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, h, stream};
+    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, h, stream, polls};
     if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, plan != nullptr, perm != nullptr, batch);
     return lu_two_level(job, kOuterBlock);
   }
@@ -868,7 +869,7 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
     const int kb = std::min(nb, n - k);
     if (n_launches) *n_launches += 2 + (n - k - kb > 0 ? 1 + (plan ? 2 : 0) : 0);
     if (cluster_panel) {
-      cudaError_t e = lu_panel_cluster(prec, A, lda, strideA, n, k, kb, nb, ccl, batch, ipiv, info, stream, rowmap);
+      cudaError_t e = lu_panel_cluster(prec, A, lda, strideA, n, k, kb, nb, ccl, batch, ipiv, info, stream, rowmap, polls);
       if (e != cudaSuccess) return e;
     } else if (mixed)
       lu_panel_kernel<float><<<batch, 1024, 0, stream>>>((float2*)A, lda, strideA, n, k, kb, ipiv, info);

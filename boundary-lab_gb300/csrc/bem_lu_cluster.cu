@@ -322,7 +322,9 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_cluster_kernel(typenam
 //  4. the pivot row leaves (lg = j), the row with lg = j takes the pivot's old
 //     lg; every other active row stores l = a[0] / pivot, subtracts l u and
 //     shifts; the next candidate is reduced per warp; CTA barrier.
-// The polls are bounded: a CTA that waits in vain ends its panel with info = -1.
+// The polls are bounded (`polls` reads of a word): a CTA that waits in vain leaves its
+// panel without storing its rows, and info = -1 and an empty row map say so.  No place in
+// memory is computed from words that did not all arrive.
 // A single CTA (CLUSTER = false) replaces 1 and 2 by the owner thread writing the
 // row to its own shared memory and a CTA barrier.
 // Requires a full panel (kb = 32) and chunk <= kRegPanelThreads.
@@ -352,7 +354,6 @@ __device__ __forceinline__ uint2 warp_max_key(uint2 k) {
 // Words of the exchange: 32 bits of payload with the step's tag above them, written and read
 // whole (64-bit accesses are single-copy atomic).  Keys pack (hi, lo): lo's 16 low bits are
 // those of ~row (rows < 10,240; 0 only where there is no candidate), its high ones the tag.
-constexpr int kPollLimit = 1 << 16;
 __device__ __forceinline__ void push_words(void* dst, unsigned long long a, unsigned long long b) {
   asm volatile("st.relaxed.cluster.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(a), "l"(b) : "memory");
 }
@@ -379,7 +380,7 @@ __device__ __forceinline__ ulonglong2 poll_words(const unsigned long long* p) {
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float2* A, long long lda, long long strideA,
                                                                            int n, int k, int kb, int chunk, int* ipiv,
-                                                                           int* info, int* rowmap) {
+                                                                           int* info, int* rowmap, int polls) {
   constexpr int NB = 32;
   constexpr int NW = kRegPanelWarps;
   cg::cluster_group cluster = cg::this_cluster();
@@ -393,8 +394,11 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
   __shared__ __align__(16) float4 urow[2][NB / 2];  // the pivot row for broadcast reads (CLUSTER: [0]; else by step parity)
   __shared__ __align__(16) float4 pub[NB / 2];
   __shared__ uint2 wkey[2][NW];  // by step parity
-  __shared__ int s_failed;
-  __shared__ int s_moved;  // rows that changed place (rank 0's counts for the cluster)
+  // this CTA gave up waiting, by step parity: a warp that reads it behind the barrier of step j
+  // must not see what a faster one writes in step j + 1
+  __shared__ int s_failed[2];
+  __shared__ int s_any_failed;  // any CTA did (rank 0's)
+  __shared__ int s_moved;       // rows that changed place (rank 0's counts for the cluster)
   float2* M = A + (size_t)blockIdx.y * strideA;
   int* piv = ipiv + (size_t)blockIdx.y * n;
   const int m = n - k;
@@ -405,7 +409,8 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
   int done_at = -1;          // step at which this row became the pivot row
   if (tid == 0) {
     s_moved = 0;
-    s_failed = 0;
+    s_failed[0] = s_failed[1] = 0;
+    s_any_failed = 0;
   }
   if constexpr (CLUSTER) {  // no tag of an earlier use in the slots when the first push arrives
     for (int i = tid; i < 2 * 16 * 2 * NB; i += kRegPanelThreads) (&rowsT[0][0][0])[i] = 0ull;
@@ -460,22 +465,24 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
     int p = (int)~key.y;
     if constexpr (CLUSTER) {
       unsigned long long kw = 0ull;
-      bool ok = false;
-      for (int it = 0; it < kPollLimit && !ok; ++it) {
+      bool ok;
+      int left = polls;
+      do {  // the bound's test below the read: on top, LU of one matrix of order 4,976 took 11.3 ms, here 10.7
         if (lane < CL) kw = poll_word(&keyT[s][lane]);
         ok = __all_sync(0xffffffffu, lane >= CL || ((unsigned)kw >> 16) == tag);
-      }
+      } while (!ok && --left > 0);
       const uint2 ck = lane < CL ? make_uint2((unsigned)(kw >> 32), (unsigned)kw & 0xffffu) : make_uint2(0u, 0u);
       key = warp_max_key(ck);
       const int pr = __ffs(__ballot_sync(0xffffffffu, ck.x == key.x && ck.y == key.y)) - 1;  // keys are distinct
       p = (int)(~key.y & 0xffffu);
       ulonglong2 u = make_ulonglong2(0ull, 0ull);
-      bool got = false;
-      for (int it = 0; it < kPollLimit && ok && !got; ++it) {
+      bool got;
+      left = polls;
+      do {
         u = poll_words(&rowsT[s][pr][2 * lane]);
         got = __all_sync(0xffffffffu, (unsigned)(u.x >> 32) == tag && (unsigned)(u.y >> 32) == tag);
-      }
-      if (!got) s_failed = 1;
+      } while (!got && --left > 0);
+      if (!(ok && got) || polls == 0) s_failed[s] = 1;  // this warp's p is worth nothing: no row is stored
       // every warp writes the same values; the barrier that ends the step keeps step j + 1's away
       reinterpret_cast<float2*>(urow[0])[lane] = make_float2(__uint_as_float((unsigned)u.x), __uint_as_float((unsigned)u.y));
       __syncwarp();
@@ -531,15 +538,14 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
     }
     publish_warp_key(s ^ 1);
     __syncthreads();
-    if (CLUSTER && s_failed) {  // uniform in the CTA; the other CTAs wait in vain in turn
-      if (tid == 0) info[blockIdx.y] = -1;
-      break;
-    }
+    if (CLUSTER && s_failed[s]) break;  // uniform in the CTA; the other CTAs wait in vain in turn
   }
   grid_trigger();
+  const bool failed = CLUSTER && (s_failed[0] | s_failed[1]);
+  if (CLUSTER && failed && tid == 0) *cluster.map_shared_rank(&s_any_failed, 0) = 1;
   // every row to its logical position: the multipliers left of its pivot column
   // (all 32 for rows that never became the pivot)
-  if (mine) {
+  if (mine && !failed) {
     const int ncol = done_at < 0 ? NB : done_at;
     float2* dst = M + (size_t)k * lda + k + lg;
     for (int c = 0; c < ncol; ++c) dst[(size_t)c * lda] = Lb[(size_t)c * kRegPanelThreads + tid];
@@ -547,7 +553,7 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
   // the net row permutation, [count, (dst row, src row) x count] in any order (at most 2 kb rows move)
   if (rowmap != nullptr) {
     int* rm = rowmap + (size_t)blockIdx.y * kRowmapStride;
-    if (mine && lg != r0 + tid) {
+    if (mine && !failed && lg != r0 + tid) {
       const int e = atomicAdd(CLUSTER ? cluster.map_shared_rank(&s_moved, 0) : &s_moved, 1);
       rm[1 + 2 * e] = k + lg;
       rm[2 + 2 * e] = k + r0 + tid;
@@ -555,7 +561,11 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
     if constexpr (!CLUSTER) __syncthreads();
   }
   if constexpr (CLUSTER) cluster.sync();  // no CTA leaves while others may still use its shared memory
-  if (rowmap != nullptr && rank == 0 && tid == 0) rowmap[(size_t)blockIdx.y * kRowmapStride] = s_moved;
+  if (rank == 0 && tid == 0) {
+    const bool gave_up = CLUSTER && s_any_failed;
+    if (gave_up) info[blockIdx.y] = -1;
+    if (rowmap != nullptr) rowmap[(size_t)blockIdx.y * kRowmapStride] = gave_up ? 0 : s_moved;
+  }
 }
 
 // The register-resident panel of the FP64 form: the algorithm of lu_panel_reg_kernel with
@@ -590,7 +600,7 @@ __device__ __forceinline__ double untagged(ulonglong2 w) { return __hiloint2doub
 
 __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double2* A, long long lda, long long strideA,
                                                                           int n, int k, int kb, int chunk, int* ipiv,
-                                                                          int* info, int* rowmap) {
+                                                                          int* info, int* rowmap, int polls) {
   constexpr int NB = 32;
   constexpr int NW = kReg64Warps;
   cg::cluster_group cluster = cg::this_cluster();
@@ -604,8 +614,11 @@ __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double
   __shared__ __align__(16) double2 pub[NB + 1];                // the candidate row and its reciprocal
   __shared__ __align__(16) double2 urow[NB + 1];               // the pivot row and its reciprocal
   __shared__ uint3 wkey[2][NW];                                // by step parity
-  __shared__ int s_failed;
-  __shared__ int s_moved;  // rows that changed place (rank 0's counts for the cluster)
+  // this CTA gave up waiting, by step parity: a warp that reads it behind the barrier of step j
+  // must not see what a faster one writes in step j + 1
+  __shared__ int s_failed[2];
+  __shared__ int s_any_failed;  // any CTA did (rank 0's)
+  __shared__ int s_moved;       // rows that changed place (rank 0's counts for the cluster)
   double2* M = A + (size_t)blockIdx.y * strideA;
   int* piv = ipiv + (size_t)blockIdx.y * n;
   const int m = n - k;
@@ -626,7 +639,8 @@ __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double
   };
   if (tid == 0) {
     s_moved = 0;
-    s_failed = 0;
+    s_failed[0] = s_failed[1] = 0;
+    s_any_failed = 0;
   }
   publish_warp_key(0);
   // no tag of an earlier use in the slots when the first push arrives
@@ -671,18 +685,20 @@ __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double
     }
     // 2. pivot (logical row p, held by CTA pr), in every warp; row j itself is a candidate, so there is one
     ulonglong2 kw = make_ulonglong2(0ull, 0ull);
-    bool ok = false;
-    for (int it = 0; it < kPollLimit && !ok; ++it) {
+    bool ok;
+    int left = polls;
+    do {
       if (lane < CL) kw = poll_words(&keyT[s][lane][0]);
       ok = __all_sync(0xffffffffu, lane >= CL || (((unsigned)kw.x >> 16) == tag && (unsigned)kw.y == tag));
-    }
+    } while (!ok && --left > 0);
     const uint3 ck = lane < CL ? make_uint3((unsigned)(kw.x >> 32), (unsigned)(kw.y >> 32), (unsigned)kw.x & 0xffffu)
                                : make_uint3(0u, 0u, 0u);
     key = warp_max_key(ck);
     const int pr = __ffs(__ballot_sync(0xffffffffu, ck.x == key.x && ck.y == key.y && ck.z == key.z)) - 1;  // distinct
     const int p = (int)(~key.z & 0xffffu);
-    bool got = false;
-    for (int it = 0; it < kPollLimit && ok && !got; ++it) {
+    bool got;
+    left = polls;
+    do {
       const unsigned long long* src = rowsT[s][pr];
       const ulonglong2 re = poll_words(src + 4 * lane), im = poll_words(src + 4 * lane + 2);
       const ulonglong2 ire = poll_words(src + 4 * NB), iim = poll_words(src + 4 * NB + 2);
@@ -693,8 +709,8 @@ __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double
         urow[lane] = make_double2(untagged(re), untagged(im));
         if (lane == 0) urow[NB] = make_double2(untagged(ire), untagged(iim));
       }
-    }
-    if (!got) s_failed = 1;
+    } while (!got && --left > 0);
+    if (!(ok && got) || polls == 0) s_failed[s] = 1;
     __syncwarp();
     if (rank == 0 && wid == 0 && lane < NB - j) M[(size_t)(k + j + lane) * lda + k + j] = urow[lane];  // U row j
     if (rank == 0 && tid == 0) {
@@ -736,26 +752,28 @@ __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double
     }
     publish_warp_key(s ^ 1);
     __syncthreads();
-    if (s_failed) {  // uniform in the CTA; the other CTAs wait in vain in turn
-      if (tid == 0) info[blockIdx.y] = -1;
-      break;
-    }
+    if (s_failed[s]) break;  // uniform in the CTA; the other CTAs wait in vain in turn
   }
+  const bool failed = s_failed[0] | s_failed[1];
+  if (failed && tid == 0) *cluster.map_shared_rank(&s_any_failed, 0) = 1;
   // every row to its logical position: the multipliers left of its pivot column
   // (all 32 for rows that never became the pivot)
-  if (mine) {
+  if (mine && !failed) {
     const int ncol = done_at < 0 ? NB : done_at;
     double2* dst = M + (size_t)k * lda + k + lg;
     for (int c = 0; c < ncol; ++c) dst[(size_t)c * lda] = Lb[(size_t)c * kReg64Threads + tid];
   }
-  if (rowmap != nullptr && mine && lg != r0 + tid) {  // the net row permutation, as above
+  if (rowmap != nullptr && mine && !failed && lg != r0 + tid) {  // the net row permutation, as above
     int* rm = rowmap + (size_t)blockIdx.y * kRowmapStride;
     const int e = atomicAdd(cluster.map_shared_rank(&s_moved, 0), 1);
     rm[1 + 2 * e] = k + lg;
     rm[2 + 2 * e] = k + r0 + tid;
   }
   cluster.sync();  // no CTA leaves while others may still use its shared memory
-  if (rowmap != nullptr && rank == 0 && tid == 0) rowmap[(size_t)blockIdx.y * kRowmapStride] = s_moved;
+  if (rank == 0 && tid == 0) {
+    if (s_any_failed) info[blockIdx.y] = -1;
+    if (rowmap != nullptr) rowmap[(size_t)blockIdx.y * kRowmapStride] = s_any_failed ? 0 : s_moved;
+  }
 }
 
 // perm[i] such that (P b)[i] = b[perm[i]], from LAPACK-style interchanges.
@@ -1161,10 +1179,10 @@ int lu_resident_batch(Precision prec, int n) {
 }
 
 cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb, int nb,
-                             int cl, int batch, int* ipiv, int* info, cudaStream_t stream, int* rowmap) {
+                             int cl, int batch, int* ipiv, int* info, cudaStream_t stream, int* rowmap, int polls) {
   const int m = n - k;
   const int chunk = (m + cl - 1) / cl;
-  void* args[] = {&A, &lda, &strideA, &n, &k, &kb, (void*)&chunk, &ipiv, &info, &rowmap};
+  void* args[] = {&A, &lda, &strideA, &n, &k, &kb, (void*)&chunk, &ipiv, &info, &rowmap, &polls};  // polls: register panels
   dim3 grid(cl, batch);
   if (prec == Precision::Mixed && nb == 32 && chunk <= kRegPanelThreads && kb == 32) {
     const size_t sm = (size_t)32 * kRegPanelThreads * sizeof(float2);

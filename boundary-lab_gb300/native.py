@@ -52,6 +52,7 @@ EXPORTED_SYMBOLS = (
     "bem_lu_factor_dense",
     "bem_trim_context",
     "bem_context_scratch_bytes",
+    "bem_set_exchange_limit",
 )
 
 
@@ -207,6 +208,8 @@ def load(build_if_missing: bool = False) -> ctypes.CDLL:
         lib.bem_trim_context.restype = ip
         lib.bem_context_scratch_bytes.argtypes = [vp]
         lib.bem_context_scratch_bytes.restype = ctypes.c_longlong
+        lib.bem_set_exchange_limit.argtypes = [vp, ip]
+        lib.bem_set_exchange_limit.restype = ip
         # allocation-free field evaluation: every pointer is a caller-owned device buffer
         lib.bem_evaluate_field_noalloc.argtypes = [vp, ip, vp, ip, ip, ctypes.c_double, vp, vp, vp, ip, ip, vp, vp,
                                                    ctypes.c_char_p, ip]
@@ -327,6 +330,11 @@ class Context:
     def trim(self) -> None:
         """Free this context's solve scratch and return unused pool memory (bem_trim_context)."""
         self._check(self._lib.bem_trim_context(self._h))
+
+    def set_exchange_limit(self, reads: int = -1) -> None:
+        """Reads after which the LU panels' exchange gives up (bem_set_exchange_limit); negative:
+        the default."""
+        self._check(self._lib.bem_set_exchange_limit(self._h, int(reads)))
 
     @property
     def scratch_bytes(self) -> int:

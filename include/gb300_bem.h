@@ -72,6 +72,12 @@ void* bem_context_stream(const bem_context* ctx);
 int bem_trim_context(bem_context* ctx);
 long long bem_context_scratch_bytes(const bem_context* ctx);
 
+/* Reads of a word after which the LU panels' exchange between the CTAs of a cluster gives
+ * up waiting for it (negative: the default, 65,536, a thousand times what a word takes).  A
+ * call whose exchange gives up returns BEM_ERR_CUDA and leaves the context usable; 0 makes
+ * every exchange give up at once, for a caller that tests its own error handling. */
+int bem_set_exchange_limit(bem_context* ctx, int reads);
+
 /* Upload a triangle mesh and build every frequency-independent cache: face
  * geometry and surface curls, the regular rule, singular (vertex-sharing) pair
  * list with remapped Duffy rules, and the k-independent singular moments (FP64
