@@ -30,14 +30,6 @@ template <> struct CT<double> { typedef double2 C2; };
 
 template <typename C2> __device__ __forceinline__ auto cabs1(C2 v) -> decltype(v.x) { return fabs(v.x) + fabs(v.y); }
 
-template <typename C2> __device__ __forceinline__ C2 cinv(C2 d) {
-  auto m = d.x * d.x + d.y * d.y;
-  C2 r;
-  r.x = d.x / m;
-  r.y = -d.y / m;
-  return r;
-}
-
 template <typename R>
 __global__ void __launch_bounds__(1024) lu_panel_kernel(typename CT<R>::C2* A, long long lda, long long strideA, int n,
                                                         int k, int kb, int* ipiv, int* info) {
@@ -112,7 +104,7 @@ __global__ void __launch_bounds__(1024) lu_panel_kernel(typename CT<R>::C2* A, l
       inv.y = R(0);
       if (tid == 0 && info[blockIdx.x] == 0) info[blockIdx.x] = col + 1;
     } else {
-      inv = cinv(d);
+      inv = pivot_inverse<true>(d);
     }
     for (int r = col + 1 + tid; r < n; r += blockDim.x) {
       C2 l = cmul(M[(size_t)col * lda + r], inv);
@@ -603,7 +595,7 @@ __global__ void __launch_bounds__(1024) lu_solve_kernel(const typename CT<R>::C2
         C2 xj;
         if (lane == j) {
           const C2 d = M[(size_t)(k0 + j) * lda + k0 + j];
-          v = cmul(v, cinv(d));
+          v = cmul(v, pivot_inverse<true>(d));
         }
         xj.x = __shfl_sync(0xffffffffu, v.x, j);
         xj.y = __shfl_sync(0xffffffffu, v.y, j);

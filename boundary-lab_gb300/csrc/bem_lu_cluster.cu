@@ -40,14 +40,6 @@ template <> struct CT2<double> { typedef double2 C2; };
 
 template <typename C2> __device__ __forceinline__ auto abs1(C2 v) -> decltype(v.x) { return fabs(v.x) + fabs(v.y); }
 
-template <typename C2> __device__ __forceinline__ C2 inverse(C2 d) {
-  auto m = d.x * d.x + d.y * d.y;
-  C2 r;
-  r.x = d.x / m;
-  r.y = -d.y / m;
-  return r;
-}
-
 constexpr int kPanelThreads = 512;
 
 // First maximum of (value, index): larger value wins, ties go to the smaller index
@@ -270,7 +262,7 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_cluster_kernel(typenam
       inv.y = R(0);
       if (rank == 0 && tid == 0 && info[blockIdx.y] == 0) info[blockIdx.y] = k + j + 1;
     } else {
-      inv = inverse(d);
+      inv = pivot_inverse<true>(d);
     }
     const int i0 = min(rows, max(0, j + 1 - r0));  // first local row below the diagonal
     C2* Pcol = P + (size_t)j * chunk;
@@ -491,14 +483,8 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
       M[(size_t)(k + j + lane) * lda + k + j] = reinterpret_cast<const float2*>(U)[lane];
     if (rank == 0 && tid == 0) piv[k + j] = k + p;
     const float2 d = make_float2(U[0].x, U[0].y);
-    float2 inv;
-    if (d.x == 0.f && d.y == 0.f) {
-      inv = make_float2(0.f, 0.f);
-      if (rank == 0 && tid == 0 && info[blockIdx.y] == 0) info[blockIdx.y] = k + j + 1;
-    } else {  // one reciprocal instead of two divisions on the step's critical path
-      const float rm = __frcp_rn(fmaf(d.x, d.x, d.y * d.y));
-      inv = make_float2(d.x * rm, -d.y * rm);
-    }
+    const float2 inv = pivot_inverse(d);
+    if (rank == 0 && tid == 0 && d.x == 0.f && d.y == 0.f && info[blockIdx.y] == 0) info[blockIdx.y] = k + j + 1;
     // 4. this thread's row
     if (mine && done_at < 0) {
       if (lg == p) {  // the pivot row: it is logical row j now, finished
@@ -663,12 +649,7 @@ __global__ void __launch_bounds__(kReg64Threads, 1) lu_panel_reg64_kernel(double
       if (own) {
 #pragma unroll
         for (int q = 0; q < NB; ++q) pub[q] = a[q];
-        if (a[0].x == 0. && a[0].y == 0.) {
-          pub[NB] = make_double2(0., 0.);
-        } else {  // one reciprocal instead of two divisions on the step's critical path
-          const double rm = __drcp_rn(fma(a[0].x, a[0].x, a[0].y * a[0].y));
-          pub[NB] = make_double2(a[0].x * rm, -a[0].y * rm);
-        }
+        pub[NB] = pivot_inverse(a[0]);
       }
       __syncwarp();
       for (int c = lane; c < NB + 1; c += 32) {
@@ -934,7 +915,7 @@ __global__ void __launch_bounds__(kSolveThreads) lu_solve_cluster_kernel(const t
       C2 dinv;
       dinv.x = 0;
       dinv.y = 0;
-      if (lane < kb) dinv = inverse(M[(size_t)(k0 + lane) * lda + k0 + lane]);
+      if (lane < kb) dinv = pivot_inverse<true>(M[(size_t)(k0 + lane) * lda + k0 + lane]);
       C2 v;
       v.x = 0;
       v.y = 0;

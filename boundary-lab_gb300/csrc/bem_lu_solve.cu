@@ -35,11 +35,6 @@ template <int CPW> constexpr size_t inverse_smem() {
   return ((size_t)kInvStages * 32 * 32 + (size_t)kInvWarps * kOuterBlock * CPW) * sizeof(float2);
 }
 
-__device__ __forceinline__ float2 cinv_or_zero(float2 d) {
-  const float m = d.x * d.x + d.y * d.y;
-  return m > 0.f ? make_float2(d.x / m, -d.y / m) : make_float2(0.f, 0.f);
-}
-
 // inv[(mat, block K, side)] = inverse of the unit lower (side 0) or the upper (side 1)
 // triangle of diagonal block K, column-major 256 x 256; rows and columns beyond the matrix
 // are zero.  The upper triangle is taken in reversed row and column order, where it is a
@@ -108,7 +103,7 @@ __device__ void block_inverse(const float2* __restrict__ D, long long lda, int K
         continue;
       }
       float2 dinv = make_float2(1.f, 0.f);
-      if (REV) dinv = cinv_or_zero(T[32 * rl + rl]);
+      if (REV) dinv = pivot_inverse<true>(T[32 * rl + rl]);  // zero beyond the matrix
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const float2 lv = T[32 * (REV ? 31 - j : j) + rl];
