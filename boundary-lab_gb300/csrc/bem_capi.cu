@@ -1157,6 +1157,46 @@ bool valid_freqs(bem_context* ctx, const double* freqs_hz, int n_freq) {
     }
   return true;
 }
+
+// How bem_solve_frequencies runs a call: the batch, and the lanes that its batches are dealt to.
+struct CallPlan {
+  int batch, lanes;
+};
+CallPlan plan_call(int nv, bem::Precision prec, int n_freq, int batch, int lanes) {
+  int B = batch > 0 ? std::min(batch, 64) : auto_batch_order(nv, prec, n_freq);
+  B = std::min(B, n_freq);
+  if (batch <= 0 && lanes >= 2 && B == n_freq) B = lane_split(n_freq);
+  const int nbatch = (n_freq + B - 1) / B;
+  return {B, std::max(1, std::min({lanes, kMaxLanes, nbatch}))};
+}
+
+// Device bytes of a mesh with npairs singular pairs: pairs, records, moments and scatter plan,
+// face records (and their lane-group copy) and maps.
+long long mesh_bytes(int nf, int npairs, bem::Precision prec) {
+  return (long long)npairs * (24 * 8 + 48 + (bem::kPairRec + bem::kPairGeoDf) * 4 + 96) +
+         (long long)bem::cheb_moment_bytes(prec, npairs) + (long long)nf * (2 * 160 + 288 + 64);
+}
+
+// Scratch of one lane (a context) that solves batches of `batch` frequencies.
+long long lane_bytes(int nv, int nf, int npairs, int nrhs, int npts, int batch, bem::Precision prec) {
+  const bool mixed = prec == bem::Precision::Mixed;
+  const long long esz = mixed ? sizeof(float2) : sizeof(double2);
+  const long long lda = round_up(nv, 32);
+  const long long n_ext = (long long)(nv * 1.3) + 64;
+  // frequencies assembled together: those of a regular launch, or a batch's within kRextBytes
+  const long long rext = round_up(n_ext, 32) * 3LL * nf * esz;
+  const long long group =
+      std::max<long long>(mixed ? 4 : 2, std::min<long long>(batch, (long long)kRextBytes / std::max(rext, 1LL)));
+  long long bytes = rext * group;                                           // extended rows
+  bytes += (long long)nf * 3 * nrhs * esz * group;                          // right-hand-side face values
+  bytes += (long long)npairs * 12 * esz * group;                            // singular blocks
+  bytes += (long long)batch * lda * nv * esz * (mixed ? 2 : 1);             // matrices (+copy)
+  bytes += (long long)batch * nrhs * lda * (esz + (2 + bem::kResidualSplits) * 16 + 16);  // rhs, x, residual parts, d
+  if (mixed) bytes += (long long)bem::lu_inverse_bytes(nv, batch);          // block inverses
+  bytes += (long long)batch * nrhs * ((long long)nf * 6 * esz + (long long)npts * 16);  // field sources + out
+  if (mixed) bytes += (long long)bem::tc_gemm_workspace_bytes(nv, batch);   // tensor-core update operands
+  return bytes + (64LL << 20);                                              // cuBLAS workspace and slack
+}
 }  // namespace
 
 extern "C" {
@@ -1169,28 +1209,15 @@ int bem_auto_batch(bem_mesh* m, int precision, int n_freq) {
 }
 
 long long bem_estimate_device_bytes(int nv, int nf, int npairs, int nrhs, int npts, int batch, int precision) {
-  const long long esz = precision == BEM_PRECISION_MIXED ? 8 : 16;
-  const long long lda = round_up(nv, 32);
-  const long long n_ext = (long long)(nv * 1.3) + 64;
-  long long bytes = 0;
-  // frequencies assembled together: those of a regular launch, or a batch's within kRextBytes
-  // (on each of two lanes)
-  const long long rext = round_up(n_ext, 32) * 3LL * nf * esz;
-  const long long group = std::max<long long>(precision == BEM_PRECISION_MIXED ? 4 : 2,
-                                              std::min<long long>(batch, 2LL * kRextBytes / std::max(rext, 1LL)));
-  bytes += rext * group;                                                    // extended rows
-  bytes += (long long)nf * 3 * nrhs * esz * group;                          // right-hand-side face values
-  bytes += (long long)batch * lda * nv * esz * (precision == BEM_PRECISION_MIXED ? 2 : 1);  // matrices (+copy)
-  bytes += (long long)npairs * (12 * esz * group + 24 * 8 + 48 + (bem::kPairRec + bem::kPairGeoDf) * 4 + 96 +
-                                (long long)bem::cheb_moment_bytes(precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64, 1));  // singular blocks, moments, pairs, records, scatter plan, Chebyshev moments
-  bytes += (long long)batch * nrhs * lda * (esz + (2 + bem::kResidualSplits) * 16 + 16);  // rhs, x, residual parts, d
-  if (precision == BEM_PRECISION_MIXED) bytes += (long long)bem::lu_inverse_bytes(nv, batch);  // block inverses
-  bytes += (long long)batch * nrhs * ((long long)nf * 6 * esz + (long long)npts * 16);  // field sources + out
-  bytes += (long long)nf * (2 * 160 + 288 + 64);                            // face records (+ lane-group copy), maps
-  if (precision == BEM_PRECISION_MIXED)                                      // tensor-core update operands
-    bytes += (long long)bem::tc_gemm_workspace_bytes(nv, batch);
-  bytes += 64LL << 20;                                                      // cuBLAS workspace and slack
-  return bytes;
+  const bem::Precision prec = precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64;
+  return mesh_bytes(nf, npairs, prec) + lane_bytes(nv, nf, npairs, nrhs, npts, batch, prec);
+}
+
+long long bem_estimate_solve_bytes(int nv, int nf, int npairs, int nrhs, int npts, int n_freq, int batch, int lanes,
+                                   int precision) {
+  const bem::Precision prec = precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64;
+  const CallPlan p = plan_call(nv, prec, std::max(1, n_freq), batch, lanes);
+  return mesh_bytes(nf, npairs, prec) + p.lanes * lane_bytes(nv, nf, npairs, nrhs, npts, p.batch, prec);
 }
 
 int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const bem_solve_options* opt,
@@ -1214,9 +1241,8 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
     }
     const bem::DeviceMesh& dm = m->dm;
     const int nv = dm.nv, nc = m->nc;
-    int B = o.batch > 0 ? std::min(o.batch, 64) : auto_batch(m, prec, n_freq);
-    B = std::min(B, n_freq);
-    if (o.batch <= 0 && o.lanes >= 2 && B == n_freq) B = lane_split(n_freq);
+    const CallPlan plan = plan_call(nv, prec, n_freq, o.batch, o.lanes);
+    const int B = plan.batch, nl = plan.lanes;
     ctx->prof = o.profile != 0;
     const int nbatch = (n_freq + B - 1) / B;
     auto slice_of = [&](int bi) {
@@ -1225,7 +1251,6 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
                    field_out ? field_out + 2 * (size_t)f0 * nc * m->nobs : nullptr, cheb};
     };
     SolveTotals T;
-    const int nl = std::max(1, std::min({o.lanes, kMaxLanes, nbatch}));
     if (nl >= 2) {
       // batch bi goes to lane bi % nl: lane 0 is this context, the others are helper contexts
       // driven from their own host threads; the mesh is shared read-only

@@ -97,19 +97,19 @@ class CudaEngine:
 
     def device_bytes(self, n_freq: int) -> int:
         """Device memory of a solve of n_freq frequencies on this mesh: the mesh caches plus the
-        scratch of the batch the solve will use (bem_estimate_device_bytes)."""
+        scratch of the batches the solve will hold (bem_estimate_solve_bytes)."""
         if self.mesh is None:
             raise RuntimeError("engine.prepare() must run before device_bytes()")
         prec = PRECISIONS[self.precision]
         with self.lock:
-            batch = self.batch or self.mesh.auto_batch(n_freq, prec)
+            batch = self.batch  # 0: the library's own, split over the lanes where one batch would hold the call
             if self.autotune and not self.batch:
                 # the tuner tries up to one frequency more than the library's own batch
-                batch = self.launch.batch if self.launch is not None else min(batch + 1, max(1, n_freq))
-            lanes = self.lanes if n_freq >= 2 * batch else 1  # each lane holds a batch's scratch
-            return self.ctx.estimate_device_bytes(self.mesh.n_vertices, self.mesh.n_faces,
-                                                  self.mesh.n_singular_pairs, self.n_rhs, self.n_points,
-                                                  batch * lanes, prec)
+                batch = (self.launch.batch if self.launch is not None
+                         else min(self.mesh.auto_batch(n_freq, prec) + 1, max(1, n_freq)))
+            return self.ctx.estimate_solve_bytes(self.mesh.n_vertices, self.mesh.n_faces,
+                                                 self.mesh.n_singular_pairs, self.n_rhs, self.n_points, n_freq,
+                                                 batch, self.lanes, prec)
 
     def preferred_chunk(self, n_freq: int) -> int:
         """Frequencies per solve call for a sweep of n_freq: one batch of the size the solve

@@ -46,6 +46,7 @@ EXPORTED_SYMBOLS = (
     "bem_assemble_lhs",
     "bem_apply_rhs_operator",
     "bem_estimate_device_bytes",
+    "bem_estimate_solve_bytes",
     "bem_auto_batch",
     "bem_evaluate_field",
     "bem_evaluate_field_noalloc",
@@ -200,6 +201,8 @@ def load(build_if_missing: bool = False) -> ctypes.CDLL:
         lib.bem_lu_factor_dense.restype = ip
         lib.bem_estimate_device_bytes.argtypes = [ip, ip, ip, ip, ip, ip, ip]
         lib.bem_estimate_device_bytes.restype = ctypes.c_longlong
+        lib.bem_estimate_solve_bytes.argtypes = [ip, ip, ip, ip, ip, ip, ip, ip, ip]
+        lib.bem_estimate_solve_bytes.restype = ctypes.c_longlong
         lib.bem_auto_batch.argtypes = [vp, ip, ip]
         lib.bem_auto_batch.restype = ip
         lib.bem_evaluate_field.argtypes = [vp, ctypes.c_double, ip, dp, dp, dp, ip, dp]
@@ -326,6 +329,12 @@ class Context:
     def estimate_device_bytes(self, n_vertices: int, n_faces: int, n_pairs: int, n_rhs: int, n_points: int,
                               batch: int, precision: int) -> int:
         return int(self._lib.bem_estimate_device_bytes(n_vertices, n_faces, n_pairs, n_rhs, n_points, batch, precision))
+
+    def estimate_solve_bytes(self, n_vertices: int, n_faces: int, n_pairs: int, n_rhs: int, n_points: int,
+                             n_freq: int, batch: int, lanes: int, precision: int) -> int:
+        """Device bytes of a Mesh.solve call with every lane it uses (bem_estimate_solve_bytes)."""
+        return int(self._lib.bem_estimate_solve_bytes(n_vertices, n_faces, n_pairs, n_rhs, n_points, n_freq, batch,
+                                                      lanes, precision))
 
     def trim(self) -> None:
         """Free this context's solve scratch and return unused pool memory (bem_trim_context)."""

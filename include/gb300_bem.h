@@ -283,10 +283,16 @@ int bem_evaluate_field_noalloc(const double* d_vertices, int n_vertices, const i
  * on a zero pivot. */
 int bem_lu_factor_dense(bem_context* ctx, int n, double* a, int* ipiv, int precision, int lu_gemm);
 
-/* Device bytes needed to solve `batch` frequencies of a mesh of this size
- * (scratch + matrices + factors), for admission control by a scheduler. */
+/* Device bytes needed to solve `batch` frequencies of a mesh of this size on one
+ * lane (scratch + matrices + factors), for admission control by a scheduler. */
 long long bem_estimate_device_bytes(int n_vertices, int n_faces, int n_singular_pairs, int n_rhs, int n_points,
                                     int batch, int precision);
+/* Device bytes of a bem_solve_frequencies call of n_freq frequencies with these
+ * batch and lanes options: as above, with the scratch of every lane that the call
+ * will use (a batch split over two lanes holds its extended rows and singular
+ * blocks twice). */
+long long bem_estimate_solve_bytes(int n_vertices, int n_faces, int n_singular_pairs, int n_rhs, int n_points,
+                                   int n_freq, int batch, int lanes, int precision);
 
 #ifdef __cplusplus
 }
