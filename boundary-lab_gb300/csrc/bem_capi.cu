@@ -911,15 +911,18 @@ struct SolveTotals {
 // each slice's field is evaluated on its own mesh.  The identity block cannot
 // change a pivot (its rows are zero in the mesh's columns), so each mesh's
 // factors are those of its own matrix.  Every slice has the same number of
-// excitations nc.
+// excitations nc.  rule_batch > 0: the batch that the rules go by which choose between orders
+// of sums (CallPlan).
 void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const bem_solve_options& o, int nc,
-                    SolveTotals& T) {
+                    SolveTotals& T, int rule_batch = 0) {
   const bem::Precision prec = o.precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64;
   const bool mixed = prec == bem::Precision::Mixed;
   const size_t esz = mixed ? sizeof(float2) : sizeof(double2);
   const long long lda = round_up(n, 32), ldb = round_up(n, 32);
   int B = 0;
   for (const Slice& x : sl) B += x.cnt;
+  if (rule_batch <= 0) rule_batch = B;
+  const bool one_slice = sl.size() == 1;
   const int nb = o.lu_block > 0 ? std::min(o.lu_block, 64) : 0;  // 0: the LU chooses
   const size_t matsz = (size_t)lda * n * esz;
   ck(ctx->mats.ensure(matsz * B), "alloc matrices");
@@ -932,7 +935,7 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
   ck(ctx->b32.ensure(vecn * esz), "alloc rhs");
   if (mixed) {
     ck(ctx->x64.ensure(vecn * sizeof(double2)), "alloc x");
-    ck(ctx->r64.ensure(vecn * sizeof(double2) * bem::residual_splits(n, B * nc)), "alloc residual parts");
+    ck(ctx->r64.ensure(vecn * sizeof(double2) * bem::residual_splits(n, rule_batch * nc)), "alloc residual parts");
     if (bem::lu_solve_blocks_fits(n)) ck(ctx->inv.ensure(bem::lu_inverse_bytes(n, B)), "alloc block inverses");
     ck(ctx->d32.ensure(vecn * sizeof(float2)), "alloc d");
     ck(ctx->xsplit.ensure(vecn * sizeof(float4)), "alloc x split");
@@ -1003,7 +1006,7 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
   int lu_launches = 0;
   ck(bem::lu_factor_batched(prec, ctx->mats.p, lda, n, B, (int*)ctx->ipiv.p, (int*)ctx->info.p, nb, ctx->cublas,
                             ctx->stream, (bem::LuGemm)o.lu_gemm, tcws, &used_tensor, &tc_err, (int*)ctx->rowmap.p,
-                            &lu_launches, (int*)ctx->perm.p, ctx->panel_polls),
+                            &lu_launches, (int*)ctx->perm.p, ctx->panel_polls, rule_batch),
      "LU factorisation");
   // kernels of this batch besides the assembly: the LU with its row permutation, the solves
   // (mixed: 5 + 4 per refinement step), the field (2, +1 mixed, per slice)
@@ -1033,9 +1036,11 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
                 : bem::lu_solve_cluster_batched(prec, ctx->mats.p, lda, n, B, (const int*)ctx->perm.p, d, ldb, nc,
                                                 ctx->stream),
          "LU solve");
-      ck(bem::refine_update_x(steps == 0, d, x, ctx->xsplit.p, nvec, ctx->stream), "update x");
+      ck(bem::refine_update_x(steps == 0 ? nullptr : (const double*)ctx->norms.p, o.refine_tol, d, x, ctx->xsplit.p,
+                              ldb, B * nc, ctx->stream),
+         "update x");
       ck(bem::refine_residual(ctx->mats2.p, lda, n, B, ctx->xsplit.p, (const float2*)ctx->b32.p, ldb, nc,
-                              (double2*)ctx->r64.p, d, (double*)ctx->norms.p, ctx->stream),
+                              (double2*)ctx->r64.p, d, (double*)ctx->norms.p, ctx->stream, rule_batch),
          "residual");
       ck(cudaMemcpyAsync(norms.data(), ctx->norms.p, (size_t)B * nc * 2 * sizeof(double), cudaMemcpyDeviceToHost,
                          ctx->stream),
@@ -1082,7 +1087,8 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
                                       : (const void*)((const double2*)ctx->b32.p + (size_t)i0 * nc * ldb);
       const void* drive = mixed ? x.m->drive32.p : x.m->drive64.p;
       ck(bem::launch_field(dm, prec, x.cnt, ks.data() + i0, qs.data() + i0, p_for_field, ldb, nc, drive,
-                           (const double*)x.m->obs.p, x.m->nobs, ctx->fsrc.p, (double2*)ctx->fout.p, ctx->stream),
+                           (const double*)x.m->obs.p, x.m->nobs, ctx->fsrc.p, (double2*)ctx->fout.p, ctx->stream,
+                           one_slice ? rule_batch : x.cnt),
          "field kernel");
       T.launches += 2;
       ck(cudaMemcpyAsync(x.field_out, ctx->fout.p, (size_t)x.cnt * nc * x.m->nobs * sizeof(double2), kind,
@@ -1161,13 +1167,16 @@ bool valid_freqs(bem_context* ctx, const double* freqs_hz, int n_freq) {
 // How bem_solve_frequencies runs a call: the batch, and the lanes that its batches are dealt to.
 struct CallPlan {
   int batch, lanes;
+  // a call of one automatic batch: the batch that a lane gets of it (0: each batch's own), also
+  // where it runs on one lane, so that its bits do not depend on the lanes
+  int rule_batch;
 };
 CallPlan plan_call(int nv, bem::Precision prec, int n_freq, int batch, int lanes) {
-  int B = batch > 0 ? std::min(batch, 64) : auto_batch_order(nv, prec, n_freq);
-  B = std::min(B, n_freq);
-  if (batch <= 0 && lanes >= 2 && B == n_freq) B = lane_split(n_freq);
+  const int whole = std::min(batch > 0 ? std::min(batch, 64) : auto_batch_order(nv, prec, n_freq), n_freq);
+  const int part = batch <= 0 && whole == n_freq ? lane_split(n_freq) : 0;
+  const int B = part > 0 && lanes >= 2 ? part : whole;
   const int nbatch = (n_freq + B - 1) / B;
-  return {B, std::max(1, std::min({lanes, kMaxLanes, nbatch}))};
+  return {B, std::max(1, std::min({lanes, kMaxLanes, nbatch})), part};
 }
 
 // Device bytes of a mesh with npairs singular pairs: pairs, records, moments and scatter plan,
@@ -1271,7 +1280,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         threads.emplace_back([&, l, cl] {
           cudaSetDevice(ctx->device);
           try {
-            for (int bi = l; bi < nbatch; bi += nl) solve_combined(cl, {slice_of(bi)}, nv, o, nc, TL[l - 1]);
+            for (int bi = l; bi < nbatch; bi += nl) solve_combined(cl, {slice_of(bi)}, nv, o, nc, TL[l - 1], plan.rule_batch);
           } catch (const BemError& e) {
             errs[l - 1] = e;
             failed[l - 1] = 1;
@@ -1282,7 +1291,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         });
       }
       try {
-        for (int bi = 0; bi < nbatch; bi += nl) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T);
+        for (int bi = 0; bi < nbatch; bi += nl) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rule_batch);
       } catch (...) {
         for (auto& t : threads) t.join();
         throw;
@@ -1304,7 +1313,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         T.launches += T2.launches;
       }
     } else {
-      for (int bi = 0; bi < nbatch; ++bi) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T);
+      for (int bi = 0; bi < nbatch; ++bi) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rule_batch);
     }
     fill_stats(stats, T);
     if (stats) {

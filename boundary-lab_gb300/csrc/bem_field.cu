@@ -296,8 +296,9 @@ int field_split(const void* kern, long long clusters, int nf) {
 }
 
 template <typename K, typename... A>
-cudaError_t launch_field_f32(K kern, unsigned pt_blocks, unsigned groups, int nf, cudaStream_t stream, A... args) {
-  const int split = field_split((const void*)kern, (long long)pt_blocks * groups, nf);
+cudaError_t launch_field_f32(K kern, unsigned pt_blocks, unsigned groups, unsigned rule_groups, int nf,
+                             cudaStream_t stream, A... args) {
+  const int split = field_split((const void*)kern, (long long)pt_blocks * rule_groups, nf);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pt_blocks * split, groups);
   cfg.blockDim = dim3(kFieldWarps * 32);
@@ -423,7 +424,8 @@ static df host_df(double x) {
 
 cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const double* k, const double2* qscale,
                          const void* pressure, long long ldp, int nc, const void* drive, const double* obs, int nobs,
-                         void* sources, double2* out, cudaStream_t stream) {
+                         void* sources, double2* out, cudaStream_t stream, int rule_batch) {
+  if (rule_batch <= 0) rule_batch = batch;
   if (batch > 64 || nc < 1 || nc > 4 || nobs <= 0) return cudaErrorInvalidValue;
   FieldRule<float> fr32;
   FieldRule<double> fr64;
@@ -460,7 +462,8 @@ cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const d
     const int4 trs = make_int4(m.tr[0], m.tr[1], m.tr[2], m.tr[3]);
     cudaError_t le = cudaSuccess;
     auto run = [&](auto kern, int per_cluster) {
-      le = launch_field_f32(kern, pt_blocks, (unsigned)((batch + per_cluster - 1) / per_cluster), m.nf, stream,
+      le = launch_field_f32(kern, pt_blocks, (unsigned)((batch + per_cluster - 1) / per_cluster),
+                            (unsigned)((rule_batch + per_cluster - 1) / per_cluster), m.nf, stream,
                             (const FaceF32*)m.faces32, m.nf, (const float2*)sources, (const float2*)drive, obs, nobs,
                             (const FieldParamsF32*)dp, batch, out, fr32, m.ntr, trs);
     };
@@ -586,7 +589,7 @@ cudaError_t launch_field_single(Precision prec, const void* faces, int nf, int Q
     const float2* s = (const float2*)sources;
     const float2* d = (const float2*)drive;
     auto run = [&](auto kern) {
-      return launch_field_f32(kern, (unsigned)((nobs + 31) / 32), 1u, nf, stream, f, nf, s, d, obs, nobs,
+      return launch_field_f32(kern, (unsigned)((nobs + 31) / 32), 1u, 1u, nf, stream, f, nf, s, d, obs, nobs,
                               (const FieldParamsF32*)dp, 1, out, fr32, 1, make_int4(0, 0, 0, 0));
     };
     const cudaError_t le = Q == 6   ? run(field_f32_kernel<6, 1, 1>)

@@ -164,6 +164,11 @@ int* tc_gemm_error_word(TcGemmPlan* p);
 // rowmap (batch * kRowmapStride ints, may be null) lets the cluster panel hand
 // the net row permutation of its interchanges to the row-swap kernel.  perm (batch * n
 // ints, may be null) receives the row permutation: (P b)[i] = b[perm[i]].
+//
+// rule_batch, here and below (0: batch itself): the batch that the rules go by which choose
+// between orders of a matrix's own sums (the last outer block's width, the residual's column
+// splits, the field's split of the faces).  A call of one automatic batch gives the same one on
+// one lane and on two, so its bits do not depend on the lanes.
 constexpr int kRowmapStride = 512;
 // Reads of a word that a register panel's CTA waits for before it gives up (info = -1): two
 // milliseconds or so, where the word takes a microsecond.
@@ -180,7 +185,7 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
                               int nb, void* cublas_handle, cudaStream_t stream, LuGemm gemm = LuGemm::Cublas,
                               void* tc_workspace = nullptr, bool* used_tensor = nullptr, int** tc_err = nullptr,
                               int* rowmap = nullptr, int* n_launches = nullptr, int* perm = nullptr,
-                              int polls = kPanelPolls);
+                              int polls = kPanelPolls, int rule_batch = 0);
 // Solve (LU) X = B in place for nrhs columns per matrix (B stride ldb*nrhs per matrix), working precision.
 cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* ipiv,
                              void* B, long long ldb, int nrhs, int nb, cudaStream_t stream);
@@ -193,16 +198,18 @@ bool lu_solve_blocks_fits(int n);
 cudaError_t lu_block_inverses(const void* LU, long long lda, int n, int batch, void* inv, cudaStream_t stream);
 cudaError_t lu_solve_blocks_batched(const void* LU, long long lda, int n, int batch, const void* inv, const int* perm,
                                     void* B, long long ldb, int nrhs, cudaStream_t stream);
-// x = d (first) or x += d, and x split into float pairs (4 floats per value) for the residual.
-cudaError_t refine_update_x(bool first, const float2* d, double2* x, void* xsplit, long long count,
-                            cudaStream_t stream);
+// x = d (norms null: the first) or x += d for the systems whose residual is still above tol, and
+// x split into float pairs (4 floats per value) for the residual.
+cudaError_t refine_update_x(const double* norms, double tol, const float2* d, double2* x, void* xsplit, long long ldb,
+                            int systems, cudaStream_t stream);
 // d = b - A x rounded to FP32 (A and b FP32, x as split above, FP64-accurate sums), and per
 // system norms[2 i] = ||b - A x||^2, norms[2 i + 1] = ||b||^2.  parts: kResidualSplits x
 // systems x ldb values at most.
 constexpr int kResidualSplits = 8;
-int residual_splits(int n, int systems);
+int residual_splits(int n, int systems);  // of rule_batch x nrhs systems
 cudaError_t refine_residual(const void* A, long long lda, int n, int batch, const void* xsplit, const float2* b,
-                            long long ldb, int nrhs, double2* parts, float2* d, double* norms, cudaStream_t stream);
+                            long long ldb, int nrhs, double2* parts, float2* d, double* norms, cudaStream_t stream,
+                            int rule_batch = 0);
 // Cluster-resident panel (bem_lu_cluster.cu).  lu_cluster_plan picks the panel
 // width (64 or 32) and cluster size for an n x n matrix; false when no cluster
 // configuration fits (then the single-CTA panel is used).
@@ -226,7 +233,7 @@ cudaError_t convert_f64_to_f32(const double2* src, float2* dst, long long n, cud
 // far field (bem_field.cu)
 cudaError_t launch_field(const DeviceMesh& m, Precision prec, int batch, const double* k, const double2* qscale,
                          const void* pressure, long long ldp, int nc, const void* drive, const double* obs, int nobs,
-                         void* sources, double2* out, cudaStream_t stream);
+                         void* sources, double2* out, cudaStream_t stream, int rule_batch = 0);
 // One frequency, one excitation, everything in caller-placed device buffers
 // (face records FaceF32/FaceF64, weighted sources, drive with qscale = 1, a
 // parameter block of field_params_bytes()).  Used by bem_noalloc.cu.

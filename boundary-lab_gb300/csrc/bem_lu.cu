@@ -655,6 +655,7 @@ struct LuJob {
   cublasHandle_t h;
   cudaStream_t stream;
   int polls;         // of the panels' exchange
+  int rule_batch;
 };
 
 // U rows [k, k+kb) of columns [c0, c1): U = L^{-1} A with L the unit lower triangle of A[k:k+kb, k:k+kb].
@@ -754,7 +755,7 @@ cudaError_t lu_two_level(const LuJob& j, int NB) {
     iota_rows_kernel<<<(total + 255) / 256, 256, 0, j.stream>>>(j.perm, n, total);
   }
   for (int k0 = 0, KB; k0 < n; k0 += KB) {
-    KB = outer_width(n - k0, NB, j.batch, narrow);
+    KB = outer_width(n - k0, NB, j.rule_batch, narrow);
     for (int j0 = 0; j0 < KB; j0 += nb) {
       const int kb = std::min(nb, KB - j0), kk = k0 + j0;
       BEM_TRY(lu_panel_cluster(j.prec, j.A, j.lda, j.strideA, n, kk, kb, nb, j.cl, j.batch, j.ipiv, j.info, j.stream,
@@ -823,7 +824,9 @@ int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm, int batch) {
 
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info, int nb,
                               void* cublas_handle, cudaStream_t stream, LuGemm gemm, void* tc_workspace,
-                              bool* used_tensor, int** tc_err, int* rowmap, int* n_launches, int* perm, int polls) {
+                              bool* used_tensor, int** tc_err, int* rowmap, int* n_launches, int* perm, int polls,
+                              int rule_batch) {
+  if (rule_batch <= 0) rule_batch = batch;
   cublasHandle_t h = (cublasHandle_t)cublas_handle;
   cublasSetStream(h, stream);
   const long long strideA = lda * (long long)n;
@@ -852,8 +855,8 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
   // form, or lu_gemm = 1) keeps one level: its kernels for the skinny panel
   // shapes of the two-level schedule are slow.
   if (cluster_panel && rowmap && plan) {
-    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, h, stream, polls};
-    if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, plan != nullptr, perm != nullptr, batch);
+    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, h, stream, polls, rule_batch};
+    if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, plan != nullptr, perm != nullptr, rule_batch);
     return lu_two_level(job, kOuterBlock);
   }
   if (n_launches) *n_launches = 0;

@@ -317,12 +317,18 @@ __global__ void __launch_bounds__(kSolveThreads, 1) lu_solve_blocks_kernel(const
 
 // -------------------------------------------------------------- refinement --
 // x (+)= d, and x as float hi / lo pairs (re hi, im hi, re lo, im lo) for the residual, so
-// that it runs no FP64 instruction in its inner loop.
+// that it runs no FP64 instruction in its inner loop.  A system (blockIdx.y) whose residual is
+// within tol stays as it is while others of its batch are refined, so that its x does not
+// depend on them; the test is the host's, to the bit.
 template <bool FIRST>
-__global__ void update_x_kernel(const float2* __restrict__ d, double2* __restrict__ x, float4* __restrict__ xs,
-                                long long count) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
+__global__ void update_x_kernel(const double* __restrict__ norms, double tol, const float2* __restrict__ d,
+                                double2* __restrict__ x, float4* __restrict__ xs, long long ldb) {
+  if (blockIdx.x * blockDim.x + threadIdx.x >= ldb) return;
+  const long long i = blockIdx.y * ldb + blockIdx.x * blockDim.x + threadIdx.x;
+  if (!FIRST) {
+    const double r2 = norms[2 * blockIdx.y], b2 = norms[2 * blockIdx.y + 1];
+    if ((b2 > 0.0 ? sqrt(r2 / b2) : sqrt(r2)) <= tol) return;
+  }
   const float2 dv = d[i];
   double2 v = make_double2((double)dv.x, (double)dv.y);
   if (!FIRST) {
@@ -528,19 +534,20 @@ cudaError_t lu_solve_blocks_batched(const void* LU, long long lda, int n, int ba
   }
 }
 
-cudaError_t refine_update_x(bool first, const float2* d, double2* x, void* xsplit, long long count,
-                            cudaStream_t stream) {
-  const unsigned blocks = (unsigned)((count + 255) / 256);
-  if (first)
-    update_x_kernel<true><<<blocks, 256, 0, stream>>>(d, x, (float4*)xsplit, count);
+cudaError_t refine_update_x(const double* norms, double tol, const float2* d, double2* x, void* xsplit, long long ldb,
+                            int systems, cudaStream_t stream) {
+  const dim3 grid((unsigned)((ldb + 255) / 256), systems);
+  if (norms == nullptr)
+    update_x_kernel<true><<<grid, 256, 0, stream>>>(norms, tol, d, x, (float4*)xsplit, ldb);
   else
-    update_x_kernel<false><<<blocks, 256, 0, stream>>>(d, x, (float4*)xsplit, count);
+    update_x_kernel<false><<<grid, 256, 0, stream>>>(norms, tol, d, x, (float4*)xsplit, ldb);
   return cudaGetLastError();
 }
 
 cudaError_t refine_residual(const void* A, long long lda, int n, int batch, const void* xsplit, const float2* b,
-                            long long ldb, int nrhs, double2* parts, float2* d, double* norms, cudaStream_t stream) {
-  const int systems = batch * nrhs, splits = residual_splits(n, systems);
+                            long long ldb, int nrhs, double2* parts, float2* d, double* norms, cudaStream_t stream,
+                            int rule_batch) {
+  const int systems = batch * nrhs, splits = residual_splits(n, (rule_batch > 0 ? rule_batch : batch) * nrhs);
   const int cols = ((n + splits - 1) / splits + 63) / 64 * 64;
   const int used = (n + cols - 1) / cols;
   dim3 g((n + 63) / 64, used, systems);

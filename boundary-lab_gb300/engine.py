@@ -80,7 +80,7 @@ class CudaEngine:
         self.autotune = autotune
         # lanes = 2: a call of two or more batches runs them side by side on two streams
         # (bem_solve_options.lanes), so the job loop asks for two batches per call; a call of
-        # at least 8 frequencies that fits one automatic batch is split in two
+        # 8 or at least 12 frequencies that fits one automatic batch is split in two
         self.lanes = max(1, min(2, int(lanes)))
         self.launch = None  # autotune.LaunchConfig once tuned
         self.tune_result = None

@@ -130,9 +130,10 @@ typedef struct bem_solve_options {
                             2: a sweep of several batches deals them round-robin to the context and a
                             helper context of its own (own stream and scratch, created on first
                             use, freed with the context), so one batch's latency-bound LU panels overlap
-                            the other's assembly and tensor-core updates; a call of at least 8
-                            frequencies that one automatic batch would hold is split in two for them;
-                            larger values act as 2.
+                            the other's assembly and tensor-core updates; a call of 8 or of at least
+                            12 frequencies that one automatic batch would hold is split in two for them
+                            (the first part a multiple of four, the second at least four); larger
+                            values act as 2.  The results are those of one lane to the bit.
                             Per-kernel times in stats are then summed over the lanes. */
 } bem_solve_options;
 
