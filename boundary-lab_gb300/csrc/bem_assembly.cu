@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
               const double rv[3] = {cm[0] + og[n][0], cm[1] + og[n][1], cm[2] + og[n][2]};
               const double r2 = fma(rv[0], rv[0], fma(rv[1], rv[1], rv[2] * rv[2]));
               if (is_zero(r2)) continue;
-              const double rinv = rsqrt_step(r2), r = r2 * rinv;
+              const double rinv = rsqrt(r2), r = r2 * rinv;
               const double tq = (cmn + ogn[n]) * rinv * rinv;  // t / r
               const double ex = -tq * rinv, tn = fma(nn, rinv, tq), wr = p.w[n] * rinv;
 #pragma unroll
@@ -1239,7 +1239,7 @@ __global__ void __launch_bounds__(128, 2)
     for (int d = 0; d < 3; ++d) rv[d] = (d0[d] + ru * e1r[d] + rvv * e2r[d]) - (tu * e1t[d] + tv * e2t[d]);
     const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
     if (is_zero(r2)) continue;
-    const double rinv = rsqrt_step(r2), r = r2 * rinv;
+    const double rinv = rsqrt(r2), r = r2 * rinv;
     const double s = rinv * inv4pi, sr2 = s * rinv * rinv;
     const double fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * sr2;
     const double fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * sr2;
@@ -1722,7 +1722,7 @@ __global__ void __launch_bounds__(32)
       for (int d = 0; d < 3; ++d) rv[d] = (d0[d] + ru * e1r[d] + rvv * e2r[d]) - (tu * e1t[d] + tv * e2t[d]);
       const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
       if (is_zero(r2)) continue;
-      const double rinv = rsqrt_step(r2), r = r2 * rinv, s = rinv * inv4pi;
+      const double rinv = rsqrt(r2), r = r2 * rinv, s = rinv * inv4pi;
       const double fy = (rv[0] * nr[0] + rv[1] * nr[1] + rv[2] * nr[2]) * s;   // (r . n_r) / (4 pi r)
       const double fx = -(rv[0] * nt[0] + rv[1] * nt[1] + rv[2] * nt[2]) * s;  // -(r . n_t) / (4 pi r)
       const double x = fmin(1.0, fma(r, two_over_R, -1.0)), x2 = x + x;
@@ -1957,7 +1957,7 @@ __device__ __forceinline__ void rhs_pair_f64(const FaceF64& F, const FaceF64& Gf
       for (int d = 0; d < 3; ++d) rv[d] = C[d] + (sg[d] * Gf.off[3 * n + d] - F.off[3 * m + d]);
       const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
       if (is_zero(r2)) continue;
-      const double rinv = rsqrt_step(r2), r = r2 * rinv;
+      const double rinv = rsqrt(r2), r = r2 * rinv;
       double s, c;
       sincos_table(r, ku, tab, &s, &c);
       // w G (1, t (ik - 1/r)), G = e^{ikr} / (4 pi r), t = -(r . n_x) / r

@@ -613,14 +613,8 @@ int bem_upload_mesh_symmetric(bem_context* ctx, const double* vertices, int n_ve
       std::vector<double> mm(12);
       for (int i = 0; i < 9; ++i) mm[i] = P.m11[i];
       for (int i = 0; i < 3; ++i) mm[9 + i] = P.m10[i];
-      // (cos, sin) of the FP64 kernels' table angles, the first quadrant's from the first
-      // octant (where the rounded angle costs nothing) by symmetry
       std::vector<double2> trig(kSincosTable);
-      for (int i = 0; i < kSincosTable; ++i) {
-        const int o = std::min(i, kSincosTable - i);
-        const double a = 2.0 * M_PI * o / kSincosUnits;
-        trig[i] = i == o ? make_double2(std::cos(a), std::sin(a)) : make_double2(std::sin(a), std::cos(a));
-      }
+      sincos_table_host(trig.data());
       UploadPack pack;
       if (P.symmetry != 0) {
         pack.add(d.fix_mask, P.fix_mask);

@@ -10,6 +10,7 @@
 
 #include <cuda_runtime.h>
 #include <math_constants.h>
+#include <math.h>
 #include <stdint.h>
 
 #define BEM_HD __host__ __device__ __forceinline__
@@ -201,16 +202,19 @@ BEM_D float reduce_two_pi(float t) {
 // FP64 issues at 1/64 of the FP32 rate here, so an FP64 kernel's time is its count of FP64
 // instructions; everything else (table reads, FP32, integer work) is nearly free beside it.
 //
-// sin and cos of k r by table, in units of h = 2 pi / 2048: u = r (k / h), n its nearest
-// integer, x = u - n.  The table holds (cos, sin) of the first quadrant's 512 units; the other
-// quadrants follow by exchanging and negating words, which is integer work.  With the units in
-// the polynomials' coefficients there is no product k r and no reduction of it, and |x| <= 1/2
-// (pi / 2048) needs two terms each: sin to x^3 with the cubic coefficient moved by 0.87 of
-// half a unit's x^5 / 120 (error 1e-17), cos to x^4 (2e-20), combined by the addition theorem:
-// 13 FP64 instructions for the pair, against 17 with 512 units to the circle, an angle in
-// radians and its two-term reduction.  Errors: the roundings of
-// x and the table's entry, with the result's about 2e-16 absolute (k / h is held in two doubles); for |k r| <= h / 2 the entry is (1, 0) and the sine has
-// full relative accuracy.  |u| < 2^31.
+// sin and cos of k r by table lookup and the addition theorem (P. T. P. Tang, Table-lookup
+// algorithms for elementary functions and their error analysis, 1991), in units of
+// h = 2 pi / 2048: u = r (k / h), n its nearest integer, x = u - n.  The table holds (cos, sin)
+// of the first quadrant's 512 units; the other quadrants follow by exchanging and negating
+// words, which is integer work.  With the units in the polynomials' coefficients there is no
+// product k r and no reduction of it (k / h is held in two doubles, so x is exact to 2^-53 of
+// a unit whatever u), and |x| <= 1/2 (pi / 2048) needs two Taylor terms each: sin to x^3 with
+// the cubic coefficient moved by 0.87 of half a unit's x^5 / 120 (error 1e-17), cos to x^4
+// (2e-20): 13 FP64 instructions for the pair, against 17 with 512 units to the circle, an
+// angle in radians and its two-term reduction.
+// Error: three roundings of 2^-54 (the table's entry, the two of the last combination) and the
+// polynomial, 2e-16 absolute; for |k r| <= h / 2 the entry is (1, 0) and the sine's error is the
+// polynomial's, below 1e-14 of it.  |u| < 2^31 (k r below 6.5e6).
 constexpr int kSincosTable = 512, kSincosUnits = 4 * kSincosTable;
 struct AngleUnits {
   double hi, lo;  // k / h
@@ -220,6 +224,17 @@ BEM_D AngleUnits angle_units(double k) {
   a.hi = k * 325.94932345220167;
   a.lo = fma(k, 325.94932345220167, -a.hi) + k * -2.0150964915386866e-14;
   return a;
+}
+// The table (kSincosTable entries) on the host: the first quadrant's (cos, sin) from the first
+// octant by symmetry, in long double (an angle rounded to double moves an entry by as much as
+// its own rounding does).
+inline void sincos_table_host(double2* t) {
+  for (int i = 0; i < kSincosTable; ++i) {
+    const int o = i < kSincosTable - i ? i : kSincosTable - i;
+    const long double a = 2.0L * 3.14159265358979323846264338327950288L * o / kSincosUnits;
+    const double c = (double)cosl(a), s = (double)sinl(a);
+    t[i] = i == o ? make_double2(c, s) : make_double2(s, c);
+  }
 }
 // The table into shared memory, by the whole CTA (synchronise before use): from its copy
 // beside the mesh, or computed where there is none (src null; about 5% of a small CTA's FP64
@@ -255,15 +270,6 @@ BEM_D void sincos_table(double r, AngleUnits k, const double2* tab, double* s, d
 }
 // a == 0 for a sum of squares, in integer instructions.
 BEM_D bool is_zero(double a) { return (__double2hiint(a) | __double2loint(a)) == 0; }
-// 1 / sqrt(a), a > 0 normal: the hardware approximation (about 2^-20) and one third-order
-// step, y + y e (1/2 + 3/8 e) with e = 1 - a y^2; five FP64 instructions, relative error
-// about 2^-52.
-BEM_D double rsqrt_step(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-(a * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
 
 // Inverse of a pivot, 0 for d = 0.  Where |d|^2 or its reciprocal would leave the exponent
 // range, d is multiplied by a power of two before and the result after, so a matrix scaled by

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256) field_f64_kernel(const FaceF64* __restric
       for (int d = 0; d < 3; ++d) rv[d] = (sg[d] * F.anchor[d] - xo[d]) + sg[d] * F.off[3 * n + d];
       const double rr = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
       if (is_zero(rr)) continue;
-      const double rinv = rsqrt_step(rr), r = rr * rinv;
+      const double rinv = rsqrt(rr), r = rr * rinv;
       const double sc = rinv * (0.25 / CUDART_PI);
       // e^{ikr} [ (t/r)(ik - 1/r) p_s w_s - q w_s / r ] / (4 pi), t = (r . n_y) / r
       const double t = (rv[0] * sg[0] * F.normal[0] + rv[1] * sg[1] * F.normal[1] + rv[2] * F.normal[2]) * rinv * sc;

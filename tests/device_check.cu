@@ -2,6 +2,8 @@
 // itself.  Built and run by test_gpu_device_check.py against libgb300_bem.so:
 //   device_check <check> [arguments]
 // prints one line of figures; 1 is returned (with a message) if a CUDA call fails.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -74,11 +76,73 @@ int block_inverse(int n, int e) {
   return 0;
 }
 
+__global__ void sincos_kernel(const double* r, const double* k, int n, const double2* trig, double2* out) {
+  __shared__ double2 tab[kSincosTable];
+  load_sincos_table(tab, trig);
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s, c;
+  sincos_table(r[i], angle_units(k[i]), tab, &s, &c);
+  out[i] = make_double2(c, s);
+}
+
+// sincos: largest absolute errors with the host's table and with the one that the CTA computes,
+// and the largest relative error of the sine up to half a unit, over k from 1e-3 to 1e4 and k r
+// from 1e-12 to 6e6, at the midpoints between two units, at the quadrants' edges and beside both.
+int sincos_errors() {
+  std::mt19937_64 rng(11);
+  std::uniform_real_distribution<double> u01(0.0, 1.0);
+  std::vector<double> r, k;
+  const double h = 2.0 * M_PI / kSincosUnits;
+  for (double kk : {1e-3, 0.37, 3.66, 57.3, 366.0, 1e4}) {
+    auto add = [&](double kr) {
+      for (int d = -1; d <= 1; ++d) {
+        double v = kr / kk;
+        if (d) v = std::nextafter(v, d < 0 ? 0.0 : 1e300);
+        if (v * kk < 6.5e6) {
+          r.push_back(v);
+          k.push_back(kk);
+        }
+      }
+    };
+    for (int i = 0; i < 4000; ++i) add(std::pow(10.0, -12.0 + 18.8 * u01(rng)));
+    for (int i = 0; i < 2000; ++i) add(700.0 * u01(rng));
+    for (int i = 0; i < 1000; ++i) add((std::floor(i < 500 ? i : 2e9 * u01(rng)) + 0.5) * h);
+    for (int i = 0; i < 600; ++i) add(0.5 * M_PI * (i < 300 ? i : std::floor(4e6 * u01(rng))));
+  }
+  r.push_back(0.0);
+  k.push_back(3.66);
+  std::vector<double2> table(kSincosTable);
+  sincos_table_host(table.data());
+  const int n = (int)r.size();
+  Dev<double> dr(r), dk(k);
+  Dev<double2> dt(table), out(n);
+  double worst[2] = {0, 0}, small = 0;
+  for (int t = 0; t < 2; ++t) {
+    sincos_kernel<<<(n + 255) / 256, 256>>>(dr.p, dk.p, n, t ? nullptr : dt.p, out.p);
+    ck(cudaGetLastError(), "sincos");
+    ck(cudaDeviceSynchronize(), "sincos");
+    const std::vector<double2> o = out.host();
+    for (int i = 0; i < n; ++i) {
+      // the exact angle as a double and its rounding error
+      const double hi = k[i] * r[i], lo = std::fma(k[i], r[i], -hi);
+      const long double sh = sinl(hi), ch = cosl(hi), sl = sinl(lo), cl = cosl(lo);
+      const long double s = sh * cl + ch * sl, c = ch * cl - sh * sl;
+      worst[t] = std::max(worst[t], (double)std::max(fabsl(o[i].y - s), fabsl(o[i].x - c)));
+      if (hi > 0.0 && hi < 0.499 * h) small = std::max(small, (double)fabsl((o[i].y - s) / s));
+    }
+  }
+  std::printf("%d %.3e %.3e %.3e\n", n, worst[0], worst[1], small);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   auto is = [&](const char* name, int args) { return argc == args + 2 && std::strcmp(argv[1], name) == 0; };
   if (is("block_inverse", 2)) return block_inverse(std::atoi(argv[2]), std::atoi(argv[3]));
+  if (is("sincos", 0)) return sincos_errors();
   std::printf("unknown check\n");
   return 1;
 }

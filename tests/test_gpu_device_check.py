@@ -34,3 +34,16 @@ def test_block_inverses_scale(check, n, e):
     factors times a power of two."""
     differ, not_finite = check("block_inverse", n, e)
     assert differ == 0 and not_finite == 0
+
+
+def test_table_sine_and_cosine(check):
+    """The FP64 kernels' sine and cosine of k r.  Absolute: three roundings of 2^-54 and the
+    polynomials' 1e-17, below 2e-16, with the host's table; where the CTA computes the table
+    (sincospi, 2 units in the last place) 2^-52 takes the place of one of them.  Up to half a unit
+    h of angle the sine is c0 x + c1 x^3 with c1 moved by 0.87 / 4 of h^5 / 120: relative error
+    h^4 / 120 times max |x^4 - 0.2175 x^2| = 0.0118, 8.7e-15, and five roundings of 2^-53."""
+    n, host_table, device_table, small = check("sincos")
+    assert n > 100000
+    assert host_table <= 2e-16
+    assert device_table <= 2e-16 - 2.0**-54 + 2.0**-52
+    assert small <= 8.8e-15 + 5 * 2.0**-53
