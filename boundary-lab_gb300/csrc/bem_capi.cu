@@ -613,8 +613,6 @@ int bem_upload_mesh_symmetric(bem_context* ctx, const double* vertices, int n_ve
       std::vector<double> mm(12);
       for (int i = 0; i < 9; ++i) mm[i] = P.m11[i];
       for (int i = 0; i < 3; ++i) mm[9 + i] = P.m10[i];
-      std::vector<double2> trig(kSincosTable);
-      sincos_table_host(trig.data());
       UploadPack pack;
       if (P.symmetry != 0) {
         pack.add(d.fix_mask, P.fix_mask);
@@ -653,7 +651,7 @@ int bem_upload_mesh_symmetric(bem_context* ctx, const double* vertices, int n_ve
       pack.add(d.curls, P.curls);
       pack.add(d.area, P.area);
       pack.add(d.m11m10, mm);
-      pack.add(d.trig, trig);
+      pack.add(d.trig, sincos_table_host());
       pack.commit(m);
       for (int q = 0; q < P.Q; ++q) {
         const double u = P.rule_pts[2 * q], v = P.rule_pts[2 * q + 1];

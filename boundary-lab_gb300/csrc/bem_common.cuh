@@ -13,6 +13,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <vector>
+
 #define BEM_HD __host__ __device__ __forceinline__
 #define BEM_D __device__ __forceinline__
 
@@ -227,14 +229,19 @@ BEM_D AngleUnits angle_units(double k) {
 }
 // The table (kSincosTable entries) on the host: the first quadrant's (cos, sin) from the first
 // octant by symmetry, in long double (an angle rounded to double moves an entry by as much as
-// its own rounding does).
-inline void sincos_table_host(double2* t) {
-  for (int i = 0; i < kSincosTable; ++i) {
-    const int o = i < kSincosTable - i ? i : kSincosTable - i;
-    const long double a = 2.0L * 3.14159265358979323846264338327950288L * o / kSincosUnits;
-    const double c = (double)cosl(a), s = (double)sinl(a);
-    t[i] = i == o ? make_double2(c, s) : make_double2(s, c);
-  }
+// its own rounding does).  Formed once per process: 0.3 ms where long double is software.
+inline const std::vector<double2>& sincos_table_host() {
+  static const std::vector<double2> table = [] {
+    std::vector<double2> t(kSincosTable);
+    for (int i = 0; i < kSincosTable; ++i) {
+      const int o = i < kSincosTable - i ? i : kSincosTable - i;
+      const long double a = 2.0L * 3.14159265358979323846264338327950288L * o / kSincosUnits;
+      const double c = (double)cosl(a), s = (double)sinl(a);
+      t[i] = i == o ? make_double2(c, s) : make_double2(s, c);
+    }
+    return t;
+  }();
+  return table;
 }
 // The table into shared memory, by the whole CTA (synchronise before use): from its copy
 // beside the mesh, or computed where there is none (src null; about 5% of a small CTA's FP64

@@ -113,11 +113,9 @@ int sincos_errors() {
   }
   r.push_back(0.0);
   k.push_back(3.66);
-  std::vector<double2> table(kSincosTable);
-  sincos_table_host(table.data());
   const int n = (int)r.size();
   Dev<double> dr(r), dk(k);
-  Dev<double2> dt(table), out(n);
+  Dev<double2> dt(sincos_table_host()), out(n);
   double worst[2] = {0, 0}, small = 0;
   for (int t = 0; t < 2; ++t) {
     sincos_kernel<<<(n + 255) / 256, 256>>>(dr.p, dk.p, n, t ? nullptr : dt.p, out.p);
