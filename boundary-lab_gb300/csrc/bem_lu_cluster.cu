@@ -483,7 +483,9 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) lu_panel_reg_kernel(float
       M[(size_t)(k + j + lane) * lda + k + j] = reinterpret_cast<const float2*>(U)[lane];
     if (rank == 0 && tid == 0) piv[k + j] = k + p;
     const float2 d = make_float2(U[0].x, U[0].y);
-    const float2 inv = pivot_inverse(d);
+    // whether |d|^2 is in range is known from the key, before the row arrives
+    const bool plain = key.x - __float_as_uint(0x1p-49f) <= __float_as_uint(0x1p49f) - __float_as_uint(0x1p-49f);
+    const float2 inv = plain ? pivot_inverse_plain<false>(d) : pivot_inverse_scaled<false>(d);
     if (rank == 0 && tid == 0 && d.x == 0.f && d.y == 0.f && info[blockIdx.y] == 0) info[blockIdx.y] = k + j + 1;
     // 4. this thread's row
     if (mine && done_at < 0) {
