@@ -886,6 +886,16 @@ struct Slice {
   bool cheb = false;     // mixed form: singular remainders through the mesh's Chebyshev moments
 };
 
+// The batches that the rules go by which choose between orders of sums, 0: each batch's own.  A
+// call of one automatic batch has the same ones on one lane and on two, so that its bits do
+// not depend on the lanes.  The LU's last outer block and the residual go by a lane's part
+// (by the whole, two lanes lost 3 % at 1,000 triangles and 16 frequencies), the field's split
+// by the whole (by a lane's part, one lane lost 7 % at 330 triangles, 28 frequencies and 2,000
+// points).
+struct SumRules {
+  int batch = 0, field = 0;
+};
+
 // Totals over the batches of one call.
 struct SolveTotals {
   double kacc[BEM_K_SLOTS] = {0};
@@ -903,18 +913,16 @@ struct SolveTotals {
 // each slice's field is evaluated on its own mesh.  The identity block cannot
 // change a pivot (its rows are zero in the mesh's columns), so each mesh's
 // factors are those of its own matrix.  Every slice has the same number of
-// excitations nc.  rule_batch > 0: the batch that the rules go by which choose between orders
-// of sums (CallPlan).
+// excitations nc.
 void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const bem_solve_options& o, int nc,
-                    SolveTotals& T, int rule_batch = 0) {
+                    SolveTotals& T, SumRules rules = {}) {
   const bem::Precision prec = o.precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64;
   const bool mixed = prec == bem::Precision::Mixed;
   const size_t esz = mixed ? sizeof(float2) : sizeof(double2);
   const long long lda = round_up(n, 32), ldb = round_up(n, 32);
   int B = 0;
   for (const Slice& x : sl) B += x.cnt;
-  if (rule_batch <= 0) rule_batch = B;
-  const bool one_slice = sl.size() == 1;
+  const int rule_batch = rules.batch > 0 ? rules.batch : B;
   const int nb = o.lu_block > 0 ? std::min(o.lu_block, 64) : 0;  // 0: the LU chooses
   const size_t matsz = (size_t)lda * n * esz;
   ck(ctx->mats.ensure(matsz * B), "alloc matrices");
@@ -1080,7 +1088,7 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
       const void* drive = mixed ? x.m->drive32.p : x.m->drive64.p;
       ck(bem::launch_field(dm, prec, x.cnt, ks.data() + i0, qs.data() + i0, p_for_field, ldb, nc, drive,
                            (const double*)x.m->obs.p, x.m->nobs, ctx->fsrc.p, (double2*)ctx->fout.p, ctx->stream,
-                           one_slice ? rule_batch : x.cnt),
+                           rules.field),
          "field kernel");
       T.launches += 2;
       ck(cudaMemcpyAsync(x.field_out, ctx->fout.p, (size_t)x.cnt * nc * x.m->nobs * sizeof(double2), kind,
@@ -1159,16 +1167,15 @@ bool valid_freqs(bem_context* ctx, const double* freqs_hz, int n_freq) {
 // How bem_solve_frequencies runs a call: the batch, and the lanes that its batches are dealt to.
 struct CallPlan {
   int batch, lanes;
-  // a call of one automatic batch: the batch that a lane gets of it (0: each batch's own), also
-  // where it runs on one lane, so that its bits do not depend on the lanes
-  int rule_batch;
+  SumRules rules;
 };
 CallPlan plan_call(int nv, bem::Precision prec, int n_freq, int batch, int lanes) {
   const int whole = std::min(batch > 0 ? std::min(batch, 64) : auto_batch_order(nv, prec, n_freq), n_freq);
   const int part = batch <= 0 && whole == n_freq ? lane_split(n_freq) : 0;
   const int B = part > 0 && lanes >= 2 ? part : whole;
   const int nbatch = (n_freq + B - 1) / B;
-  return {B, std::max(1, std::min({lanes, kMaxLanes, nbatch})), part};
+  return {B, std::max(1, std::min({lanes, kMaxLanes, nbatch})),
+          part > 0 ? SumRules{part, whole} : SumRules{}};
 }
 
 // Device bytes of a mesh with npairs singular pairs: pairs, records, moments and scatter plan,
@@ -1272,7 +1279,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         threads.emplace_back([&, l, cl] {
           cudaSetDevice(ctx->device);
           try {
-            for (int bi = l; bi < nbatch; bi += nl) solve_combined(cl, {slice_of(bi)}, nv, o, nc, TL[l - 1], plan.rule_batch);
+            for (int bi = l; bi < nbatch; bi += nl) solve_combined(cl, {slice_of(bi)}, nv, o, nc, TL[l - 1], plan.rules);
           } catch (const BemError& e) {
             errs[l - 1] = e;
             failed[l - 1] = 1;
@@ -1283,7 +1290,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         });
       }
       try {
-        for (int bi = 0; bi < nbatch; bi += nl) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rule_batch);
+        for (int bi = 0; bi < nbatch; bi += nl) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rules);
       } catch (...) {
         for (auto& t : threads) t.join();
         throw;
@@ -1305,7 +1312,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         T.launches += T2.launches;
       }
     } else {
-      for (int bi = 0; bi < nbatch; ++bi) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rule_batch);
+      for (int bi = 0; bi < nbatch; ++bi) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rules);
     }
     fill_stats(stats, T);
     if (stats) {
