@@ -2968,8 +2968,8 @@ cudaError_t launch_rhs_freqs(const DeviceMesh& m, Precision prec, int nfreq, con
 // Kernel launches of launch_rhs_freqs for nfreq frequencies.
 int rhs_launches(Precision prec, int nc, int nfreq) {
   const int width = rhs_width(prec, nc);
-  if (width == 1) return (nfreq + kRhsGroups - 1) / kRhsGroups + 1;
-  return (nfreq >= width ? 1 : 0) + (nfreq % width ? 1 : 0) + 1;  // full groups, the remainder, the gather
+  // the full groups, kRhsGroups to a launch, the remainder, the gather
+  return (nfreq / width + kRhsGroups - 1) / kRhsGroups + (nfreq % width ? 1 : 0) + 1;
 }
 
 }  // namespace bem

@@ -135,11 +135,79 @@ int sincos_errors() {
   return 0;
 }
 
+// Kernels that a capture of `launch` holds.
+template <typename F> int captured_kernels(F launch) {
+  cudaStream_t stream;
+  cudaGraph_t graph;
+  ck(cudaStreamCreate(&stream), "stream");
+  ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+  ck(launch(stream), "captured launch");
+  ck(cudaStreamEndCapture(stream, &graph), "end capture");
+  size_t n = 0;
+  ck(cudaGraphGetNodes(graph, nullptr, &n), "nodes");
+  std::vector<cudaGraphNode_t> nodes(n);
+  ck(cudaGraphGetNodes(graph, nodes.data(), &n), "nodes");
+  int kernels = 0;
+  for (cudaGraphNode_t node : nodes) {
+    cudaGraphNodeType type;
+    ck(cudaGraphNodeGetType(node, &type), "node type");
+    kernels += type == cudaGraphNodeTypeKernel;
+  }
+  ck(cudaGraphDestroy(graph), "destroy graph");
+  ck(cudaStreamDestroy(stream), "destroy stream");
+  return kernels;
+}
+
+// launch_counts: calls whose reported number of launches is not what they launch, of the
+// right-hand side (excitations 1..4) and the regular pairs, both forms, 1..64 frequencies.  The
+// launches are captured, not run; every pointer is a zeroed buffer all the same.
+int launch_counts() {
+  Dev<char> zeros(std::vector<char>((size_t)64 << 20));
+  void* z = zeros.p;
+  bem::DeviceMesh m;
+  m.faces32 = (bem::FaceF32*)z;
+  m.faces64 = (bem::FaceF64*)z;
+  m.lane_slots = (bem::LaneSlot*)z;
+  m.group_faces32 = (float*)z;
+  m.tile_group_ptr = m.tile_row_base = m.col_ptr = m.col_fb = m.vertex_row = m.driven = (int*)z;
+  m.pairs_by_test_ptr = m.pairs_by_test = (int*)z;
+  m.pairs = (bem::SingularPair*)z;
+  m.trig = (double2*)z;
+  m.nv = 8;
+  m.nf = 12;
+  m.Q = 6;
+  m.n_tiles = 1;
+  m.max_tile_rows = 40;
+  m.ntr = 1;
+  std::vector<double> k(64);
+  std::vector<bem::OperatorCoeffs> c(64);
+  std::vector<double2> q(64, make_double2(0.0, 1.0)), cD(64, make_double2(1.0, 0.0)), cH(64);
+  for (int i = 0; i < 64; ++i) {
+    k[i] = 1.0 + i;
+    cH[i] = make_double2(0.0, -1.0 / k[i]);
+  }
+  int wrong = 0, calls = 0;
+  for (bem::Precision prec : {bem::Precision::Mixed, bem::Precision::FP64})
+    for (int n = 1; n <= 64; ++n) {
+      for (int nc = 1; nc <= 4; ++nc, ++calls)
+        wrong += bem::rhs_launches(prec, nc, n) != captured_kernels([&](cudaStream_t s) {
+          return bem::launch_rhs_freqs(m, prec, n, k.data(), c.data(), q.data(), z, nc, z, 12, z, z, 32, s);
+        });
+      ++calls;
+      wrong += bem::regular_launches(m, prec, n) != captured_kernels([&](cudaStream_t s) {
+        return bem::launch_regular(m, prec, n, k.data(), cD.data(), cH.data(), z, 64, 4096, s);
+      });
+    }
+  std::printf("%d %d\n", calls, wrong);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   auto is = [&](const char* name, int args) { return argc == args + 2 && std::strcmp(argv[1], name) == 0; };
   if (is("block_inverse", 2)) return block_inverse(std::atoi(argv[2]), std::atoi(argv[3]));
+  if (is("launch_counts", 0)) return launch_counts();
   if (is("sincos", 0)) return sincos_errors();
   std::printf("unknown check\n");
   return 1;

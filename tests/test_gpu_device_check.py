@@ -47,3 +47,10 @@ def test_table_sine_and_cosine(check):
     assert host_table <= 2e-16
     assert device_table <= 2e-16 - 2.0**-54 + 2.0**-52
     assert small <= 8.8e-15 + 5 * 2.0**-53
+
+
+def test_reported_launches(check):
+    """stats["kernel_launches"] counts the right-hand side's and the regular pairs' launches by
+    formula: they are those of the launches captured in a graph."""
+    calls, wrong = check("launch_counts")
+    assert calls == 2 * 64 * 5 and wrong == 0
