@@ -1678,10 +1678,10 @@ __global__ void __launch_bounds__(128)
 // The same expansion for the FP64 form: moments and contraction in FP64, with the terms at
 // which the coefficients reach rounding (cheb_terms with tolerance kChebTol64), so the sums
 // are those of the Duffy points to rounding.  Per point and chunk of four terms about 160
-// FP64 instructions, 640 for 16 terms: four frequencies point by point, once per mesh; a
-// frequency through the moments then costs a fortieth of one (1,280 triangles: 4.1 ->
-// 0.10 ms, the moments 15.4 ms once for 16 terms; 17.5 with butterfly sums).  Per pair 21 sums per term: IR[9], IDh[9],
-// IKh[3] (SR[a] is the sum of IR[a][b] over b), stored [pair][term][kCheb64Sums].
+// FP64 instructions: the moments of 1,280 triangles take 15 ms once for 16 terms (17.5 with
+// butterfly sums), as much as six frequencies point by point, and a frequency through them
+// 0.10 ms instead of 2.5.  Per pair 21 sums per term: IR[9], IDh[9], IKh[3] (SR[a] is the sum of
+// IR[a][b] over b), stored [pair][term][kCheb64Sums].
 constexpr int kCheb64Sums = 21;
 
 __global__ void __launch_bounds__(32)

@@ -281,10 +281,11 @@ Layout layout_for(const bem::DeviceMesh& dm, bem::Precision prec) {
 }
 
 // Frequencies a call needs before its singular remainders go through the mesh's
-// Chebyshev moments: forming them costs about as much as six frequencies of the point-by-
-// point singular kernel at 16 terms (more at more terms, at most 24), and each frequency
-// through them costs a fifteenth of one.  A shorter call runs point by point even when the
-// moments exist, so a call's results depend on its own inputs only.
+// Chebyshev moments: in the mixed form, for which the number was chosen, forming them costs
+// about as much as six frequencies of the point-by-point singular kernel at 16 terms (more at
+// more terms, at most 24), and each frequency through them costs a fifteenth of one.  (In the
+// FP64 form 16 terms cost 6.4 frequencies; see ensure_cheb.)  A shorter call runs point by
+// point even when the moments exist, so a call's results depend on its own inputs only.
 constexpr int kChebMinFreqs = 12;
 
 // Batch of a call that one automatic batch would hold and that may use two lanes: split in
@@ -302,15 +303,26 @@ int lane_split(int n_freq) {
 // Forms (or extends) the mesh's Chebyshev moments on the side stream for the call's
 // wavenumbers k[0..n): with the fewest terms (a multiple of four) that cover every
 // frequency whose expansion converges within kChebN terms, or twice the terms the moments
-// had, up to kChebN.  Nothing when no frequency converges (those run point by point).
-void ensure_cheb(bem_context* ctx, bem_mesh* m, bem::Precision prec, const double* k, int n) {
+// had, up to kChebN.  Returns whether the call goes through them: not when no frequency
+// converges (those run point by point).  The FP64 form also runs a call point by point of which
+// too few frequencies converge to pay for the terms they need, whether or not the mesh has the
+// moments.  A term costs 0.4 of a frequency
+// point by point: first calls of 12 frequencies at 1,280 triangles, 105.6 ms point by point,
+// take 107.0 and 105.2 where 4 and 5 converge in 12 terms, 106.1 and 104.4 where 6 and 7 do in
+// 16, 105.3 where 8 do in 20.
+bool ensure_cheb(bem_context* ctx, bem_mesh* m, bem::Precision prec, const double* k, int n) {
   bem::DeviceMesh& d = m->dm;
-  if (d.npairs == 0 || !(d.cheb_R > 0.0)) return;
+  if (d.npairs == 0 || !(d.cheb_R > 0.0)) return false;
   const bool mixed = prec == bem::Precision::Mixed;
   int& have = mixed ? d.cheb_n : d.cheb64_n;
-  int need = 0;
-  for (int i = 0; i < n; ++i) need = std::max(need, bem::cheb_terms(prec, k[i], d.cheb_R));
-  if (need == 0 || have >= need) return;
+  int need = 0, converging = 0;
+  for (int i = 0; i < n; ++i) {
+    const int terms = bem::cheb_terms(prec, k[i], d.cheb_R);
+    need = std::max(need, terms);
+    converging += terms > 0;
+  }
+  if (need == 0 || (!mixed && 5 * converging < 2 * need)) return false;
+  if (have >= need) return true;
   const int nterms = std::min(bem::kChebN, std::max(need, 2 * have));
   const size_t bytes = bem::cheb_moment_bytes(prec, d.npairs);
   if (mixed && !d.cheb) d.cheb = (float*)mesh_alloc(m, bytes, "allocate Chebyshev moments");
@@ -333,6 +345,7 @@ void ensure_cheb(bem_context* ctx, bem_mesh* m, bem::Precision prec, const doubl
   if (!m->cheb_ready) ck(cudaEventCreateWithFlags(&m->cheb_ready, cudaEventDisableTiming), "create event");
   ck(cudaEventRecord(m->cheb_ready, ctx->side), "record event");
   have = nterms;
+  return true;
 }
 
 // Extended rows held at once: as many frequencies as fit 1 GiB, and at least those that share
@@ -1241,11 +1254,11 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
     if (field_out && m->nobs < 1) return fail(ctx, BEM_ERR_INVALID_ARGUMENT, "no observation points set");
     if (!valid_options(ctx, o)) return BEM_ERR_INVALID_ARGUMENT;
     const bem::Precision prec = o.precision == BEM_PRECISION_MIXED ? bem::Precision::Mixed : bem::Precision::FP64;
-    const bool cheb = n_freq >= kChebMinFreqs;
+    bool cheb = n_freq >= kChebMinFreqs;
     if (cheb) {
       std::vector<double> kw(n_freq);
       for (int i = 0; i < n_freq; ++i) kw[i] = 2.0 * M_PI * freqs_hz[i] / o.sound_speed;
-      ensure_cheb(ctx, m, prec, kw.data(), n_freq);
+      cheb = ensure_cheb(ctx, m, prec, kw.data(), n_freq);
     }
     const bem::DeviceMesh& dm = m->dm;
     const int nv = dm.nv, nc = m->nc;
