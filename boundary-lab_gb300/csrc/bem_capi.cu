@@ -306,7 +306,7 @@ int lane_split(int n_freq) {
 // had, up to kChebN.  Returns whether the call goes through them: not when no frequency
 // converges (those run point by point).  The FP64 form also runs a call point by point of which
 // too few frequencies converge to pay for the terms they need, whether or not the mesh has the
-// moments.  A term costs 0.4 of a frequency
+// moments, and one for whose moments there is no memory.  A term costs 0.4 of a frequency
 // point by point: first calls of 12 frequencies at 1,280 triangles, 105.6 ms point by point,
 // take 107.0 and 105.2 where 4 and 5 converge in 12 terms, 106.1 and 104.4 where 6 and 7 do in
 // 16, 105.3 where 8 do in 20.
@@ -326,7 +326,15 @@ bool ensure_cheb(bem_context* ctx, bem_mesh* m, bem::Precision prec, const doubl
   const int nterms = std::min(bem::kChebN, std::max(need, 2 * have));
   const size_t bytes = bem::cheb_moment_bytes(prec, d.npairs);
   if (mixed && !d.cheb) d.cheb = (float*)mesh_alloc(m, bytes, "allocate Chebyshev moments");
-  if (!mixed && !d.cheb64) d.cheb64 = (double*)mesh_alloc(m, bytes, "allocate Chebyshev moments");
+  if (!mixed && !d.cheb64) {
+    try {
+      d.cheb64 = (double*)mesh_alloc(m, bytes, "allocate Chebyshev moments");
+    } catch (const BemError& e) {
+      if (e.code != BEM_ERR_OUT_OF_MEMORY) throw;
+      cudaGetLastError();
+      return false;
+    }
+  }
   // the side stream must see the allocation (made on the context's stream), the pair
   // records (written on the side stream) are in order there, and no singular kernel of an
   // earlier sweep may still read the moments being rewritten
