@@ -457,6 +457,17 @@ void assemble_one(bem_mesh* m, bem::Precision prec, double k, const bem::Operato
                        cheb);
 }
 
+// Frees a context's scratch and its lanes' and returns the pool's unused memory to the device.
+void release_scratch(bem_context* ctx) {
+  for (DevBuf* b : ctx->scratch()) b->release();
+  for (bem_context* l : ctx->lanes) {
+    for (DevBuf* b : l->scratch()) b->release();
+    ck(cudaStreamSynchronize(l->stream), "trim scratch");
+  }
+  ck(cudaStreamSynchronize(ctx->stream), "trim scratch");
+  ck(cudaMemPoolTrimTo(ctx->pool, 0), "trim memory pool");
+}
+
 void free_mesh_device(bem_mesh* m) {
   if (m->cheb_ready) {  // the side stream may still read the mesh data
     cudaStreamWaitEvent(m->ctx->stream, m->cheb_ready, 0);
@@ -556,13 +567,7 @@ void bem_destroy_context(bem_context* ctx) {
 int bem_trim_context(bem_context* ctx) {
   if (!ctx) return BEM_ERR_INVALID_ARGUMENT;
   return guarded(ctx, [&]() -> int {
-    for (DevBuf* b : ctx->scratch()) b->release();
-    for (bem_context* l : ctx->lanes) {
-      for (DevBuf* b : l->scratch()) b->release();
-      ck(cudaStreamSynchronize(l->stream), "trim scratch");
-    }
-    ck(cudaStreamSynchronize(ctx->stream), "trim scratch");
-    ck(cudaMemPoolTrimTo(ctx->pool, 0), "trim memory pool");
+    release_scratch(ctx);
     return BEM_OK;
   });
 }
@@ -1271,22 +1276,21 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
     const bem::DeviceMesh& dm = m->dm;
     const int nv = dm.nv, nc = m->nc;
     const CallPlan plan = plan_call(nv, prec, n_freq, o.batch, o.lanes);
-    const int B = plan.batch, nl = plan.lanes;
     ctx->prof = o.profile != 0;
-    const int nbatch = (n_freq + B - 1) / B;
-    auto slice_of = [&](int bi) {
+    auto slice_of = [&](int B, int bi) {
       const int f0 = bi * B, bt = std::min(B, n_freq - f0);
       return Slice{m, freqs_hz + f0, bt, pressure_out ? pressure_out + 2 * (size_t)f0 * nc * nv : nullptr,
                    field_out ? field_out + 2 * (size_t)f0 * nc * m->nobs : nullptr, cheb};
     };
     SolveTotals T;
-    if (nl >= 2) {
+    auto run_lanes = [&](int B, int nl) {
+      const int nbatch = (n_freq + B - 1) / B;
       // batch bi goes to lane bi % nl: lane 0 is this context, the others are helper contexts
       // driven from their own host threads; the mesh is shared read-only
       while ((int)ctx->lanes.size() < nl - 1) {
         bem_context* c2 = nullptr;
         const int rc = bem_create_context(ctx->device, &c2);
-        if (rc != BEM_OK) return fail(ctx, rc, "cannot create a lane's context");
+        if (rc != BEM_OK) throw BemError{rc, "cannot create a lane's context"};
         ctx->lanes.push_back(c2);
       }
       std::vector<SolveTotals> TL(nl - 1);
@@ -1300,7 +1304,8 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         threads.emplace_back([&, l, cl] {
           cudaSetDevice(ctx->device);
           try {
-            for (int bi = l; bi < nbatch; bi += nl) solve_combined(cl, {slice_of(bi)}, nv, o, nc, TL[l - 1], plan.rules);
+            for (int bi = l; bi < nbatch; bi += nl)
+              solve_combined(cl, {slice_of(B, bi)}, nv, o, nc, TL[l - 1], plan.rules);
           } catch (const BemError& e) {
             errs[l - 1] = e;
             failed[l - 1] = 1;
@@ -1311,7 +1316,7 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         });
       }
       try {
-        for (int bi = 0; bi < nbatch; bi += nl) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rules);
+        for (int bi = 0; bi < nbatch; bi += nl) solve_combined(ctx, {slice_of(B, bi)}, nv, o, nc, T, plan.rules);
       } catch (...) {
         for (auto& t : threads) t.join();
         throw;
@@ -1332,8 +1337,25 @@ int bem_solve_frequencies(bem_mesh* m, const double* freqs_hz, int n_freq, const
         T.gemm_used = std::max(T.gemm_used, T2.gemm_used);
         T.launches += T2.launches;
       }
-    } else {
-      for (int bi = 0; bi < nbatch; ++bi) solve_combined(ctx, {slice_of(bi)}, nv, o, nc, T, plan.rules);
+    };
+    bool split = plan.lanes >= 2;
+    if (split) {
+      try {
+        run_lanes(plan.batch, plan.lanes);
+      } catch (const BemError& e) {
+        // one batch that was split over the lanes by itself, and there is no room for the second
+        // lane (its context or its scratch): the batch on this one, with the same bits
+        const bool room = e.code != BEM_ERR_OUT_OF_MEMORY && (int)ctx->lanes.size() >= plan.lanes - 1;
+        if (plan.rules.batch == 0 || room) throw;
+        cudaGetLastError();
+        release_scratch(ctx);
+        T = SolveTotals{};
+        split = false;
+      }
+    }
+    if (!split) {
+      const int B = plan.rules.batch > 0 ? n_freq : plan.batch;
+      for (int f = 0; f < n_freq; f += B) solve_combined(ctx, {slice_of(B, f / B)}, nv, o, nc, T, plan.rules);
     }
     fill_stats(stats, T);
     if (stats) {

@@ -61,3 +61,22 @@ def test_fp64_sweep_without_room_for_moments():
         assert st["singular_cheb_freqs"] == 12
     finally:
         ctx.close()
+
+
+def test_split_call_without_room_for_the_second_lane():
+    freqs = np.geomspace(200.0, 1500.0, 8)
+    kw = dict(precision=native.BEM_PRECISION_MIXED)
+    ctx = native.Context(0)
+    try:
+        m = _upload(ctx, 5000)
+        p, u, st = m.solve(freqs, **kw)
+        assert st["batches"] == 1
+        with device_full():
+            p1, u1, st = m.solve(freqs, lanes=2, **kw)
+        assert st["batches"] == 1
+        assert np.array_equal(p1, p) and np.array_equal(u1, u)
+        p2, u2, st = m.solve(freqs, lanes=2, **kw)  # with memory again
+        assert st["batches"] == 2
+        assert np.array_equal(p2, p) and np.array_equal(u2, u)
+    finally:
+        ctx.close()
