@@ -244,6 +244,7 @@ template <typename F> int guarded(bem_context* ctx, F&& f) {
     }
     return f();
   } catch (const BemError& e) {
+    cudaGetLastError();  // reported here; left in place, the next call's launch checks would report it again
     return fail(ctx, e.code, e.msg);
   } catch (const std::bad_alloc&) {
     return fail(ctx, BEM_ERR_OUT_OF_MEMORY, "host allocation failed");

@@ -80,3 +80,15 @@ def test_split_call_without_room_for_the_second_lane():
         assert np.array_equal(p2, p) and np.array_equal(u2, u)
     finally:
         ctx.close()
+
+
+def test_an_allocation_that_failed_is_reported_once():
+    ctx = native.Context(0)
+    try:
+        m = _upload(ctx, 5000)
+        with device_full(), pytest.raises(native.BemError, match="OUT_OF_MEMORY"):
+            m.solve([700.0])
+        assert m.solve([700.0])[2]["max_rel_residual"] <= 1e-10
+        _upload(ctx, 600).release()
+    finally:
+        ctx.close()
