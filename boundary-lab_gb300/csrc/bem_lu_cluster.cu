@@ -24,6 +24,9 @@
 #include <cooperative_groups.h>
 #include <limits.h>
 
+#include <array>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "bem_common.cuh"
@@ -1039,11 +1042,11 @@ template <typename K> int active_clusters(K kern, int threads, size_t smem, int 
 }
 
 // Panel width and cluster size for an n x n batch.  The panel is latency-bound
-// (a cluster barrier per column), so the batch's panels should run in as few
-// waves of clusters as possible: among the (width, cluster size) pairs whose
-// panel fits in shared memory, take the fewest waves (batch / resident
-// clusters), then the wider panel, then the smaller cluster.  want_nb > 0 fixes
-// the width.
+// (an exchange between the cluster's CTAs per column), so the batch's panels should
+// run in as few waves of clusters as possible: the register panel (32 wide) where its
+// rows fit, else, among the (width, cluster size) pairs whose panel fits in shared
+// memory, the fewest waves (batch / resident clusters), then the wider panel, then
+// the smaller cluster.  want_nb > 0 fixes the width.
 template <typename R> bool choose_panel(int n, int want_nb, int batch, int& nb, int& cl) {
   bool found = false;
   int best_waves = 0;
@@ -1114,35 +1117,53 @@ template <typename R> bool choose_panel(int n, int want_nb, int batch, int& nb, 
 
 }  // namespace
 
-bool lu_cluster_plan(Precision prec, int n, int want_nb, int batch, int* nb, int* cl) {
-  struct Key {
-    int n = -1, want = 0, batch = 0;
-  };
-  static thread_local Key last[2];
-  static thread_local int last_nb[2] = {0, 0}, last_cl[2] = {0, 0};
-  static thread_local bool last_ok[2] = {false, false};
-  const int pi = prec == Precision::Mixed ? 1 : 0;
-  if (last[pi].n != n || last[pi].want != want_nb || last[pi].batch != batch) {
-    int b = 0, c = 0;
-    last_ok[pi] = prec == Precision::Mixed ? choose_panel<float>(n, want_nb, batch, b, c)
-                                           : choose_panel<double>(n, want_nb, batch, b, c);
-    last[pi].n = n;
-    last[pi].want = want_nb;
-    last[pi].batch = batch;
-    last_nb[pi] = b;
-    last_cl[pi] = c;
+namespace {
+// Answers of the occupancy queries below, by device and question: a solve asks two of them each
+// call (10 queries or so of the driver), and a lane of its own thread asks again.
+using PlanKey = std::array<int, 5>;  // device, form, order, width wanted (-1: resident batch), batch
+struct PanelPlan {
+  bool ok = false;
+  int nb = 0, cl = 0, resident = 0;
+};
+template <typename F> PanelPlan remembered_plan(PlanKey key, F&& find) {
+  static std::mutex mu;
+  static std::map<PlanKey, PanelPlan> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  key[0] = dev;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
   }
-  *nb = last_nb[pi];
-  *cl = last_cl[pi];
-  return last_ok[pi];
+  const PanelPlan p = find();
+  if (!p.ok) return p;  // a query may fail for want of memory: asked again next time
+  std::lock_guard<std::mutex> lock(mu);
+  if (known.size() >= 4096) known.clear();
+  return known[key] = p;
+}
+}  // namespace
+
+bool lu_cluster_plan(Precision prec, int n, int want_nb, int batch, int* nb, int* cl) {
+  const PanelPlan p = remembered_plan({0, (int)prec, n, want_nb, batch}, [&] {
+    PanelPlan q;
+    q.ok = prec == Precision::Mixed ? choose_panel<float>(n, want_nb, batch, q.nb, q.cl)
+                                    : choose_panel<double>(n, want_nb, batch, q.nb, q.cl);
+    return q;
+  });
+  *nb = p.nb;
+  *cl = p.cl;
+  return p.ok;
 }
 
 // Matrices whose cluster panels are resident at once (one wave) for an n x n
 // factorisation with the panel plan of a large batch: a batch beyond this
 // runs every panel in two waves.
-int lu_resident_batch(Precision prec, int n) {
+namespace {
+bool resident_batch(Precision prec, int n, int* resident) {
   int nb = 0, cl = 0;
-  if (!lu_cluster_plan(prec, n, 0, 64, &nb, &cl)) return 64;
+  *resident = 64;
+  if (!lu_cluster_plan(prec, n, 0, 64, &nb, &cl)) return false;
   const int chunk = (n + cl - 1) / cl;
   int act = 0;
   if (prec == Precision::Mixed && nb == 32 && chunk <= kRegPanelThreads)
@@ -1158,7 +1179,17 @@ int lu_resident_batch(Precision prec, int n) {
   else
     act = nb == 64 ? active_clusters(lu_panel_cluster_kernel<double, 64>, kPanelThreads, panel_smem<double, 64>(chunk), cl)
                    : active_clusters(lu_panel_cluster_kernel<double, 32>, kPanelThreads, panel_smem<double, 32>(chunk), cl);
-  return std::max(1, act);
+  *resident = std::max(1, act);
+  return true;
+}
+}  // namespace
+
+int lu_resident_batch(Precision prec, int n) {
+  return remembered_plan({0, (int)prec, n, -1, 64}, [&] {
+           PanelPlan q;
+           q.ok = resident_batch(prec, n, &q.resident);
+           return q;
+         }).resident;
 }
 
 cudaError_t lu_panel_cluster(Precision prec, void* A, long long lda, long long strideA, int n, int k, int kb, int nb,
