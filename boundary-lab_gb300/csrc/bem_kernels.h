@@ -179,16 +179,13 @@ constexpr int kPanelPolls = 1 << 16;
 // 3xFP16 update that halves the HBM traffic that bounds it (LU 2.91 -> 2.79 ms
 // per frequency at n = 4,976 against 128).
 constexpr int kOuterBlock = 256;
-// Kernels the two-level LU launches for one batch (cuBLAS kernels not counted).
-int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm, int batch);
+// Kernels the two-level LU launches for one batch.
+int lu_launch_count(int n, int nb, int NB, bool perm, int batch);
 cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int batch, int* ipiv, int* info,
                               int nb, void* cublas_handle, cudaStream_t stream, LuGemm gemm = LuGemm::Cublas,
                               void* tc_workspace = nullptr, bool* used_tensor = nullptr, int** tc_err = nullptr,
                               int* rowmap = nullptr, int* n_launches = nullptr, int* perm = nullptr,
                               int polls = kPanelPolls, int rule_batch = 0);
-// Solve (LU) X = B in place for nrhs columns per matrix (B stride ldb*nrhs per matrix), working precision.
-cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* ipiv,
-                             void* B, long long ldb, int nrhs, int nb, cudaStream_t stream);
 // Solves and refinement of the mixed form (bem_lu_solve.cu).  lu_block_inverses inverts the
 // 256 x 256 diagonal blocks of the factors into inv (lu_inverse_bytes); the solves then take
 // B (column stride ldb, nrhs per matrix) to x in place.  lu_solve_blocks_fits: whether order

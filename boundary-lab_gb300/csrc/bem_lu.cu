@@ -523,108 +523,6 @@ __global__ void iota_rows_kernel(int* __restrict__ perm, int n, int total) {
   if (i < total) perm[i] = i % n;
 }
 
-// One CTA per (matrix, right-hand side): P, then L (unit lower), then U.
-template <typename R>
-__global__ void __launch_bounds__(1024) lu_solve_kernel(const typename CT<R>::C2* A, long long lda, long long strideA,
-                                                        int n, const int* ipiv, typename CT<R>::C2* B, long long ldb,
-                                                        int nrhs) {
-  typedef typename CT<R>::C2 C2;
-  const int mat = blockIdx.x / nrhs, rhs = blockIdx.x % nrhs;
-  const C2* M = A + (size_t)mat * strideA;
-  const int* piv = ipiv + (size_t)mat * n;
-  C2* b = B + ((size_t)mat * nrhs + rhs) * ldb;
-  __shared__ C2 xs[32];
-  const int tid = threadIdx.x, lane = tid & 31;
-  if (tid == 0)
-    for (int i = 0; i < n; ++i) {
-      const int p = piv[i];
-      if (p != i) {
-        C2 t = b[i];
-        b[i] = b[p];
-        b[p] = t;
-      }
-    }
-  __syncthreads();
-  // forward substitution, blocks of 32 rows
-  for (int k0 = 0; k0 < n; k0 += 32) {
-    const int kb = min(32, n - k0);
-    if (tid < 32) {
-      C2 v;
-      v.x = 0;
-      v.y = 0;
-      if (lane < kb) v = b[k0 + lane];
-      for (int j = 0; j < kb; ++j) {
-        C2 xj;
-        xj.x = __shfl_sync(0xffffffffu, v.x, j);
-        xj.y = __shfl_sync(0xffffffffu, v.y, j);
-        if (lane > j && lane < kb) {
-          const C2 l = M[(size_t)(k0 + j) * lda + k0 + lane];
-          v.x -= l.x * xj.x - l.y * xj.y;
-          v.y -= l.x * xj.y + l.y * xj.x;
-        }
-      }
-      if (lane < kb) {
-        b[k0 + lane] = v;
-        xs[lane] = v;
-      }
-    }
-    __syncthreads();
-    for (int r = k0 + kb + tid; r < n; r += blockDim.x) {
-      C2 v = b[r];
-      for (int j = 0; j < kb; ++j) {
-        const C2 l = M[(size_t)(k0 + j) * lda + r];
-        const C2 x = xs[j];
-        v.x -= l.x * x.x - l.y * x.y;
-        v.y -= l.x * x.y + l.y * x.x;
-      }
-      b[r] = v;
-    }
-    __syncthreads();
-  }
-  // backward substitution
-  const int nblk = (n + 31) / 32;
-  for (int bi = nblk - 1; bi >= 0; --bi) {
-    const int k0 = bi * 32;
-    const int kb = min(32, n - k0);
-    if (tid < 32) {
-      C2 v;
-      v.x = 0;
-      v.y = 0;
-      if (lane < kb) v = b[k0 + lane];
-      for (int j = kb - 1; j >= 0; --j) {
-        C2 xj;
-        if (lane == j) {
-          const C2 d = M[(size_t)(k0 + j) * lda + k0 + j];
-          v = cmul(v, pivot_inverse<true>(d));
-        }
-        xj.x = __shfl_sync(0xffffffffu, v.x, j);
-        xj.y = __shfl_sync(0xffffffffu, v.y, j);
-        if (lane < j) {
-          const C2 u = M[(size_t)(k0 + j) * lda + k0 + lane];
-          v.x -= u.x * xj.x - u.y * xj.y;
-          v.y -= u.x * xj.y + u.y * xj.x;
-        }
-      }
-      if (lane < kb) {
-        b[k0 + lane] = v;
-        xs[lane] = v;
-      }
-    }
-    __syncthreads();
-    for (int r = tid; r < k0; r += blockDim.x) {
-      C2 v = b[r];
-      for (int j = 0; j < kb; ++j) {
-        const C2 u = M[(size_t)(k0 + j) * lda + r];
-        const C2 x = xs[j];
-        v.x -= u.x * x.x - u.y * x.y;
-        v.y -= u.x * x.y + u.y * x.x;
-      }
-      b[r] = v;
-    }
-    __syncthreads();
-  }
-}
-
 __global__ void f64_to_f32_kernel(const double2* s, float2* d, long long n) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) d[i] = make_float2((float)s[i].x, (float)s[i].y);
@@ -641,18 +539,16 @@ size_t tc_gemm_plan_size();
 
 namespace {
 
-// State of one batched factorisation for the two-level driver.
+// State of one batched factorisation for the two-level driver (mixed form).
 struct LuJob {
-  Precision prec;
-  void* A;
+  float2* A;
   long long lda, strideA;
   int n, batch, nb, cl;
   int* ipiv;
   int* info;
   int* rowmap;
   int* perm;         // row permutation of the whole factorisation, built panel by panel (null: not wanted)
-  TcGemmPlan* plan;  // tcgen05 updates (mixed form); null: cuBLAS
-  cublasHandle_t h;
+  TcGemmPlan* plan;  // tcgen05 updates
   cudaStream_t stream;
   int polls;         // of the panels' exchange
   int rule_batch;
@@ -663,39 +559,16 @@ cudaError_t trsm_cols(const LuJob& j, int k, int kb, int c0, int c1) {
   if (c1 <= c0 || kb <= 0) return cudaSuccess;
   const int tpb = 128;
   dim3 g((unsigned)((c1 - c0 + tpb - 1) / tpb), j.batch);
-  if (j.prec == Precision::Mixed) {
-    const size_t sm = (size_t)kb * kb * sizeof(float2) + (size_t)kb * (tpb + 1) * sizeof(float2);
-    if (sm > 48 * 1024) ensure_smem_limit((const void*)lu_trsm_kernel<float2>, sm);
-    lu_trsm_kernel<float2><<<g, tpb, sm, j.stream>>>((float2*)j.A, j.lda, j.strideA, j.n, k, kb, c0, c1);
-  } else {
-    const size_t sm = (size_t)kb * kb * sizeof(double2) + (size_t)kb * (tpb + 1) * sizeof(double2);
-    if (sm > 48 * 1024) ensure_smem_limit((const void*)lu_trsm_kernel<double2>, sm);
-    lu_trsm_kernel<double2><<<g, tpb, sm, j.stream>>>((double2*)j.A, j.lda, j.strideA, j.n, k, kb, c0, c1);
-  }
+  const size_t sm = (size_t)kb * kb * sizeof(float2) + (size_t)kb * (tpb + 1) * sizeof(float2);
+  if (sm > 48 * 1024) ensure_smem_limit((const void*)lu_trsm_kernel<float2>, sm);
+  lu_trsm_kernel<float2><<<g, tpb, sm, j.stream>>>(j.A, j.lda, j.strideA, j.n, k, kb, c0, c1);
   return cudaGetLastError();
 }
 
 // A[r0:r0+M, c0:c0+N] -= A[r0:r0+M, kc:kc+K] * A[kc:kc+K, c0:c0+N] for every matrix.
 cudaError_t block_update(const LuJob& j, int r0, int M, int c0, int N, int kc, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
-  if (j.plan) return tc_update(j.plan, (float2*)j.A, j.lda, j.strideA, r0, M, c0, N, kc, K, j.stream);
-  const int ld = (int)j.lda;
-  if (j.prec == Precision::Mixed) {
-    const cuComplex alpha = make_cuComplex(-1.f, 0.f), beta = make_cuComplex(1.f, 0.f);
-    const cuComplex* base = (const cuComplex*)j.A;
-    const cublasStatus_t st = cublasCgemmStridedBatched(
-        j.h, CUBLAS_OP_N, CUBLAS_OP_N, M, N, K, &alpha, base + r0 + (size_t)kc * j.lda, ld, j.strideA,
-        base + kc + (size_t)c0 * j.lda, ld, j.strideA, &beta, (cuComplex*)j.A + r0 + (size_t)c0 * j.lda, ld, j.strideA,
-        j.batch);
-    return st == CUBLAS_STATUS_SUCCESS ? cudaSuccess : cudaErrorUnknown;
-  }
-  const cuDoubleComplex alpha = make_cuDoubleComplex(-1.0, 0.0), beta = make_cuDoubleComplex(1.0, 0.0);
-  const cuDoubleComplex* base = (const cuDoubleComplex*)j.A;
-  const cublasStatus_t st = cublasZgemmStridedBatched(
-      j.h, CUBLAS_OP_N, CUBLAS_OP_N, M, N, K, &alpha, base + r0 + (size_t)kc * j.lda, ld, j.strideA,
-      base + kc + (size_t)c0 * j.lda, ld, j.strideA, &beta, (cuDoubleComplex*)j.A + r0 + (size_t)c0 * j.lda, ld,
-      j.strideA, j.batch);
-  return st == CUBLAS_STATUS_SUCCESS ? cudaSuccess : cudaErrorUnknown;
+  return tc_update(j.plan, j.A, j.lda, j.strideA, r0, M, c0, N, kc, K, j.stream);
 }
 
 #define BEM_TRY(x)                          \
@@ -711,7 +584,7 @@ cudaError_t outer_urows(const LuJob& j, int k0, int c0, int c1) {
     constexpr size_t sm = urows_smem<CPW>();
     ensure_smem_limit((const void*)lu_urows_kernel<CPW>, sm);
     dim3 g((unsigned)((c1 - c0 + kUrowsWarps * CPW - 1) / (kUrowsWarps * CPW)), j.batch);
-    return launch_chained(lu_urows_kernel<CPW>, g, kUrowsWarps * 32, sm, j.stream, (float2*)j.A, j.lda, j.strideA, k0,
+    return launch_chained(lu_urows_kernel<CPW>, g, kUrowsWarps * 32, sm, j.stream, j.A, j.lda, j.strideA, k0,
                           c0, c1);
   };
   // 8 columns per warp where that still gives every SM a CTA, else 4
@@ -748,8 +621,7 @@ int outer_width(int rest, int NB, int batch, bool narrow) {
 // its successor after its last step, so that no waiting CTA holds an SM of another stream.
 cudaError_t lu_two_level(const LuJob& j, int NB) {
   const int n = j.n, nb = j.nb;
-  const bool narrow = j.prec == Precision::Mixed && nb == 32;
-  float2* A32 = (float2*)j.A;
+  const bool narrow = nb == 32;
   if (j.perm) {
     const int total = n * j.batch;
     iota_rows_kernel<<<(total + 255) / 256, 256, 0, j.stream>>>(j.perm, n, total);
@@ -758,24 +630,24 @@ cudaError_t lu_two_level(const LuJob& j, int NB) {
     KB = outer_width(n - k0, NB, j.rule_batch, narrow);
     for (int j0 = 0; j0 < KB; j0 += nb) {
       const int kb = std::min(nb, KB - j0), kk = k0 + j0;
-      BEM_TRY(lu_panel_cluster(j.prec, j.A, j.lda, j.strideA, n, kk, kb, nb, j.cl, j.batch, j.ipiv, j.info, j.stream,
+      BEM_TRY(lu_panel_cluster(Precision::Mixed, j.A, j.lda, j.strideA, n, kk, kb, nb, j.cl, j.batch, j.ipiv, j.info, j.stream,
                                j.rowmap, j.polls));
       if (narrow && kb == 32) {
         const int rest = k0 + KB - kk - 32;  // the rest of the outer block
         const int solve_ctas = (rest + 7) / 8;
         dim3 gs((unsigned)(solve_ctas + (kk + n - k0 - KB + (j.perm ? 1 : 0) + 7) / 8), j.batch);
         if (gs.x > 0)
-          BEM_TRY(launch_chained(lu_swap_urows_kernel, gs, 256, 0, j.stream, A32, j.lda, j.strideA, n, kk, k0 + KB,
+          BEM_TRY(launch_chained(lu_swap_urows_kernel, gs, 256, 0, j.stream, j.A, j.lda, j.strideA, n, kk, k0 + KB,
                                  solve_ctas, j.rowmap, j.perm));
         if (rest > 0) {
           dim3 gu((unsigned)((n - kk - 32 + 127) / 128), (unsigned)((rest + 31) / 32), j.batch);
-          BEM_TRY(launch_chained(lu_update32_kernel, gu, 256, 0, j.stream, A32, j.lda, j.strideA, kk + 32, n - kk - 32,
+          BEM_TRY(launch_chained(lu_update32_kernel, gu, 256, 0, j.stream, j.A, j.lda, j.strideA, kk + 32, n - kk - 32,
                                  kk + 32, rest, kk));
         }
         BEM_TRY(cudaGetLastError());
         continue;
       }
-      BEM_TRY(lu_swap_rows_batched(j.prec, j.A, j.lda, j.strideA, n, kk, kb, j.batch, j.rowmap, j.perm, j.stream));
+      BEM_TRY(lu_swap_rows_batched(Precision::Mixed, j.A, j.lda, j.strideA, n, kk, kb, j.batch, j.rowmap, j.perm, j.stream));
       if (j0 + kb < KB) {  // the rest of the outer block
         BEM_TRY(trsm_cols(j, kk, kb, kk + kb, k0 + KB));
         BEM_TRY(block_update(j, kk + kb, n - kk - kb, kk + kb, k0 + KB - kk - kb, kk, kb));
@@ -800,9 +672,9 @@ cudaError_t lu_two_level(const LuJob& j, int NB) {
 
 }  // namespace
 
-int lu_launch_count(int n, int nb, int NB, bool tensor, bool perm, int batch) {
-  const int per_update = tensor ? 2 : 0;  // operand split + tcgen05 kernel (cuBLAS kernels are not counted)
-  const bool narrow = tensor && nb == 32;
+int lu_launch_count(int n, int nb, int NB, bool perm, int batch) {
+  const int per_update = 2;  // operand split + tcgen05 kernel
+  const bool narrow = nb == 32;
   int count = perm ? 1 : 0;
   for (int k0 = 0, KB; k0 < n; k0 += KB) {
     KB = outer_width(n - k0, NB, batch, narrow);
@@ -855,8 +727,8 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
   // form, or lu_gemm = 1) keeps one level: its kernels for the skinny panel
   // shapes of the two-level schedule are slow.
   if (cluster_panel && rowmap && plan) {
-    LuJob job{prec, A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, h, stream, polls, rule_batch};
-    if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, plan != nullptr, perm != nullptr, rule_batch);
+    LuJob job{(float2*)A, lda, strideA, n, batch, nb, ccl, ipiv, info, rowmap, perm, plan, stream, polls, rule_batch};
+    if (n_launches) *n_launches = lu_launch_count(n, nb, kOuterBlock, perm != nullptr, rule_batch);
     return lu_two_level(job, kOuterBlock);
   }
   if (n_launches) *n_launches = 0;
@@ -924,18 +796,6 @@ cudaError_t lu_factor_batched(Precision prec, void* A, long long lda, int n, int
     if (n_launches) *n_launches += 1;
     return lu_perm_batched(ipiv, n, batch, perm, stream);
   }
-  return cudaGetLastError();
-}
-
-cudaError_t lu_solve_batched(Precision prec, const void* LU, long long lda, int n, int batch, const int* ipiv, void* B,
-                             long long ldb, int nrhs, int /*nb*/, cudaStream_t stream) {
-  const long long strideA = lda * (long long)n;
-  if (prec == Precision::Mixed)
-    lu_solve_kernel<float><<<batch * nrhs, 1024, 0, stream>>>((const float2*)LU, lda, strideA, n, ipiv, (float2*)B,
-                                                             ldb, nrhs);
-  else
-    lu_solve_kernel<double><<<batch * nrhs, 1024, 0, stream>>>((const double2*)LU, lda, strideA, n, ipiv,
-                                                              (double2*)B, ldb, nrhs);
   return cudaGetLastError();
 }
 
