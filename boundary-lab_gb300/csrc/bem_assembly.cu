@@ -2375,8 +2375,8 @@ cudaError_t launch_regular_f64_bm(const DeviceMesh& m, int groups, const double*
 }  // namespace
 
 // Frequencies per launch of the FP64 Burton-Miller kernel: two where their accumulators
-// (and the 8 KB table) fit in a CTA's shared memory (570 tile rows), else one; 0 beyond
-// 1,160 rows, where the general kernel without the table runs.
+// (and the 8 KB table) fit in a CTA's shared memory (581 tile rows), else one; 0 beyond
+// 1,162 rows, where the general kernel without the table runs.
 int regular_width_f64(const DeviceMesh& m) {
   for (int w = 2; w >= 1; --w)
     if ((size_t)4 * w * 3 * m.max_tile_rows * sizeof(double2) <= (size_t)218 * 1024) return w;

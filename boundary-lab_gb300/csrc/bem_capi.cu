@@ -910,7 +910,7 @@ struct Slice {
   int cnt;
   double* pressure_out;  // [cnt][nc][nv] complex
   double* field_out;     // [cnt][nc][nobs] complex
-  bool cheb = false;     // mixed form: singular remainders through the mesh's Chebyshev moments
+  bool cheb = false;     // singular remainders through the mesh's Chebyshev moments
 };
 
 // The batches that the rules go by which choose between orders of sums, 0: each batch's own.  A
@@ -1036,7 +1036,7 @@ void solve_combined(bem_context* ctx, const std::vector<Slice>& sl, int n, const
                             &lu_launches, (int*)ctx->perm.p, ctx->panel_polls, rule_batch),
      "LU factorisation");
   // kernels of this batch besides the assembly: the LU with its row permutation, the solves
-  // (mixed: 5 + 4 per refinement step), the field (2, +1 mixed, per slice)
+  // (mixed: the block inverses, 4 for each solve with its residual), the field (2, +1 mixed, per slice)
   T.launches += lu_launches;
   T.gemm_used = mixed ? (used_tensor ? 2 : 1) : 0;
   prof_mark(ctx, BEM_K_LU);

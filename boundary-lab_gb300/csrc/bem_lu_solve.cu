@@ -483,7 +483,7 @@ size_t lu_inverse_bytes(int n, int batch) {
   return (size_t)batch * ((n + kOuterBlock - 1) / kOuterBlock) * 2 * kOuterBlock * kOuterBlock * sizeof(float2);
 }
 
-// Orders whose rows fit the cluster's shared memory (46,000 with one right-hand side at a
+// Orders whose rows fit the cluster's shared memory (up to 43,264, with one right-hand side at a
 // time); a larger one keeps the substitution of lu_solve_cluster_batched.
 bool lu_solve_blocks_fits(int n) { return solve_smem(n, kSolveCluster, 1) <= kSolveSmemMax; }
 

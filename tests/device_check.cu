@@ -4,6 +4,7 @@
 // prints one line of figures; 1 is returned (with a message) if a CUDA call fails.
 #include <algorithm>
 #include <cmath>
+#include <complex>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -12,6 +13,10 @@
 
 #include "bem_common.cuh"
 #include "bem_kernels.h"
+
+namespace bem {
+int regular_width_f64(const DeviceMesh& m);
+}
 
 namespace {
 
@@ -158,6 +163,131 @@ template <typename F> int captured_kernels(F launch) {
   return kernels;
 }
 
+// solves n nrhs: relative difference between the block solves and the cluster substitution that
+// takes over where their rows do not fit, on the same FP32 factors and right-hand sides, and
+// the larger of both residuals ||P b - L U x|| / (|| |L| |U| |x| ||) in double.
+int solves(int n, int nrhs) {
+  const int batch = 2;
+  const long long lda = (n + 31) / 32 * 32, ldb = lda;
+  std::vector<float2> a = factors(n, lda, batch, 0, 3);
+  // a diagonal that dominates keeps the solutions of a random triangle bounded
+  for (int b = 0; b < batch; ++b)
+    for (int i = 0; i < n; ++i) a[((size_t)b * n + i) * lda + i].x += 3.f;
+  for (auto& v : a) {
+    v.x *= 2.f / std::sqrt((float)n);
+    v.y *= 2.f / std::sqrt((float)n);
+  }
+  for (int b = 0; b < batch; ++b)
+    for (int i = 0; i < n; ++i) a[((size_t)b * n + i) * lda + i].x += 1.f;
+  std::vector<float2> rhs((size_t)batch * nrhs * ldb, make_float2(0.f, 0.f));
+  std::mt19937 rng(5);
+  std::uniform_real_distribution<float> u(-1.f, 1.f);
+  std::vector<int> perm((size_t)batch * n);
+  for (int b = 0; b < batch; ++b) {
+    for (int i = 0; i < n; ++i) perm[(size_t)b * n + i] = i;
+    std::shuffle(perm.begin() + (size_t)b * n, perm.begin() + (size_t)(b + 1) * n, rng);
+    for (int c = 0; c < nrhs; ++c)
+      for (int i = 0; i < n; ++i) rhs[((size_t)b * nrhs + c) * ldb + i] = make_float2(u(rng), u(rng));
+  }
+  Dev<float2> da(a), d1(rhs), d2(rhs), inv(bem::lu_inverse_bytes(n, batch) / sizeof(float2));
+  Dev<int> dp(perm);
+  ck(bem::lu_block_inverses(da.p, lda, n, batch, inv.p, 0), "block inverses");
+  ck(bem::lu_solve_blocks_batched(da.p, lda, n, batch, inv.p, dp.p, d1.p, ldb, nrhs, 0), "block solves");
+  ck(bem::lu_solve_cluster_batched(bem::Precision::Mixed, da.p, lda, n, batch, dp.p, d2.p, ldb, nrhs, 0), "cluster solves");
+  ck(cudaDeviceSynchronize(), "solves");
+  const std::vector<float2> x[2] = {d1.host(), d2.host()};
+  double diff = 0, norm = 0, worst = 0;
+  for (size_t i = 0; i < rhs.size(); ++i) {
+    diff += std::pow((double)x[0][i].x - x[1][i].x, 2) + std::pow((double)x[0][i].y - x[1][i].y, 2);
+    norm += std::pow((double)x[0][i].x, 2) + std::pow((double)x[0][i].y, 2);
+  }
+  using cd = std::complex<double>;
+  for (int k = 0; k < 2; ++k)
+    for (int s = 0; s < batch * nrhs; ++s) {
+      const float2* M = a.data() + (size_t)(s / nrhs) * n * lda;
+      std::vector<cd> y(n), z(n);
+      std::vector<double> ya(n), za(n);
+      auto at = [&](int i, int j) { return cd(M[(size_t)j * lda + i].x, M[(size_t)j * lda + i].y); };
+      for (int j = 0; j < n; ++j) {  // y = U x
+        const cd xv(x[k][(size_t)s * ldb + j].x, x[k][(size_t)s * ldb + j].y);
+        for (int i = 0; i <= j; ++i) {
+          y[i] += at(i, j) * xv;
+          ya[i] += std::abs(at(i, j)) * std::abs(xv);
+        }
+      }
+      for (int j = 0; j < n; ++j) {  // z = L y
+        z[j] += y[j];
+        za[j] += ya[j];
+        for (int i = j + 1; i < n; ++i) {
+          z[i] += at(i, j) * y[j];
+          za[i] += std::abs(at(i, j)) * ya[j];
+        }
+      }
+      double r = 0, scale = 0;
+      for (int i = 0; i < n; ++i) {
+        const float2 b = rhs[(size_t)s * ldb + perm[(size_t)(s / nrhs) * n + i]];
+        r += std::norm(cd(b.x, b.y) - z[i]);
+        scale += za[i] * za[i];
+      }
+      worst = std::max(worst, std::sqrt(r / scale));
+    }
+  std::printf("%.3e %.3e\n", std::sqrt(diff / norm), worst);
+  return 0;
+}
+
+// Entries of small factors and right-hand sides by a hash of their index.
+__global__ void fill_kernel(float2* a, long long count, long long lda, float scale, float diagonal) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  unsigned long long h = (unsigned long long)i * 0x9e3779b97f4a7c15ull + 12345;
+  h ^= h >> 31;
+  h *= 0xbf58476d1ce4e5b9ull;
+  h ^= h >> 29;
+  const float re = (float)(int)(unsigned)h * 0x1p-31f, im = (float)(int)(unsigned)(h >> 32) * 0x1p-31f;
+  a[i] = make_float2(scale * re + (i / lda == i % lda ? diagonal : 0.f), scale * im);
+}
+
+// rhs_groups n nrhs: entries of the block solves of nrhs right-hand sides together that differ, to
+// the bit, from each by itself, and entries that are not finite.
+int rhs_groups(int n, int nrhs) {
+  const long long lda = (n + 31) / 32 * 32, ldb = lda;
+  std::vector<int> perm(n);
+  for (int i = 0; i < n; ++i) perm[i] = n - 1 - i;
+  Dev<float2> a((size_t)lda * n), b((size_t)ldb * nrhs), x((size_t)ldb * nrhs), inv(bem::lu_inverse_bytes(n, 1) / sizeof(float2));
+  Dev<int> dp(perm);
+  fill_kernel<<<(unsigned)((a.n + 255) / 256), 256>>>(a.p, (long long)a.n, lda, 0.5f / n, 1.f);
+  fill_kernel<<<(unsigned)((b.n + 255) / 256), 256>>>(b.p, (long long)b.n, ldb, 1.f, 0.f);
+  ck(bem::lu_block_inverses(a.p, lda, n, 1, inv.p, 0), "block inverses");
+  ck(cudaMemcpy(x.p, b.p, b.n * sizeof(float2), cudaMemcpyDeviceToDevice), "copy");
+  ck(bem::lu_solve_blocks_batched(a.p, lda, n, 1, inv.p, dp.p, x.p, ldb, nrhs, 0), "solves together");
+  for (int c = 0; c < nrhs; ++c)
+    ck(bem::lu_solve_blocks_batched(a.p, lda, n, 1, inv.p, dp.p, b.p + c * ldb, ldb, 1, 0), "solve by itself");
+  ck(cudaDeviceSynchronize(), "solves");
+  const std::vector<float2> together = x.host(), alone = b.host();
+  long long differ = 0, bad = 0;
+  for (int c = 0; c < nrhs; ++c)
+    for (int i = 0; i < n; ++i) {
+      const float2 u = together[c * ldb + i], v = alone[c * ldb + i];
+      differ += u.x != v.x || u.y != v.y;
+      bad += !std::isfinite(u.x) || !std::isfinite(u.y);
+    }
+  std::printf("%lld %lld\n", differ, bad);
+  return 0;
+}
+
+// edges: whether the dispatch of the solves (orders) and of the FP64 regular kernel (tile rows)
+// changes where the figures beside it say.
+int edges() {
+  auto width = [](int rows) {
+    bem::DeviceMesh m;
+    m.max_tile_rows = rows;
+    return bem::regular_width_f64(m);
+  };
+  std::printf("%d %d %d %d %d %d\n", bem::lu_solve_blocks_fits(43264), bem::lu_solve_blocks_fits(43265), width(581),
+              width(582), width(1162), width(1163));
+  return 0;
+}
+
 // launch_counts: calls whose reported number of launches is not what they launch, of the
 // right-hand side (excitations 1..4) and the regular pairs, both forms, 1..64 frequencies.  The
 // launches are captured, not run; every pointer is a zeroed buffer all the same.
@@ -207,6 +337,9 @@ int launch_counts() {
 int main(int argc, char** argv) {
   auto is = [&](const char* name, int args) { return argc == args + 2 && std::strcmp(argv[1], name) == 0; };
   if (is("block_inverse", 2)) return block_inverse(std::atoi(argv[2]), std::atoi(argv[3]));
+  if (is("solves", 2)) return solves(std::atoi(argv[2]), std::atoi(argv[3]));
+  if (is("rhs_groups", 2)) return rhs_groups(std::atoi(argv[2]), std::atoi(argv[3]));
+  if (is("edges", 0)) return edges();
   if (is("launch_counts", 0)) return launch_counts();
   if (is("sincos", 0)) return sincos_errors();
   std::printf("unknown check\n");

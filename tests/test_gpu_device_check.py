@@ -54,3 +54,26 @@ def test_reported_launches(check):
     formula: they are those of the launches captured in a graph."""
     calls, wrong = check("launch_counts")
     assert calls == 2 * 64 * 5 and wrong == 0
+
+
+@pytest.mark.parametrize("n,nrhs", [(33, 1), (256, 3), (300, 4), (1000, 2)])
+def test_substitution_of_orders_that_the_block_solves_do_not_hold(check, n, nrhs):
+    """The cluster substitution (mixed form, orders above 43,264) against the block solves.  Both
+    are backward stable: ||P b - L U x|| <= 2 n 2^-24 (sqrt 8 for complex products) of
+    || |L| |U| |x| ||, in practice far below; the difference is that times the condition of
+    these well-conditioned triangles (below 100)."""
+    diff, residual = check("solves", n, nrhs)
+    bound = 2 * n * 2.0**-24 * 8**0.5
+    assert residual <= bound and diff <= 100 * bound
+
+
+@pytest.mark.parametrize("n,nrhs", [(300, 4), (520, 3), (9602, 4)])
+def test_right_hand_sides_together_and_alone(check, n, nrhs):
+    """A right-hand side's sums do not depend on how many share the factors' reads; at 9,602
+    rows a cluster holds two of the four at a time."""
+    differ, not_finite = check("rhs_groups", n, nrhs)
+    assert differ == 0 and not_finite == 0
+
+
+def test_edges_of_the_dispatch(check):
+    assert check("edges") == [1, 0, 2, 1, 1, 0]
