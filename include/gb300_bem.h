@@ -133,7 +133,9 @@ typedef struct bem_solve_options {
                             the other's assembly and tensor-core updates; a call of 8 or of at least
                             12 frequencies that one automatic batch would hold is split in two for them
                             (the first part a multiple of four, the second at least four); larger
-                            values act as 2.  The results are those of one lane to the bit.
+                            values act as 2.  The results are those of one lane to the bit (in
+                            the FP64 form as far as cuBLAS's batched product does not depend on
+                            the batch; it has not where tested).
                             Per-kernel times in stats are then summed over the lanes. */
 } bem_solve_options;
 
